@@ -206,10 +206,14 @@ __device__ __forceinline__ void block_add(double v, double* dst)
 // split into (their partial sums meet in shared memory) are chosen so that the
 // FP64 work spreads evenly over the SMs and over each SM's four sub-partitions
 // (sp2_shape).
+// Once tr(X - X^2) < tol_idem the recursion takes `polish` (0 or 2) more steps, one
+// square and one 2X - X^2: an occupation 1 - d goes to 1 - 2d and 1 - 4d^2 (or 1 - d^2
+// and 1 - 2d^2), one at d to the mirror image, so a sum of 1e-7 left by the test ends
+// at 4e-14, the rounding of the sum, on both sides.
 template <typename T>
 __global__ void __launch_bounds__(1024) sp2_persistent_kernel(int n, int nocc, int tt, int ks, T* X0, T* X1,
                                                               double* tr, int maxs, double tol_idem, double tol_n,
-                                                              Sp2Sync* sync)
+                                                              int polish, Sp2Sync* sync)
 {
     extern __shared__ __align__(16) unsigned char sp2_smem[];
     const int ld = n + 1;
@@ -234,11 +238,14 @@ __global__ void __launch_bounds__(1024) sp2_persistent_kernel(int n, int nocc, i
     const int i = i0 + ty, j = j0 + tx;
     const int kc = (n + ks - 1) / ks, k0 = slice * kc, k1 = min(n, k0 + kc);
     const bool own = worker && slice == 0 && i < n && j < n;
+    int left = -1;  // polishing steps still to do (-1: not converged yet)
+    bool last_square = false;
     for (int it = 0; it < maxs; ++it) {
         T* Xc = (it & 1) ? X1 : X0;
         T* Xn = (it & 1) ? X0 : X1;
         const double t0 = __ldcg(tr + 2 * it), t1 = __ldcg(tr + 2 * it + 1);
-        if (fabs(t0 - t1) < tol_idem && fabs(t0 - nocc) < tol_n) {
+        if (left < 0 && fabs(t0 - t1) < tol_idem && fabs(t0 - nocc) < tol_n) left = polish;
+        if (left == 0) {
             if ((it & 1) && own) {  // X_k is in X1: move this block's tile to X0
                 X0[i + (int64_t)j * n] = __ldcg(X1 + i + (int64_t)j * n);
                 if (ti != tj) X0[j + (int64_t)i * n] = __ldcg(X1 + j + (int64_t)i * n);
@@ -246,7 +253,10 @@ __global__ void __launch_bounds__(1024) sp2_persistent_kernel(int n, int nocc, i
             if (blockIdx.x == 0 && threadIdx.x == 0) sync->steps = it;
             return;
         }
-        const bool square = fabs(t1 - nocc) <= fabs(2 * t0 - t1 - nocc);
+        // the last of the polishing steps is the opposite of the one before it
+        const bool square = left == 1 ? !last_square : fabs(t1 - nocc) <= fabs(2 * t0 - t1 - nocc);
+        last_square = square;
+        if (left > 0) --left;
         for (int e = threadIdx.x; e < tt * n; e += blockDim.x) {
             const int r = e % tt, k = e / tt;  // r fastest: tt consecutive elements of a column
             Ar[r * ld + k] = (i0 + r < n) ? __ldcg(Xc + i0 + r + (int64_t)k * n) : T(0);
@@ -431,14 +441,14 @@ struct Purifier {
     // One cooperative launch of the whole recursion on the iterate Xs, with
     // barrier state slot `which` (0: FP32 steps, 1: FP64 steps).
     template <typename T>
-    void run_persistent(Context& ctx, T* Xs, T* Xw, double* trs, int maxs, double tol_idem, double tol_n, int tt,
-                        int which)
+    void run_persistent(Context& ctx, T* Xs, T* Xw, double* trs, int maxs, double tol_idem, double tol_n, int polish,
+                        int tt, int which)
     {
         cudaStream_t st = ctx.stream;
         HF_CUDA(cudaMemsetAsync(sync.p + which, 0, sizeof(Sp2Sync), st));
         int n_ = n, nocc_ = nocc, tt_ = tt, ks_ = kslices;
         Sp2Sync* sp = sync.p + which;
-        void* args[] = {&n_, &nocc_, &tt_, &ks_, &Xs, &Xw, &trs, &maxs, &tol_idem, &tol_n, &sp};
+        void* args[] = {&n_, &nocc_, &tt_, &ks_, &Xs, &Xw, &trs, &maxs, &tol_idem, &tol_n, &polish, &sp};
         HF_CUDA(cudaLaunchCooperativeKernel((const void*)sp2_persistent_kernel<T>, dim3(sp2_tiles(n, tt)),
                                             dim3(sp2_threads(tt, kslices)), args,
                                             sp2_smem_bytes(n, tt, kslices, sizeof(T)), st));
@@ -451,15 +461,26 @@ struct Purifier {
     double* htr = nullptr;
     bool pending = false;
     static constexpr int MAXS = 160;
-    void check()
+    // Did the last density() end with tr X = nocc?  strict: and by the idempotency
+    // test, not at the step limit.  (True when nothing is pending.)
+    bool converged(bool strict)
     {
-        if (!pending) return;
+        if (!pending) return true;
         pending = false;
         HF_CHECK(hsync[0].err == 0 && hsync[1].err == 0, HFGPU_ERR_CUDA,
                  "density purification: grid barrier timed out");
         const int last = std::min(std::max(hsync[1].steps, 0), MAXS);
-        HF_CHECK(fabs(htr[2 * last] - nocc) < 1e-6, HFGPU_ERR_LINALG,
-                 "density purification did not converge (no gap?)");
+        return fabs(htr[2 * last] - nocc) < 1e-6 && !(strict && last == MAXS);
+    }
+    // is the whole recursion one cooperative launch at this size?
+    bool one_launch(Context& ctx)
+    {
+        if (tile == 0) {
+            const Sp2Shape sh = sp2_shape(ctx, n);
+            tile = sh.tt == 0 ? -1 : sh.tt;
+            kslices = sh.ks;
+        }
+        return tile > 0;
     }
     ~Purifier()
     {
@@ -491,12 +512,7 @@ struct Purifier {
         const unsigned tiles = (unsigned)(nt * (nt + 1) / 2);  // of the per-step fallback
         double h[2] = {0, 1};
         bool done = false;
-        if (tile == 0) {
-            const Sp2Shape sh = sp2_shape(ctx, n);
-            tile = sh.tt == 0 ? -1 : sh.tt;
-            kslices = sh.ks;
-        }
-        if (tile > 0) {
+        if (one_launch(ctx)) {
             if (!sync.p) {
                 sync.alloc(2, st);
                 HF_CUDA(cudaMemsetAsync(sync.p, 0, 2 * sizeof(Sp2Sync), st));
@@ -509,7 +525,7 @@ struct Purifier {
                 double* trf = tr.p + 2 * (MAXS + 1);
                 convert_trace_kernel<double, float><<<nblk(nn), 256, 0, st>>>(n, T1.p, Xf.p, trf);
                 count_launch();
-                run_persistent<float>(ctx, Xf.p, Xf.p + nn, trf, MAXS, 1e-3, 1e-3, tile, 0);
+                run_persistent<float>(ctx, Xf.p, Xf.p + nn, trf, MAXS, 1e-3, 1e-3, 0, tile, 0);
                 ctx.trace_mark("sp2 fp32");
                 HF_CUDA(cudaMemsetAsync(tr64, 0, sizeof(double) * 2 * (MAXS + 1), st));
                 convert_trace_kernel<float, double><<<nblk(nn), 256, 0, st>>>(n, Xf.p, T1.p, tr64);
@@ -518,7 +534,7 @@ struct Purifier {
                 HF_CUDA(cudaMemsetAsync(sync.p, 0, sizeof(Sp2Sync), st));  // no FP32 phase this time
             }
             // T2 (X^T F X) is free once the first iterate is built: the second buffer
-            run_persistent<double>(ctx, T1.p, T2.p, tr64, MAXS, 1e-13 * n, 1e-6, tile, 1);
+            run_persistent<double>(ctx, T1.p, T2.p, tr64, MAXS, 1e-7, 1e-6, 2, tile, 1);
             ctx.trace_mark("sp2 fp64");
             HF_CUDA(cudaMemcpyAsync(hsync, sync.p, 2 * sizeof(Sp2Sync), cudaMemcpyDeviceToHost, st));
             HF_CUDA(cudaMemcpyAsync(htr, tr64, 2 * (MAXS + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -622,6 +638,8 @@ __global__ void diis_solve_kernel(int nd, int nhist, int head, double* __restric
     for (int k = 0; k < nd; k++) cvec[k] = ok ? (k < nhist ? b[k] : 0.0) : (k == head ? 1.0 : 0.0);
 }
 
+constexpr int SP2_MIN = 8;  // smallest basis whose iteration densities come from purification by default
+
 ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dLam)
 {
     cudaStream_t st = ctx.stream;
@@ -655,24 +673,25 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     }
     int nhist = 0, head = 0;
 
+    // eigensolver: our own (eigh.cu) where it fits, with the purifier's X; cuSOLVER's
+    // dsygvd otherwise
     Purifier pur;
-    if (in.purify) pur.setup(ctx, n, in.nocc, in.dS);
-    // eigensolver: our own (eigh.cu) where it fits, with the purifier's X or one
-    // made here; cuSOLVER's dsygvd otherwise
     Eigh eig;
-    DBuf<double> Xown;
-    const double* Xorth = nullptr;
     const bool own_eigh = in.eigensolver == 0 && Eigh::supported(ctx, n);
-    if (own_eigh) {
-        eig.setup(ctx, n);
-        if (in.purify) {
-            Xorth = pur.X.p;
-        } else {
-            Xown.alloc(nn, st);
-            cholesky_orthogonalizer(ctx, n, in.dS, Xown.p);
-            Xorth = Xown.p;
-        }
-    }
+    if (in.purify || own_eigh) pur.setup(ctx, n, in.nocc, in.dS);
+    if (own_eigh) eig.setup(ctx, n);
+    const double* Xorth = pur.X.p;
+    // Densities of the iterations: with the own eigensolver they too come from FP64
+    // purification, whose projector is the occupied eigenvectors' to rounding (its
+    // last two steps square the idempotency error away), and an eigensolve follows
+    // only where that does not converge (no gap) and for the final orbitals.  The
+    // eigensolve walks n columns with a grid barrier each and waits for the host's
+    // tridiagonal solve; purification takes about 30 steps and no host.  At n = 225:
+    // 3.0 ms an iteration by eigensolve.  Below SP2_MIN functions, for a tolP near
+    // rounding, and where the recursion does not fit one launch, the eigensolve
+    // stays.
+    const bool sp2_density = in.purify || (own_eigh && in.nocc > 0 && in.nocc < n && n >= SP2_MIN &&
+                                           in.tolP >= 1e-11 && pur.one_launch(ctx));
     // orbitals C (may alias F) and energies of F C = S C diag(lam); with the own
     // eigensolver only the lowest ncol orbitals are formed (ncol <= 0: all)
     auto eigh = [&](const double* Fm, double* Cm, int ncol) {
@@ -757,11 +776,9 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
             ctx.trace_mark("diis extrap");
         }
         HF_CUDA(cudaMemcpyAsync(Pold.p, dP, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
-        if (in.purify) {
-            HF_CUDA(cudaMemcpyAsync(Fw.p, Fsolve, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
-            // FP32 steps while the density is still far from converged
-            pur.density(ctx, Fw.p, dP, it > 1 && !endgame && last_dP > 1e-4);
-            HF_CUDA(cudaMemsetAsync(info.p, 0, sizeof(int), st));
+        if (sp2_density) {
+            // with the purify option, FP32 steps while the density is still far from converged
+            pur.density(ctx, Fsolve, dP, in.purify && it > 1 && !endgame && last_dP > 1e-4);
         } else {
             // the density needs the occupied orbitals only; all are formed once converged
             eigh(Fsolve, Fw.p, in.nocc);
@@ -775,7 +792,14 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
         scal.download(h, 2);
         info.download(&hinfo, 1);
         HF_CUDA(cudaStreamSynchronize(st));
-        if (in.purify) pur.check();
+        if (sp2_density && !pur.converged(!in.purify)) {
+            HF_CHECK(!in.purify, HFGPU_ERR_LINALG, "density purification did not converge (no gap?)");
+            eigh(Fsolve, Fw.p, in.nocc);
+            form_density(ctx, n, in.nocc, Fw.p, dP);
+            reduce(ctx, 1, nn, dP, Pold.p, nullptr, scal.p + 1);
+            scal.download(h, 2);
+            HF_CUDA(cudaStreamSynchronize(st));
+        }
         ctx.trace_mark("convergence");
         HF_CHECK(hinfo == 0, HFGPU_ERR_LINALG,
                  "eigh: dsygvd returned info = " + std::to_string(hinfo) +
@@ -793,9 +817,9 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
             if (dPv < in.tolP && emax - emin < in.tolE && !last_full) {
                 endgame = true;  // accept convergence only on a fully built Fock matrix
             } else if (dPv < in.tolP && emax - emin < in.tolE) {
-                if (in.purify) {
+                if (sp2_density) {
                     // orbitals and orbital energies of the last Fock matrix, as the reference returns them
-                    eigh(Fw.p, Fw.p, 0);
+                    eigh(last_F, Fw.p, 0);
                     form_density(ctx, n, in.nocc, Fw.p, dP);
                     info.download(&hinfo, 1);
                     HF_CUDA(cudaStreamSynchronize(st));
@@ -816,8 +840,10 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
         }
     }
     // orbitals of the last Fock matrix
-    if (in.purify) eigh(Fw.p, Fw.p, 0);
-    else if (own_eigh && last_F) eigh(last_F, Fw.p, 0);
+    if ((sp2_density || own_eigh) && last_F) {
+        eigh(last_F, Fw.p, 0);
+        if (sp2_density && !in.purify) form_density(ctx, n, in.nocc, Fw.p, dP);
+    }
     HF_CUDA(cudaMemcpyAsync(dC, Fw.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
     HF_CUDA(cudaStreamSynchronize(st));
     out.converged = false;
