@@ -3,7 +3,8 @@
 // The shape knobs are, per quartet class:
 //   * ERI: primitive quartets per lane before a quartet's primitive loop is
 //     split over more lanes (the `split` of each segment),
-//   * digest: lanes per quartet in the Fock build.
+//   * digest: warps that share the bra component rows of the same quartets in the
+//     Fock build.
 // With tuning on (hfgpu_options.autotune or HFGPU_AUTOTUNE=1), the first time a
 // (kernel, class, size bucket) is met its candidates are timed on the real
 // launch and the fastest is kept in a process-wide table; later molecules of

@@ -113,9 +113,9 @@ void BatchWave::run_digest_locked()
                 HF_CUDA(cudaStreamWaitEvent(st, ev_[m], 0));
                 tables_.h_P[s] = reqP_[m];
                 tables_.h_G[s] = reqG_[m];
-                tables_.h_screen[s] = reqScreen_[m];
+                tables_.h_screen[s] = screen_f32(reqScreen_[m]);
             } else {
-                tables_.h_screen[s] = -1.0;
+                tables_.h_screen[s] = -1.0f;
             }
         }
         HF_CUDA(cudaEventRecord(t0_, st));

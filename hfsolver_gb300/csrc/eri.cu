@@ -230,6 +230,16 @@ __global__ void pair_qmax_kernel(int npair, const double* __restrict__ diag, dou
     Q[id] = sqrt(m);
 }
 
+static std::vector<float> round_up_f32(const std::vector<double>& v)
+{
+    std::vector<float> f(v.size());
+    for (size_t i = 0; i < v.size(); ++i) {
+        f[i] = (float)v[i];
+        if ((double)f[i] < v[i]) f[i] = std::nextafterf(f[i], INFINITY);
+    }
+    return f;
+}
+
 EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
 {
     cudaStream_t st = ctx.stream;
@@ -365,7 +375,7 @@ EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
         }
         P->gpairs = to_device(gp, st);
         P->h_gpairs = gp;
-        P->dQ = to_device(P->Q, st);
+        P->dQf = to_device(round_up_f32(P->Q), st);
 
         // segments per class
         std::vector<int64_t> prefix;
@@ -453,29 +463,46 @@ EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
 
 void eri_plan_destroy(EriPlan* p) { delete p; }
 
-__global__ void sym_kernel(int n, const double* __restrict__ Gh, double* G)
+// element (i, j) of G = 2 (Jh + Jh^T) - (Kh + Kh^T) / 2 from the half matrices of a build
+__device__ __forceinline__ double g_element(int n, const double* __restrict__ Gh, int i, int j)
 {
-    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)n * n) return;
-    const int i = idx % n, j = idx / n;
-    G[idx] = Gh[idx] + Gh[j + (int64_t)i * n];
+    const double* Kh = Gh + n * n;
+    return 2.0 * (Gh[i + j * n] + Gh[j + i * n]) - 0.5 * (Kh[i + j * n] + Kh[j + i * n]);
 }
 
-// lanes per quartet in the Fock digest: spread a class with few quartets and
-// large blocks over more lanes (at most one (a, b) row each), up to about
-// 150k threads in flight
+__global__ void sym_kernel(int n, const double* __restrict__ Gh, double* G)
+{
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= n * n) return;
+    G[idx] = g_element(n, Gh, idx % n, idx / n);
+}
+
+// Warps that share the bra component rows of a class's quartets (a divisor of the
+// row count).  Every warp sends its own J_cd, K_bc and K_bd sums, so few splits
+// mean few atomics; but a warp's part of a quartet should stay short against the
+// build (ELEMS_MAX elements: ~0.1 ms of an FP64 pipe) and the class should make
+// MIN_WARPS warps, until a part is down to ELEMS_MIN elements.  Full builds at
+// (216, 9, 1200) against these: 2 waters 0.048 and 0.038 ms, 3 waters 0.079 and
+// 0.067, 8 waters 0.728 and 0.64, 16 waters 3.30 and 3.27; ELEMS_MIN = 162 would
+// give 0.054, 0.063, 0.64 and 3.23.
+constexpr int DIGEST_ELEMS_MAX = 648, DIGEST_ELEMS_MIN = 54, DIGEST_MIN_WARPS = 150;
 static int digest_split(const ClassPlan& c)
 {
     const int nab = ncart(ptype_la(c.tb)) * ncart(ptype_lb(c.tb));
-    int s = 1;
-    while (s * 2 <= 32 && s * 2 <= nab && c.nq * s < 150000) s *= 2;
-    return s;
+    const int ncd = ncart(ptype_la(c.tk)) * ncart(ptype_lb(c.tk));
+    const int64_t chunks = (c.nq + 31) / 32;
+    for (int s = 1; s < nab; ++s) {
+        if (nab % s) continue;
+        const int elems = nab / s * ncd;
+        if (elems <= DIGEST_ELEMS_MIN || (elems <= DIGEST_ELEMS_MAX && chunks * s >= DIGEST_MIN_WARPS)) return s;
+    }
+    return nab;
 }
 
 // largest |P| element of each shell pair
 __global__ void shell_dmax_kernel(int ns, const int* __restrict__ L, const int* __restrict__ cfn0,
                                   const int* __restrict__ comp_fn, const double* __restrict__ P, int n,
-                                  double* __restrict__ Dm)
+                                  float* __restrict__ Dm)
 {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= ns * ns) return;
@@ -490,7 +517,7 @@ __global__ void shell_dmax_kernel(int ns, const int* __restrict__ L, const int* 
             if (g >= 0) m = fmax(m, fabs(P[f + (int64_t)g * n]));
         }
     }
-    Dm[idx] = m;
+    Dm[idx] = __double2float_ru(m);
 }
 
 // quartets a warp screens before digesting the survivors: one pass when nothing
@@ -499,47 +526,80 @@ __global__ void shell_dmax_kernel(int ns, const int* __restrict__ L, const int* 
 static int digest_rounds(const Context& ctx, const ClassPlan& c, int split, bool screened)
 {
     if (!screened) return 1;
-    const int64_t warps1 = (c.nq * split + 31) / 32;
+    const int64_t warps1 = (c.nq + 31) / 32 * split;
     int r = 1;
     while (r < 8 && warps1 / (2 * r) >= (int64_t)ctx.num_sms * 16) r *= 2;
     return r;
 }
 
-static void launch_digest(const ClassPlan& c, const DigestArgs& a, cudaStream_t s)
+static DigestClass digest_class(const EriPlan* P, const ClassPlan& c, int split, int rounds)
 {
-    const int64_t qpw = (int64_t)(32 / a.split) * a.rounds;
-    const int64_t warps = (c.nq + qpw - 1) / qpw;
-    const unsigned blocks = (unsigned)((warps + DIGEST_WARPS - 1) / DIGEST_WARPS);
-    if (a.split == 1)
-        digest_fn(c.tb, c.tk)<<<blocks, DIGEST_BLOCK, 0, s>>>(a);
-    else
-        digest_wide_fn(c.tb, c.tk)<<<blocks, DIGEST_BLOCK, 0, s>>>(a);
-    count_launch();
-    HF_CUDA(cudaGetLastError());
+    DigestClass d;
+    d.id = 6 * c.tb + c.tk;
+    d.block0 = 0;
+    d.nq = (int)c.nq;
+    d.split = split;
+    d.rounds = rounds;
+    d.nseg = (int)c.segs.size();
+    d.segs = c.dsegs.p;
+    d.blocks = P->blocks.p + c.boff;
+    d.qlist = P->qlist.p ? P->qlist.p + c.qbase : nullptr;
+    return d;
 }
 
-// Lanes per quartet of the class's Fock digest: the built-in rule, or with
-// tuning on the fastest of 1, 2, 4, ... lanes timed once per (class, size
-// bucket) into a scratch matrix.
-static int digest_split_tuned(Context& ctx, const ClassPlan& c, DigestArgs a, int64_t nn)
+static int digest_blocks(const DigestClass& d)
+{
+    const int64_t qpw = (int64_t)32 * d.rounds;
+    const int64_t warps = (d.nq + qpw - 1) / qpw * d.split;
+    return (int)((warps + DIGEST_WARPS - 1) / DIGEST_WARPS);
+}
+
+__global__ void fill_kernel(int64_t n, double v, double* p)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = v;
+}
+
+// Row splits of the class's Fock digest: the built-in rule, or with tuning on the
+// fastest divisor of the row count, timed once per (class, size bucket) into
+// scratch matrices.  Timed as it runs in a build: TUNE_COPIES of the class at once
+// (alone, a class prefers more splits than it gains with the others around it) and
+// a density without zeros (the block-diagonal one of an atomic start skips most of
+// the atomics).
+static int digest_split_tuned(Context& ctx, const EriPlan* P, const ClassPlan& c, const DigestArgs& a)
 {
     int split = digest_split(c);
     if (!ctx.tune || c.nq == 0) return split;
     const int bucket = tune_bucket(c.nq);
     if (tune_get(TUNE_DIGEST, c.tb, c.tk, bucket, &split)) return split;
     const int nab = ncart(ptype_la(c.tb)) * ncart(ptype_lb(c.tb));
-    DBuf<double> scratch(nn, ctx.stream);
+    const int64_t nn = (int64_t)a.n * a.n;
+    DBuf<double> scratch(3 * nn, ctx.stream);
     scratch.zero();
-    a.Gh = scratch.p;
+    fill_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, ctx.stream>>>(nn, 1.0, scratch.p + 2 * nn);
+    count_launch();
+    constexpr int TUNE_COPIES = 8;
+    static_assert(TUNE_COPIES <= DIGEST_TIER_MAX, "one launch");
+    DigestLaunch l;
+    l.a = a;
+    l.a.Gh = scratch.p;
+    l.a.P = scratch.p + 2 * nn;
+    l.a.screen = 0.0f;
+    l.ncls = TUNE_COPIES;
     cudaEvent_t e0, e1;
     HF_CUDA(cudaEventCreate(&e0));
     HF_CUDA(cudaEventCreate(&e1));
     float best = 1e30f;
-    for (int cand = 1; cand <= 32 && (cand == 1 || cand / 2 < nab); cand <<= 1) {
-        a.split = cand;
-        a.rounds = digest_rounds(ctx, c, cand, a.screen > 0);
+    for (int cand = 1; cand <= nab; ++cand) {
+        if (nab % cand) continue;
+        l.nblocks = 0;
+        for (int k = 0; k < TUNE_COPIES; ++k) {
+            l.cls[k] = digest_class(P, c, cand, 1);
+            l.cls[k].block0 = l.nblocks;
+            l.nblocks += digest_blocks(l.cls[k]);
+        }
         HF_CUDA(cudaEventRecord(e0, ctx.stream));
-        launch_digest(c, a, ctx.stream);
+        launch_digest_tier(digest_tier(c.tk), l, ctx.stream);
         HF_CUDA(cudaEventRecord(e1, ctx.stream));
         const float ms = elapsed(e0, e1);
         if (ms < best) {
@@ -553,19 +613,62 @@ static int digest_split_tuned(Context& ctx, const ClassPlan& c, DigestArgs a, in
     return split;
 }
 
+// The build's classes in one launch per tier: the heavy tiers on two side streams,
+// the light one on stream s (which the side streams fork from and join), larger
+// blocks first in each.  split(c): the class's row splits.
+template <class Split>
+static void digest_launches(Context& ctx, const EriPlan* P, const DigestArgs& a, bool screened, cudaStream_t s,
+                            Split&& split)
+{
+    DigestLaunch l[DIGEST_TIERS];
+    for (auto& t : l) {
+        t.a = a;
+        t.ncls = t.nblocks = 0;
+    }
+    for (int ci = (int)P->classes.size() - 1; ci >= 0; --ci) {
+        const ClassPlan& c = P->classes[ci];
+        if (c.nq == 0) continue;
+        DigestLaunch& t = l[digest_tier(c.tk)];
+        const int sp = split(c);
+        DigestClass d = digest_class(P, c, sp, digest_rounds(ctx, c, sp, screened));
+        d.block0 = t.nblocks;
+        t.nblocks += digest_blocks(d);
+        t.cls[t.ncls++] = d;
+    }
+    static_assert(DIGEST_TIERS - 1 <= Context::NAUX, "one side stream per heavy tier");
+    HF_CUDA(cudaEventRecord(ctx.fork_ev, s));
+    for (int t = DIGEST_TIERS - 1; t >= 1; --t)
+        if (l[t].ncls) {
+            HF_CUDA(cudaStreamWaitEvent(ctx.aux[t - 1], ctx.fork_ev, 0));
+            launch_digest_tier(t, l[t], ctx.aux[t - 1]);
+            HF_CUDA(cudaEventRecord(ctx.join_ev[t - 1], ctx.aux[t - 1]));
+        }
+    if (l[0].ncls) launch_digest_tier(0, l[0], s);
+    for (int t = 1; t < DIGEST_TIERS; ++t)
+        if (l[t].ncls) HF_CUDA(cudaStreamWaitEvent(s, ctx.join_ev[t - 1], 0));
+}
+
+// the digest's single-precision screen: rounded down, and positive if it was
+float screen_f32(double s)
+{
+    float f = (float)s;
+    if ((double)f > s) f = std::nextafterf(f, -INFINITY);
+    return s > 0 ? std::max(f, 1e-45f) : f;
+}
+
 void eri_digest(Context& ctx, EriPlan* P, const double* dP, double* dG, double screen)
 {
     HF_CHECK(P->blocks.p != nullptr, HFGPU_ERR_INVALID, "eri_digest: integrals were not kept");
     const int n = P->basis.nbf;
     const int64_t nn = (int64_t)n * n;
-    DBuf<double> Gh(nn, ctx.stream);
+    DBuf<double> Gh(2 * nn, ctx.stream);
     Gh.zero();
     cudaEvent_t e0, e1;
     HF_CUDA(cudaEventCreate(&e0));
     HF_CUDA(cudaEventCreate(&e1));
     HF_CUDA(cudaEventRecord(e0, ctx.stream));
     const int ns = (int)P->basis.shells.size();
-    DBuf<double> Dm;
+    DBuf<float> Dm;
     if (screen > 0) {
         Dm.alloc((size_t)ns * ns, ctx.stream);
         shell_dmax_kernel<<<(ns * ns + 127) / 128, 128, 0, ctx.stream>>>(ns, P->sL.p, P->scf.p, P->cfn.p, dP, n,
@@ -573,46 +676,20 @@ void eri_digest(Context& ctx, EriPlan* P, const double* dP, double* dG, double s
         count_launch();
         HF_CUDA(cudaGetLastError());
     }
-    // the classes are independent until the symmetrisation: spread them over the
-    // side streams, largest blocks first
-    ctx.fork();
-    int slot = 0;
-    for (int ci = (int)P->classes.size() - 1; ci >= 0; --ci) {
-        auto& c = P->classes[ci];
-        if (c.nq == 0) continue;
-        DigestArgs a;
-        a.sh = P->shdev();
-        a.pr = P->prdev();
-        a.gpairs = P->gpairs.p;
-        a.prefix = P->prefix.p;
-        a.list = nullptr;
-        a.segs = c.dsegs.p;
-        a.nseg = (int)c.segs.size();
-        a.nq = c.nq;
-        a.blocks = P->blocks.p + c.boff;
-        a.P = dP;
-        a.n = n;
-        a.Gh = Gh.p;
-        a.screen = screen;
-        a.Q = P->dQ.p;
-        a.Dm = Dm.p;
-        a.ns = ns;
-        a.mol_n = nullptr;
-        a.mol_P = nullptr;
-        a.mol_Gh = nullptr;
-        a.mol_screen = nullptr;
-        a.mol_Dm = nullptr;
-        a.mol_ns = nullptr;
-        a.mol_sh0 = nullptr;
-        a.qlist = P->qlist.p ? P->qlist.p + c.qbase : nullptr;
-        a.pair_mol = nullptr;
-        a.rounds = 1;
-        a.split = digest_split_tuned(ctx, c, a, nn);
-        a.rounds = digest_rounds(ctx, c, a.split, screen > 0);
-        cudaStream_t s = ctx.aux[slot++ % Context::NAUX];
-        launch_digest(c, a, s);
-    }
-    ctx.join();
+    DigestArgs a{};
+    a.sh = P->shdev();
+    a.pr = P->prdev();
+    a.gpairs = P->gpairs.p;
+    a.prefix = P->prefix.p;
+    a.P = dP;
+    a.n = n;
+    a.Gh = Gh.p;
+    a.screen = screen_f32(screen);
+    a.Q = P->dQf.p;
+    a.Dm = Dm.p;
+    a.ns = ns;
+    digest_launches(ctx, P, a, screen > 0, ctx.stream,
+                    [&](const ClassPlan& c) { return digest_split_tuned(ctx, P, c, a); });
     sym_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, ctx.stream>>>(n, Gh.p, dG);
     count_launch();
     HF_CUDA(cudaGetLastError());
@@ -822,7 +899,7 @@ EriPlan* eri_plan_merge(Context& ctx, const std::vector<EriPlan*>& plans)
         M->sxyz = to_device(xyz, st); M->alpha = to_device(alpha, st); M->coef = to_device(coef, st);
         M->dA = to_device(M->pA, st); M->dB = to_device(M->pB, st); M->dK = to_device(M->pK, st);
         M->doff = to_device(M->poff, st);
-        M->dQ = to_device(M->Q, st);
+        M->dQf = to_device(round_up_f32(M->Q), st);
         {
             std::vector<int> pm;
             pm.reserve(pair0);
@@ -875,7 +952,7 @@ __global__ void batch_dmax_kernel(int nmol, const int64_t* __restrict__ dm_prefi
                                   const int* __restrict__ cfn0, const int* __restrict__ comp_fn,
                                   const int* __restrict__ mol_n, const int* __restrict__ mol_ns,
                                   const int* __restrict__ mol_sh0, const double* const* __restrict__ mol_P,
-                                  const double* __restrict__ mol_screen, double* __restrict__ Dm)
+                                  const float* __restrict__ mol_screen, float* __restrict__ Dm)
 {
     const int64_t total = dm_prefix[nmol];
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -885,7 +962,7 @@ __global__ void batch_dmax_kernel(int nmol, const int64_t* __restrict__ dm_prefi
             const int mid = (lo + hi + 1) >> 1;
             if (dm_prefix[mid] <= idx) lo = mid; else hi = mid - 1;
         }
-        if (mol_screen[lo] <= 0.0) continue;
+        if (mol_screen[lo] <= 0.0f) continue;
         const int ns = mol_ns[lo], n = mol_n[lo];
         const int64_t e = idx - dm_prefix[lo];
         const int s1 = mol_sh0[lo] + (int)(e / ns), s2 = mol_sh0[lo] + (int)(e % ns);
@@ -899,14 +976,14 @@ __global__ void batch_dmax_kernel(int nmol, const int64_t* __restrict__ dm_prefi
                 if (g >= 0) m = fmax(m, fabs(P[f + (int64_t)g * n]));
             }
         }
-        Dm[idx] = m;
+        Dm[idx] = __double2float_ru(m);
     }
 }
 
-// G_m = Gh_m + Gh_m^T for every molecule of the build
+// G of every molecule of the build from its half matrices
 __global__ void batch_sym_kernel(int nmol, const int64_t* __restrict__ nn_prefix, const int* __restrict__ mol_n,
                                  const double* __restrict__ Gh, double* const* __restrict__ mol_G,
-                                 const double* __restrict__ mol_screen)
+                                 const float* __restrict__ mol_screen)
 {
     const int64_t total = nn_prefix[nmol];
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -916,12 +993,10 @@ __global__ void batch_sym_kernel(int nmol, const int64_t* __restrict__ nn_prefix
             const int mid = (lo + hi + 1) >> 1;
             if (nn_prefix[mid] <= idx) lo = mid; else hi = mid - 1;
         }
-        if (mol_screen[lo] < 0.0) continue;
+        if (mol_screen[lo] < 0.0f) continue;
         const int n = mol_n[lo];
-        const int64_t e = idx - nn_prefix[lo];
-        const int i = (int)(e % n), j = (int)(e / n);
-        const double* gh = Gh + nn_prefix[lo];
-        mol_G[lo][e] = gh[e] + gh[j + (int64_t)i * n];
+        const int e = (int)(idx - nn_prefix[lo]);
+        mol_G[lo][e] = g_element(n, Gh + 2 * nn_prefix[lo], e % n, e / n);
     }
 }
 
@@ -938,12 +1013,12 @@ void BatchDigest::setup(Context& ctx, const EriPlan* P, cudaStream_t s)
     mol_n = to_device(P->mol_nbf, s);
     mol_ns = to_device(P->mol_ns, s);
     mol_sh0 = to_device(P->mol_sh0, s);
-    Gh.alloc(std::max<int64_t>(nnp[nmol], 1), s);
+    Gh.alloc(std::max<int64_t>(2 * nnp[nmol], 1), s);
     Dm.alloc(std::max<int64_t>(dmp[nmol], 1), s);
     std::vector<double*> gh(nmol);
-    std::vector<const double*> dm(nmol);
+    std::vector<const float*> dm(nmol);
     for (int m = 0; m < nmol; ++m) {
-        gh[m] = Gh.p + nnp[m];
+        gh[m] = Gh.p + 2 * nnp[m];
         dm[m] = Dm.p + dmp[m];
     }
     mol_Gh = to_device(gh, s);
@@ -954,11 +1029,11 @@ void BatchDigest::setup(Context& ctx, const EriPlan* P, cudaStream_t s)
     HF_CUDA(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
     HF_CUDA(cudaMallocHost((void**)&h_P, nmol * sizeof(const double*)));
     HF_CUDA(cudaMallocHost((void**)&h_G, nmol * sizeof(double*)));
-    HF_CUDA(cudaMallocHost((void**)&h_screen, nmol * sizeof(double)));
+    HF_CUDA(cudaMallocHost((void**)&h_screen, nmol * sizeof(float)));
     for (int m = 0; m < nmol; ++m) {
         h_P[m] = nullptr;
         h_G[m] = nullptr;
-        h_screen[m] = -1.0;
+        h_screen[m] = -1.0f;
     }
 }
 
@@ -977,62 +1052,37 @@ BatchDigest::~BatchDigest()
 }
 
 // One Fock build for every molecule whose h_screen >= 0: Gh zeroed, shell-pair
-// maxima for the screened ones, one digest launch per quartet class over all
-// molecules' quartets, and the symmetrisation into each molecule's G.
+// maxima for the screened ones, the digest over all molecules'
+// quartets, and the symmetrisation into each molecule's G.
 static void batch_digest_launches(Context& ctx, EriPlan* P, BatchDigest& t, cudaStream_t s)
 {
     HF_CUDA(cudaMemsetAsync(t.Gh.p, 0, t.Gh.n * sizeof(double), s));
-    const int64_t dm_total = t.Dm.n, nn_total = t.Gh.n;
+    const int64_t dm_total = t.Dm.n, nn_total = t.Gh.n / 2;
     const unsigned gd = (unsigned)std::max<int64_t>(1, std::min<int64_t>((dm_total + 255) / 256, ctx.num_sms * 8));
     batch_dmax_kernel<<<gd, 256, 0, s>>>(t.nmol, t.dm_prefix.p, P->sL.p, P->scf.p, P->cfn.p, t.mol_n.p, t.mol_ns.p,
                                         t.mol_sh0.p, t.mol_P.p, t.mol_screen.p, t.Dm.p);
     count_launch();
     HF_CUDA(cudaGetLastError());
-    // the classes are independent until the symmetrisation: spread over the side
-    // streams (inside a capture these become parallel branches of the graph)
-    HF_CUDA(cudaEventRecord(ctx.fork_ev, s));
-    for (int i = 0; i < Context::NAUX; ++i) HF_CUDA(cudaStreamWaitEvent(ctx.aux[i], ctx.fork_ev, 0));
-    int slot = 0;
-    for (int ci = (int)P->classes.size() - 1; ci >= 0; --ci) {
-        auto& c = P->classes[ci];
-        if (c.nq == 0) continue;
-        DigestArgs a;
-        a.sh = P->shdev();
-        a.pr = P->prdev();
-        a.gpairs = P->gpairs.p;
-        a.prefix = P->prefix.p;
-        a.list = nullptr;
-        a.segs = c.dsegs.p;
-        a.nseg = (int)c.segs.size();
-        a.nq = c.nq;
-        a.blocks = P->blocks.p + c.boff;
-        a.P = nullptr;
-        a.n = 0;
-        a.Gh = nullptr;
-        a.screen = 0.0;
-        a.Q = P->dQ.p;
-        a.Dm = nullptr;
-        a.ns = 0;
-        a.mol_n = t.mol_n.p;
-        a.mol_P = t.mol_P.p;
-        a.mol_Gh = t.mol_Gh.p;
-        a.mol_screen = t.mol_screen.p;
-        a.mol_Dm = t.mol_Dm.p;
-        a.mol_ns = t.mol_ns.p;
-        a.mol_sh0 = t.mol_sh0.p;
-        a.qlist = P->qlist.p ? P->qlist.p + c.qbase : nullptr;
-        a.pair_mol = P->pair_mol.p;
+    DigestArgs a{};
+    a.sh = P->shdev();
+    a.pr = P->prdev();
+    a.gpairs = P->gpairs.p;
+    a.prefix = P->prefix.p;
+    a.Q = P->dQf.p;
+    a.mol_n = t.mol_n.p;
+    a.mol_P = t.mol_P.p;
+    a.mol_Gh = t.mol_Gh.p;
+    a.mol_screen = t.mol_screen.p;
+    a.mol_Dm = t.mol_Dm.p;
+    a.mol_ns = t.mol_ns.p;
+    a.mol_sh0 = t.mol_sh0.p;
+    a.pair_mol = P->pair_mol.p;
+    // captured once for all builds, screened or not
+    digest_launches(ctx, P, a, true, s, [&](const ClassPlan& c) {
         int split = digest_split(c);
         if (ctx.tune) tune_get(TUNE_DIGEST, c.tb, c.tk, tune_bucket(c.nq), &split);
-        a.split = split;
-        // captured once for all builds, screened or not
-        a.rounds = digest_rounds(ctx, c, split, true);
-        launch_digest(c, a, ctx.aux[slot++ % Context::NAUX]);
-    }
-    for (int i = 0; i < Context::NAUX; ++i) {
-        HF_CUDA(cudaEventRecord(ctx.join_ev[i], ctx.aux[i]));
-        HF_CUDA(cudaStreamWaitEvent(s, ctx.join_ev[i], 0));
-    }
+        return split;
+    });
     const unsigned gs = (unsigned)std::max<int64_t>(1, std::min<int64_t>((nn_total + 255) / 256, ctx.num_sms * 8));
     batch_sym_kernel<<<gs, 256, 0, s>>>(t.nmol, t.nn_prefix.p, t.mol_n.p, t.Gh.p, t.mol_G.p, t.mol_screen.p);
     count_launch();
@@ -1045,7 +1095,7 @@ void eri_digest_batch(Context& ctx, EriPlan* P, BatchDigest& t, cudaStream_t s)
     // this build's densities, outputs and screens
     HF_CUDA(cudaMemcpyAsync(t.mol_P.p, t.h_P, t.nmol * sizeof(const double*), cudaMemcpyHostToDevice, s));
     HF_CUDA(cudaMemcpyAsync(t.mol_G.p, t.h_G, t.nmol * sizeof(double*), cudaMemcpyHostToDevice, s));
-    HF_CUDA(cudaMemcpyAsync(t.mol_screen.p, t.h_screen, t.nmol * sizeof(double), cudaMemcpyHostToDevice, s));
+    HF_CUDA(cudaMemcpyAsync(t.mol_screen.p, t.h_screen, t.nmol * sizeof(float), cudaMemcpyHostToDevice, s));
     HF_CUDA(cudaEventRecord(t.copied, s));
     if (!t.exec) {
         // the launches of a build are the same every iteration: captured once into a

@@ -56,7 +56,7 @@ struct EriArgs {
     int nseg;
     int64_t nwarps;
     double* out;     // packed integrals (may be null), or diagonal buffer [pair][36]
-    double* blocks;  // class-wise quartet blocks [element][quartet] (may be null)
+    double* blocks;  // class-wise quartet blocks [element][quartet], weighted for the digest (may be null)
     int64_t nq_class;
     const int64_t* mol_out;  // batched plans: offset of each molecule's packed array in out (else null)
     int2* qlist;             // with blocks: the (bra, ket) pair ids of each quartet of the class (else null)
@@ -127,15 +127,21 @@ __device__ __forceinline__ void run_chunk(const EriArgs& a, double* out, int bra
         }
     } else {
         if (a.qlist && CH == 0) a.qlist[qg] = make_int2(bra, ket);
-        if (a.blocks) {  // the whole block, one element plane per component quartet (coalesced in q)
+        const int A = a.pr.A[bra], B = a.pr.B[bra], C = a.pr.A[ket], D = a.pr.B[ket];
+        if (a.blocks) {
+            // the whole block, one element plane per component quartet (coalesced in q),
+            // times the Fock digest's weight: 1/2 per coincidence of shells (exact)
+            const int same = (A == B) + (C == D) + (bra == ket);
+            const double w = same == 0 ? 1.0 : same == 1 ? 0.5 : same == 2 ? 0.25 : 0.125;
 #pragma unroll
             for (int s = 0; s < CI::NCD; ++s)
 #pragma unroll
-                for (int ab = 0; ab < CI::NAB; ++ab)
-                    a.blocks[(int64_t)(ab * CI::NCDT + CH * CI::NCD + s) * a.nq_class + qg] = acc[ab * CI::NCD + s];
+                for (int ab = 0; ab < CI::NAB; ++ab) {
+                    const double v = acc[ab * CI::NCD + s];
+                    a.blocks[(int64_t)(ab * CI::NCDT + CH * CI::NCD + s) * a.nq_class + qg] = same ? v * w : v;
+                }
         }
         if (!out) return;
-        const int A = a.pr.A[bra], B = a.pr.B[bra], C = a.pr.A[ket], D = a.pr.B[ket];
         const int* fa = a.sh.comp_fn + a.sh.cfn0[A];
         const int* fb = a.sh.comp_fn + a.sh.cfn0[B];
         const int* fc = a.sh.comp_fn + a.sh.cfn0[C];

@@ -36,7 +36,7 @@ struct EriPlan {
     DBuf<double> pdata;
     // screening
     std::vector<double> Q;
-    DBuf<double> dQ;
+    DBuf<float> dQf;  // rounded up
     DBuf<int> gpairs;
     DBuf<int64_t> prefix;
     std::vector<ClassPlan> classes;

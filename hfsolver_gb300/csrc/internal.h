@@ -222,6 +222,9 @@ void eri_compute_finish(Context& ctx, EriPlan* p, EriStats* st);
 // touch is below screen (for density differences)
 void eri_digest(Context& ctx, EriPlan* p, const double* dP, double* dG, double screen = 0.0);
 
+// the digest's single-precision screen (eri.cu): rounded down, positive if s is
+float screen_f32(double s);
+
 // one-electron integrals (onee.cu): S, T, V on the device (n x n, symmetric)
 // (on: the stream to run on, ctx.stream if null; the results are ready in stream
 // order there, the host does not wait)
@@ -258,13 +261,15 @@ struct BatchDigest {
     int nmol = 0;
     DBuf<int64_t> nn_prefix, dm_prefix;  // element offsets of the molecules' n x n and ns x ns blocks
     DBuf<int> mol_n, mol_ns, mol_sh0;
-    DBuf<double> Gh, Dm;                 // half matrices and shell-pair maxima of all molecules
+    DBuf<double> Gh;                     // half matrices Jh, Kh of all molecules
+    DBuf<float> Dm;                      // shell-pair maxima of all molecules
     DBuf<double*> mol_Gh, mol_G;
-    DBuf<const double*> mol_Dm, mol_P;
-    DBuf<double> mol_screen;
+    DBuf<const double*> mol_P;
+    DBuf<const float*> mol_Dm;
+    DBuf<float> mol_screen;
     const double** h_P = nullptr;
     double** h_G = nullptr;
-    double* h_screen = nullptr;
+    float* h_screen = nullptr;
     cudaGraphExec_t exec = nullptr;      // the build's launches, captured on first use
     int64_t graph_kernels = 0;
     cudaEvent_t copied = nullptr;        // recorded after each build's table copies

@@ -1,35 +1,22 @@
-// Instantiations of the block Fock-build kernels (jk_blocks.cuh), kept out of
-// eri.cu so that they compile in parallel with it.
+// The light and middle tiers of the block Fock-build kernel (jk_blocks.cuh); the
+// heavy tier is in jk_blocks_d.cu, so that they compile in parallel.
+#include "internal.h"
 #include "jk_blocks.cuh"
 
 namespace hfgpu {
 
-DigestFn digest_fn(int tb, int tk)
-{
-#define HF_D(B, K) \
-    if (tb == B && tk == K) return digest_kernel<B, K>;
-    HF_D(0, 0) HF_D(0, 1) HF_D(0, 2) HF_D(0, 3) HF_D(0, 4) HF_D(0, 5)
-    HF_D(1, 1) HF_D(1, 2) HF_D(1, 3) HF_D(1, 4) HF_D(1, 5)
-    HF_D(2, 2) HF_D(2, 3) HF_D(2, 4) HF_D(2, 5)
-    HF_D(3, 3) HF_D(3, 4) HF_D(3, 5)
-    HF_D(4, 4) HF_D(4, 5)
-    HF_D(5, 5)
-#undef HF_D
-    return nullptr;
-}
+void launch_digest_heavy(const DigestLaunch& l, cudaStream_t s);  // jk_blocks_d.cu
 
-DigestFn digest_wide_fn(int tb, int tk)
+void launch_digest_tier(int tier, const DigestLaunch& l, cudaStream_t s)
 {
-#define HF_D(B, K) \
-    if (tb == B && tk == K) return digest_wide_kernel<B, K>;
-    HF_D(0, 0) HF_D(0, 1) HF_D(0, 2) HF_D(0, 3) HF_D(0, 4) HF_D(0, 5)
-    HF_D(1, 1) HF_D(1, 2) HF_D(1, 3) HF_D(1, 4) HF_D(1, 5)
-    HF_D(2, 2) HF_D(2, 3) HF_D(2, 4) HF_D(2, 5)
-    HF_D(3, 3) HF_D(3, 4) HF_D(3, 5)
-    HF_D(4, 4) HF_D(4, 5)
-    HF_D(5, 5)
-#undef HF_D
-    return nullptr;
+    if (tier == 0)
+        digest_kernel<0><<<l.nblocks, DIGEST_BLOCK, 0, s>>>(l);
+    else if (tier == 1)
+        digest_kernel<1><<<l.nblocks, DIGEST_BLOCK, 0, s>>>(l);
+    else
+        launch_digest_heavy(l, s);
+    count_launch();
+    HF_CUDA(cudaGetLastError());
 }
 
 }  // namespace hfgpu

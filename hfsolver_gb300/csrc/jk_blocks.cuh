@@ -10,51 +10,79 @@
 // including both orders when A == B, C == D or bra pair == ket pair; weighting
 // every element by 1/2 per coincidence of shells makes the sum over the block
 // equal to the sum over unique integrals with the usual 8-fold weights.  The
-// half-matrix updates are those of jk.cu:
-//   Gh[a][b] += 2 w P_cd, Gh[c][d] += 2 w P_ab,
-//   Gh[a][c] -= w P_bd/2, Gh[b][c] -= w P_ad/2, Gh[a][d] -= w P_bc/2, Gh[b][d] -= w P_ac/2,
-// and G = Gh + Gh^T.
+// ERI pass stores the blocks with that (exact) weight w applied, and the J and
+// K terms go to two half matrices without their factors,
+//   Jh[a][b] += w v P_cd, Jh[c][d] += w v P_ab,
+//   Kh[a][c] += w v P_bd, Kh[b][c] += w v P_ad, Kh[a][d] += w v P_bc, Kh[b][d] += w v P_ac,
+// so that G = 2 (Jh + Jh^T) - (Kh + Kh^T) / 2 takes them once per matrix element.
+//
+// Bound: the FP64 pipe.  A warp-wide FP64 instruction holds its sub-partition's
+// pipe ~64 cycles here, whatever it computes, so the six FMAs per element should
+// be all there is: no weights, no partial-sum adds (each chain continues from
+// the stored sum, partial J and K sums meet in the atomics, which the L2
+// performs), no FP64 in the screening (single precision, rounded up), no idle
+// lanes.  Measured, a full build at 8 waters (36 M elements, 0.35 ms of FP64
+// pipe): 1.16 ms with weights per output, 64-bit compares, value-returning atomics
+// and 21 launches; 0.64 ms now; at 16 waters (2.0 ms of pipe) 5.3 and 3.3 ms.  The
+// rest is the atomics (0.1 ms of the 0.64) and load latency.
 #pragma once
 #include "eri_kernel.cuh"
 
 namespace hfgpu {
+
+// one quartet class of a build
+struct DigestClass {
+    int id;       // 6 tb + tk
+    int block0;   // first thread block of the class within its launch
+    int nq;       // quartets (below 2^31, checked when the plan is made)
+    int split;    // warps that share the bra component rows of the same 32 x rounds quartets
+    int rounds;   // a warp screens rounds x 32 quartets and digests the survivors (1 to 8)
+    int nseg;
+    const Seg* segs;
+    const double* blocks;
+    // the (bra, ket) pair ids of every quartet, written by the ERI pass (null: found
+    // by searching the segments)
+    const int2* qlist;
+};
 
 struct DigestArgs {
     ShellDev sh;
     PairDev pr;
     const int* gpairs;
     const int64_t* prefix;
-    const int2* list;
-    const Seg* segs;
-    int nseg;
-    int64_t nq;
-    const double* blocks;
     const double* P;
     int n;
-    double* Gh;
-    int split;   // lanes per quartet (digest_wide_kernel; a power of two <= 32)
-    int rounds;  // a warp screens rounds x (32 / split) quartets and digests the survivors (1 to 8)
+    double* Gh;  // Jh (n x n), then Kh
     // density-difference screening (screen > 0): pair Schwarz bounds Q and the
-    // largest |P| element of each shell pair, Dm[S1 * ns + S2]
-    double screen;
-    const double* Q;
-    const double* Dm;
+    // largest |P| element of each shell pair, Dm[S1 * ns + S2] (both rounded up)
+    float screen;
+    const float* Q;
+    const float* Dm;
     int ns;
     // batched plans (mol_n != null): per molecule its basis size, density,
-    // half-matrix output, screen (< 0: not part of this build), shell-pair
-    // maximum table, shell count and first shell; the scalars above are unused
+    // half-matrix outputs, screen (< 0: not part of this build), shell-pair
+    // maximum table, shell count and first shell, and the molecule of every pair;
+    // the scalars above are unused
     const int* mol_n;
     const double* const* mol_P;
     double* const* mol_Gh;
-    const double* mol_screen;
-    const double* const* mol_Dm;
+    const float* mol_screen;
+    const float* const* mol_Dm;
     const int* mol_ns;
     const int* mol_sh0;
-    // the (bra, ket) pair ids of every quartet of the class, written by the ERI
-    // pass (null: found by searching the segments), and in batched plans the
-    // molecule of every pair
-    const int2* qlist;
     const int* pair_mol;
+};
+
+// The classes of a build go out in three launches by ket type, so that one
+// launch's classes need about the same registers: kets ss and ps (<= 80), ds and
+// pp (<= 150), dp and dd (255).  21 launches over eight streams cost 0.08 ms a
+// build before any work (3 waters: 0.105 ms a build for 0.017 ms of FP64 time).
+constexpr int DIGEST_TIERS = 3, DIGEST_TIER_MAX = 11;
+__host__ __device__ constexpr int digest_tier(int tk) { return tk / 2; }
+struct DigestLaunch {
+    DigestArgs a;
+    int ncls, nblocks;
+    DigestClass cls[DIGEST_TIER_MAX];
 };
 
 // the per-molecule view of a batched build (the arguments themselves for one molecule)
@@ -62,8 +90,8 @@ struct DigestMol {
     int n, ns, sh0;
     const double* P;
     double* Gh;
-    double screen;
-    const double* Dm;
+    float screen;
+    const float* Dm;
 };
 
 __device__ __forceinline__ bool digest_mol(const DigestArgs& a, int mol, DigestMol& m)
@@ -73,7 +101,7 @@ __device__ __forceinline__ bool digest_mol(const DigestArgs& a, int mol, DigestM
         return true;
     }
     m.screen = a.mol_screen[mol];
-    if (m.screen < 0.0) return false;
+    if (m.screen < 0.0f) return false;
     m.n = a.mol_n[mol];
     m.ns = a.mol_ns[mol];
     m.sh0 = a.mol_sh0[mol];
@@ -85,30 +113,23 @@ __device__ __forceinline__ bool digest_mol(const DigestArgs& a, int mol, DigestM
 
 // quartet qg of the class: its bra and ket pair ids and its molecule, from the
 // list the ERI pass wrote, else by searching the segments and prefix sums
-__device__ __forceinline__ void digest_quartet(const DigestArgs& a, int64_t qg, int& bra, int& ket, int& mol)
+__device__ __forceinline__ void digest_quartet(const DigestArgs& a, const DigestClass& c, int qg, int& bra, int& ket, int& mol)
 {
-    if (a.qlist) {
-        const int2 e = __ldg(a.qlist + qg);
+    if (c.qlist) {
+        const int2 e = __ldg(c.qlist + qg);
         bra = e.x;
         ket = e.y;
         mol = a.pair_mol ? __ldg(a.pair_mol + bra) : 0;
         return;
     }
-    const int qg32 = (int)qg;
-    int lo = 0, hi = a.nseg - 1;  // last segment with qoff <= qg
+    int lo = 0, hi = c.nseg - 1;  // last segment with qoff <= qg
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if ((int)(a.segs[mid].qoff) <= qg32) lo = mid; else hi = mid - 1;
+        if ((int)(c.segs[mid].qoff) <= qg) lo = mid; else hi = mid - 1;
     }
-    const Seg sg = a.segs[lo];
-    const int q = qg32 - (int)sg.qoff;  // class quartet counts stay below 2^31 (plan check)
+    const Seg sg = c.segs[lo];
+    const int q = qg - (int)sg.qoff;
     mol = sg.mol;
-    if (sg.list) {
-        const int2 e = a.list[sg.pref0 + q];
-        bra = e.x;
-        ket = e.y;
-        return;
-    }
     const int64_t* pf = a.prefix + sg.pref0;
     int l2 = 0, h2 = sg.nbra - 1;
     while (l2 < h2) {
@@ -121,21 +142,30 @@ __device__ __forceinline__ void digest_quartet(const DigestArgs& a, int64_t qg, 
 
 // true if the quartet's whole contribution is below the screening threshold:
 // |(ab|cd)| <= Q_bra Q_ket, and the largest density factor it meets is
-// 2|P_ab|, 2|P_cd| (Coulomb) or |P_ac|/2 ... (exchange)
+// 2|P_ab|, 2|P_cd| (Coulomb) or |P_ac|/2 ... (exchange).  In single precision,
+// rounded up: never true where the FP64 test would be false.
 __device__ __forceinline__ bool digest_skip(const DigestArgs& a, const DigestMol& m, int bra, int ket, int A, int B,
                                             int C, int D)
 {
-    if (m.screen <= 0.0) return false;
-    const double* Dm = m.Dm;
+    if (m.screen <= 0.0f) return false;
+    const float* Dm = m.Dm;
     const int ns = m.ns;
     A -= m.sh0; B -= m.sh0; C -= m.sh0; D -= m.sh0;
-    const double dj = fmax(Dm[A * ns + B], Dm[C * ns + D]);
-    const double dk = fmax(fmax(Dm[A * ns + C], Dm[B * ns + D]), fmax(Dm[A * ns + D], Dm[B * ns + C]));
-    return a.Q[bra] * a.Q[ket] * fmax(2.0 * dj, 0.5 * dk) < m.screen;
+    const float dj = fmaxf(Dm[A * ns + B], Dm[C * ns + D]);
+    const float dk = fmaxf(fmaxf(Dm[A * ns + C], Dm[B * ns + D]), fmaxf(Dm[A * ns + D], Dm[B * ns + C]));
+    return __fmul_ru(__fmul_ru(a.Q[bra], a.Q[ket]), fmaxf(2.0f * dj, 0.5f * dk)) < m.screen;
 }
 
-// v != 0 tested on the bit pattern (integer pipe; -0 counts as zero)
-__device__ __forceinline__ bool digest_nonzero(double v) { return (__double_as_longlong(v) << 1) != 0; }
+// v != 0 on the two 32-bit halves (-0 counts as zero): FP64 and 64-bit integer
+// compares both run on the FP64 pipe
+__device__ __forceinline__ bool digest_nonzero(double v) { return (__double2loint(v) | (__double2hiint(v) << 1)) != 0; }
+
+// *p += v with no result: a red on a global address.  atomicAdd on a generic
+// pointer compiles to an atom that returns a value, and the warp waits for it.
+__device__ __forceinline__ void red_add(double* p, double v)
+{
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
+}
 
 constexpr int DIGEST_MAX_Q = 256;  // quartets screened per warp: 32 x 8 rounds
 // threads per block of the digest kernels (two warps: a class with few quartets
@@ -146,16 +176,16 @@ constexpr int DIGEST_BLOCK = 64, DIGEST_WARPS = DIGEST_BLOCK / 32;
 // molecules not in this build) and leave the offsets of the survivors in the
 // warp's list; returns their number.  The survivors are then digested in full
 // warps, instead of each warp idling on the lanes whose quartets were skipped.
-__device__ __forceinline__ int digest_compact(const DigestArgs& a, int64_t q0, int cnt, int* list, int lane)
+__device__ __forceinline__ int digest_compact(const DigestArgs& a, const DigestClass& c, int q0, int cnt, int* list, int lane)
 {
     int ns = 0;
     for (int r = 0; r < cnt; r += 32) {
         const int k = r + lane;
-        const int64_t qg = q0 + k;
+        const int qg = q0 + k;
         bool keep = false;
-        if (k < cnt && qg < a.nq) {
+        if (k < cnt && (unsigned)qg < (unsigned)c.nq) {
             int bra, ket, mol;
-            digest_quartet(a, qg, bra, ket, mol);
+            digest_quartet(a, c, qg, bra, ket, mol);
             DigestMol mm;
             if (digest_mol(a, mol, mm))
                 keep = !digest_skip(a, mm, bra, ket, a.pr.A[bra], a.pr.B[bra], a.pr.A[ket], a.pr.B[ket]);
@@ -168,152 +198,16 @@ __device__ __forceinline__ int digest_compact(const DigestArgs& a, int64_t q0, i
     return ns;
 }
 
-// one thread digests one whole quartet (already screened)
+// One thread digests the bra component rows r0 .. r1 - 1 (row ia NB + ib) of one
+// quartet: J_cd and P_cd, and K_ac and K_ad of the current ia, in registers, K_bc
+// and K_bd in registers (NB = 1) or local memory.
 template <int TB, int TK>
-__device__ __forceinline__ void digest_one(const DigestArgs& a, int64_t qg)
+__device__ __forceinline__ void digest_rows(const DigestArgs& a, const DigestClass& c, int qg, int r0, int r1)
 {
     using CI = ClassInfo<TB, TK>;
-    constexpr int NA = ncart(CI::LA), NB = ncart(CI::LB), NC = ncart(CI::LC), ND = ncart(CI::LD);
+    constexpr int NB = ncart(CI::LB), NC = ncart(CI::LC), ND = ncart(CI::LD);
     int bra, ket, mol;
-    digest_quartet(a, qg, bra, ket, mol);
-    DigestMol mm;
-    digest_mol(a, mol, mm);
-    const int A = a.pr.A[bra], B = a.pr.B[bra], C = a.pr.A[ket], D = a.pr.B[ket];
-    int fa[NA], fb[NB], fc[NC], fd[ND];
-#pragma unroll
-    for (int i = 0; i < NA; ++i) fa[i] = a.sh.comp_fn[a.sh.cfn0[A] + i];
-#pragma unroll
-    for (int i = 0; i < NB; ++i) fb[i] = a.sh.comp_fn[a.sh.cfn0[B] + i];
-#pragma unroll
-    for (int i = 0; i < NC; ++i) fc[i] = a.sh.comp_fn[a.sh.cfn0[C] + i];
-#pragma unroll
-    for (int i = 0; i < ND; ++i) fd[i] = a.sh.comp_fn[a.sh.cfn0[D] + i];
-    const int n = mm.n;
-    const double* Pm = mm.P;
-    auto Pv = [&](int x, int y) { return (x < 0 || y < 0) ? 0.0 : __ldg(Pm + x + (int64_t)y * n); };
-    const double f = (A == B ? 0.5 : 1.0) * (C == D ? 0.5 : 1.0) * (bra == ket ? 0.5 : 1.0);
-    // every output is multiplied once by its weight (J: 2f, K: -f/2) instead of
-    // every integral by f: on this GPU each FP64 instruction is as dear as an FMA
-    const double cj = 2.0 * f, ck = -0.5 * f;
-    // accumulators indexed by the rolled (a, b) loop live in local memory; each
-    // FMA chain starts from the stored partial sum, so no separate FP64 adds
-    double jab[NA * NB], kac[NA * NC], kbc[NB * NC], kad[NA * ND], kbd[NB * ND];
-    double jcd[NC * ND], Pcd[NC * ND];
-#pragma unroll
-    for (int i = 0; i < NA * NC; ++i) kac[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NB * NC; ++i) kbc[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NA * ND; ++i) kad[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NB * ND; ++i) kbd[i] = 0.0;
-#pragma unroll
-    for (int ic = 0; ic < NC; ++ic)
-#pragma unroll
-        for (int id = 0; id < ND; ++id) {
-            jcd[ic * ND + id] = 0.0;
-            Pcd[ic * ND + id] = Pv(fc[ic], fd[id]);
-        }
-#pragma unroll 1
-    for (int ia = 0; ia < NA; ++ia)
-#pragma unroll 1
-        for (int ib = 0; ib < NB; ++ib) {
-            const double Pab = Pv(fa[ia], fb[ib]);
-            double Pac[NC], Pbc[NC], Pad[ND], Pbd[ND];
-#pragma unroll
-            for (int ic = 0; ic < NC; ++ic) {
-                Pac[ic] = Pv(fa[ia], fc[ic]);
-                Pbc[ic] = Pv(fb[ib], fc[ic]);
-            }
-#pragma unroll
-            for (int id = 0; id < ND; ++id) {
-                Pad[id] = Pv(fa[ia], fd[id]);
-                Pbd[id] = Pv(fb[ib], fd[id]);
-            }
-            double s_ab = 0.0, s_ad[ND], s_bd[ND];
-#pragma unroll
-            for (int id = 0; id < ND; ++id) {
-                s_ad[id] = kad[ia * ND + id];
-                s_bd[id] = kbd[ib * ND + id];
-            }
-            const double* blk = a.blocks + (int64_t)((ia * NB + ib) * CI::NCDT) * a.nq + qg;
-#pragma unroll
-            for (int ic = 0; ic < NC; ++ic) {
-                double s_ac = kac[ia * NC + ic], s_bc = kbc[ib * NC + ic];
-#pragma unroll
-                for (int id = 0; id < ND; ++id) {
-                    const double v = __ldg(blk + (int64_t)(ic * ND + id) * a.nq);
-                    s_ab = fma(v, Pcd[ic * ND + id], s_ab);
-                    jcd[ic * ND + id] = fma(v, Pab, jcd[ic * ND + id]);
-                    s_ac = fma(v, Pbd[id], s_ac);
-                    s_bc = fma(v, Pad[id], s_bc);
-                    s_ad[id] = fma(v, Pbc[ic], s_ad[id]);
-                    s_bd[id] = fma(v, Pac[ic], s_bd[id]);
-                }
-                kac[ia * NC + ic] = s_ac;
-                kbc[ib * NC + ic] = s_bc;
-            }
-            jab[ia * NB + ib] = s_ab;
-#pragma unroll
-            for (int id = 0; id < ND; ++id) {
-                kad[ia * ND + id] = s_ad[id];
-                kbd[ib * ND + id] = s_bd[id];
-            }
-        }
-    double* Gh = mm.Gh;
-    auto add = [&](int x, int y, double v) {
-        if (x >= 0 && y >= 0 && digest_nonzero(v)) atomicAdd(Gh + x + (int64_t)y * n, v);
-    };
-#pragma unroll 1
-    for (int ia = 0; ia < NA; ++ia)
-        for (int ib = 0; ib < NB; ++ib) add(fa[ia], fb[ib], cj * jab[ia * NB + ib]);
-#pragma unroll 1
-    for (int ic = 0; ic < NC; ++ic)
-        for (int id = 0; id < ND; ++id) add(fc[ic], fd[id], cj * jcd[ic * ND + id]);
-#pragma unroll 1
-    for (int ia = 0; ia < NA; ++ia)
-        for (int ic = 0; ic < NC; ++ic) add(fa[ia], fc[ic], ck * kac[ia * NC + ic]);
-#pragma unroll 1
-    for (int ib = 0; ib < NB; ++ib)
-        for (int ic = 0; ic < NC; ++ic) add(fb[ib], fc[ic], ck * kbc[ib * NC + ic]);
-#pragma unroll 1
-    for (int ia = 0; ia < NA; ++ia)
-        for (int id = 0; id < ND; ++id) add(fa[ia], fd[id], ck * kad[ia * ND + id]);
-#pragma unroll 1
-    for (int ib = 0; ib < NB; ++ib)
-        for (int id = 0; id < ND; ++id) add(fb[ib], fd[id], ck * kbd[ib * ND + id]);
-}
-
-template <int TB, int TK>
-__global__ void __launch_bounds__(DIGEST_BLOCK) digest_kernel(DigestArgs a)
-{
-    __shared__ int sl[DIGEST_WARPS][DIGEST_MAX_Q];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qpw = 32 * a.rounds;
-    const int64_t q0 = ((int64_t)blockIdx.x * DIGEST_WARPS + warp) * qpw;
-    if (q0 >= a.nq) return;  // the whole warp
-    if (a.screen <= 0.0 && !a.mol_n) {  // nothing is screened: no list
-        for (int k = lane; k < qpw; k += 32)
-            if (q0 + k < a.nq) digest_one<TB, TK>(a, q0 + k);
-        return;
-    }
-    const int ns = digest_compact(a, q0, qpw, sl[warp], lane);
-    for (int base = 0; base < ns; base += 32)
-        if (base + lane < ns) digest_one<TB, TK>(a, q0 + sl[warp][base + lane]);
-}
-
-// The same Fock contribution with `split` lanes per quartet, for classes with
-// few quartets and large blocks ((dd|dd) has a few hundred quartets of 1296
-// elements each): the lanes of a quartet take its (a, b) rows in turn, send
-// each row's J_ab and K contributions straight to Gh, and sum their partial
-// J_cd with warp shuffles before one lane per (c, d) adds it.
-template <int TB, int TK>
-__device__ __forceinline__ void digest_wide_one(const DigestArgs& a, int64_t qg, int split, int sub, unsigned mask)
-{
-    using CI = ClassInfo<TB, TK>;
-    constexpr int NA = ncart(CI::LA), NB = ncart(CI::LB), NC = ncart(CI::LC), ND = ncart(CI::LD);
-    int bra, ket, mol;
-    digest_quartet(a, qg, bra, ket, mol);
+    digest_quartet(a, c, qg, bra, ket, mol);
     DigestMol mm;
     digest_mol(a, mol, mm);
     const int A = a.pr.A[bra], B = a.pr.B[bra], C = a.pr.A[ket], D = a.pr.B[ket];
@@ -326,14 +220,17 @@ __device__ __forceinline__ void digest_wide_one(const DigestArgs& a, int64_t qg,
     const int* fb = a.sh.comp_fn + a.sh.cfn0[B];
     const int n = mm.n;
     const double* Pm = mm.P;
-    auto Pv = [&](int x, int y) { return (x < 0 || y < 0) ? 0.0 : __ldg(Pm + x + (int64_t)y * n); };
-    double* Gh = mm.Gh;
-    auto add = [&](int x, int y, double v) {
-        if (x >= 0 && y >= 0 && digest_nonzero(v)) atomicAdd(Gh + x + (int64_t)y * n, v);
+    auto Pv = [&](int x, int y) { return (x < 0 || y < 0) ? 0.0 : __ldg(Pm + x + y * n); };
+    double* Jh = mm.Gh;
+    double* Kh = Jh + n * n;
+    auto add = [&](double* H, int x, int y, double v) {
+        if (x >= 0 && y >= 0 && digest_nonzero(v)) red_add(H + x + y * n, v);
     };
-    const double f = (A == B ? 0.5 : 1.0) * (C == D ? 0.5 : 1.0) * (bra == ket ? 0.5 : 1.0);
-    const double cj = 2.0 * f, ck = -0.5 * f;
-    double jcd[NC * ND], Pcd[NC * ND];
+    double jcd[NC * ND], Pcd[NC * ND], kbc[NB * NC], kbd[NB * ND];
+#pragma unroll
+    for (int i = 0; i < NB * NC; ++i) kbc[i] = 0.0;
+#pragma unroll
+    for (int i = 0; i < NB * ND; ++i) kbd[i] = 0.0;
 #pragma unroll
     for (int ic = 0; ic < NC; ++ic)
 #pragma unroll
@@ -341,84 +238,130 @@ __device__ __forceinline__ void digest_wide_one(const DigestArgs& a, int64_t qg,
             jcd[ic * ND + id] = 0.0;
             Pcd[ic * ND + id] = Pv(fc[ic], fd[id]);
         }
+    const int64_t nq = c.nq;
+    const double* blk = c.blocks + (r0 * CI::NCDT) * nq + qg;
 #pragma unroll 1
-    for (int ab = sub; ab < NA * NB; ab += split) {
-        const int ia = ab / NB, ib = ab - ia * NB;
-        const int xa = __ldg(fa + ia), xb = __ldg(fb + ib);
-        const double Pab = Pv(xa, xb);
-        double Pac[NC], Pbc[NC], Pad[ND], Pbd[ND];
+    for (int r = r0; r < r1;) {
+        const int ia = r / NB;
+        const int rend = min(r1, (ia + 1) * NB);
+        const int xa = __ldg(fa + ia);
+        double Pac[NC], Pad[ND], s_ac[NC], s_ad[ND];
 #pragma unroll
         for (int ic = 0; ic < NC; ++ic) {
             Pac[ic] = Pv(xa, fc[ic]);
-            Pbc[ic] = Pv(xb, fc[ic]);
+            s_ac[ic] = 0.0;
         }
 #pragma unroll
         for (int id = 0; id < ND; ++id) {
             Pad[id] = Pv(xa, fd[id]);
-            Pbd[id] = Pv(xb, fd[id]);
+            s_ad[id] = 0.0;
         }
-        double s_ab = 0.0, s_ad[ND], s_bd[ND];
-#pragma unroll
-        for (int id = 0; id < ND; ++id) s_ad[id] = s_bd[id] = 0.0;
-        const double* blk = a.blocks + (int64_t)(ab * CI::NCDT) * a.nq + qg;
-#pragma unroll
-        for (int ic = 0; ic < NC; ++ic) {
-            double s_ac = 0.0, s_bc = 0.0;
+#pragma unroll 1
+        for (; r < rend; ++r) {
+            const int ib = NB == 1 ? 0 : r - ia * NB;
+            const int xb = __ldg(fb + ib);
+            const double Pab = Pv(xa, xb);
+            double Pbd[ND], s_ab = 0.0, s_bd[ND];
 #pragma unroll
             for (int id = 0; id < ND; ++id) {
-                const double v = __ldg(blk + (int64_t)(ic * ND + id) * a.nq);
-                s_ab = fma(v, Pcd[ic * ND + id], s_ab);
-                jcd[ic * ND + id] = fma(v, Pab, jcd[ic * ND + id]);
-                s_ac = fma(v, Pbd[id], s_ac);
-                s_bc = fma(v, Pad[id], s_bc);
-                s_ad[id] = fma(v, Pbc[ic], s_ad[id]);
-                s_bd[id] = fma(v, Pac[ic], s_bd[id]);
+                Pbd[id] = Pv(xb, fd[id]);
+                s_bd[id] = kbd[ib * ND + id];
             }
-            add(xa, fc[ic], ck * s_ac);
-            add(xb, fc[ic], ck * s_bc);
-        }
-        add(xa, xb, cj * s_ab);
 #pragma unroll
-        for (int id = 0; id < ND; ++id) {
-            add(xa, fd[id], ck * s_ad[id]);
-            add(xb, fd[id], ck * s_bd[id]);
+            for (int ic = 0; ic < NC; ++ic) {
+                const double Pbc = Pv(xb, fc[ic]);
+                double s_bc = kbc[ib * NC + ic];
+#pragma unroll
+                for (int id = 0; id < ND; ++id) {
+                    const double v = __ldg(blk);
+                    blk += nq;
+                    s_ab = fma(v, Pcd[ic * ND + id], s_ab);
+                    jcd[ic * ND + id] = fma(v, Pab, jcd[ic * ND + id]);
+                    s_ac[ic] = fma(v, Pbd[id], s_ac[ic]);
+                    s_bc = fma(v, Pad[id], s_bc);
+                    s_ad[id] = fma(v, Pbc, s_ad[id]);
+                    s_bd[id] = fma(v, Pac[ic], s_bd[id]);
+                }
+                kbc[ib * NC + ic] = s_bc;
+            }
+#pragma unroll
+            for (int id = 0; id < ND; ++id) kbd[ib * ND + id] = s_bd[id];
+            add(Jh, xa, xb, s_ab);
         }
+#pragma unroll
+        for (int ic = 0; ic < NC; ++ic) add(Kh, xa, fc[ic], s_ac[ic]);
+#pragma unroll
+        for (int id = 0; id < ND; ++id) add(Kh, xa, fd[id], s_ad[id]);
     }
-    for (int o = split >> 1; o > 0; o >>= 1)
 #pragma unroll
-        for (int i = 0; i < NC * ND; ++i) jcd[i] += __shfl_xor_sync(mask, jcd[i], o);
+    for (int ic = 0; ic < NC; ++ic)
 #pragma unroll
-    for (int i = 0; i < NC * ND; ++i)
-        if ((i & (split - 1)) == sub) add(fc[i / ND], fd[i % ND], cj * jcd[i]);
+        for (int id = 0; id < ND; ++id) add(Jh, fc[ic], fd[id], jcd[ic * ND + id]);
+    // the ib that rows r0 .. r1 - 1 met
+    const int nb = min(NB, r1 - r0);
+#pragma unroll 1
+    for (int k = 0; k < nb; ++k) {
+        const int ib = NB == 1 ? 0 : (r0 + k) % NB;
+        const int xb = __ldg(fb + ib);
+#pragma unroll
+        for (int ic = 0; ic < NC; ++ic) add(Kh, xb, fc[ic], kbc[ib * NC + ic]);
+#pragma unroll
+        for (int id = 0; id < ND; ++id) add(Kh, xb, fd[id], kbd[ib * ND + id]);
+    }
 }
 
+// One warp = 32 x rounds quartets (32 at a time, one per lane) and 1 / split of
+// their bra component rows: all lanes do the same rows, so none idles, the block
+// reads are 32 consecutive quartets of one element plane, and classes of few
+// large blocks ((dd|dd): a few hundred quartets of 1296 elements at 200
+// functions) still make many warps.
 template <int TB, int TK>
-__global__ void __launch_bounds__(DIGEST_BLOCK) digest_wide_kernel(DigestArgs a)
+__device__ __forceinline__ void digest_block(const DigestArgs& a, const DigestClass& c, int* list)
 {
-    __shared__ int sl[DIGEST_WARPS][DIGEST_MAX_Q];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = a.split, per = 32 / split;
-    const int qpw = per * a.rounds;
-    const int64_t q0 = ((int64_t)blockIdx.x * DIGEST_WARPS + warp) * qpw;
-    if (q0 >= a.nq) return;  // the whole warp
-    const int sub = lane & (split - 1);
-    const unsigned mask = split == 32 ? 0xffffffffu : (((1u << split) - 1u) << (lane & ~(unsigned)(split - 1)));
-    if (a.screen <= 0.0 && !a.mol_n) {  // nothing is screened: no list
-        for (int base = 0; base < qpw; base += per) {
-            const int64_t qg = q0 + base + lane / split;  // the same for all lanes of a quartet
-            if (qg < a.nq) digest_wide_one<TB, TK>(a, qg, split, sub, mask);
-        }
+    const int qpw = 32 * c.rounds;
+    const int w = ((int)blockIdx.x - c.block0) * DIGEST_WARPS + warp;
+    const int chunk = w / c.split, sub = w - chunk * c.split;
+    const int q0 = chunk * qpw;
+    if ((unsigned)q0 >= (unsigned)c.nq) return;  // the whole warp
+    constexpr int ROWS = ClassInfo<TB, TK>::NAB;
+    const int per = ROWS / c.split;  // split divides the rows
+    const int r0 = sub * per, r1 = r0 + per;
+    if (a.screen <= 0.0f && !a.mol_n) {  // nothing is screened: no list
+        for (int k = lane; k < qpw; k += 32)
+            if ((unsigned)(q0 + k) < (unsigned)c.nq) digest_rows<TB, TK>(a, c, q0 + k, r0, r1);
         return;
     }
-    const int ns = digest_compact(a, q0, qpw, sl[warp], lane);
-    for (int base = 0; base < ns; base += per) {
-        const int k = base + lane / split;  // the same for all lanes of a quartet
-        if (k < ns) digest_wide_one<TB, TK>(a, q0 + sl[warp][k], split, sub, mask);
-    }
+    list += warp * DIGEST_MAX_Q;
+    const int ns = digest_compact(a, c, q0, qpw, list, lane);
+    for (int base = 0; base < ns; base += 32)
+        if (base + lane < ns) digest_rows<TB, TK>(a, c, q0 + list[base + lane], r0, r1);
 }
 
-using DigestFn = void (*)(DigestArgs);
-DigestFn digest_fn(int tb, int tk);       // jk_blocks.cu
-DigestFn digest_wide_fn(int tb, int tk);  // jk_blocks.cu
+template <int TIER>
+__global__ void __launch_bounds__(DIGEST_BLOCK) digest_kernel(const __grid_constant__ DigestLaunch l)
+{
+    __shared__ int list[DIGEST_WARPS * DIGEST_MAX_Q];
+    int k = 0;
+    while (k + 1 < l.ncls && (int)blockIdx.x >= l.cls[k + 1].block0) ++k;
+    const DigestClass& c = l.cls[k];
+#define HF_D(B, K) \
+    case 6 * B + K: digest_block<B, K>(l.a, c, list); break;
+    if constexpr (TIER == 0) {
+        switch (c.id) { HF_D(0, 0) HF_D(0, 1) HF_D(1, 1) }
+    } else if constexpr (TIER == 1) {
+        switch (c.id) { HF_D(0, 2) HF_D(1, 2) HF_D(2, 2) HF_D(0, 3) HF_D(1, 3) HF_D(2, 3) HF_D(3, 3) }
+    } else {
+        switch (c.id) {
+            HF_D(0, 4) HF_D(1, 4) HF_D(2, 4) HF_D(3, 4) HF_D(4, 4)
+            HF_D(0, 5) HF_D(1, 5) HF_D(2, 5) HF_D(3, 5) HF_D(4, 5) HF_D(5, 5)
+        }
+    }
+#undef HF_D
+}
+
+// launches the classes of l (all of one tier) on stream s (jk_blocks.cu, one
+// translation unit per tier)
+void launch_digest_tier(int tier, const DigestLaunch& l, cudaStream_t s);
 
 }  // namespace hfgpu
