@@ -160,7 +160,7 @@ static void dgemm_rows(Context& ctx, const Src& src, int64_t M, int K, const dou
 void dgemm_rowmajor(Context& ctx, int64_t m, int n, int k, double alpha, const double* A, int64_t lda,
                     const double* B, int64_t ldb, double beta, double* C, int64_t ldc)
 {
-    const DenseRowsG rows{A, lda, nullptr};
+    const DenseRowsG rows(A, lda, nullptr);
     dgemm_rows(ctx, rows, m, k, B, ldb, 1, n, C, OutMap{0, ldc}, alpha, beta);
 }
 
@@ -173,10 +173,6 @@ void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int
     cudaStream_t st = ctx.stream;
     HF_CHECK(n <= 4096, HFGPU_ERR_UNSUPPORTED, "FP64 transform supports up to 4096 functions");
     const int64_t npair = (int64_t)n * (n + 1) / 2;
-    std::vector<int2> hp(npair);
-    for (int i = 0; i < n; i++)
-        for (int j = 0; j <= i; j++) hp[(size_t)i * (i + 1) / 2 + j] = make_int2(i, j);
-    DBuf<int2> pairs = to_device(hp, st);
     const int64_t nq = (int64_t)n1 * n2;
     const int nlg = (n + 15) / 16;
     DBuf<double> Z((size_t)npair * nq, st);
@@ -185,10 +181,10 @@ void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int
     DBuf<double> Y((size_t)std::min(pb, npair) * n1 * n, st);
     for (int64_t p0 = 0; p0 < npair; p0 += pb) {
         const int64_t np = std::min(pb, npair - p0);
-        const PackedRowsBlocked rows1{d_int2, pairs.p, p0, np, n, nlg, nullptr};
+        const PackedRowsBlocked rows1{d_int2, p0, np, n, nlg, nullptr};
         dgemm_rows(ctx, rows1, (np + 7) / 8 * nlg * 128, n, C1, 1, n, n1, Y.p, OutMap{n, n1});
         ctx.trace_mark("fp64 step 1");
-        const DenseRowsG rows2{Y.p, n, nullptr};
+        const DenseRowsG rows2(Y.p, n, nullptr);
         dgemm_rows(ctx, rows2, np * n1, n, C2, 1, n, n2, Z.p + p0 * nq, OutMap{0, n2});
         ctx.trace_mark("fp64 step 2");
     }
@@ -203,7 +199,7 @@ void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int
         SymPairRows rows3{Zt.p + q0 * npair, npair, n};
         dgemm_rows(ctx, rows3, nqb * n, n, C1, 1, n, n1, W.p, OutMap{n, n1});
         ctx.trace_mark("fp64 step 3");
-        const DenseRowsG rows4{W.p, n, nullptr};
+        const DenseRowsG rows4(W.p, n, nullptr);
         dgemm_rows(ctx, rows4, nqb * n1, n, C2, 1, n, n2, T + q0 * n1 * n2, OutMap{0, n2});
         ctx.trace_mark("fp64 step 4");
     }

@@ -136,6 +136,15 @@ struct Context {
     double stat_fock_ms = 0, stat_tc_ms = 0, stat_tc_flops = 0;
     // the gather-fed GEMM over the packed integrals (transform step 1) alone
     double stat_tc_step1_ms = 0, stat_tc_step1_n = 0;
+    // event pairs around sliced GEMMs and their error flag (device), read by
+    // sliced_gemm_settle() at the end of a transform instead of after each GEMM
+    struct TcTimer {
+        cudaEvent_t a, b;
+        double flops;
+        bool step1;
+    };
+    std::vector<TcTimer> tc_events;
+    int* tc_err = nullptr;
     bool tune = false;  // time candidate kernel shapes on first use (autotune.cpp)
     // phase trace (HFGPU_TRACE=1 in the environment): an event on `stream` and a
     // host clock reading at each named point of a pipeline call; trace_report()

@@ -1,15 +1,17 @@
-// Mixed-precision AO -> MO transform on the tensor cores, for MBPT2.
+// AO -> MO half transform on the tensor cores, and MBPT2 from it.
 //
-// Same (ia|jb) as ao2mo_fp64 (the quantity transform_int2, src/mbpt.f90:11-79,
-// feeds to term1, src/mbpt2.f90:8-31), ordered as a half transform so that
-// every contraction is one "tall A times coefficient block" GEMM in the exact
-// bf16-sliced form of tcgemm.cu (FP64 inputs and outputs):
+// The (ia|jb) that transform_int2 (src/mbpt.f90:11-79) feeds to term1
+// (src/mbpt2.f90:8-31), ordered as a half transform so that every contraction is one
+// "tall A times coefficient block" GEMM in the exact bf16-sliced form of tcgemm.cu
+// (FP64 inputs and outputs; six digits for the mixed-precision path, nine for the
+// plain FP64 one):
 //   1. Y[p][j][la]  = sum_si (mu nu|la si) C1[si, j]     p = pair(mu >= nu)
 //   2. Z[p][j][b]   = sum_la Y[p][j][la] C2[la, b]
 //   3. W[q][i][mu]  = sum_nu Z[pair(mu, nu)][q] C1[nu, i]    q = (j, b)
 //   4. T[q][i][a]   = sum_mu W[q][i][mu] C2[mu, a]       T[j][b][i][a] = (ia|jb)
-// Steps 1-2 run over blocks of pairs and steps 3-4 over blocks of q, so each
-// sliced operand stays within a fixed device-memory budget.
+// The rows of A are gathered where they lie (the packed integrals, Z transposed, Y and
+// W) and cut inside the GEMM.  Steps 1-2 run over blocks of pairs and steps 3-4 over
+// blocks of q, so Y and W stay within a fixed device-memory budget.
 #include <algorithm>
 #include <vector>
 
@@ -19,7 +21,7 @@
 
 namespace hfgpu {
 
-static const int64_t SLICE_BUDGET_ROWS = 1 << 20;  // rows per sliced operand (x K_pad x 10 bytes)
+static const int64_t BLOCK_ROWS = 1 << 20;  // GEMM rows of a block
 
 // out[c][r] = in[r][c] for a rows x cols row-major matrix (32 x 32 tiles through
 // shared memory, both sides coalesced)
@@ -47,68 +49,32 @@ void transpose_device(Context& ctx, const double* in, int64_t rows, int64_t cols
 }
 
 void ao2mo_sliced(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,
-                  double* T)
+                  int digits, double* T)
 {
     cudaStream_t st = ctx.stream;
-    HF_CHECK(n <= 512, HFGPU_ERR_UNSUPPORTED, "mixed-precision transform supports up to 512 functions");
-    const int64_t npair = (int64_t)n * (n + 1) / 2;
-    std::vector<int2> hp(npair);
-    for (int i = 0; i < n; i++)
-        for (int j = 0; j <= i; j++) hp[(size_t)i * (i + 1) / 2 + j] = make_int2(i, j);
-    DBuf<int2> pairs = to_device(hp, st);
-    Sliced B1, B2, A;
-    // steps 2 and 4 (N = v) read their FP64 rows straight into the gather-fed GEMM
-    // (coalesced rows, no slice planes through HBM) while the virtual block spans
-    // at most DENSE_GATHER_TILES output tiles of 80 columns; wider ones use slicing
-    // + TMA.  Measured at 16 waters (v = 320, four tiles): gathering each row four
-    // times beats slicing it once through HBM (steps 2 + 4: 131 -> 91 ms).  The gather GEMM walks whole 80-column tiles of B, so C2's slices are
-    // then padded to a multiple of 80 rows.
-    constexpr int DENSE_GATHER_TILES = 4;
-    const bool dense_gather = n2 <= 80 * DENSE_GATHER_TILES;
-    slice_dense(ctx, C1, n1, n, n, B1, SLICE_TILE_B);  // rows of B^T = columns of C1
-    slice_dense(ctx, C2, n2, n, n, B2, dense_gather ? 80 : SLICE_TILE_B);
+    const int64_t npair = (int64_t)n * (n + 1) / 2, nq = (int64_t)n1 * n2;
+    Sliced B1, B2;
+    slice_dense(ctx, C1, n1, n, n, digits, B1);  // rows of B^T = columns of C1
+    slice_dense(ctx, C2, n2, n, n, digits, B2);
     ctx.trace_mark("mp2 slice C");
-    const int64_t nq = (int64_t)n1 * n2;
-    // gather-fed GEMMs for steps 1 and 3 when C1's columns fit one output tile of
-    // the gather kernel (64 or 80 columns); with two column tiles the rows would be
-    // gathered twice and the slicing + TMA path wins
-    const bool gather = n1 <= 80;
-    // row maxima of the gathered rows (exponents of their slices), by coalesced
-    // passes over the packed array instead of a second gather inside the GEMM
-    DBuf<unsigned> rmax;
-    if (gather) {
-        // reused by steps 3-4 for blocks of at most qb rows q
-        const int64_t qb_rows = std::max<int64_t>(1, SLICE_BUDGET_ROWS / std::max(n, n1));
-        rmax.alloc((size_t)std::max(npair, std::min(qb_rows, nq)) * n, st);
-        packed_row_max(ctx, d_int2, n, rmax.p);
-        ctx.trace_mark("mp2 row max");
-    }
+    // row maxima of the gathered rows (the exponents of their digits), by coalesced
+    // passes instead of a second gather inside the GEMM
+    const int64_t pb = std::min(npair, std::max<int64_t>(8, BLOCK_ROWS / n / 8 * 8));
+    const int64_t qb = std::min(nq, std::max<int64_t>(1, BLOCK_ROWS / std::max(n, n1)));
+    DBuf<unsigned> rmax((size_t)std::max(npair, qb) * n, st), dmax((size_t)std::max(pb, qb) * n1, st);
+    packed_row_max(ctx, d_int2, n, rmax.p);
+    ctx.trace_mark("mp2 row max");
     DBuf<double> Z((size_t)npair * nq, st);
-    // steps 1-2 over blocks of pairs
-    const int64_t pb = std::max<int64_t>(1, SLICE_BUDGET_ROWS / n);
-    const int64_t qb_rows2 = std::max<int64_t>(1, SLICE_BUDGET_ROWS / std::max(n, n1));
-    DBuf<unsigned> dmax;
-    if (dense_gather) dmax.alloc((size_t)std::max(std::min(pb, npair), std::min(qb_rows2, nq)) * n1, st);
-    DBuf<double> Y((size_t)std::min(pb, npair) * n1 * n, st);
-    for (int64_t p0 = 0; p0 < npair; p0 += pb) {
-        const int64_t np = std::min(pb, npair - p0);
-        // rows (p, la) -> Y[p][j][la]; with one output column tile the ERIs are
-        // sliced inside the GEMM (gathered once), else through bf16 planes
-        if (gather) {
-            sliced_gemm_packed(ctx, d_int2, pairs.p, p0, np, n, rmax.p, B1, Y.p, OutMap{n, n1});
-        } else {
-            slice_packed(ctx, d_int2, pairs.p, p0, np, n, A);
-            sliced_gemm(ctx, A, B1, Y.p, OutMap{n, n1}, false);
-        }
-        ctx.trace_mark("mp2 step 1");
-        if (dense_gather) {  // rows (p, j) -> Z[p][j][b]
+    {
+        DBuf<double> Y((size_t)pb * n1 * n, st);
+        for (int64_t p0 = 0; p0 < npair; p0 += pb) {
+            const int64_t np = std::min(pb, npair - p0);
+            sliced_gemm_packed(ctx, d_int2, p0, np, n, rmax.p, B1, Y.p, OutMap{n, n1});
+            ctx.trace_mark("mp2 step 1");
             dense_row_max(ctx, Y.p, np * n1, n, n, dmax.p);
-            sliced_gemm_dense_gather(ctx, Y.p, np * n1, n, n, dmax.p, B2, Z.p + p0 * nq, OutMap{0, n2});
-        } else {
-            slice_dense(ctx, Y.p, np * n1, n, n, A, SLICE_TILE_A);
-            sliced_gemm(ctx, A, B2, Z.p + p0 * nq, OutMap{0, n2}, false);
+            sliced_gemm_dense(ctx, Y.p, np * n1, n, n, dmax.p, B2, Z.p + p0 * nq, OutMap{0, n2});
+            ctx.trace_mark("mp2 step 2");
         }
-        ctx.trace_mark("mp2 step 2");
     }
     // Z^T: one contiguous row of pairs per q, so that the (q, mu) rows of step 3
     // gather from one L2-resident row instead of one cache line per element
@@ -116,29 +82,19 @@ void ao2mo_sliced(Context& ctx, int n, const double* d_int2, const double* C1, i
     transpose_device(ctx, Z.p, npair, nq, Zt.p);
     Z.release();
     ctx.trace_mark("mp2 transpose");
-    // steps 3-4 over blocks of q
-    const int64_t qb = std::max<int64_t>(1, SLICE_BUDGET_ROWS / std::max(n, n1));
-    DBuf<double> W((size_t)std::min(qb, nq) * n1 * n, st);
+    DBuf<double> W((size_t)qb * n1 * n, st);
     for (int64_t q0 = 0; q0 < nq; q0 += qb) {
         const int64_t nqb = std::min(qb, nq - q0);
         // rows (q, mu) over nu of Zt[q0 + q][pair(mu, nu)] -> W[q][i][mu]
-        if (gather) {
-            sympair_row_max(ctx, Zt.p + q0 * npair, npair, nqb, n, rmax.p);
-            sliced_gemm_sympair(ctx, Zt.p + q0 * npair, npair, nqb, n, rmax.p, B1, W.p, OutMap{n, n1});
-        } else {
-            slice_sympair(ctx, Zt.p + q0 * npair, npair, nqb, n, A);
-            sliced_gemm(ctx, A, B1, W.p, OutMap{n, n1}, false);
-        }
+        sympair_row_max(ctx, Zt.p + q0 * npair, npair, nqb, n, rmax.p);
+        sliced_gemm_sympair(ctx, Zt.p + q0 * npair, npair, nqb, n, rmax.p, B1, W.p, OutMap{n, n1});
         ctx.trace_mark("mp2 step 3");
-        if (dense_gather) {  // rows (q, i) -> T[q][i][a]
-            dense_row_max(ctx, W.p, nqb * n1, n, n, dmax.p);
-            sliced_gemm_dense_gather(ctx, W.p, nqb * n1, n, n, dmax.p, B2, T + q0 * n1 * n2, OutMap{0, n2});
-        } else {
-            slice_dense(ctx, W.p, nqb * n1, n, n, A, SLICE_TILE_A);
-            sliced_gemm(ctx, A, B2, T + q0 * n1 * n2, OutMap{0, n2}, false);
-        }
+        // rows (q, i) -> T[q][i][a]
+        dense_row_max(ctx, W.p, nqb * n1, n, n, dmax.p);
+        sliced_gemm_dense(ctx, W.p, nqb * n1, n, n, dmax.p, B2, T + q0 * n1 * n2, OutMap{0, n2});
         ctx.trace_mark("mp2 step 4");
     }
+    sliced_gemm_settle(ctx);
 }
 
 // one block per pair i >= j: sum_ab (ia|jb) [2 (ia|jb) - (ib|ja)] / (e_i + e_j - e_a - e_b)
@@ -201,7 +157,9 @@ double mp2_energy_mixed(Context& ctx, int n, const double* d_int2, const double*
     const int v = n - o;
     if (o <= 0 || v <= 0) return 0.0;
     DBuf<double> T((size_t)o * v * o * v, ctx.stream);
-    ao2mo_sliced(ctx, n, d_int2, dC, o, dC + (size_t)n * o, v, T.p);
+    HF_CHECK(n <= slice_kmax(SLICE_MIXED), HFGPU_ERR_UNSUPPORTED,
+             "mixed-precision transform supports up to 512 functions");
+    ao2mo_sliced(ctx, n, d_int2, dC, o, dC + (size_t)n * o, v, SLICE_MIXED, T.p);
     const int npairs = o * (o + 1) / 2;
     DBuf<double> part((size_t)npairs, ctx.stream);
     mp2_pair_energy_kernel<<<npairs, 256, 0, ctx.stream>>>(o, v, T.p, d_eps, part.p);

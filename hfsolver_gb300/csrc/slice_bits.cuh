@@ -1,19 +1,23 @@
-// Integer-only pieces of the exact bf16 slicing (tcgemm.cu), shared by the
-// device kernels and host-side checks.
+// Integer pieces of the exact bf16 slicing (tcgemm.cu), host and device.
 //
 // A row with exponent e (|x| < 2^e for every element) is scaled to the integer
-// Y = round(|x| 2^(42 - e)) < 2^42 (+1 by rounding), cut into six 7-bit digits
-// Y = sum_t d_t 2^(7 (5 - t)) (d_0 may reach 128), and each digit is stored as
-// the bf16 value sign(x) d_t.  GB300 runs 64-bit conversions on its narrow
-// FP64 pipe, so everything here is integer arithmetic, except for one packed
-// bf16 subtraction per two digits: the bit pattern 0x4300 | d is the bf16
-// value 128 + d for 0 <= d <= 128 (the digit lands in the mantissa, or for
-// d = 128 carries into the exponent), and subtracting 128 leaves exactly d.
+// Y = round(x 2^(F - e)), |Y| <= 2^F, and cut into N balanced digits of radix 128,
+// Y = sum_t d_t 2^(7 (N - 1 - t)), every digit an integer that bf16 holds exactly:
+//   N = 6, F = 42: |d_0| <= 128, -64 <= d_t <= 63 below it (the mixed-precision path)
+//   N = 9, F = 62: |d_0| <= 64, the same below (FP64 accuracy: 2^-62 of the row's scale)
+// Digits are balanced rather than sign and magnitude for two reasons.  The sum over
+// K of all digit products of one group i + j = t stays below 2^24, so FP32
+// accumulation is exact for every input: N = 6: (2 128 64 + 4 64 64) K <= 2^24 for
+// K <= 512; N = 9: 9 64 64 K < 2^24 for K <= 455.  And the products that are left
+// out (i + j >= N) are half as large and of random sign: the error is about half
+// that of 7-bit magnitudes at the same number of products.
 //
-// The epilogue's conversion back, RN((double) S) 2^E for the int64 sum S of
-// the digit products, is done the same way: the double's fields are assembled
-// from the integer's leading bit and a round-to-nearest-even of the bits below
-// the 53rd, so the FP64 pipe is not used for the output either.
+// Adding the bias 64 (1 + 128 + ... ) (128 at the top of N = 6) to the two's
+// complement Y turns the digits into plain bit fields u_t = d_t + bias.  The bf16
+// pattern 0x4300 | u is the value 128 + u (u <= 128: a carry makes it 256), so one
+// packed subtraction of 192 leaves two digits exactly.  GB300 runs 64-bit
+// conversions and compares on its narrow FP64 pipe; everything here is 32-bit
+// integer and bf16x2 arithmetic.
 #pragma once
 #include <cstdint>
 
@@ -25,83 +29,46 @@
 
 namespace hfgpu {
 
-constexpr int SLICE_NSL = 6, SLICE_BITS = 7;
-
-HF_HD int clz64(uint64_t v)
-{
-#ifdef __CUDA_ARCH__
-    return __clzll((long long)v);
-#else
-    return v ? __builtin_clzll(v) : 64;
-#endif
-}
-
-// round(|x| 2^(42 - e)) from the bits of x (0 for zero and subnormal x)
-HF_HD uint64_t scaled_magnitude(uint64_t bits, int e)
-{
-    const int ex = (int)((bits >> 52) & 0x7FF);
-    uint64_t Y = 0;
-    if (ex != 0) {
-        const uint64_t m = (bits & ((1ull << 52) - 1)) | (1ull << 52);
-        const int sh = ex - 1075 + SLICE_NSL * SLICE_BITS - e;  // |x| < 2^e gives sh < -10
-        if (sh >= 0)
-            Y = m << sh;
-        else if (sh > -63)
-            Y = (m + (1ull << (-sh - 1))) >> (-sh);
+template <int NSL>
+struct SliceFmt {
+    static_assert(NSL == 6 || NSL == 9, "digit counts with a stated range");
+    static constexpr int F = NSL == 6 ? 42 : 62;
+    static constexpr int HALF = NSL == 6 ? 1 : 0;  // the biased value is kept doubled (one bit below the digits)
+    static constexpr int KMAX = NSL == 6 ? 512 : 455;
+    static constexpr uint64_t lower()  // 64 (1 + 128 + ... + 128^(NSL - 2))
+    {
+        uint64_t b = 0;
+        for (int k = 0; k < NSL - 1; ++k) b |= 64ull << (7 * k);
+        return b;
     }
-    return Y;
+    static constexpr uint64_t BIAS = (lower() + ((NSL == 6 ? 128ull : 64ull) << (7 * (NSL - 1)))) << HALF;
+    // out = 2^(ea + eb - SHIFT) sum_t acc_t 2^(7 (NSL - 1 - t)): two scales F, less the
+    // weights 7 (2 NSL - 2) - 7 (NSL - 1) taken by the recombination
+    static constexpr int SHIFT = 2 * F - 7 * (NSL - 1);
+};
+
+// the biased digits of x (its bits), scaled by the row exponent e: U = Y + bias
+// (doubled where HALF = 1).  Zero and subnormal x give Y = 0.
+template <int NSL>
+HF_HD uint64_t biased_digits(uint64_t bits, int e)
+{
+    using S = SliceFmt<NSL>;
+    const int ex = (int)(bits >> 52) & 0x7FF;
+    const uint64_t m = (bits << 11) | (1ull << 63);  // |x| = m 2^(ex - 1022 - 64)
+    const int r = 63 - S::F + e + 1022 - ex;         // m >> r is |x| 2^(F + 1 - e)
+    uint64_t t = 0;
+    if (ex != 0 && r <= 63) t = (m >> r) + 1;        // + 1: round half up at the bit below the digits
+    t = S::HALF ? t & ~1ull : t >> 1;
+    const uint64_t sgn = (uint64_t)((int64_t)bits >> 63);
+    return ((t ^ sgn) - sgn) + S::BIAS;
 }
 
-// digit t (0: most significant) of Y
-HF_HD uint32_t digit(uint64_t Y, int t)
+// the digit field of weight 128^(NSL - 1 - t) of U (biased)
+template <int NSL>
+HF_HD uint32_t digit_field(uint64_t U, int t)
 {
-    const int shift = SLICE_BITS * (SLICE_NSL - 1 - t);
-    return (uint32_t)(Y >> shift) & (t == 0 ? 0xFFFFFFFFu : ((1u << SLICE_BITS) - 1));
-}
-
-// plane t of two elements before the subtraction: bf16 patterns of 128 + d
-// (element 0 in the low half)
-HF_HD uint32_t digit_word(uint64_t Y0, uint64_t Y1, int t)
-{
-    return 0x43004300u | digit(Y0, t) | (digit(Y1, t) << 16);
-}
-
-// sign bits of two elements, in place for the packed bf16 pair
-HF_HD uint32_t sign_word(uint64_t bits0, uint64_t bits1)
-{
-    return (uint32_t)(bits0 >> 63) << 15 | (uint32_t)(bits1 >> 63) << 31;
-}
-
-// RN((double) S) 2^E assembled from integer fields.  ok = false when the result
-// would be subnormal or overflow (the caller then uses the FP64 unit).
-HF_HD uint64_t scaled_int_to_double_bits(long long S, int E, bool& ok)
-{
-    ok = true;
-    if (S == 0) return 0;
-    const uint64_t sign = S < 0 ? 1ull : 0ull;
-    const uint64_t m = sign ? (uint64_t)0 - (uint64_t)S : (uint64_t)S;
-    int msb = 63 - clz64(m);
-    uint64_t mant;
-    if (msb <= 52) {
-        mant = m << (52 - msb);
-    } else {
-        const int sh = msb - 52;
-        const uint64_t rem = m & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-        mant = m >> sh;
-        if (rem > half || (rem == half && (mant & 1ull))) {
-            ++mant;
-            if (mant == (1ull << 53)) {
-                mant >>= 1;
-                ++msb;
-            }
-        }
-    }
-    const int ef = msb + E + 1023;
-    if (ef <= 0 || ef >= 2047) {
-        ok = false;
-        return 0;
-    }
-    return sign << 63 | (uint64_t)ef << 52 | (mant & ((1ull << 52) - 1));
+    const uint32_t v = (uint32_t)(U >> (7 * (NSL - 1 - t) + SliceFmt<NSL>::HALF));
+    return t == 0 ? v : v & 127u;
 }
 
 }  // namespace hfgpu

@@ -1,35 +1,48 @@
 // FP64-accurate GEMM on the tcgen05 tensor cores (sm_103a) by exact bf16 slicing.
 //
-// C[r, c] = sum_k A[r, k] B[k, c] for FP64 A and B, as used by the mixed-
-// precision AO->MO transform.  Each row of A (and each column of B) is scaled
-// by a power of two 2^e so that |x| < 2^e, rounded to a 42-bit fixed-point
-// integer and cut into six 7-bit digits d_0..d_5 (x ~ 2^e sum_t d_t 2^{-7(t+1)}),
-// stored as bf16 "slice planes" (integers <= 128 are exact in bf16).  This is
-// the error-free splitting of Ozaki, Ogita, Oishi and Rump (Numer. Algorithms
-// 59, 95 (2012)) with bf16 tensor-core products:
-//   * a product of two digits is < 2^14, so a K-sum of one digit pair over
-//     K <= 1024 stays below 2^24 and the FP32 tensor-core accumulation is exact;
-//   * digit pairs (i, j) with i + j = t share the weight 2^{-7(t+2)} and are
-//     accumulated together in TMEM accumulator t (t = 0..5, 21 products);
-//     groups t = 0, 1 stay exact for K <= 512, and the rounding of the later
-//     groups is below 2^{-24} of terms that are already 2^{-28} smaller;
-//   * the epilogue recombines sum_t acc_t 2^{-7(t+2)} exactly in int64 and
-//     applies the row and column scales with one FP64 multiply.
-// The result matches an FP64 GEMM to about 2^-42 K max|A_r.| max|B_.c| per element.
+// C[r, c] = sum_k A[r, k] B[k, c] for FP64 A and B, as used by the AO->MO
+// transforms.  Each row of A (and each column of B) is scaled by a power of two 2^e
+// so that |x| < 2^e, rounded to a fixed-point integer and cut into NSL balanced
+// 7-bit digits d_0 .. d_{NSL-1} (slice_bits.cuh), stored as bf16.  This is the
+// error-free splitting of Ozaki, Ogita, Oishi and Rump (Numer. Algorithms 59, 95
+// (2012)) with bf16 tensor-core products: digit pairs (i, j) with i + j = t share a
+// weight and are accumulated together in group t (t < NSL); every group's FP32 sum
+// is exact; the epilogue recombines the groups in int64 and applies the row and
+// column scales.  Six digits (21 products) keep each entry to 2^-42 of its row's or
+// column's scale; nine digits (45 products) keep 2^-62, more than an FP64 entry has.
 //
-// Kernel: persistent CTAs (128 threads, one per SM) walk the 128 x 64 output
-// tiles.  A K step of 32 is one pipeline stage: the 6 A and 6 B slice tiles
-// (TMA, 64-byte swizzle, 72 KiB); three stages are in flight.  One thread
-// issues the loads and the 21 x 2 tcgen05.mma (M=128, N=64, K=16, BF16 in,
-// FP32 out) per step, queueing step k's products before it waits for step
-// k-1's to free that stage for step k-1+3.  The next tile's first loads are
-// issued before the epilogue reads TMEM.  Every wait on an mbarrier is bounded
-// and reports a timeout through an error flag instead of spinning forever.
-#include <cuda.h>
+// Kernel: persistent CTAs, one per SM, walk the 128 x T output tiles; a K step of 32
+// is one pipeline stage.
+//   * A: 16 producer warps gather their rows' FP64 elements (Src, gather_rows.cuh),
+//     cut them and store the digits straight into the stage's shared-memory tiles in
+//     the 64-byte-swizzled K-major layout the MMA reads (16-byte chunk c of row r at
+//     c ^ ((r >> 1) & 3)).  Thread t: row t % 128, K quarter t / 128 (8 elements, one
+//     chunk per plane); the elements of the next two steps are in flight.
+//   * B: its digit planes are stacked as NSL T rows of one K-major tile (one bulk copy
+//     a stage, laid out by slice_kernel), so that digit plane i of A multiplies
+//     consecutive planes of B in one product: column block j lands on group i + j by
+//     starting at TMEM column (i + j) T.  The groups are taken in slots of three, so
+//     that consecutive products write the same columns: 9 tcgen05.mma of up to 240
+//     columns per 16 k instead of 21 of T.  (One product over all the planes that i
+//     meets, whose column ranges overlap in part from one i to the next, ran 30%
+//     slower: 44 against 34 ms for 16 waters' step 1 with the cutting left out.)
+//   * The 17th warp issues the B loads (ahead, into every free stage) and the products.
+//   * Producers read the accumulators of a finished tile back (tcgen05.ld) after they
+//     have filled the first stage of the next one, so that the products have a stage to
+//     go on with; with NSL T <= 256 columns two sets of accumulators fit TMEM and the
+//     products go on meanwhile too.
+// Bound: the producers' instructions (gather, cut, read back), then shared-memory
+// bandwidth (a 32 k step of 80 columns reads 180 KB for its products beside the 78 KB
+// written).  Transform step 1 against separate products per digit pair, accumulators
+// read back at a tile barrier and B as tensor-map tiles: 8 waters (N = 40) 6.9 ->
+// 3.5 ms, 16 waters (N = 80) 77 -> 55 ms; all four steps 12.4 -> 7.0 and 187 -> 130.
+// Every wait on an mbarrier is bounded and reports a timeout through an error flag
+// instead of spinning forever.
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <mutex>
+#include <string>
 #include <type_traits>
 
 #include "internal.h"
@@ -39,15 +52,13 @@
 
 namespace hfgpu {
 
-constexpr int NSL = 6, SL_BITS = 7;
-constexpr int BM = 128, BN = 64, BK = 32;
-constexpr int STAGES = 3;
-constexpr int A_TILE = BM * BK * 2;  // 8 KiB
-constexpr int B_TILE = BN * BK * 2;  // 4 KiB
-constexpr int STAGE_BYTES = NSL * (A_TILE + B_TILE);  // 72 KiB: the 12 slice tiles of one K step
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 128;
-constexpr uint32_t TMEM_COLS = 512;  // 6 accumulators x 64 columns, rounded to a power of two
-constexpr int WAIT_SPINS = 1 << 22;
+constexpr int BM = 128, BK = 32;
+constexpr int A_TILE = BM * BK * 2;  // 8 KiB: one digit plane of a stage
+constexpr uint32_t TMEM_COLS = 512;
+constexpr int WAIT_SPINS = 1 << 20;  // of up to 2 us each
+constexpr int GATHER_PRODUCERS = 512, PRODUCER_WARPS = GATHER_PRODUCERS / 32;
+constexpr int GATHER_THREADS = GATHER_PRODUCERS + 32;
+constexpr int MAX_STAGES = 4, MAX_OPS = 18;
 
 // ------------------------------------------------------------------ PTX helpers
 __device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -73,29 +84,39 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase)
     return ok != 0;
 }
 
+// the same, suspended for up to about `ns` while the phase is open: polling would take
+// issue slots from the warps that cut digits
+__device__ __forceinline__ bool mbar_try_wait_ns(uint64_t* bar, uint32_t phase, uint32_t ns)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(su32(bar)), "r"(phase), "r"(ns)
+        : "memory");
+    return ok != 0;
+}
+
 // bounded wait on an mbarrier phase; false after WAIT_SPINS polls
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase)
 {
-    for (int i = 0; i < WAIT_SPINS; ++i) {
-        if (mbar_try_wait(bar, phase)) return true;
-        if (i > 32) __nanosleep(64);
-    }
+    for (int i = 0; i < WAIT_SPINS; ++i)
+        if (mbar_try_wait_ns(bar, phase, 2000)) return true;
     return false;
 }
 
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar)
+// contiguous copy into shared memory (16-byte aligned, bytes a multiple of 16)
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar)
 {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            su32(dst)),
-        "l"((uint64_t)map), "r"(x), "r"(y), "r"(su32(bar))
-        : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(su32(dst)),
+                 "l"(src), "r"(bytes), "r"(su32(bar))
+                 : "memory");
 }
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// K-major operand tile written by TMA with 64-byte swizzle (rows of BK = 32
+// K-major operand tile with 64-byte swizzle (rows of BK = 32
 // bf16): 8-row groups 512 B apart
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr)
 {
@@ -107,21 +128,17 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr)
     return d;
 }
 
-// kind::f16 instruction descriptor: BF16 x BF16 -> FP32, both K-major, M = 128, N = BN
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-
-__device__ __forceinline__ void umma_d(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc)
+// kind::f16 instruction descriptor: BF16 x BF16 -> FP32, both K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t idesc(int n)
 {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dt),
-        "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t acc)
+__device__ __forceinline__ void umma(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t id, uint32_t acc)
 {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dt),
-        "l"(ad), "l"(bd), "r"(IDESC), "r"(acc));
+        "l"(ad), "l"(bd), "r"(id), "r"(acc));
 }
 
 __device__ __forceinline__ void umma_commit(uint64_t* bar)
@@ -130,17 +147,28 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar)
                  : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(bar)) : "memory");
+}
+
+// four consecutive columns of the calling warp's 32 lanes (no wait)
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+}
+// wait for the loads queued so far; the registers pass through so that nothing reads
+// them earlier
+template <int N>
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[N][4])
+{
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    for (int t = 0; t < N; ++t)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm volatile("" : "+r"(r[t][i]));
 }
 
 // 2^e for any integer e (0 below the normal range, where the scaled values of
@@ -152,688 +180,522 @@ __device__ __forceinline__ double pow2(int e)
     return __longlong_as_double((int64_t)(e + 1023) << 52);
 }
 
-static_assert(NSL == SLICE_NSL && SL_BITS == SLICE_BITS, "slice layout shared with slice_bits.cuh");
-
-// RN((double) S) 2^E, from integer fields where the result is a normal double
-// (slice_bits.cuh), else on the FP64 unit; identical results either way
-__device__ __forceinline__ double scaled_sum_to_double(long long S, int E)
+// v 2^E, by the exponent field where v is zero or |E| leaves the result normal (v is an
+// integer below 2^120 in magnitude)
+__device__ __forceinline__ double scale_pow2(double v, int E)
 {
-    if (E >= -1022 && E <= 1023) {
-        bool ok;
-        const uint64_t b = scaled_int_to_double_bits(S, E, ok);
-        if (ok) return __longlong_as_double((long long)b);
-    }
-    return (double)S * pow2(E);
+    const int hi = __double2hiint(v);
+    if ((unsigned)(E + 900) <= 1800u) return __hiloint2double((hi << 1) == 0 ? hi : hi + (E << 20), __double2loint(v));
+    return v * pow2(E);
 }
 
-// two bf16 lanes minus 128 (exact): 0x4300 | d -> d (slice_bits.cuh)
-__device__ __forceinline__ uint32_t bf16x2_minus_128(uint32_t w)
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c)
 {
-    uint32_t r;
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0x43004300u));
-    return r;
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
 }
 
-// ------------------------------------------------------------------ GEMM kernel
-__device__ __forceinline__ int64_t out_index(const OutMap& om, int64_t r, int64_t c)
+// group sums (integers, |a_t| <= 2^24) -> sum_t a_t 2^(7 (NSL - 1 - t)), rounded once to
+// FP64 and times 2^E: 32 x 32 + 64-bit multiply-adds, and one or two conversions on
+// the FP64 pipe (they overlap the integer work of other warps).
+template <int NSL>
+__device__ __forceinline__ double recombine(const uint32_t (&a)[NSL], int E)
 {
-    return om.R > 0 ? (r / om.R) * (om.R * om.ld) + c * om.R + (r % om.R) : r * om.ld + c;
-}
-
-__global__ void __launch_bounds__(128, 1)
-    sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                       int64_t a_rows_pad, int b_rows_pad, int ksteps, const int* __restrict__ ea,
-                       const int* __restrict__ eb, int64_t M, int N, double* out, OutMap om, int accumulate,
-                       int* err, int64_t ntiles, int ntn)
-{
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);  // TMA landed, one per stage
-    uint64_t* empty = full + STAGES;                            // products of the stage done
-    uint32_t* tslot = (uint32_t*)(empty + STAGES);
-    __shared__ int s_ok;
-    auto sA = [&](int s, int t) { return smem + s * STAGE_BYTES + t * A_TILE; };
-    auto sB = [&](int s, int t) { return smem + s * STAGE_BYTES + NSL * A_TILE + t * B_TILE; };
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)),
-                     "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    const uint32_t tmem = *tslot;
-
-    // thread 0's bookkeeping: the K step whose load is in flight on each stage
-    // (-1: none), and the last K step whose products were committed
-    int64_t pend[STAGES];
-    for (int s = 0; s < STAGES; ++s) pend[s] = -1;
-    int64_t last_commit = -1;
-    auto load = [&](int64_t g, int64_t m0, int n0, int ks) {
-        const int s = (int)(g % STAGES);
-        mbar_expect_tx(&full[s], STAGE_BYTES);
+    int v[NSL];
 #pragma unroll
-        for (int t = 0; t < NSL; ++t) {
-            tma_load_2d(sA(s, t), &tmA, ks * BK, (int)(t * a_rows_pad + m0), &full[s]);
-            tma_load_2d(sB(s, t), &tmB, ks * BK, t * b_rows_pad + n0, &full[s]);
-        }
-        pend[s] = g;
-    };
-    const int pro = ksteps < STAGES ? ksteps : STAGES;
-
-    bool ok = true;
-    int64_t g0 = 0;  // K steps run by this CTA before the current tile
-    int64_t tile = blockIdx.x;
-    if (tile < ntiles && threadIdx.x == 0)
-        for (int ks = 0; ks < pro; ++ks) load(ks, (tile / ntn) * BM, (int)(tile % ntn) * BN, ks);
-    for (; tile < ntiles && ok; tile += gridDim.x) {
-        const int64_t m0 = (tile / ntn) * BM;
-        const int n0 = (int)(tile % ntn) * BN;
-        if (threadIdx.x == 0) {
-            // products of step ks are queued before waiting for those of step ks-1,
-            // whose stage is then refilled STAGES steps ahead
-            for (int ks = 0; ks < ksteps && ok; ++ks) {
-                const int64_t g = g0 + ks;
-                const int s = (int)(g % STAGES);
-                if (!mbar_wait(&full[s], (uint32_t)((g / STAGES) & 1))) {
-                    ok = false;
-                    break;
-                }
-                pend[s] = -1;
-                fence_after();
-#pragma unroll
-                for (int i = 0; i < NSL; ++i)
-#pragma unroll
-                    for (int j = 0; j < NSL - i; ++j) {
-                        const uint32_t dt = tmem + (uint32_t)((i + j) * BN);
-#pragma unroll
-                        for (int kk = 0; kk < BK / 16; ++kk) {
-                            const uint64_t ad = sdesc(su32(sA(s, i)) + kk * 32);
-                            const uint64_t bd = sdesc(su32(sB(s, j)) + kk * 32);
-                            // group t = i + j is first written by (i = 0, j = t) at ks = 0, kk = 0
-                            umma(dt, ad, bd, (ks == 0 && i == 0 && kk == 0) ? 0u : 1u);
-                        }
-                    }
-                umma_commit(&empty[s]);
-                last_commit = g;
-                if (ks >= 1 && ks - 1 + STAGES < ksteps) {
-                    const int64_t gp = g - 1;
-                    if (!mbar_wait(&empty[gp % STAGES], (uint32_t)((gp / STAGES) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    load(gp + STAGES, m0, n0, ks - 1 + STAGES);
-                }
-            }
-            s_ok = ok;
-        }
-        __syncthreads();
-        ok = s_ok;
-        const int64_t glast = g0 + ksteps - 1;
-        if (ok) ok = mbar_wait(&empty[glast % STAGES], (uint32_t)((glast / STAGES) & 1));
-        ok = __syncthreads_and(ok);
-        // every stage is free again: start the next tile's loads before the epilogue
-        const int64_t next = tile + gridDim.x;
-        if (ok && threadIdx.x == 0 && next < ntiles)
-            for (int ks = 0; ks < pro; ++ks) load(glast + 1 + ks, (next / ntn) * BM, (int)(next % ntn) * BN, ks);
-        if (ok) {
-            fence_after();
-            // epilogue: warp w owns TMEM lanes (rows) 32w .. 32w+31
-            // Every group sum is an integer-valued FP32 (sums of digit products), so the
-            // groups recombine exactly in int64: S = sum_t acc_t 2^{7(NSL-1-t)} < 2^59,
-            // and the value is S 2^{-7(NSL+1)} times the row and column scales.
-            const int64_t r = m0 + warp * 32 + lane;
-            const int er = (r < M) ? ea[r] : 0;
-            for (int c0 = 0; c0 < BN && n0 + c0 < N; c0 += 16) {
-                long long S[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) S[i] = 0;
-#pragma unroll
-                for (int t = 0; t < NSL; ++t) {
-                    float f[16];
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * BN + c0), f);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)  // |group sum| < 6 K 2^14 < 2^31 for K <= 512
-                        S[i] += (long long)__float2int_rn(f[i]) << (SL_BITS * (NSL - 1 - t));
-                }
-                if (r < M) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int c = n0 + c0 + i;
-                        if (c < N) {
-                            const double x = scaled_sum_to_double(S[i], er + eb[c] - SL_BITS * (NSL + 1));
-                            const int64_t o = out_index(om, r, c);
-                            out[o] = accumulate ? out[o] + x : x;
-                        }
-                    }
-                }
-            }
-        }
-        // the epilogue's TMEM reads finish before the next tile's products overwrite it
-        fence_before();
-        __syncthreads();
-        fence_after();
-        g0 += ksteps;
-    }
-    if (!ok) {
-        if (lane == 0) atomicExch(err, 1);
-        if (threadIdx.x == 0) {
-            // let copies and products still in flight land before TMEM and shared memory go (bounded)
-            for (int s = 0; s < STAGES; ++s)
-                if (pend[s] >= 0) mbar_wait(&full[s], (uint32_t)((pend[s] / STAGES) & 1));
-            if (last_commit >= 0) mbar_wait(&empty[last_commit % STAGES], (uint32_t)((last_commit / STAGES) & 1));
-        }
-    }
-    fence_before();
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
-}
-
-// ------------------------------------------------------------------ slicing
-// bf16 bit pattern of sign * v for an integer 0 <= v <= 128 (exact: bf16 holds
-// 8 significant bits), built with integer operations only
-__device__ __forceinline__ uint16_t small_int_bf16(uint32_t v, uint32_t sign)
-{
-    if (v == 0) return (uint16_t)(sign << 15);
-    const int e = 31 - __clz(v);  // 2^e <= v < 2^(e+1), e <= 7
-    return (uint16_t)((sign << 15) | ((uint32_t)(127 + e) << 7) | ((v << (7 - e)) & 0x7Fu));
-}
-
-// digits of |x| * 2^(42 - e) (rounded), with the sign of x applied, as bf16
-// bit patterns: no floating-point instruction at all (GB300 runs 64-bit
-// conversions on its narrow FP64 pipe)
-__device__ __forceinline__ void digits_bf16(double x, int e, uint16_t (&d)[NSL])
-{
-    const uint64_t bits = (uint64_t)__double_as_longlong(x);
-    const int ex = (int)((bits >> 52) & 0x7FF);
-    uint64_t Y = 0;
-    if (ex != 0) {
-        const uint64_t m = (bits & ((1ull << 52) - 1)) | (1ull << 52);
-        const int sh = ex - 1075 + NSL * SL_BITS - e;  // |x| < 2^e gives sh < -10
-        if (sh >= 0)
-            Y = m << sh;
-        else if (sh > -63)
-            Y = (m + (1ull << (-sh - 1))) >> (-sh);
-    }
-    const uint32_t sgn = (uint32_t)(bits >> 63);
-#pragma unroll
-    for (int t = 0; t < NSL; ++t) {
-        const int shift = SL_BITS * (NSL - 1 - t);
-        const uint32_t dig = (uint32_t)(Y >> shift) & (t == 0 ? 0xFFFFFFFFu : ((1u << SL_BITS) - 1));
-        d[t] = small_int_bf16(dig, sgn);
+    for (int t = 0; t < NSL; ++t) v[t] = __float2int_rn(__uint_as_float(a[t]));
+    // groups 0 .. 3, below 2^47
+    const long long hi = mad_wide(v[0], 1 << 21, mad_wide(v[1], 1 << 14, mad_wide(v[2], 1 << 7, v[3])));
+    if constexpr (NSL == 6) {
+        return scale_pow2((double)(mad_wide(v[4], 1 << 7, v[5]) + (hi << 14)), E);
+    } else {  // both parts are exact in FP64 (below 2^53)
+        const long long lo = mad_wide(v[4], 1 << 28, mad_wide(v[5], 1 << 21, mad_wide(v[6], 1 << 14, mad_wide(v[7], 1 << 7, v[8]))));
+        return scale_pow2(fma((double)hi, 34359738368.0, (double)lo), E);
     }
 }
 
-// row exponent from the bits of the largest |x| of the row: |x| < 2^e for every
-// x in the row (0 for an all-zero row)
-__device__ __forceinline__ int row_exponent(uint64_t amax_bits)
+// digit plane t of two elements as packed bf16 (element a in the low half)
+template <int NSL, int T>
+__device__ __forceinline__ uint32_t digit_word(uint64_t Ua, uint64_t Ub)
 {
-    if (amax_bits == 0) return 0;
-    return (int)((amax_bits >> 52) & 0x7FF) - 1022;
+    uint32_t w;
+    if constexpr (NSL == 6 && T == 0) {  // u - 128 with u <= 256, by FP32
+        const float fa = __uint_as_float(0x4B000000u | digit_field<6>(Ua, 0)) - 8388736.0f;
+        const float fb = __uint_as_float(0x4B000000u | digit_field<6>(Ub, 0)) - 8388736.0f;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(fb), "f"(fa));
+    } else {
+        const uint32_t u = 0x43004300u | digit_field<NSL>(Ua, T) | (digit_field<NSL>(Ub, T) << 16);
+        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(w) : "r"(u), "r"(0x43404340u));
+    }
+    return w;
 }
 
-// One warp per row.  Src::row(r) sets up the row once; element (r, k) is
-// Src::at(row, k).
-template <class Src>
-__global__ void slice_kernel(Src src, int64_t rows, int K, int64_t rows_pad, int K_pad, __nv_bfloat16* planes,
-                             int* rexp)
+template <int NSL, int T = 0>
+__device__ __forceinline__ void digit_words(uint64_t Ua, uint64_t Ub, uint32_t (&w)[NSL])
 {
-    constexpr int KMAX = 16;  // K <= 512
+    if constexpr (T < NSL) {
+        w[T] = digit_word<NSL, T>(Ua, Ub);
+        digit_words<NSL, T + 1>(Ua, Ub, w);
+    }
+}
+
+// row exponent from the upper word of the largest |x| of the row: |x| < 2^e for every
+// x in the row (0 for a row without normal numbers, whose digits are all zero)
+__device__ __forceinline__ int row_exponent(unsigned amax_hi)
+{
+    return amax_hi < (1u << 20) ? 0 : (int)(amax_hi >> 20) - 1022;
+}
+
+// the digits of 8 consecutive elements of a row whose largest |x| has upper word amax_hi
+template <int NSL>
+__device__ __forceinline__ void cut8(const double (&x)[8], unsigned amax_hi, uint32_t (&w)[4][NSL])
+{
+    const int e = row_exponent(amax_hi);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2)
+        digit_words<NSL>(biased_digits<NSL>((uint64_t)__double_as_longlong(x[j]), e),
+                         biased_digits<NSL>((uint64_t)__double_as_longlong(x[j + 1]), e), w[j / 2]);
+}
+
+// ------------------------------------------------------------------ slicing of B
+// One warp per row (a column of B): its exponent, then every element's digits, laid out
+// as the GEMM's stages take them: per column tile and K step, NSL T rows (plane major)
+// of 32 bf16, already swizzled, so that a stage's B is one contiguous bulk copy.  (As
+// NSL tensor-map tiles of T 64-byte rows a step's B took longer to arrive than its A
+// to be cut: 16 waters, step 1 70 ms; see the kernel.)
+template <int NSL>
+__global__ void slice_kernel(const double* __restrict__ A, int64_t ld, int64_t rows, int K, int T, int ksteps,
+                             uint16_t* planes, int* rexp)
+{
     const int lane = threadIdx.x & 31;
     const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarp) {
-        const typename Src::Row row = src.row(r);
-        double x[KMAX];
-        // the largest |x| as an integer compare of the magnitude bits (finite
-        // doubles order like their bit patterns), off the FP64 pipe
-        unsigned long long amax = 0;
+        const double* row = A + r * ld;
+        unsigned m = 0u;
+        for (int k = lane; k < K; k += 32) m = max(m, (unsigned)__double2hiint(row[k]) & 0x7FFFFFFFu);
 #pragma unroll
-        for (int q = 0; q < KMAX; ++q) {
-            const int k = lane + 32 * q;
-            x[q] = (k < K) ? src.at(row, k) : 0.0;
-            const unsigned long long m = (unsigned long long)__double_as_longlong(x[q]) & 0x7FFFFFFFFFFFFFFFull;
-            amax = m > amax ? m : amax;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long v = __shfl_xor_sync(0xffffffffu, amax, o);
-            amax = v > amax ? v : amax;
-        }
-        const int e = row_exponent(amax);
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const int e = row_exponent(m);
         if (lane == 0) rexp[r] = e;
+        const int nt = (int)(r / T), c = (int)(r - (int64_t)nt * T);
+        for (int k = lane; k < K; k += 32) {
+            const uint64_t U = biased_digits<NSL>((uint64_t)__double_as_longlong(row[k]), e);
+            uint32_t w[NSL];
+            digit_words<NSL>(U, U, w);
 #pragma unroll
-        for (int q = 0; q < KMAX; ++q) {
-            const int k = lane + 32 * q;
-            if (k < K) {
-                uint16_t d[NSL];
-                digits_bf16(x[q], e, d);
-                uint16_t* pl = reinterpret_cast<uint16_t*>(planes);
-#pragma unroll
-                for (int t = 0; t < NSL; ++t) pl[((int64_t)t * rows_pad + r) * K_pad + k] = d[t];
+            for (int t = 0; t < NSL; ++t) {
+                const int row = t * T + c;
+                const int chunk = ((k & 31) >> 3) ^ ((row >> 1) & 3);  // 64-byte swizzle
+                planes[(((int64_t)nt * ksteps + (k >> 5)) * (NSL * T) + row) * BK + chunk * 8 + (k & 7)] = (uint16_t)w[t];
             }
         }
     }
 }
 
-// ------------------------------------------------------------------ gather-fed GEMM
-// The same product with the A operand sliced on the fly: instead of writing six
-// bf16 planes of A to HBM and reading them back through TMA, the CTA's threads
-// gather A's FP64 elements (Src::row / Src::at), cut them into digits and store
-// them straight into the stage's shared-memory tiles in the 64-byte-swizzled
-// K-major layout the MMA reads (16-byte chunk c of row r at chunk c ^ ((r >> 1) & 3)).
-// B still arrives by TMA.  Each tile first takes its rows' exponents (the
-// largest magnitude of each row, from the same gathers).
-// 512 threads: thread t produces row t % 128, K quarter t / 128 (8 elements, one
-// 16-byte chunk per plane) of every stage, fetching the next stage's elements
-// before it stores this one; the 16 producer warps share the epilogue (warp w:
-// TMEM lanes 32 (w % 4), columns 16 (w / 4) .. +15).  A 17th warp issues the
-// B loads (ahead, into every stage already free) and the products, so that no
-// producer waits for a stage's other producers.
-constexpr int GATHER_PRODUCERS = 512;
-constexpr int GATHER_THREADS = GATHER_PRODUCERS + 32;
-
-// Output-tile width and pipeline depth of the gather-fed GEMM: 64 columns with
-// three stages, or 80 columns (16 waters: 80 occupied orbitals in one tile, so
-// the rows are gathered once) with two stages to stay within shared memory.
-template <int GBN_, int GST_>
-struct GatherCfg {
-    static constexpr int GBN = GBN_, GST = GST_;
-    static constexpr int B_T = GBN * BK * 2;
-    static constexpr int STAGE = NSL * (A_TILE + B_T);
-    static constexpr int SMEM = GST * STAGE + 1024 + 128;
-    static constexpr uint32_t IDESC =
-        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GBN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-    static_assert(GBN % 16 == 0 && NSL * GBN <= (int)TMEM_COLS, "tile width");
+// ------------------------------------------------------------------ GEMM kernel
+struct GatherArgs {
+    const unsigned char* b;  // B's stages (slice_kernel)
+    int K, ksteps;
+    int T, nst, stage, nbuf, slot;  // tile columns, pipeline stages, bytes of one, accumulator sets, groups of a slot
+    int N, ntn, M, ntiles;
+    const int* eb;
+    double* out;
+    OutMap om;
+    int* err;
 };
-using Gather64 = GatherCfg<64, 3>;
-using Gather80 = GatherCfg<80, 2>;
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(bar)) : "memory");
-}
-
-template <class Src, class C>
+template <class Src, int NSL>
 __global__ void __launch_bounds__(GATHER_THREADS, 1)
-    sliced_gemm_gather_kernel(Src src, const __grid_constant__ CUtensorMap tmB,
-                              int b_rows_pad, int K, int ksteps, const int* __restrict__ eb, int64_t M, int N,
-                              double* out, OutMap om, int* err, int64_t ntiles, int ntn)
+    gather_gemm_kernel(const Src src, const GatherArgs g)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = (uint64_t*)(smem + C::GST * C::STAGE);
-    uint64_t* empty = full + C::GST;
-    uint32_t* tslot = (uint32_t*)(empty + C::GST);
+    __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES];  // stage filled / its products done
+    __shared__ uint64_t acc_full[2], acc_empty[2];            // accumulators complete / read back
+    // the products of 16 k: TMEM column (bit 31: plane 0 of A, which writes its groups
+    // first), descriptor offsets of A and B (16-byte units), instruction descriptor
+    __shared__ uint4 ops[MAX_OPS];
+    __shared__ uint32_t tslot;
     __shared__ int s_ok;
-    constexpr int PARTS = GATHER_PRODUCERS / BM;  // K parts of a stage per row
-    __shared__ int s_exp[BM];  // row exponents of the current tile (for the epilogue)
-    auto sA = [&](int s, int t) { return smem + s * C::STAGE + t * A_TILE; };
-    auto sB = [&](int s, int t) { return smem + s * C::STAGE + NSL * A_TILE + t * C::B_T; };
-
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int PK = BK / PARTS;              // elements per thread and stage (8: one 16-byte chunk)
-    static_assert(PK == 8, "one 16-byte chunk per thread and plane");
-    const int prow = tid & (BM - 1), part = tid / BM;
-    const bool producer = tid < GATHER_PRODUCERS, issuer = tid == GATHER_PRODUCERS;
+    const int T = g.T, nst = g.nst, nbuf = g.nbuf, ksteps = g.ksteps;
     if (tid == 0) {
-        for (int s = 0; s < C::GST; ++s) {
-            mbar_init(&full[s], GATHER_PRODUCERS + 1);  // every producer + the B expect_tx
+        for (int s = 0; s < nst; ++s) {
+            mbar_init(&full[s], PRODUCER_WARPS + 1);  // every producer warp + the B expect_tx
             mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], PRODUCER_WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_ok = 1;
+        // slots of g.slot groups; plane i of A writes groups max(i, g0) .. g1 - 1 of each
+        int k = 0;
+        for (int g0 = (NSL - 1) / g.slot * g.slot; g0 >= 0; g0 -= g.slot) {
+            const int g1 = min(g0 + g.slot, NSL);
+            for (int i = 0; i < g1; ++i) {
+                const int first = max(i, g0);
+                ops[k++] = make_uint4((uint32_t)(first * T) | (i == 0 ? 0x80000000u : 0u), (uint32_t)(i * (A_TILE >> 4)),
+                                      (uint32_t)((first - i) * T * (BK * 2) >> 4), idesc(((g1 - first) * T + 15) & ~15));
+            }
+        }
     }
+    const int nops = g.slot == NSL ? NSL : NSL == 6 ? 9 : 18;
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)),
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&tslot)),
                      "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = *tslot;
+    const uint32_t tmem = tslot;
+    auto stage_a = [&](int s) { return smem + s * g.stage; };
+    auto stage_b = [&](int s) { return smem + s * g.stage + NSL * A_TILE; };
 
     bool ok = true;
-    int64_t g0 = 0;
-    int64_t last_commit = -1;  // issuer
-    int64_t pend_b = -1;       // issuer: last step whose B load was issued
-    for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const int64_t m0 = (tile / ntn) * BM;
-        const int n0 = (int)(tile % ntn) * C::GBN;
-        const int64_t R = m0 + prow;
-        const bool live = producer && R < M && src.live(R);
-        const typename Src::Row row = src.row(live ? R : 0);
-        // the row's exponent from the precomputed row maximum (row_max kernels);
-        // the barrier keeps this tile's s_exp writes behind the last epilogue's reads
-        const unsigned long long amax = live ? src.row_max(R) : 0ull;
-        __syncthreads();
-        const int e = row_exponent(amax);
-        if (producer && part == 0) s_exp[prow] = e;
-        // this thread's 8 elements of step 0, fetched ahead
-        double x[PK];
-#pragma unroll
-        for (int j = 0; j < PK; ++j) {
-            const int k = part * PK + j;
-            x[j] = (live && k < K) ? src.at(row, k) : 0.0;
-        }
-        if (issuer) {
-            // B loads for every step up to g + GST - 1 whose stage is free (step g's own
-            // is waited for), then step g's products once its stage is full
-            int64_t next_b = g0;
-            const int64_t gend = g0 + ksteps;
-            for (int ks = 0; ks < ksteps && ok; ++ks) {
-                const int64_t g = g0 + ks;
-                while (next_b < gend && next_b < g + C::GST) {
-                    const int sl = (int)(next_b % C::GST);
-                    if (next_b >= C::GST) {
-                        const uint32_t ph = (uint32_t)(((next_b - C::GST) / C::GST) & 1);
-                        if (next_b == g) {
-                            if (!mbar_wait(&empty[sl], ph)) {
-                                ok = false;
+    if (warp == PRODUCER_WARPS) {
+        if (lane == 0) {
+            // B loads run ahead into every stage already free; step q of the CTA's whole
+            // sequence uses stage q % nst for the (q / nst)-th time
+            int sl = 0, sl_use = 0;        // next stage to load, how often it was used
+            int ks_l = 0;                  // its K step
+            int tile_l = blockIdx.x;       // its tile
+            int ahead = 0;                 // loads issued beyond the step being multiplied
+            int last_load = -1, last_load_use = 0, last_commit = -1, last_commit_use = 0;
+            int s = 0, use = 0, lt = 0;
+            const int b_bytes = NSL * T * BK * 2;
+            for (int tile = blockIdx.x; tile < g.ntiles && ok; tile += gridDim.x, ++lt) {
+                const int buf = nbuf == 2 ? lt & 1 : 0;
+                const uint32_t acc = tmem + (uint32_t)(buf * 256);
+                for (int ks = 0; ks < ksteps && ok; ++ks) {
+                    while (tile_l < g.ntiles && ahead < nst) {
+                        if (sl_use > 0) {
+                            const uint32_t ph = (uint32_t)(sl_use - 1) & 1u;
+                            if (ahead == 0) {
+                                if (!mbar_wait(&empty[sl], ph)) {
+                                    ok = false;
+                                    break;
+                                }
+                            } else if (!mbar_try_wait(&empty[sl], ph)) {
                                 break;
                             }
-                        } else if (!mbar_try_wait(&empty[sl], ph)) {
+                        }
+                        mbar_expect_tx(&full[sl], b_bytes);
+                        bulk_load(stage_b(sl), g.b + (int64_t)((tile_l % g.ntn) * ksteps + ks_l) * b_bytes, b_bytes,
+                                  &full[sl]);
+                        last_load = sl;
+                        last_load_use = sl_use;
+                        ++ahead;
+                        if (++sl == nst) {
+                            sl = 0;
+                            ++sl_use;
+                        }
+                        if (++ks_l == ksteps) {
+                            ks_l = 0;
+                            tile_l += gridDim.x;
+                        }
+                    }
+                    if (!ok) break;
+                    if (ks == 0 && lt >= nbuf) {  // the tile that used these accumulators has been read back
+                        if (!mbar_wait(&acc_empty[buf], (uint32_t)(lt / nbuf - 1) & 1u)) {
+                            ok = false;
                             break;
                         }
                     }
-                    mbar_expect_tx(&full[sl], NSL * C::B_T);
-#pragma unroll
-                    for (int t = 0; t < NSL; ++t)
-                        tma_load_2d(sB(sl, t), &tmB, (int)(next_b - g0) * BK, t * b_rows_pad + n0, &full[sl]);
-                    pend_b = next_b;
-                    ++next_b;
-                }
-                if (!ok) break;
-                const int s = (int)(g % C::GST);
-                if (!mbar_wait(&full[s], (uint32_t)((g / C::GST) & 1))) {
-                    ok = false;
-                    break;
-                }
-                fence_after();
-#pragma unroll
-                for (int i = 0; i < NSL; ++i)
-#pragma unroll
-                    for (int jj = 0; jj < NSL - i; ++jj) {
-                        const uint32_t dt = tmem + (uint32_t)((i + jj) * C::GBN);
-#pragma unroll
-                        for (int kk = 0; kk < BK / 16; ++kk) {
-                            const uint64_t ad = sdesc(su32(sA(s, i)) + kk * 32);
-                            const uint64_t bd = sdesc(su32(sB(s, jj)) + kk * 32);
-                            umma_d(dt, ad, bd, C::IDESC, (ks == 0 && i == 0 && kk == 0) ? 0u : 1u);
-                        }
+                    if (!mbar_wait(&full[s], (uint32_t)use & 1u)) {
+                        ok = false;
+                        break;
                     }
-                umma_commit(&empty[s]);
-                last_commit = g;
+                    fence_after();
+                    const uint64_t a0 = sdesc(su32(stage_a(s))), b0 = sdesc(su32(stage_b(s)));
+                    const bool second = g.K - ks * BK > 16;  // the step's second 16 k hold elements
+#pragma unroll 3
+                    for (int k = 0; k < nops; ++k) {  // kk innermost: the same columns twice in a row
+                        const uint4 op = ops[k];
+                        const uint32_t dt = acc + (op.x & 0xFFFFu);
+                        umma(dt, a0 + op.y, b0 + op.z, op.w, ks == 0 ? (op.x >> 31) ^ 1u : 1u);
+                        if (second) umma(dt, a0 + op.y + 2, b0 + op.z + 2, op.w, 1u);
+                    }
+                    umma_commit(&empty[s]);
+                    if (ks == ksteps - 1) umma_commit(&acc_full[buf]);
+                    last_commit = s;
+                    last_commit_use = use;
+                    --ahead;
+                    if (++s == nst) {
+                        s = 0;
+                        ++use;
+                    }
+                }
+            }
+            if (!ok) {
+                atomicExch(&s_ok, 0);
+                // B copies and products still in flight land before shared memory and TMEM go
+                // (bounded; a stage whose producers gave up never fills: its copy is waited
+                // out by the spin limit)
+                if (last_load >= 0) mbar_wait(&full[last_load], (uint32_t)last_load_use & 1u);
+                if (last_commit >= 0) mbar_wait(&empty[last_commit], (uint32_t)last_commit_use & 1u);
             }
         }
-        for (int ks = 0; ks < ksteps && ok && producer; ++ks) {
-            const int64_t g = g0 + ks;
-            const int s = (int)(g % C::GST);
-            if (g >= C::GST && !mbar_wait(&empty[s], (uint32_t)(((g - C::GST) / C::GST) & 1))) {
-                ok = false;
-                break;
+    } else {
+        const int prow = tid & (BM - 1), part = tid / BM;  // row of the tile, K quarter of a stage
+        const int chunk = part ^ ((prow >> 1) & 3);
+        // the tile and step that are fetched next, up to two steps ahead of the cutting
+        // (32-bit tile arithmetic: 64-bit divisions would cost as much as the digits)
+        int tile_f = blockIdx.x, ks_f = 0;
+        bool live_f = false;
+        typename Src::Row row_f{};
+        unsigned amax_f = 0;
+        auto open_row = [&] {
+            amax_f = 0;
+            live_f = tile_f < g.ntiles && src.open((int)((unsigned)tile_f / (unsigned)g.ntn) * BM + prow, g.M, row_f, amax_f);
+        };
+        auto fetch = [&](double(&x)[8], unsigned& amax) {
+            const int k0 = ks_f * BK + part * 8;
+            amax = amax_f;
+            if (live_f && k0 + 8 <= g.K) {
+                src.load8(row_f, k0, x);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = (live_f && k0 + j < g.K) ? src.at(row_f, k0 + j) : 0.0;
             }
-            // two elements per 32-bit word and plane: digit patterns 0x4300 | d, one
-            // packed bf16 subtraction of 128, then the signs (slice_bits.cuh)
-            uint32_t w[NSL][PK / 2];
-#pragma unroll
-            for (int j = 0; j < PK; j += 2) {
-                const uint64_t b0 = (uint64_t)__double_as_longlong(x[j]), b1 = (uint64_t)__double_as_longlong(x[j + 1]);
-                const uint64_t Y0 = scaled_magnitude(b0, e), Y1 = scaled_magnitude(b1, e);
-                const uint32_t sw = sign_word(b0, b1);
-#pragma unroll
-                for (int t = 0; t < NSL; ++t) w[t][j / 2] = bf16x2_minus_128(digit_word(Y0, Y1, t)) ^ sw;
+            if (++ks_f == ksteps) {
+                ks_f = 0;
+                tile_f += gridDim.x;
+                open_row();
             }
-            // the next step's elements are in flight while this one is stored and multiplied
-            if (ks + 1 < ksteps) {
+        };
+        // read the accumulators of the CTA's tile number lt back: TMEM lanes 32 (warp % 4),
+        // every fourth group of four columns
+        const int cstep = g.om.R > 0 ? (int)g.om.R : 1;
+        auto epilogue = [&](int tile, int lt) {
+            const int buf = nbuf == 2 ? lt & 1 : 0;
+            const int mt = (int)((unsigned)tile / (unsigned)g.ntn), n0 = (tile - mt * g.ntn) * T;
+            int64_t off = 0;
+            unsigned amax = 0;
+            const bool lv = src.place(mt * BM + (warp & 3) * 32 + lane, g.M, (int)g.om.R, g.om.ld, off, amax);
+            const int er = row_exponent(amax) - SliceFmt<NSL>::SHIFT;
+            double* orow = g.out + off;
+            if (!mbar_wait(&acc_full[buf], (uint32_t)(nbuf == 2 ? lt >> 1 : lt) & 1u)) return false;
+            fence_after();
+            const uint32_t ta = tmem + (uint32_t)(buf * 256) + ((uint32_t)((warp & 3) * 32) << 16);
+            for (int c0 = (warp >> 2) * 4; c0 < T && n0 + c0 < g.N; c0 += PRODUCER_WARPS) {
+                uint32_t f[NSL][4];
 #pragma unroll
-                for (int j = 0; j < PK; ++j) {
-                    const int k = (ks + 1) * BK + part * PK + j;
-                    x[j] = (live && k < K) ? src.at(row, k) : 0.0;
+                for (int t = 0; t < NSL; ++t) tmem_ld4(ta + (uint32_t)(t * T + c0), f[t]);
+                tmem_wait_ld(f);
+                const int c = n0 + c0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    uint32_t a[NSL];
+#pragma unroll
+                    for (int t = 0; t < NSL; ++t) a[t] = f[t][i];
+                    if (lv && c + i < g.N)
+                        orow[(int64_t)(c + i) * cstep] = recombine<NSL>(a, er + __ldg(g.eb + c + i));
                 }
             }
-            const int c = part ^ ((prow >> 1) & 3);  // 64-byte swizzle: chunk c of row r at c ^ ((r >> 1) & 3)
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            return true;
+        };
+
+        open_row();
+        double x0[8], x1[8];
+        unsigned m0, m1;
+        fetch(x0, m0);
+        fetch(x1, m1);
+        int s = 0, use = 0, lt = 0, prev = -1, tile = blockIdx.x, ks = 0;
+        // one K step from x; false at the end of the tiles or after a timeout.  (One copy of
+        // this code, with the two buffers swapped after it: two copies, or a second way to
+        // cut digits on the FP32 pipe, ran slower from instruction fetches.)
+        auto step = [&](double(&x)[8], unsigned& amax) {
+            uint32_t w[4][NSL];
+            const bool has = ks * BK + part * 8 < g.K;
+            if (has) cut8<NSL>(x, amax, w);
+            fetch(x, amax);  // in flight while this step is stored and the next one is cut
+            if (use > 0 && !mbar_wait(&empty[s], (uint32_t)(use - 1) & 1u)) return ok = false;
+            unsigned char* dst = stage_a(s) + prow * 64 + chunk * 16;
 #pragma unroll
             for (int t = 0; t < NSL; ++t)
-                *reinterpret_cast<uint4*>(sA(s, t) + prow * 64 + c * 16) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
+                *reinterpret_cast<uint4*>(dst + t * A_TILE) =
+                    has ? make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]) : make_uint4(0u, 0u, 0u, 0u);
             // the tensor core reads shared memory through the async proxy
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive(&full[s]);
-        }
-        if (!ok) atomicExch(&s_ok, 0);
-        __syncthreads();
-        ok = s_ok != 0;
-        const int64_t glast = g0 + ksteps - 1;
-        if (ok) ok = mbar_wait(&empty[glast % C::GST], (uint32_t)((glast / C::GST) & 1));
-        ok = __syncthreads_and(ok);
-        if (ok && producer) {
-            fence_after();
-            // warp w: TMEM lanes 32 (w % 4), 16 columns starting at 16 (w / 4)
-            const int64_t r = m0 + (warp & 3) * 32 + lane;
-            const int er = s_exp[(warp & 3) * 32 + lane];
-            for (int c0 = (warp >> 2) * 16; c0 < C::GBN && n0 + c0 < N; c0 += 64) {
-                long long S[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) S[i] = 0;
-#pragma unroll
-                for (int t = 0; t < NSL; ++t) {
-                    float f[16];
-                    tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(t * C::GBN + c0), f);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) S[i] += (long long)__float2int_rn(f[i]) << (SL_BITS * (NSL - 1 - t));
-                }
-                if (r < M && src.live(r)) {
-                    const int64_t ro = src.out_row(r);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int c = n0 + c0 + i;
-                        if (c < N) out[out_index(om, ro, c)] = scaled_sum_to_double(S[i], er + eb[c] - SL_BITS * (NSL + 1));
-                    }
-                }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+            if (++s == nst) {
+                s = 0;
+                ++use;
             }
+            // the previous tile is read back once the first step of this one is filled
+            if (ks == 0 && prev >= 0 && !epilogue(prev, lt - 1)) return ok = false;
+            if (++ks == ksteps) {
+                ks = 0;
+                prev = tile;
+                tile += gridDim.x;
+                ++lt;
+            }
+            return tile < g.ntiles;
+        };
+        while (step(x0, m0)) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const double t = x0[j];
+                x0[j] = x1[j];
+                x1[j] = t;
+            }
+            const unsigned t = m0;
+            m0 = m1;
+            m1 = t;
         }
-        fence_before();
-        __syncthreads();
-        fence_after();
-        g0 += ksteps;
-    }
-    if (!ok) {
-        if (lane == 0) atomicExch(err, 1);
-        if (issuer) {
-            // B copies and products still in flight land before shared memory and TMEM go (bounded)
-            if (pend_b >= 0) mbar_wait(&full[pend_b % C::GST], (uint32_t)((pend_b / C::GST) & 1));
-            if (last_commit >= 0) mbar_wait(&empty[last_commit % C::GST], (uint32_t)((last_commit / C::GST) & 1));
-        }
+        if (ok && prev >= 0) ok = epilogue(prev, lt - 1);
+        if (!ok) atomicExch(&s_ok, 0);
     }
     fence_before();
     __syncthreads();
+    if (tid == 0 && !s_ok) atomicExch(g.err, 1);
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+int slice_kmax(int digits) { return digits == SLICE_MIXED ? SliceFmt<6>::KMAX : SliceFmt<9>::KMAX; }
 
-static EncodeTiledFn encode_fn()
+// Columns of a tile for N columns of B: the fewest tiles (every tile gathers and cuts
+// the A rows again) that fit the TMEM columns, evenly filled, a multiple of 16 (the
+// granularity of a product's columns); or 40, for 33 to 40 columns of six digits: 240
+// accumulator columns leave room for a second set, 48 x 6 would not (8 waters, step 1:
+// 4.1 against 5.1 ms).
+static int tile_columns(int64_t N, int digits)
 {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    });
-    HF_CHECK(fn != nullptr, HFGPU_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    return fn;
+    if (digits == SLICE_MIXED && N > 32 && N <= 40) return 40;
+    const int most = (int)TMEM_COLS / digits / 16 * 16;  // 80 with six digits, 48 with nine
+    const int64_t ntn = (N + most - 1) / most;
+    return (int)(((N + ntn - 1) / ntn + 15) / 16 * 16);
 }
 
-static CUtensorMap make_map(const Sliced& s, int box_rows)
+void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, int digits, Sliced& s)
 {
-    CUtensorMap m;
-    cuuint64_t dims[2] = {(cuuint64_t)s.K_pad, (cuuint64_t)(NSL * s.rows_pad)};
-    cuuint64_t strides[1] = {(cuuint64_t)s.K_pad * 2};
-    cuuint32_t box[2] = {BK, (cuuint32_t)box_rows};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)s.planes.p, dims, strides, box, es,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    HF_CHECK(r == CUDA_SUCCESS, HFGPU_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
-    return m;
-}
-
-static int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
-
-void Sliced::alloc(Context& ctx, int64_t r, int k, int row_tile)
-{
-    HF_CHECK(k >= 1 && k <= 512, HFGPU_ERR_UNSUPPORTED, "sliced GEMM supports 1 <= K <= 512");
-    rows = r;
-    K = k;
-    rows_pad = round_up(r, row_tile);
-    K_pad = (int)round_up(k, BK);
-    const size_t need = (size_t)NSL * rows_pad * K_pad;
-    if (planes.n < need) planes.alloc(need, ctx.stream);
-    if (rexp.n < (size_t)rows_pad) rexp.alloc(rows_pad, ctx.stream);
-    HF_CUDA(cudaMemsetAsync(planes.p, 0, need * sizeof(__nv_bfloat16), ctx.stream));
-}
-
-template <class Src>
-static void launch_slice(Context& ctx, const Src& src, Sliced& s)
-{
-    const int64_t warps = std::min<int64_t>(s.rows, (int64_t)ctx.num_sms * 64);
+    HF_CHECK(K >= 1 && K <= slice_kmax(digits), HFGPU_ERR_UNSUPPORTED,
+             "sliced GEMM supports 1 <= K <= " + std::to_string(slice_kmax(digits)));
+    s.rows = rows;
+    s.K = K;
+    s.digits = digits;
+    s.tile = tile_columns(rows, digits);
+    s.rows_pad = (rows + s.tile - 1) / s.tile * s.tile;
+    s.ksteps = (K + BK - 1) / BK;
+    const size_t need = (size_t)digits * s.rows_pad * s.ksteps * BK;
+    s.planes.alloc(need, ctx.stream);
+    s.rexp.alloc(s.rows_pad, ctx.stream);
+    HF_CUDA(cudaMemsetAsync(s.planes.p, 0, need * sizeof(__nv_bfloat16), ctx.stream));
+    const int64_t warps = std::min<int64_t>(rows, (int64_t)ctx.num_sms * 64);
     const unsigned blocks = (unsigned)std::max<int64_t>(1, (warps * 32 + 255) / 256);
-    slice_kernel<Src><<<blocks, 256, 0, ctx.stream>>>(src, s.rows, s.K, s.rows_pad, s.K_pad, s.planes.p, s.rexp.p);
+    uint16_t* pl = reinterpret_cast<uint16_t*>(s.planes.p);
+    if (digits == SLICE_MIXED)
+        slice_kernel<6><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p);
+    else
+        slice_kernel<9><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p);
     count_launch();
     HF_CUDA(cudaGetLastError());
 }
 
-void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, Sliced& s, int row_tile)
-{
-    s.alloc(ctx, rows, K, row_tile);
-    launch_slice(ctx, DenseRows{A, ld}, s);
-}
-
-void slice_packed(Context& ctx, const double* ints, const int2* pairs, int64_t p0, int64_t npairs, int n, Sliced& s)
-{
-    s.alloc(ctx, npairs * n, n, BM);
-    launch_slice(ctx, PackedRows{ints, pairs, p0, n}, s);
-}
-
-void slice_sympair(Context& ctx, const double* Zt, int64_t ldz, int64_t nq, int n, Sliced& s)
-{
-    s.alloc(ctx, nq * n, n, BM);
-    launch_slice(ctx, SymPairRows{Zt, ldz, n}, s);
-}
-
-void sliced_gemm(Context& ctx, const Sliced& A, const Sliced& B, double* out, OutMap om, bool accumulate)
-{
-    HF_CHECK(A.K == B.K && A.K_pad == B.K_pad, HFGPU_ERR_INVALID, "sliced GEMM: K mismatch");
-    HF_CHECK(B.rows_pad % BN == 0 && A.rows_pad % BM == 0, HFGPU_ERR_INVALID, "sliced GEMM: padding");
-    static bool attr = false;
-    if (!attr) {
-        HF_CUDA(cudaFuncSetAttribute(sliced_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        attr = true;
-    }
-    const CUtensorMap ta = make_map(A, BM), tb = make_map(B, BN);
-    DBuf<int> err(1, ctx.stream);
-    err.zero();
-    cudaEvent_t e0, e1;
-    HF_CUDA(cudaEventCreate(&e0));
-    HF_CUDA(cudaEventCreate(&e1));
-    HF_CUDA(cudaEventRecord(e0, ctx.stream));
-    // persistent CTAs, one per SM, walking the output tiles (column tile fastest)
-    const int ntn = (int)(B.rows_pad / BN);
-    const int64_t ntiles = (A.rows_pad / BM) * ntn;
-    HF_CHECK(ntiles > 0, HFGPU_ERR_INVALID, "sliced GEMM: empty");
-    const unsigned grid = (unsigned)std::min<int64_t>(ntiles, ctx.num_sms);
-    sliced_gemm_kernel<<<grid, 128, SMEM_BYTES, ctx.stream>>>(ta, tb, A.rows_pad, (int)B.rows_pad, A.K_pad / BK,
-                                                               A.rexp.p, B.rexp.p, A.rows, (int)B.rows, out, om,
-                                                               accumulate ? 1 : 0, err.p, ntiles, ntn);
-    count_launch();
-    HF_CUDA(cudaGetLastError());
-    HF_CUDA(cudaEventRecord(e1, ctx.stream));
-    int h = 0;
-    err.download(&h, 1);
-    HF_CUDA(cudaStreamSynchronize(ctx.stream));
-    float ms = 0;
-    HF_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    ctx.stat_tc_ms += ms;
-    ctx.stat_tc_flops += 2.0 * (NSL * (NSL + 1) / 2) * (double)A.rows * (double)B.rows * (double)A.K;
-    HF_CHECK(h == 0, HFGPU_ERR_CUDA, "sliced GEMM: an mbarrier wait timed out");
-}
-
-}  // namespace hfgpu
-
-namespace hfgpu {
-
-template <class Src, class C>
-static void gather_gemm_cfg(Context& ctx, const Src& src, int64_t M, int64_t M_rows, int K, const Sliced& B, double* out,
-                            OutMap om)
+// (M: rows of the launch, dead ones included; M_rows: the live rows, for the flop count)
+template <class Src, int NSL>
+static void gather_gemm_n(Context& ctx, const Src& src, int64_t M, int64_t M_rows, int K, const Sliced& B, double* out,
+                          OutMap om)
 {
     HF_CHECK(K == B.K, HFGPU_ERR_INVALID, "gather GEMM: K mismatch");
-    const int ntn = (int)((B.rows + C::GBN - 1) / C::GBN);
-    HF_CHECK((int64_t)ntn * C::GBN <= B.rows_pad, HFGPU_ERR_INVALID, "gather GEMM: padding");
-    static bool attr = false;
-    if (!attr) {
-        HF_CUDA(cudaFuncSetAttribute(sliced_gemm_gather_kernel<Src, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     C::SMEM));
-        attr = true;
+    GatherArgs g;
+    g.b = reinterpret_cast<const unsigned char*>(B.planes.p);
+    g.K = K;
+    g.ksteps = B.ksteps;
+    g.T = B.tile;
+    g.N = (int)B.rows;
+    g.ntn = (int)(B.rows_pad / B.tile);
+    const int64_t ntiles = (M + BM - 1) / BM * g.ntn;
+    HF_CHECK(ntiles > 0 && M < (1ll << 30) && ntiles < (1ll << 30), HFGPU_ERR_INVALID, "gather GEMM: row count");
+    HF_CHECK((std::is_same_v<Src, DenseRowsG> || om.R == K), HFGPU_ERR_INVALID, "gather GEMM: output placement");
+    g.M = (int)M;
+    g.ntiles = (int)ntiles;
+    g.nbuf = NSL * g.T <= 256 ? 2 : 1;
+    // slots of three groups where every product's columns are a multiple of 16; else all
+    // groups in one: a padded product then writes only past the last group, into the 8
+    // spare columns of a set (and reads B rows of the next plane)
+    g.slot = g.T % 16 == 0 ? 3 : NSL;
+    HF_CHECK(g.slot == 3 || NSL * g.T + 8 <= 256, HFGPU_ERR_INVALID, "gather GEMM: tile columns");
+    g.stage = (NSL * A_TILE + NSL * g.T * BK * 2 + 1023) / 1024 * 1024;  // the digit planes of A and of B
+    g.eb = B.rexp.p;
+    g.out = out;
+    g.om = om;
+    static std::once_flag once;
+    static size_t most = 0;
+    std::call_once(once, [] {
+        int dev = 0, optin = 0;
+        cudaFuncAttributes fa{};
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+            cudaFuncGetAttributes(&fa, gather_gemm_kernel<Src, NSL>) != cudaSuccess)
+            return;
+        const size_t m = (size_t)optin - fa.sharedSizeBytes;
+        if (cudaFuncSetAttribute(gather_gemm_kernel<Src, NSL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m) ==
+            cudaSuccess)
+            most = m;
+    });
+    g.nst = (int)std::min<size_t>(MAX_STAGES, most > 1024 ? (most - 1024) / g.stage : 0);
+    HF_CHECK(g.nst >= 2, HFGPU_ERR_CUDA, "gather GEMM: shared memory attribute");
+    if (!ctx.tc_err) {
+        HF_CUDA(cudaMalloc((void**)&ctx.tc_err, sizeof(int)));
+        HF_CUDA(cudaMemsetAsync(ctx.tc_err, 0, sizeof(int), ctx.stream));
     }
-    const CUtensorMap tb = make_map(B, C::GBN);
-    DBuf<int> err(1, ctx.stream);
-    err.zero();
-    cudaEvent_t e0, e1;
-    HF_CUDA(cudaEventCreate(&e0));
-    HF_CUDA(cudaEventCreate(&e1));
-    HF_CUDA(cudaEventRecord(e0, ctx.stream));
-    const int64_t ntiles = (M + BM - 1) / BM * ntn;
-    HF_CHECK(ntiles > 0, HFGPU_ERR_INVALID, "gather GEMM: empty");
-    const unsigned grid = (unsigned)std::min<int64_t>(ntiles, ctx.num_sms);
-    sliced_gemm_gather_kernel<Src, C><<<grid, GATHER_THREADS, C::SMEM, ctx.stream>>>(
-        src, tb, (int)B.rows_pad, K, B.K_pad / BK, B.rexp.p, M, (int)B.rows, out, om, err.p, ntiles, ntn);
+    g.err = ctx.tc_err;
+    Context::TcTimer t;
+    HF_CUDA(cudaEventCreate(&t.a));
+    HF_CUDA(cudaEventCreate(&t.b));
+    t.step1 = std::is_same_v<Src, PackedRowsBlocked>;
+    t.flops = 2.0 * (NSL * (NSL + 1) / 2) * (double)M_rows * (double)B.rows * (double)K;
+    HF_CUDA(cudaEventRecord(t.a, ctx.stream));
+    const unsigned grid = (unsigned)std::min<int64_t>(g.ntiles, ctx.num_sms);
+    gather_gemm_kernel<Src, NSL><<<grid, GATHER_THREADS, g.nst * g.stage + 1024, ctx.stream>>>(src, g);
     count_launch();
     HF_CUDA(cudaGetLastError());
-    HF_CUDA(cudaEventRecord(e1, ctx.stream));
-    int h = 0;
-    err.download(&h, 1);
-    HF_CUDA(cudaStreamSynchronize(ctx.stream));
-    float ms = 0;
-    HF_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    ctx.stat_tc_ms += ms;
-    ctx.stat_tc_flops += 2.0 * (NSL * (NSL + 1) / 2) * (double)M_rows * (double)B.rows * (double)K;
-    if constexpr (std::is_same_v<Src, PackedRowsBlocked>) {
-        ctx.stat_tc_step1_ms += ms;
-        ctx.stat_tc_step1_n += 1;
-    }
-    HF_CHECK(h == 0, HFGPU_ERR_CUDA, "gather GEMM: an mbarrier wait timed out");
+    HF_CUDA(cudaEventRecord(t.b, ctx.stream));
+    ctx.tc_events.push_back(t);
 }
 
-// widest output tile first: every row is gathered once per column tile
-// (M: rows of the launch, dead ones included; M_rows: the live rows, for the flop count)
 template <class Src>
 static void gather_gemm(Context& ctx, const Src& src, int64_t M, int64_t M_rows, int K, const Sliced& B, double* out,
                         OutMap om)
 {
-    if (B.rows <= Gather64::GBN)
-        gather_gemm_cfg<Src, Gather64>(ctx, src, M, M_rows, K, B, out, om);
+    if (B.digits == SLICE_MIXED)
+        gather_gemm_n<Src, 6>(ctx, src, M, M_rows, K, B, out, om);
     else
-        gather_gemm_cfg<Src, Gather80>(ctx, src, M, M_rows, K, B, out, om);
+        gather_gemm_n<Src, 9>(ctx, src, M, M_rows, K, B, out, om);
+}
+
+void sliced_gemm_settle(Context& ctx)
+{
+    int h = 0;
+    if (ctx.tc_err) {
+        HF_CUDA(cudaMemcpyAsync(&h, ctx.tc_err, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+        HF_CUDA(cudaMemsetAsync(ctx.tc_err, 0, sizeof(int), ctx.stream));
+    }
+    HF_CUDA(cudaStreamSynchronize(ctx.stream));
+    for (auto& t : ctx.tc_events) {
+        float ms = 0;
+        HF_CUDA(cudaEventElapsedTime(&ms, t.a, t.b));
+        cudaEventDestroy(t.a);
+        cudaEventDestroy(t.b);
+        ctx.stat_tc_ms += ms;
+        ctx.stat_tc_flops += t.flops;
+        if (t.step1) {
+            ctx.stat_tc_step1_ms += ms;
+            ctx.stat_tc_step1_n += 1;
+        }
+    }
+    ctx.tc_events.clear();
+    HF_CHECK(h == 0, HFGPU_ERR_CUDA, "sliced GEMM: an mbarrier wait timed out");
 }
 
 // ---- row maxima for the gather-fed GEMM
@@ -982,26 +844,24 @@ void dense_row_max(Context& ctx, const double* A, int64_t rows, int K, int64_t l
     HF_CUDA(cudaGetLastError());
 }
 
-void sliced_gemm_dense_gather(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, const unsigned* rmax,
-                              const Sliced& B, double* out, OutMap om)
+void sliced_gemm_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, const unsigned* rmax,
+                       const Sliced& B, double* out, OutMap om)
 {
-    const DenseRowsG src{A, ld, rmax};
-    gather_gemm(ctx, src, rows, rows, K, B, out, om);
+    gather_gemm(ctx, DenseRowsG(A, ld, rmax), rows, rows, K, B, out, om);
 }
 
-void sliced_gemm_packed(Context& ctx, const double* ints, const int2* pairs, int64_t p0, int64_t npairs, int n,
-                        const unsigned* rmax, const Sliced& B, double* out, OutMap om)
+void sliced_gemm_packed(Context& ctx, const double* ints, int64_t p0, int64_t npairs, int n, const unsigned* rmax,
+                        const Sliced& B, double* out, OutMap om)
 {
     const int nlg = (n + 15) / 16;
-    const PackedRowsBlocked src{ints, pairs, p0, npairs, n, nlg, rmax};
+    const PackedRowsBlocked src{ints, p0, npairs, n, nlg, rmax};
     gather_gemm(ctx, src, (npairs + 7) / 8 * nlg * 128, npairs * n, n, B, out, om);
 }
 
 void sliced_gemm_sympair(Context& ctx, const double* Zt, int64_t ldz, int64_t nq, int n, const unsigned* rmax,
                          const Sliced& B, double* out, OutMap om)
 {
-    SymPairRows src{Zt, ldz, n};
-    src.rmax = rmax;
+    const SymPairRows src{Zt, ldz, n, rmax};
     gather_gemm(ctx, src, nq * n, nq * n, n, B, out, om);
 }
 

@@ -1,4 +1,4 @@
-// Exactly sliced FP64 GEMM on tcgen05 tensor cores (tcgemm.cu).
+// Exactly sliced FP64 GEMMs on tcgen05 tensor cores (tcgemm.cu).
 #pragma once
 #include <cuda_bf16.h>
 
@@ -13,45 +13,49 @@ struct OutMap {
     int64_t ld;
 };
 
-// A matrix cut into six bf16 planes of 7-bit digits plus one power-of-two
-// exponent per row; rows and K padded to the tile sizes.
+// Digits a double is cut into: 6 (2^-42 of its row's scale) or 9 (2^-62).
+enum SliceDigits { SLICE_MIXED = 6, SLICE_FP64 = 9 };
+// the longest K whose FP32 accumulation is exact with that many digits
+int slice_kmax(int digits);
+
+// The B operand of a sliced GEMM: the rows of B^T cut into bf16 digit planes, laid out
+// as the GEMM's pipeline stages (whole tiles of `tile` columns, K steps of 32), plus
+// one power-of-two exponent per row.
 struct Sliced {
     DBuf<__nv_bfloat16> planes;
     DBuf<int> rexp;
     int64_t rows = 0, rows_pad = 0;
-    int K = 0, K_pad = 0;
-    void alloc(Context& ctx, int64_t rows, int K, int row_tile);
+    int K = 0, ksteps = 0, digits = 0, tile = 0;
 };
-
-constexpr int SLICE_TILE_A = 128, SLICE_TILE_B = 64;
-
 // rows of a row-major FP64 matrix (stride ld)
-void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, Sliced& s, int row_tile);
-// rows (pair p, la) over si of the packed (mu nu|la si), pairs[p0 .. p0+npairs)
-void slice_packed(Context& ctx, const double* ints, const int2* pairs, int64_t p0, int64_t npairs, int n, Sliced& s);
-// rows (q, mu), q < nq, over nu of Zt[q * ldz + pair(mu, nu)]
-void slice_sympair(Context& ctx, const double* Zt, int64_t ldz, int64_t nq, int n, Sliced& s);
-// out (+)= A B^T for slices A (M x K) and B (N x K)
-void sliced_gemm(Context& ctx, const Sliced& A, const Sliced& B, double* out, OutMap om, bool accumulate);
+void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, int digits, Sliced& s);
+
 // out = A B^T with A's rows gathered and sliced inside the GEMM (no A planes in
-// HBM): rows (pair p, la) over si of the packed (mu nu|la si) ...
-// (rmax: the rows' maxima from packed_row_max, for all pairs) ...
-void sliced_gemm_packed(Context& ctx, const double* ints, const int2* pairs, int64_t p0, int64_t npairs, int n,
-                        const unsigned* rmax, const Sliced& B, double* out, OutMap om);
+// HBM), B's digits deciding the precision:
+// rows (pair p, la) over si of the packed (mu nu|la si), pairs p0 .. p0 + npairs (rmax:
+// the rows' maxima from packed_row_max, for all pairs) ...
+void sliced_gemm_packed(Context& ctx, const double* ints, int64_t p0, int64_t npairs, int n, const unsigned* rmax,
+                        const Sliced& B, double* out, OutMap om);
 // ... or rows (q, mu), q < nq, over nu of Zt[q * ldz + pair(mu, nu)] (rmax from
-// sympair_row_max for these nq rows)
+// sympair_row_max for these nq rows) ...
 void sliced_gemm_sympair(Context& ctx, const double* Zt, int64_t ldz, int64_t nq, int n, const unsigned* rmax,
                          const Sliced& B, double* out, OutMap om);
+// ... or dense row-major rows (rows x K, stride ld; rmax from dense_row_max)
+void sliced_gemm_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, const unsigned* rmax,
+                       const Sliced& B, double* out, OutMap om);
 // max |x| of every gather row, as the upper 32 bits of |x| (enough for its
 // exponent): packed integrals, rows (pair p, la) of all n (n + 1) / 2 pairs ->
 // out[p * n + la]; Zt rows (q, mu) -> out[q * n + mu]
 void packed_row_max(Context& ctx, const double* ints, int n, unsigned* out);
-// dense row-major rows (rows x K, stride ld): their maxima, and the gather-fed GEMM
-// over them (no A planes in HBM; B may span several 64/80-column tiles)
 void dense_row_max(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, unsigned* out);
-void sliced_gemm_dense_gather(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, const unsigned* rmax,
-                              const Sliced& B, double* out, OutMap om);
 void sympair_row_max(Context& ctx, const double* Zt, int64_t ldz, int64_t nq, int n, unsigned* out);
+// wait for the sliced GEMMs queued so far: adds their times to the context's
+// counters and throws if one of them timed out
+void sliced_gemm_settle(Context& ctx);
+// (ia|jb) by the half transform on sliced GEMMs of `digits` digits, T[j][b][i][a]
+// (mp2_mixed.cu); n <= slice_kmax(digits)
+void ao2mo_sliced(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,
+                  int digits, double* T);
 // out[c][r] = in[r][c] for a rows x cols row-major FP64 matrix (mp2_mixed.cu)
 void transpose_device(Context& ctx, const double* in, int64_t rows, int64_t cols, double* out);
 
