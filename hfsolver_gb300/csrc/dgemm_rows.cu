@@ -1,9 +1,14 @@
-// Plain FP64 AO -> MO transform: the drop-in beside the tensor-core path.
+// Plain FP64 AO -> MO transform: the drop-in beside the mixed-precision path.
 //
-// The same (ia|jb) as the mixed-precision transform (mp2_mixed.cu), in the same
-// half-transform order over mu >= nu pairs, with every contraction an FP64
-// GEMM whose A rows are gathered straight from where the transform keeps them
-// (gather_rows.cuh): the packed AO integrals, Z transposed, or dense rows.
+// Up to slice_kmax(9) = 455 functions every contraction is the sliced tensor-core GEMM
+// with nine digits per factor (tcgemm.cu), which keeps 2^-62 of a row's scale and sums
+// exactly: at 20 to 48 functions the transformed integrals are within 1e-16 (2-norm) of
+// 113-bit arithmetic, where FP64 GEMMs left 3e-16, and GB300's FP64 pipe (2 FMAs per
+// clock per SM) no longer bounds it: 6 waters' MBPT2 34 -> 6 ms, 8 waters' 137 -> 19 ms.
+//
+// Beyond that the same half transform over mu >= nu pairs runs on FP64 GEMMs whose A
+// rows are gathered straight from where the transform keeps them (gather_rows.cuh): the
+// packed AO integrals, Z transposed, or dense rows.
 //   1. Y[p][j][la] = sum_si (mu nu|la si) C1[si, j]        p = pair(mu >= nu)
 //   2. Z[p][j][b]  = sum_la Y[p][j][la] C2[la, b]
 //   3. W[q][i][mu] = sum_nu Z[pair(mu, nu)][q] C1[nu, i]   q = (j, b)
@@ -11,7 +16,7 @@
 // transform_int2 (src/mbpt.f90:11-79) forms all four quarters over the full
 // n^4 index space by dot products; this order uses the (mu nu) symmetry of
 // the AO integrals in steps 1-2 (half the work of a dense first quarter) and
-// never unpacks them.
+// never unpacks them.  The GEMM also serves MBPT3's products.
 //
 // dgemm_rows_kernel: out = A B over 128 x (8 TN) output tiles, 256 threads, K in
 // chunks of 16.  Thread (tx, ty) = (lane, warp) owns rows tx + 32 i (i < 4) and
@@ -170,6 +175,10 @@ static const int64_t FP64_BLOCK_ROWS = 1 << 20;
 void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,
                 double* T)
 {
+    if (n <= slice_kmax(SLICE_FP64)) {
+        ao2mo_sliced(ctx, n, d_int2, C1, n1, C2, n2, SLICE_FP64, T);
+        return;
+    }
     cudaStream_t st = ctx.stream;
     HF_CHECK(n <= 4096, HFGPU_ERR_UNSUPPORTED, "FP64 transform supports up to 4096 functions");
     const int64_t npair = (int64_t)n * (n + 1) / 2;

@@ -35,3 +35,33 @@ def test_sliced_gemm_exact_where_digits_agree():
     x = 1.0 - 2.0 ** -42
     C = sliced(np.full((130, 512), x), np.full((512, 80), -x))
     assert np.all(np.abs(C + 512.0 * x * x) <= 512.0 * 2.0 ** -41)
+
+
+@pytest.mark.parametrize("n,seed", [(3, 0), (17, 1), (26, 2)])
+def test_fp64_transform_against_extended_precision(n, seed):
+    """transform_int2 with nine digits per factor against the same contraction in extended
+    precision.  Each of the four steps keeps its sums to 2^-62 n of the factors' scales and
+    rounds once to FP64 (2^-53), with intermediate values at most n times the largest
+    integral (orthogonal C): 4 n 2^-52 of the largest result and integral bounds it."""
+    import hfsolver_gb300 as hf
+
+    rng = np.random.default_rng(seed)
+    m = n * (n + 1) // 2
+    B = rng.standard_normal((m, n)) * 10.0 ** rng.uniform(-4, 0, size=(m, 1))
+    M = B @ B.T
+    k, l = np.tril_indices(m)
+    int2 = np.ascontiguousarray(M[k, l])
+    C = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    out = hf.transform_int2(int2, C)
+    M = np.zeros((m, m))
+    M[k, l] = int2
+    M[l, k] = int2
+    i, j = np.tril_indices(n)
+    X, Cl = M.astype(np.longdouble), C.astype(np.longdouble)
+    for _ in range(2):
+        Q = np.zeros((m, n, n), dtype=np.longdouble)
+        Q[:, i, j] = X
+        Q[:, j, i] = X
+        X = np.ascontiguousarray(np.stack([Cl.T @ (q @ Cl) for q in Q])[:, i, j].T)
+    err = np.max(np.abs((out - X[k, l]).astype(np.float64)))
+    assert err <= 4 * n * 2.0 ** -52 * max(np.max(np.abs(int2)), float(np.max(np.abs(X))))
