@@ -115,6 +115,18 @@ void Context::fork()
     for (int i = 0; i < NAUX; ++i) HF_CUDA(cudaStreamWaitEvent(aux[i], fork_ev, 0));
 }
 
+void* Context::pinned(Pin which, size_t bytes)
+{
+    if (pin_n[which] < bytes) {
+        if (pin_p[which]) cudaFreeHost(pin_p[which]);
+        pin_p[which] = nullptr;
+        pin_n[which] = 0;
+        HF_CUDA(cudaMallocHost(&pin_p[which], bytes));
+        pin_n[which] = bytes;
+    }
+    return pin_p[which];
+}
+
 void Context::settle_timers()
 {
     for (auto& e : fock_events) {

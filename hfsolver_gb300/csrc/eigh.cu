@@ -263,13 +263,12 @@ void Eigh::setup(Context& ctx, int n_)
     M.alloc((size_t)n * m, st);
     W.alloc((size_t)m * n, st);
     sync.alloc(1, st);
-    HF_CUDA(cudaMallocHost((void**)&hbuf, sizeof(double) * (3 * n + nn) + sizeof(TrdSync)));
+    hbuf = (double*)ctx.pinned(Context::PIN_EIGH, sizeof(double) * (3 * n + nn) + sizeof(TrdSync));
     HF_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
 }
 
 Eigh::~Eigh()
 {
-    if (hbuf) cudaFreeHost(hbuf);
     if (ready) cudaEventDestroy(ready);
 }
 
@@ -280,7 +279,8 @@ void Eigh::solve(Context& ctx, const double* X, const double* F, double* C, doub
     const int m = n - 2;
     if (ncol <= 0 || ncol > n) ncol = n;
     const double one = 1.0, zero = 0.0, mone = -1.0;
-    // F' = X^T F X
+    // F' = X^T F X (dense sums: where levels are degenerate, an open-shell atom's p for
+    // one, their rounding picks the occupied ones, and the atomic start with them)
     gemm(ctx, true, false, n, n, n, 1.0, X, n, F, n, 0.0, T1.p, n);
     gemm(ctx, false, false, n, n, n, 1.0, T1.p, n, X, n, 0.0, Fp.p, n);
     ctx.trace_mark("eigh X^T F X");

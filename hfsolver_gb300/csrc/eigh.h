@@ -26,7 +26,7 @@ struct Eigh {
     int n = 0;
     DBuf<double> Fp, T1, V, tau, de, xch, Tinv, Tw, XV, M, W;
     DBuf<TrdSync> sync;
-    double* hbuf = nullptr;  // pinned: d, e (2n), lam (n), Z (n x n), barrier state
+    double* hbuf = nullptr;  // pinned, the context's: d, e (2n), lam (n), Z (n x n), barrier state
     cudaEvent_t ready = nullptr;
     static bool supported(Context& ctx, int n);
     void setup(Context& ctx, int n_);

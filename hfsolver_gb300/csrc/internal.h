@@ -159,14 +159,25 @@ struct Context {
     void trace_begin();
     void trace_mark(const char* name);
     void trace_report();
+    // pinned host buffers, one per use, grown on demand and kept with the context
+    // (pinning pages costs more than the SCF of a small molecule's set-up)
+    enum Pin { PIN_SCF, PIN_EIGH, PIN_COUNT };
+    void* pin_p[PIN_COUNT] = {};
+    size_t pin_n[PIN_COUNT] = {};
+    void* pinned(Pin which, size_t bytes);
     // held by every public call for its whole duration: calls from several host
     // threads on one context run one after another (handles and stream are shared)
     std::recursive_mutex call_mutex;
 };
 // C = alpha op(A) op(B) + beta C in FP64, column-major: the own small-matrix
 // kernel for m, n, k <= 512 (gemm_small.cu), cuBLAS beyond
+// flags: what the caller knows of the operands.  GEMM_K_LE_I: op(A)(i, k) = 0 for k > i;
+// GEMM_K_GE_I: for k < i; GEMM_K_LE_J, GEMM_K_GE_J: the same of op(B)(k, j);
+// GEMM_SYMMETRIC: C is symmetric (m = n; with beta = 0).  (Zeros and both triangles must
+// be stored all the same: beyond 512 cuBLAS reads them.)
+enum { GEMM_K_LE_I = 1, GEMM_K_GE_I = 2, GEMM_K_LE_J = 4, GEMM_K_GE_J = 8, GEMM_SYMMETRIC = 16 };
 void gemm(Context& ctx, bool ta, bool tb, int m, int n, int k, double alpha, const double* A, int lda,
-          const double* B, int ldb, double beta, double* C, int ldc);
+          const double* B, int ldb, double beta, double* C, int ldc, int flags = 0);
 // algorithmic FP64 flops of one primitive shell quartet (la lb | lc ld): the fixed
 // McMurchie-Davidson count of the ERI roofline (eri.cu)
 double md_flops(int la, int lb, int lc, int ld);

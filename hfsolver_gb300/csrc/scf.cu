@@ -12,7 +12,9 @@
 // back two scalars (E0, dP) for the convergence test.
 #include <algorithm>
 #include <cmath>
+#include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -22,67 +24,133 @@
 
 namespace hfgpu {
 
-__global__ void add_kernel(int64_t nn, const double* __restrict__ A, const double* __restrict__ B, double* C)
+// ---- the elementwise passes of an iteration, with their sums ----------------
+// Every sum over n^2 elements: each block's part goes to partial[], and the block that
+// finishes last adds them in block order (deterministic), writes the result and resets
+// the counter for the next launch.  One block alone took 30 us for 400 functions.
+constexpr int RED_BLOCK = 256, RED_MAX_BLOCKS = 128, RED_MAX = 20;  // RED_MAX sums at once
+struct RedWork {
+    double* partial;  // RED_MAX_BLOCKS x RED_MAX
+    unsigned* count;
+};
+
+static unsigned red_blocks(int64_t nn)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nn) C[i] = A[i] + B[i];
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>(RED_MAX_BLOCKS, (nn + 2 * RED_BLOCK - 1) / (2 * RED_BLOCK)));
 }
 
-__global__ void sub_kernel(int64_t nn, const double* __restrict__ A, const double* __restrict__ B, double* C)
+// The block's sums of v[0 .. m) (m <= M) to partial; true in the last block to finish, with
+// the totals over all blocks in tot[0 .. m) (shared memory).
+template <int M>
+__device__ bool grid_sums(const double (&v)[M], int m, const RedWork w, double* tot)
 {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nn) C[i] = A[i] - B[i];
-}
-
-__global__ void mix_kernel(int64_t nn, double alpha, const double* __restrict__ Pold, double* P)
-{
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nn) P[i] = (1 - alpha) * Pold[i] + alpha * P[i];
-}
-
-__global__ void comm_kernel(int n, const double* __restrict__ Y, double* E)
-{
-    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)n * n) return;
-    int i = idx % n, j = idx / n;
-    E[idx] = Y[idx] - Y[j + (int64_t)i * n];
-}
-
-// Deterministic single-block reductions (n^2 <= a few 1e5 elements).
-// mode 0: sum A*(B+C)/2, mode 1: sqrt(sum (A-B)^2 / 4), mode 2: sum A*B
-__global__ void reduce_kernel(int mode, int64_t nn, const double* __restrict__ A, const double* __restrict__ B,
-                              const double* __restrict__ C, double* out)
-{
-    __shared__ double sh[1024];
-    double s = 0.0;
-    for (int64_t i = threadIdx.x; i < nn; i += blockDim.x) {
-        if (mode == 0)
-            s += A[i] * (B[i] + C[i]);
-        else if (mode == 1)
-            s += (A[i] - B[i]) * (A[i] - B[i]);
-        else
-            s += A[i] * B[i];
+    __shared__ double sh[M][RED_BLOCK / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < M; ++k) {
+        if (k >= m) break;
+        double x = v[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) sh[k][warp] = x;
     }
-    sh[threadIdx.x] = s;
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
+    if ((int)threadIdx.x < m) {
+        double x = 0;
+        for (int i = 0; i < RED_BLOCK / 32; ++i) x += sh[threadIdx.x][i];
+        w.partial[blockIdx.x * RED_MAX + threadIdx.x] = x;
+        __threadfence();
     }
-    if (threadIdx.x == 0) {
-        double r = sh[0];
-        if (mode == 0) r *= 0.5;
-        if (mode == 1) r = sqrt(r / 4);
-        *out = r;
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(w.count, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    for (int k = warp; k < m; k += RED_BLOCK / 32) {
+        double x = 0;
+        for (int i = lane; i < (int)gridDim.x; i += 32) x += __ldcg(w.partial + i * RED_MAX + k);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) tot[k] = x;
+    }
+    if (threadIdx.x == 0) *w.count = 0;
+    __syncthreads();
+    return true;
+}
+
+// what an iteration reports to the host, in one copy
+struct Sp2Sync {
+    unsigned count;
+    int err, steps;
+    double trace;  // tr X of the result
+};
+struct ScfReport {
+    double E0, dP;
+    Sp2Sync sp2[2];  // density purification: [0] FP32, [1] FP64
+};
+
+// F = H + G (with acc: G is added to the running acc first, F = H + acc), F's copy in the
+// DIIS history, Pold = P, E0 = sum P (H + F) / 2; clears the purification's barriers
+__global__ void __launch_bounds__(RED_BLOCK) fock_kernel(int64_t nn, const double* __restrict__ H,
+                                                         const double* __restrict__ G, double* acc,
+                                                         const double* __restrict__ P, double* __restrict__ F,
+                                                         double* __restrict__ Fhist, double* __restrict__ Pold, RedWork w,
+                                                         ScfReport* rep)
+{
+    __shared__ double tot[1];
+    double s[1] = {0.0};
+    for (int64_t i = (int64_t)blockIdx.x * RED_BLOCK + threadIdx.x; i < nn; i += (int64_t)gridDim.x * RED_BLOCK) {
+        double g = G[i];
+        if (acc) {
+            g += acc[i];
+            acc[i] = g;
+        }
+        const double h = H[i], f = h + g, p = P[i];
+        F[i] = f;
+        if (Fhist) Fhist[i] = f;
+        Pold[i] = p;
+        s[0] += p * (h + f);
+    }
+    if (grid_sums(s, 1, w, tot) && threadIdx.x == 0) {
+        rep->E0 = 0.5 * tot[0];
+        rep->sp2[0] = rep->sp2[1] = Sp2Sync{0u, 0, 0, 0.0};
     }
 }
 
-static void reduce(Context& ctx, int mode, int64_t nn, const double* A, const double* B, const double* C,
-                   double* dout)
+// D = P - Pold (the next incremental build's density), dP = sqrt(sum D^2 / 4)
+__global__ void __launch_bounds__(RED_BLOCK) density_change_kernel(int64_t nn, const double* __restrict__ P,
+                                                                   const double* __restrict__ Pold, double* D, RedWork w,
+                                                                   ScfReport* rep)
 {
-    reduce_kernel<<<1, 1024, 0, ctx.stream>>>(mode, nn, A, B, C, dout);
-    count_launch();
-    HF_CUDA(cudaGetLastError());
+    __shared__ double tot[1];
+    double s[1] = {0.0};
+    for (int64_t i = (int64_t)blockIdx.x * RED_BLOCK + threadIdx.x; i < nn; i += (int64_t)gridDim.x * RED_BLOCK) {
+        const double d = P[i] - Pold[i];
+        if (D) D[i] = d;
+        s[0] += d * d;
+    }
+    if (grid_sums(s, 1, w, tot) && threadIdx.x == 0) rep->dP = sqrt(tot[0] / 4);
+}
+
+__global__ void __launch_bounds__(RED_BLOCK) dot_kernel(int64_t nn, const double* __restrict__ A,
+                                                        const double* __restrict__ B, RedWork w, double* out)
+{
+    __shared__ double tot[1];
+    double s[1] = {0.0};
+    for (int64_t i = (int64_t)blockIdx.x * RED_BLOCK + threadIdx.x; i < nn; i += (int64_t)gridDim.x * RED_BLOCK)
+        s[0] += A[i] * B[i];
+    if (grid_sums(s, 1, w, tot) && threadIdx.x == 0) *out = tot[0];
+}
+
+// P = (1 - alpha) Pold + alpha P and D = P - Pold
+__global__ void mix_kernel(int64_t nn, double alpha, const double* __restrict__ Pold, double* P, double* D)
+{
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nn) return;
+    const double p = (1 - alpha) * Pold[i] + alpha * P[i];
+    P[i] = p;
+    if (D) D[i] = p - Pold[i];
 }
 
 static unsigned nblk(int64_t n) { return (unsigned)((n + 255) / 256); }
@@ -156,26 +224,324 @@ __global__ void __launch_bounds__(SQ_T* SQ_T) sym_square_kernel(int n, const dou
     }
 }
 
-// The whole SP2 recursion in one cooperative launch: one block per upper-
-// triangle 16x16 tile of the iterate X, grid-wide barriers between the square
-// and the update, the square-or-not choice and the convergence test made by
-// every block from the same traces.  A block keeps its own tile of X^2 in
-// registers, so only X travels through memory (read past L1: other blocks
-// wrote it).  Every barrier wait is bounded; a timeout sets err and all blocks
-// leave.
-struct Sp2Sync {
-    unsigned count, gen;
-    int err, steps;
+// The whole density purification of one Fock matrix as one cooperative launch: the
+// spectral bounds, the initial iterate and the SP2 recursion, one block per tt x tt
+// upper-triangle tile of the iterate, one grid barrier per step.
+// what a block leaves for the others at a barrier: its share of tr X and ||X||_F^2 in
+// units of 2^-50, or of the traces of F and its spectral bounds
+struct __align__(16) Sp2Slot {
+    long long a, c;
 };
+struct __align__(16) Sp2Bounds {
+    double tr, nrm, lo, hi;
+};
+// The shares are summed as integers: a warp-wide FP64 add holds its sub-partition's pipe
+// 64 cycles and a shuffle sum of two doubles takes a thousand, a third of a step.  (|X| <= 1
+// and ||X||^2 <= n: sums below 2^60, each element within 2^-51.)
+constexpr double SP2_UNIT = 1125899906842624.0;  // 2^50
 
-// grid barrier number `epoch` of one SP2 launch (gridsync.cuh)
-__device__ bool sp2_grid_barrier(Sp2Sync* s, unsigned nblocks, unsigned epoch)
+enum { SP2_FROM_F = 0, SP2_FROM_F32 = 1 };
+
+// Start: SP2_FROM_F: X_0 = (hi I - F) / (hi - lo), the spectrum of F mapped into [0, 1] by
+// its Gershgorin bounds with the occupied states near 1 (the blocks share the rows of F
+// and meet at one barrier; X_0 itself is never stored: step 0 maps F as it stages it);
+// SP2_FROM_F32: X_0 is the FP32 result of an earlier coarse launch.
+// A step: every block sums the others' shares of tr X_k and ||X_k||_F^2 = tr X_k^2 (X_k
+// symmetric) in a fixed order, so all blocks take the same choice between X^2 and 2X - X^2
+// and the same convergence decision; squares its tile from its tt rows and tt columns of
+// X_k, staged whole in shared memory (stride n + 1: no bank conflicts); writes it with its
+// shares and arrives at the barrier.  The iterate alternates between X0 and X1 and ends in
+// X0.  T = float for the coarse steps of early SCF iterations.  The tile edge tt (8 .. 32)
+// and the number of k-slices ks each output's dot product is split into (their partial
+// sums meet in shared memory) are chosen so that the FP64 work spreads evenly over the SMs
+// and over each SM's four sub-partitions (sp2_shape).
+// Once tr(X - X^2) < tol_idem the recursion takes `polish` (0 or 2) more steps, one
+// square and one 2X - X^2: an occupation 1 - d goes to 1 - 2d and 1 - 4d^2 (or 1 - d^2
+// and 1 - 2d^2), one at d to the mirror image, so a sum of 1e-7 left by the test ends
+// at 4e-14, the rounding of the sum, on both sides.
+// Bound: the FP64 pipe at a few hundred functions, the latency of a step below: one
+// barrier and one round of L2 loads (shares and tiles together); every warp-wide FP64
+// instruction outside the dot products (sums, tests) lengthens it by 64 cycles.  Per
+// purification of 28 steps, with the bounds and X_0 in a chain of small kernels before:
+// 25 functions 0.154 -> 0.11 ms, 50: 0.20 -> 0.14, 150: 0.54 -> 0.38; the 17 densities of
+// an 8-water SCF (8 of them FP32 first) 7.4 -> 5.3 ms, the 18 of 16 waters 31.3 -> 26.7.
+// x^2 in units of 2^-50: the scale goes to x's exponent (|x| < 2^-900 counts as zero)
+__device__ __forceinline__ long long square_fixed(double x)
 {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) ok = grid_arrive_wait(&s->count, &s->err, nblocks, epoch);
-    __syncthreads();
-    return ok;
+    const int hi = __double2hiint(x);
+    const double y = (hi & 0x7FF00000) < (123 << 20) ? 0.0 : __hiloint2double(hi + (25 << 20), __double2loint(x));
+    return __double2ll_rn(y * y);
+}
+
+template <typename T, int FROM>
+__global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int ks, const void* src, T* X0, T* X1,
+                                                   Sp2Slot* slots, int maxs, double tol_idem, double tol_n, int polish,
+                                                   Sp2Sync* sync)
+{
+    extern __shared__ __align__(16) unsigned char sp2_smem[];
+    __shared__ long long red[2][32];
+    __shared__ double rb[4][32], tot[2];
+    __shared__ long long s_trace;
+    __shared__ int s_go, s_conv, s_square;
+    const int ld = n + 1, nblk = gridDim.x;
+    T* Ar = (T*)sp2_smem;    // rows i0 .. i0+tt-1 of X_k, all k
+    T* Bc = Ar + tt * ld;    // columns j0 .. j0+tt-1 (rows by symmetry)
+    T* part = Bc + tt * ld;  // partial dot products of k-slices 1 .. ks-1
+    const int nt = (n + tt - 1) / tt;
+    int b = blockIdx.x, ti = 0;
+    while (b >= nt - ti) {
+        b -= nt - ti;
+        ++ti;
+    }
+    const int tj = ti + b;
+    const int i0 = ti * tt, j0 = tj * tt;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    // ks x tt x tt workers: output (ty, tx) of k-slice `slice`; the block is rounded up to
+    // whole warps
+    const int outs = tt * tt;
+    const bool worker = (int)threadIdx.x < ks * outs;
+    const int slice = (int)threadIdx.x / outs, o = (int)threadIdx.x - slice * outs;
+    const int ty = o / tt, tx = o % tt;
+    const int i = i0 + ty, j = j0 + tx;
+    const int kc = (n + ks - 1) / ks, k0 = slice * kc, k1 = min(n, k0 + kc);
+    const bool own = worker && slice == 0 && i < n && j < n;
+
+    // this thread's place in the staging of a panel, and its stride
+    const int st_r = (int)threadIdx.x % tt, st_k = (int)threadIdx.x / tt;
+    const int st_dr = (int)blockDim.x % tt, st_dk = (int)blockDim.x / tt;
+    auto fixed = [](double x) { return __double2ll_rn(x * SP2_UNIT); };
+    Sp2Bounds* bounds = reinterpret_cast<Sp2Bounds*>(slots + 2 * nblk);
+    // arrive at barrier number `epoch` (thread 0, after the block's writes); false after a timeout
+    auto barrier = [&](unsigned epoch) {
+        if (threadIdx.x == 0) s_go = grid_arrive_wait(&sync->count, &sync->err, (unsigned)nblk, epoch);
+        __syncthreads();
+        return s_go != 0;
+    };
+    // the block's share of the traces into its slot of set `set`, then the barrier
+    auto share = [&](long long a, long long c, int set, unsigned epoch) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, d);
+            c += __shfl_xor_sync(0xffffffffu, c, d);
+        }
+        if (lane == 0) {
+            red[0][warp] = a;
+            red[1][warp] = c;
+        }
+        __syncthreads();  // (and every thread's part of X is written)
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < nw; ++w) {
+                a += red[0][w];
+                c += red[1][w];
+            }
+            slots[set * nblk + blockIdx.x] = Sp2Slot{a, c};
+        }
+        return barrier(epoch);
+    };
+    // What step `it` does, from tr X and ||X||^2 in units of 2^-50 (one thread, in integers:
+    // every FP64 compare would cost all warps 64 cycles each)
+    const long long N = (long long)nocc << 50, tol_i = fixed(tol_idem), tol_t = fixed(tol_n);
+    auto decide = [&](long long a, long long c) {
+        s_trace = a;
+        s_conv = llabs(a - c) < tol_i && llabs(a - N) < tol_t;
+        s_square = llabs(c - N) <= llabs(2 * a - c - N);
+    };
+    // the sums over all slots of set `set` and the decision, by warp 0; ready after the next
+    // __syncthreads
+    auto gather = [&](int set) {
+        if (warp == 0) {
+            long long a = 0, c = 0;
+            for (int s = lane; s < nblk; s += 32) {
+                const longlong2 u = __ldcg(reinterpret_cast<const longlong2*>(slots + set * nblk + s));
+                a += u.x;
+                c += u.y;
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                a += __shfl_xor_sync(0xffffffffu, a, d);
+                c += __shfl_xor_sync(0xffffffffu, c, d);
+            }
+            if (lane == 0) decide(a, c);
+        }
+    };
+
+    unsigned epoch = 0;
+    double scale = 0.0, shift = 0.0;  // X_0 = shift I - scale F
+    if (FROM == SP2_FROM_F) {
+        const double* F = (const double*)src;
+        double tr = 0, nrm = 0, lo = 1e300, hi = -1e300;
+        for (int r = (int)blockIdx.x * nw + warp; r < n; r += nblk * nw) {  // one warp per row (column: F is symmetric)
+            double s = 0, q = 0;
+            for (int k = lane; k < n; k += 32) {
+                const double f = F[k + (int64_t)r * n];
+                s += fabs(f);
+                q = fma(f, f, q);
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                s += __shfl_xor_sync(0xffffffffu, s, d);
+                q += __shfl_xor_sync(0xffffffffu, q, d);
+            }
+            const double f = F[r + (int64_t)r * n], rad = s - fabs(f);
+            lo = fmin(lo, f - rad);
+            hi = fmax(hi, f + rad);
+            if (lane == 0) {
+                tr += f;
+                nrm += q;
+            }
+        }
+        if (lane == 0) {
+            rb[0][warp] = tr;
+            rb[1][warp] = nrm;
+            rb[2][warp] = lo;
+            rb[3][warp] = hi;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < nw; ++w) {
+                tr += rb[0][w];
+                nrm += rb[1][w];
+                lo = fmin(lo, rb[2][w]);
+                hi = fmax(hi, rb[3][w]);
+            }
+            bounds[blockIdx.x] = Sp2Bounds{tr, nrm, lo, hi};
+        }
+        if (!barrier(++epoch)) return;
+        if (warp == 0) {
+            tr = nrm = 0;
+            lo = 1e300, hi = -1e300;
+            for (int s = lane; s < nblk; s += 32) {
+                const double2* p = reinterpret_cast<const double2*>(bounds + s);
+                const double2 u = __ldcg(p), v = __ldcg(p + 1);
+                tr += u.x;
+                nrm += u.y;
+                lo = fmin(lo, v.x);
+                hi = fmax(hi, v.y);
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                tr += __shfl_xor_sync(0xffffffffu, tr, d);
+                nrm += __shfl_xor_sync(0xffffffffu, nrm, d);
+                lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+                hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+            }
+            if (lane == 0) {  // X_0 = shift I - scale F, its trace and squared norm
+                const double sc = 1.0 / (hi - lo), sf = hi * sc;
+                decide(fixed(n * sf - sc * tr), fixed(n * sf * sf - 2.0 * sf * sc * tr + sc * sc * nrm));
+                tot[0] = sc;
+                tot[1] = sf;
+            }
+        }
+        __syncthreads();
+        scale = tot[0];
+        shift = tot[1];
+    } else {
+        long long tr = 0, nrm = 0;
+        const float* S = (const float*)src;
+        if (own) {
+            const double x = (double)S[i + (int64_t)j * n];
+            if (i == j) tr = fixed(x);
+            nrm = square_fixed(x) << (ti != tj ? 1 : 0);
+        }
+        if (!share(tr, nrm, 0, ++epoch)) return;
+        gather(0);
+    }
+
+    int left = -1;  // polishing steps still to do (-1: not converged yet)
+    bool last_square = false;
+    for (int it = 0; it < maxs; ++it) {
+        T* Xc = (it & 1) ? X1 : X0;
+        T* Xn = (it & 1) ? X0 : X1;
+        if (it > 0) gather(it & 1);
+        // U elements of each panel in flight per thread: one at a time, a step at 150
+        // functions (four warps a block) spent 8 us here; r fastest: tt consecutive elements
+        // of a column
+        constexpr int U = 6;
+        for (int r = st_r, k = st_k; k < n;) {
+            T x[U], y[U];
+            int rr[U], kk[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                rr[u] = r;
+                kk[u] = k;
+                x[u] = y[u] = T(0);
+                if (k < n) {
+                    const int a = i0 + r, c = j0 + r;
+                    if (it == 0 && FROM == SP2_FROM_F) {
+                        const double* F = (const double*)src;
+                        if (a < n) x[u] = (T)((a == k ? shift : 0.0) - scale * F[a + k * n]);
+                        if (c < n) y[u] = (T)((c == k ? shift : 0.0) - scale * F[c + k * n]);
+                    } else if (it == 0) {
+                        const float* S = (const float*)src;
+                        if (a < n) x[u] = (T)S[a + k * n];
+                        if (c < n) y[u] = (T)S[c + k * n];
+                    } else {
+                        if (a < n) x[u] = __ldcg(Xc + a + k * n);
+                        if (c < n) y[u] = __ldcg(Xc + c + k * n);
+                    }
+                }
+                r += st_dr;
+                k += st_dk;
+                if (r >= tt) {
+                    r -= tt;
+                    ++k;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (kk[u] < n) {
+                    Ar[rr[u] * ld + kk[u]] = x[u];
+                    Bc[rr[u] * ld + kk[u]] = y[u];
+                }
+        }
+        __syncthreads();
+        const bool conv = s_conv != 0, sq = s_square != 0;
+        if (left < 0 && conv) left = polish;
+        if (left == 0) {
+            if (own && ((it & 1) || it == 0)) {  // X_k is in X1, or was never stored: this block's tile to X0
+                X0[i + (int64_t)j * n] = Ar[ty * ld + j];
+                if (ti != tj) X0[j + (int64_t)i * n] = Ar[ty * ld + j];
+            }
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                sync->steps = it;
+                sync->trace = (double)s_trace * (1.0 / SP2_UNIT);
+            }
+            return;
+        }
+        // the last of the polishing steps is the opposite of the one before it
+        const bool square = left == 1 ? !last_square : sq;
+        last_square = square;
+        if (left > 0) --left;
+        T acc = 0;
+        if (worker) {
+            const T* ar = Ar + ty * ld;
+            const T* bc = Bc + tx * ld;
+            for (int k = k0; k < k1; ++k) acc = fma(ar[k], bc[k], acc);
+            if (slice > 0) part[(slice - 1) * outs + o] = acc;
+        }
+        if (ks > 1) {
+            __syncthreads();
+            if (worker && slice == 0)
+                for (int q = 1; q < ks; ++q) acc += part[(q - 1) * outs + o];
+        }
+        long long pt = 0, pn = 0;
+        if (own) {
+            const T x = square ? acc : T(2) * Ar[ty * ld + j] - acc;
+            Xn[i + (int64_t)j * n] = x;
+            if (ti != tj) Xn[j + (int64_t)i * n] = x;
+            if (i == j) pt = fixed((double)x);
+            pn = square_fixed((double)x) << (ti != tj ? 1 : 0);
+        }
+        // (its __syncthreads also guard Ar, Bc, part and tot)
+        if (!share(pt, pn, (it + 1) & 1, ++epoch)) return;
+    }
+    if (blockIdx.x == 0) {  // maxs is even: X is in X0
+        gather(maxs & 1);
+        if (threadIdx.x == 0) {
+            sync->steps = maxs;
+            sync->trace = (double)s_trace * (1.0 / SP2_UNIT);
+        }
+    }
 }
 
 // Sum of v over the block into *dst (one atomic per block).
@@ -195,117 +561,7 @@ __device__ __forceinline__ void block_add(double v, double* dst)
     __syncthreads();
 }
 
-// The whole SP2 recursion as one cooperative launch, one grid barrier per step.
-// tr[2k] = tr X_k and tr[2k+1] = ||X_k||_F^2 = tr X_k^2 (X_k symmetric) are
-// reduced while X_k is written, so every block can choose X^2 or 2X - X^2 for
-// step k before it squares.  The iterate alternates between X0 and X1; a block
-// squares its tt x tt upper-triangle tile from its tt rows and tt columns of X_k,
-// staged whole in shared memory (stride n + 1: no bank conflicts).  The result
-// ends in X0.  T = float for the coarse steps of early SCF iterations.  The tile
-// edge tt (8 .. 32) and the number of k-slices ks each output's dot product is
-// split into (their partial sums meet in shared memory) are chosen so that the
-// FP64 work spreads evenly over the SMs and over each SM's four sub-partitions
-// (sp2_shape).
-// Once tr(X - X^2) < tol_idem the recursion takes `polish` (0 or 2) more steps, one
-// square and one 2X - X^2: an occupation 1 - d goes to 1 - 2d and 1 - 4d^2 (or 1 - d^2
-// and 1 - 2d^2), one at d to the mirror image, so a sum of 1e-7 left by the test ends
-// at 4e-14, the rounding of the sum, on both sides.
-template <typename T>
-__global__ void __launch_bounds__(1024) sp2_persistent_kernel(int n, int nocc, int tt, int ks, T* X0, T* X1,
-                                                              double* tr, int maxs, double tol_idem, double tol_n,
-                                                              int polish, Sp2Sync* sync)
-{
-    extern __shared__ __align__(16) unsigned char sp2_smem[];
-    const int ld = n + 1;
-    T* Ar = (T*)sp2_smem;  // rows i0 .. i0+tt-1 of X_k, all k
-    T* Bc = Ar + tt * ld;  // columns j0 .. j0+tt-1 (rows by symmetry)
-    T* part = Bc + tt * ld;  // partial dot products of k-slices 1 .. ks-1
-    const int nt = (n + tt - 1) / tt;
-    int b = blockIdx.x, ti = 0;
-    while (b >= nt - ti) {
-        b -= nt - ti;
-        ++ti;
-    }
-    const int tj = ti + b;
-    const int i0 = ti * tt, j0 = tj * tt;
-    // ks x tt x tt workers: output (ty, tx) of k-slice `slice` (ks slices spread the
-    // tile's FP64 work over all four sub-partitions of the SM); the block is rounded
-    // up to whole warps for the reductions
-    const int outs = tt * tt;
-    const bool worker = (int)threadIdx.x < ks * outs;
-    const int slice = (int)threadIdx.x / outs, o = (int)threadIdx.x - slice * outs;
-    const int ty = o / tt, tx = o % tt;
-    const int i = i0 + ty, j = j0 + tx;
-    const int kc = (n + ks - 1) / ks, k0 = slice * kc, k1 = min(n, k0 + kc);
-    const bool own = worker && slice == 0 && i < n && j < n;
-    int left = -1;  // polishing steps still to do (-1: not converged yet)
-    bool last_square = false;
-    for (int it = 0; it < maxs; ++it) {
-        T* Xc = (it & 1) ? X1 : X0;
-        T* Xn = (it & 1) ? X0 : X1;
-        const double t0 = __ldcg(tr + 2 * it), t1 = __ldcg(tr + 2 * it + 1);
-        if (left < 0 && fabs(t0 - t1) < tol_idem && fabs(t0 - nocc) < tol_n) left = polish;
-        if (left == 0) {
-            if ((it & 1) && own) {  // X_k is in X1: move this block's tile to X0
-                X0[i + (int64_t)j * n] = __ldcg(X1 + i + (int64_t)j * n);
-                if (ti != tj) X0[j + (int64_t)i * n] = __ldcg(X1 + j + (int64_t)i * n);
-            }
-            if (blockIdx.x == 0 && threadIdx.x == 0) sync->steps = it;
-            return;
-        }
-        // the last of the polishing steps is the opposite of the one before it
-        const bool square = left == 1 ? !last_square : fabs(t1 - nocc) <= fabs(2 * t0 - t1 - nocc);
-        last_square = square;
-        if (left > 0) --left;
-        for (int e = threadIdx.x; e < tt * n; e += blockDim.x) {
-            const int r = e % tt, k = e / tt;  // r fastest: tt consecutive elements of a column
-            Ar[r * ld + k] = (i0 + r < n) ? __ldcg(Xc + i0 + r + (int64_t)k * n) : T(0);
-            Bc[r * ld + k] = (j0 + r < n) ? __ldcg(Xc + j0 + r + (int64_t)k * n) : T(0);
-        }
-        __syncthreads();
-        T acc = 0;
-        if (worker) {
-            const T* ar = Ar + ty * ld;
-            const T* bc = Bc + tx * ld;
-            for (int k = k0; k < k1; ++k) acc = fma(ar[k], bc[k], acc);
-            if (slice > 0) part[(slice - 1) * outs + o] = acc;
-        }
-        if (ks > 1) {
-            __syncthreads();
-            if (worker && slice == 0)
-                for (int q = 1; q < ks; ++q) acc += part[(q - 1) * outs + o];
-        }
-        double pt = 0.0, pn = 0.0;
-        if (own) {
-            const T x = square ? acc : T(2) * __ldcg(Xc + i + (int64_t)j * n) - acc;
-            Xn[i + (int64_t)j * n] = x;
-            if (ti != tj) Xn[j + (int64_t)i * n] = x;
-            if (i == j) pt = (double)x;
-            pn = (double)x * (double)x * (ti != tj ? 2.0 : 1.0);
-        }
-        block_add(pt, tr + 2 * (it + 1));  // (its __syncthreads also guard Ar/Bc reuse)
-        block_add(pn, tr + 2 * (it + 1) + 1);
-        if (!sp2_grid_barrier(sync, gridDim.x, (unsigned)it + 1)) return;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) sync->steps = maxs;
-}
-
-// dst = src in another precision; trn[0] += its trace, trn[1] += its squared norm
-template <typename S, typename D>
-__global__ void convert_trace_kernel(int n, const S* __restrict__ src, D* __restrict__ dst, double* trn)
-{
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double t = 0.0, q = 0.0;
-    if (idx < (int64_t)n * n) {
-        const D v = (D)src[idx];
-        dst[idx] = v;
-        if (idx % n == idx / n) t = (double)v;
-        q = (double)v * (double)v;
-    }
-    block_add(t, trn);
-    block_add(q, trn + 1);
-}
-
+// The launch-per-step form (bases whose recursion does not fit one launch):
 // X = (emax I - F) / (emax - emin): spectrum mapped into [0, 1], occupied states
 // near 1; trX[0] = tr X and trX[1] = ||X||_F^2 of this initial iterate
 __global__ void sp2_init2_kernel(int n, const double* __restrict__ F, const double* __restrict__ b, double* X,
@@ -363,32 +619,37 @@ static bool coop_ok(Context& ctx, int n, int tt, int ks)
     const int dev = ctx.device;
     std::call_once(once, [dev] {
         int optin = 0;
-        cudaFuncAttributes fd{}, ff{};
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-            cudaFuncGetAttributes(&fd, sp2_persistent_kernel<double>) != cudaSuccess ||
-            cudaFuncGetAttributes(&ff, sp2_persistent_kernel<float>) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return;
+        const void* fns[] = {(const void*)sp2_kernel<double, SP2_FROM_F>, (const void*)sp2_kernel<double, SP2_FROM_F32>,
+                             (const void*)sp2_kernel<float, SP2_FROM_F>};
+        size_t fixed = 0;
+        bool ok = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess;
+        for (const void* f : fns) {
+            cudaFuncAttributes fa{};
+            ok = ok && cudaFuncGetAttributes(&fa, f) == cudaSuccess;
+            fixed = std::max(fixed, fa.sharedSizeBytes);
         }
-        most = (size_t)optin - std::max(fd.sharedSizeBytes, ff.sharedSizeBytes);
-        attr_ok = cudaFuncSetAttribute(sp2_persistent_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)most) == cudaSuccess &&
-                  cudaFuncSetAttribute(sp2_persistent_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)most) == cudaSuccess;
+        most = (size_t)optin - fixed;
+        for (const void* f : fns)
+            ok = ok && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
+        attr_ok = ok;
         if (!attr_ok) (void)cudaGetLastError();  // no pending error for the next launch check
     });
     if (!attr_ok || n > 512 || sp2_smem_bytes(n, tt, ks, sizeof(double)) > most) return false;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sp2_persistent_kernel<double>, sp2_threads(tt, ks),
-                                                      sp2_smem_bytes(n, tt, ks, sizeof(double))) != cudaSuccess)
+    int per_sm32 = 0;
+    const size_t smem = sp2_smem_bytes(n, tt, ks, sizeof(double));
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sp2_kernel<double, SP2_FROM_F>, sp2_threads(tt, ks),
+                                                      smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm32, sp2_kernel<double, SP2_FROM_F32>, sp2_threads(tt, ks),
+                                                      smem) != cudaSuccess)
         return false;
-    return (int64_t)per_sm * ctx.num_sms >= (int64_t)sp2_tiles(n, tt);
+    return (int64_t)std::min(per_sm, per_sm32) * ctx.num_sms >= (int64_t)sp2_tiles(n, tt);
 }
 
 // tile edge tt and k-slices ks of the persistent SP2 kernel.  Per step, a warp's
 // FP64 FMA keeps its sub-partition's FP64 pipe ~64 cycles busy on this GPU, so the
 // busiest sub-partition of the busiest SM takes ceil(resident warps / 4) x n/ks
-// such instructions; every block adds ~40 cycles of atomics at the barrier and the
-// trace sums.  Take the (tt in 8 .. 32, ks in 1 .. 4, at most 1024 threads) with
+// such instructions; every block adds ~40 cycles of the barrier's atomic and of the
+// shares that all others read.  Take the (tt in 8 .. 32, ks in 1 .. 4, at most 1024 threads) with
 // the least of both among those whose grid can be co-resident (n = 400: edge 17
 // or 25, where 8 .. 16 would need more blocks per SM than shared memory allows).
 // tt = 0: none fits.
@@ -398,6 +659,12 @@ struct Sp2Shape {
 
 static Sp2Shape sp2_shape(Context& ctx, int n)
 {
+    // ~100 occupancy queries a size: kept per (device, size)
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, Sp2Shape> cache;
+    std::lock_guard<std::mutex> lk(mu);
+    const auto known = cache.find({ctx.device, n});
+    if (known != cache.end()) return known->second;
     Sp2Shape best;
     int64_t best_cost = 0;
     for (int tt = 32; tt >= 8; --tt)
@@ -413,52 +680,48 @@ static Sp2Shape sp2_shape(Context& ctx, int n)
                 best_cost = cost;
             }
         }
-    return best;
+    return cache[{ctx.device, n}] = best;
 }
 
 struct Purifier {
     int n = 0, nocc = 0;
     int tile = 0;  // persistent-kernel tile edge (sp2_shape); -1: per-step fallback
     int kslices = 1;
-    DBuf<double> X, T1, T2, B, tr;  // orthogonaliser S^-1/2 and work
-    DBuf<float> Xf;                 // FP32 iterate of the coarse steps
-    DBuf<Sp2Sync> sync;
-    void setup(Context& ctx, int n_, int nocc_, const double* dS)
+    DBuf<double> X, T1, T2, T3, B, tr;  // orthogonaliser L^-T and work
+    DBuf<float> Xf;                     // FP32 iterate of the coarse steps
+    DBuf<Sp2Slot> slots;
+    ScfReport* rep = nullptr;         // device: barriers and outcome, cleared before each density()
+    const ScfReport* hrep = nullptr;  // its host copy, read by converged()
+    void setup(Context& ctx, int n_, int nocc_, const double* dS, ScfReport* rep_, const ScfReport* hrep_)
     {
         n = n_;
         nocc = nocc_;
+        rep = rep_;
+        hrep = hrep_;
         const int64_t nn = (int64_t)n * n;
         cudaStream_t st = ctx.stream;
         X.alloc(nn, st);
         T1.alloc(nn, st);
         T2.alloc(nn, st);
-        B.alloc(4, st);
-        tr.alloc(4, st);
         // orthogonaliser X = L^-T from the Cholesky factor S = L L^T (X^T S X = I):
         // a factorisation and a triangular solve instead of an eigensolve
         cholesky_orthogonalizer(ctx, n, dS, X.p);
     }
-    // One cooperative launch of the whole recursion on the iterate Xs, with
-    // barrier state slot `which` (0: FP32 steps, 1: FP64 steps).
-    template <typename T>
-    void run_persistent(Context& ctx, T* Xs, T* Xw, double* trs, int maxs, double tol_idem, double tol_n, int polish,
-                        int tt, int which)
+    // One cooperative launch of the whole recursion, barrier state slot `which`.
+    template <typename T, int FROM>
+    void run(Context& ctx, const void* src, T* X0, T* X1, double tol_idem, double tol_n, int polish, int which)
     {
-        cudaStream_t st = ctx.stream;
-        HF_CUDA(cudaMemsetAsync(sync.p + which, 0, sizeof(Sp2Sync), st));
-        int n_ = n, nocc_ = nocc, tt_ = tt, ks_ = kslices;
-        Sp2Sync* sp = sync.p + which;
-        void* args[] = {&n_, &nocc_, &tt_, &ks_, &Xs, &Xw, &trs, &maxs, &tol_idem, &tol_n, &polish, &sp};
-        HF_CUDA(cudaLaunchCooperativeKernel((const void*)sp2_persistent_kernel<T>, dim3(sp2_tiles(n, tt)),
-                                            dim3(sp2_threads(tt, kslices)), args,
-                                            sp2_smem_bytes(n, tt, kslices, sizeof(T)), st));
+        int n_ = n, nocc_ = nocc, tt_ = tile, ks_ = kslices, maxs = MAXS;
+        Sp2Slot* sl = slots.p;
+        Sp2Sync* sp = rep->sp2 + which;
+        void* args[] = {&n_, &nocc_, &tt_, &ks_, &src, &X0, &X1, &sl, &maxs, &tol_idem, &tol_n, &polish, &sp};
+        HF_CUDA(cudaLaunchCooperativeKernel((const void*)sp2_kernel<T, FROM>, dim3(sp2_tiles(n, tile)),
+                                            dim3(sp2_threads(tile, kslices)), args,
+                                            sp2_smem_bytes(n, tile, kslices, sizeof(T)), ctx.stream));
         count_launch();
     }
-    // The outcome of the last cooperative purification (barrier timeouts, final
-    // trace) is copied to pinned host memory without waiting; check() reads it
-    // after the caller's next synchronisation.
-    Sp2Sync* hsync = nullptr;
-    double* htr = nullptr;
+    // The outcome of the last cooperative purification (barrier timeouts, final trace)
+    // travels to the host with the iteration's report.
     bool pending = false;
     static constexpr int MAXS = 160;
     // Did the last density() end with tr X = nocc?  strict: and by the idempotency
@@ -467,10 +730,9 @@ struct Purifier {
     {
         if (!pending) return true;
         pending = false;
-        HF_CHECK(hsync[0].err == 0 && hsync[1].err == 0, HFGPU_ERR_CUDA,
+        HF_CHECK(hrep->sp2[0].err == 0 && hrep->sp2[1].err == 0, HFGPU_ERR_CUDA,
                  "density purification: grid barrier timed out");
-        const int last = std::min(std::max(hsync[1].steps, 0), MAXS);
-        return fabs(htr[2 * last] - nocc) < 1e-6 && !(strict && last == MAXS);
+        return fabs(hrep->sp2[1].trace - nocc) < 1e-6 && !(strict && hrep->sp2[1].steps >= MAXS);
     }
     // is the whole recursion one cooperative launch at this size?
     bool one_launch(Context& ctx)
@@ -482,11 +744,6 @@ struct Purifier {
         }
         return tile > 0;
     }
-    ~Purifier()
-    {
-        if (hsync) cudaFreeHost(hsync);
-        if (htr) cudaFreeHost(htr);
-    }
     // P = 2 X proj(X^T F X) X^T: the closed-shell density of F without diagonalising it.
     // coarse: run the recursion in FP32 until tr(X - X^2) < 1e-3, then finish in
     // FP64 (a few steps); the result is idempotent to FP64 precision but its
@@ -496,54 +753,52 @@ struct Purifier {
     {
         const int64_t nn = (int64_t)n * n;
         cudaStream_t st = ctx.stream;
-        const double one = 1.0, zero = 0.0, two = 2.0;
-        gemm(ctx, true, false, n, n, n, 1.0, X.p, n, dF, n, 0.0, T1.p, n);
-        gemm(ctx, false, false, n, n, n, 1.0, T1.p, n, X.p, n, 0.0, T2.p, n);
-        gersh_kernel<<<1, 1024, 0, st>>>(n, T2.p, B.p);
-        count_launch();
-        // per-step trace slots [step][tr X, tr X^2], zeroed once
-        const int CHECK = 8;
-        if (tr.n < (size_t)4 * (MAXS + 1)) tr.alloc(4 * (MAXS + 1), st);
-        HF_CUDA(cudaMemsetAsync(tr.p, 0, sizeof(double) * 4 * (MAXS + 1), st));
-        sp2_init2_kernel<<<nblk(nn), 256, 0, st>>>(n, T2.p, B.p, T1.p, tr.p);  // T1 = iterate
-        count_launch();
+        // X is upper triangular: X^T F sums k <= i, (X^T F) X k <= j and is symmetric
+        gemm(ctx, true, false, n, n, n, 1.0, X.p, n, dF, n, 0.0, T1.p, n, GEMM_K_LE_I);
+        gemm(ctx, false, false, n, n, n, 1.0, T1.p, n, X.p, n, 0.0, T2.p, n, GEMM_K_LE_J | GEMM_SYMMETRIC);
         ctx.trace_mark("sp2 X^T F X");
-        const int nt = (n + SQ_T - 1) / SQ_T;
-        const unsigned tiles = (unsigned)(nt * (nt + 1) / 2);  // of the per-step fallback
-        double h[2] = {0, 1};
-        bool done = false;
         if (one_launch(ctx)) {
-            if (!sync.p) {
-                sync.alloc(2, st);
-                HF_CUDA(cudaMemsetAsync(sync.p, 0, 2 * sizeof(Sp2Sync), st));
-                HF_CUDA(cudaMallocHost((void**)&hsync, 2 * sizeof(Sp2Sync)));
-                HF_CUDA(cudaMallocHost((void**)&htr, 2 * (MAXS + 1) * sizeof(double)));
+            if (!slots.p) {
+                slots.alloc(4 * (size_t)sp2_tiles(n, tile), st);  // two sets, and the bounds
+                T3.alloc(nn, st);
             }
-            double* tr64 = tr.p;
             if (coarse) {
                 if (Xf.n < (size_t)(2 * nn)) Xf.alloc(2 * nn, st);
-                double* trf = tr.p + 2 * (MAXS + 1);
-                convert_trace_kernel<double, float><<<nblk(nn), 256, 0, st>>>(n, T1.p, Xf.p, trf);
-                count_launch();
-                run_persistent<float>(ctx, Xf.p, Xf.p + nn, trf, MAXS, 1e-3, 1e-3, 0, tile, 0);
+                run<float, SP2_FROM_F>(ctx, T2.p, Xf.p, Xf.p + nn, 1e-3, 1e-3, 0, 0);
                 ctx.trace_mark("sp2 fp32");
-                HF_CUDA(cudaMemsetAsync(tr64, 0, sizeof(double) * 2 * (MAXS + 1), st));
-                convert_trace_kernel<float, double><<<nblk(nn), 256, 0, st>>>(n, Xf.p, T1.p, tr64);
-                count_launch();
+                run<double, SP2_FROM_F32>(ctx, Xf.p, T1.p, T3.p, 1e-7, 1e-6, 2, 1);
             } else {
-                HF_CUDA(cudaMemsetAsync(sync.p, 0, sizeof(Sp2Sync), st));  // no FP32 phase this time
+                run<double, SP2_FROM_F>(ctx, T2.p, T1.p, T3.p, 1e-7, 1e-6, 2, 1);
             }
-            // T2 (X^T F X) is free once the first iterate is built: the second buffer
-            run_persistent<double>(ctx, T1.p, T2.p, tr64, MAXS, 1e-7, 1e-6, 2, tile, 1);
             ctx.trace_mark("sp2 fp64");
-            HF_CUDA(cudaMemcpyAsync(hsync, sync.p, 2 * sizeof(Sp2Sync), cudaMemcpyDeviceToHost, st));
-            HF_CUDA(cudaMemcpyAsync(htr, tr64, 2 * (MAXS + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
             pending = true;
-            done = true;
-            h[0] = nocc;  // checked later by check()
+        } else {
+            per_step(ctx);
         }
-        // launch-per-step fallback: tr[2k+1] is accumulated by the square kernel
-        if (!done) HF_CUDA(cudaMemsetAsync(tr.p + 1, 0, sizeof(double), st));
+        // X Y sums k >= i, (X Y) X^T k >= j and is symmetric
+        gemm(ctx, false, false, n, n, n, 1.0, X.p, n, T1.p, n, 0.0, T2.p, n, GEMM_K_GE_I);
+        gemm(ctx, false, true, n, n, n, 2.0, T2.p, n, X.p, n, 0.0, dP, n, GEMM_K_GE_J | GEMM_SYMMETRIC);
+    }
+    // launch-per-step form: T2 = X^T F X to the projector in T1
+    void per_step(Context& ctx)
+    {
+        const int64_t nn = (int64_t)n * n;
+        cudaStream_t st = ctx.stream;
+        const int CHECK = 8;
+        B.alloc(4, st);
+        gersh_kernel<<<1, 1024, 0, st>>>(n, T2.p, B.p);
+        count_launch();
+        // per-step trace slots [step][tr X, tr X^2], zeroed once; tr[2k+1] is accumulated
+        // by the square kernel
+        tr.alloc(2 * (MAXS + 1), st);
+        HF_CUDA(cudaMemsetAsync(tr.p, 0, sizeof(double) * 2 * (MAXS + 1), st));
+        sp2_init2_kernel<<<nblk(nn), 256, 0, st>>>(n, T2.p, B.p, T1.p, tr.p);  // T1 = iterate
+        count_launch();
+        HF_CUDA(cudaMemsetAsync(tr.p + 1, 0, sizeof(double), st));
+        const int nt = (n + SQ_T - 1) / SQ_T;
+        const unsigned tiles = (unsigned)(nt * (nt + 1) / 2);
+        double h[2] = {0, 1};
+        bool done = false;
         for (int it = 0; it < MAXS && !done; ++it) {
             sym_square_kernel<<<tiles, SQ_T * SQ_T, 0, st>>>(n, T1.p, T2.p, tr.p + 2 * it + 1);
             count_launch();
@@ -557,8 +812,6 @@ struct Purifier {
             }
         }
         HF_CHECK(fabs(h[0] - nocc) < 1e-6, HFGPU_ERR_LINALG, "density purification did not converge (no gap?)");
-        gemm(ctx, false, false, n, n, n, 1.0, X.p, n, T1.p, n, 0.0, T2.p, n);
-        gemm(ctx, false, true, n, n, n, 2.0, T2.p, n, X.p, n, 0.0, dP, n);
     }
 };
 
@@ -573,69 +826,87 @@ static void form_density(Context& ctx, int n, int nocc, const double* C, double*
     gemm(ctx, false, true, n, n, nocc, 2.0, C, n, C, n, 0.0, P, n);
 }
 
-// small dense solve with partial pivoting (DIIS system, size <= 21)
-// The DIIS step on the device (one thread), so that the SCF iteration needs no
-// host round trip for it: Bd (nd x nd) keeps <e_k, e_l>; its row and column
-// `head` come from bvec (<e_k, e_head>, k < nhist).  The system
-// [[B / scale, -1], [-1, 0]] c = [0 .. 0, -1] is solved by Gaussian elimination
-// with partial pivoting; cvec receives the nhist coefficients, or selects the
-// newest Fock matrix alone when the system is singular.
-constexpr int DIIS_MAX = 20;  // the history length run_scf allows
-__global__ void diis_solve_kernel(int nd, int nhist, int head, double* __restrict__ Bd,
-                                  const double* __restrict__ bvec, double* __restrict__ cvec)
+// The DIIS step: e = Y - Y^T (the commutator F P S - S P F) into the history slot `head`,
+// its products with the nhist errors kept, and in the last block the DIIS system
+// [[B / scale, -1], [-1, 0]] c = [0 .. 0, -1], solved by Gaussian elimination with partial
+// pivoting by one warp (B, nd x nd, keeps <e_k, e_l> from one call to the next); c gets the
+// nhist coefficients, or selects the newest Fock matrix alone when the system is singular.
+constexpr int DIIS_MAX = RED_MAX;  // the history length run_scf allows
+__global__ void __launch_bounds__(RED_BLOCK) diis_error_kernel(int n, const double* __restrict__ Y, double* Eh, int nd,
+                                                               int nhist, int head, double* __restrict__ Bd,
+                                                               double* __restrict__ cvec, RedWork w)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int k = 0; k < nhist; k++) {
-        Bd[head * nd + k] = bvec[k];
-        Bd[k * nd + head] = bvec[k];
+    __shared__ double tot[DIIS_MAX];
+    __shared__ double A[DIIS_MAX + 1][DIIS_MAX + 2], x[DIIS_MAX + 1];
+    const int64_t nn = (int64_t)n * n;
+    double s[DIIS_MAX];
+#pragma unroll
+    for (int k = 0; k < DIIS_MAX; ++k) s[k] = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * RED_BLOCK + threadIdx.x; i < nn; i += (int64_t)gridDim.x * RED_BLOCK) {
+        const int r = (int)(i % n), c = (int)(i / n);
+        const double e = Y[i] - Y[c + (int64_t)r * n];
+        Eh[head * nn + i] = e;
+#pragma unroll
+        for (int k = 0; k < DIIS_MAX; ++k)
+            if (k < nhist) s[k] = fma(k == head ? e : Eh[k * nn + i], e, s[k]);
     }
-    const int m = nhist + 1;
-    double A[(DIIS_MAX + 1) * (DIIS_MAX + 1)], b[DIIS_MAX + 1];
+    if (!grid_sums(s, nhist, w, tot)) return;
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x, m = nhist + 1;
+    if (lane < nhist) {
+        Bd[head * nd + lane] = tot[lane];
+        Bd[lane * nd + head] = tot[lane];
+    }
+    __syncwarp();
     double scale = 0;
-    for (int a = 0; a < nhist; a++) scale = fmax(scale, fabs(Bd[a * nd + a]));
+    for (int k = 0; k < nhist; ++k) scale = fmax(scale, fabs(Bd[k * nd + k]));
     if (scale <= 0) scale = 1;
-    for (int a = 0; a < m; a++) {
-        for (int c = 0; c < m; c++) A[a * m + c] = 0.0;
-        b[a] = 0.0;
-    }
-    for (int a = 0; a < nhist; a++) {
-        for (int c = 0; c < nhist; c++) A[a * m + c] = Bd[a * nd + c] / scale;
-        A[a * m + nhist] = -1;
-        A[nhist * m + a] = -1;
-    }
-    b[nhist] = -1;
+    // lane = column; column m is the right-hand side
+    for (int r = 0; r < m; ++r)
+        if (lane <= m)
+            A[r][lane] = lane < nhist ? (r < nhist ? Bd[r * nd + lane] / scale : -1.0)
+                         : lane == nhist ? (r < nhist ? -1.0 : 0.0) : (r == nhist ? -1.0 : 0.0);
+    __syncwarp();
     bool ok = true;
-    for (int c = 0; c < m && ok; c++) {
+    for (int c = 0; c < m && ok; ++c) {
         int piv = c;
-        for (int r = c + 1; r < m; r++)
-            if (fabs(A[r * m + c]) > fabs(A[piv * m + c])) piv = r;
-        if (fabs(A[piv * m + c]) < 1e-300) {
-            ok = false;
-            break;
+        for (int r = c + 1; r < m; ++r)
+            if (fabs(A[r][c]) > fabs(A[piv][c])) piv = r;
+        if (fabs(A[piv][c]) < 1e-300) ok = false;
+        __syncwarp();
+        if (ok && lane <= m && piv != c) {
+            const double t = A[c][lane];
+            A[c][lane] = A[piv][lane];
+            A[piv][lane] = t;
         }
-        if (piv != c) {
-            for (int k = 0; k < m; k++) {
-                const double t = A[c * m + k];
-                A[c * m + k] = A[piv * m + k];
-                A[piv * m + k] = t;
+        __syncwarp();
+        if (ok)
+            for (int r = c + 1; r < m; ++r) {
+                const double f = A[r][c] / A[c][c];
+                __syncwarp();
+                if (lane >= c && lane <= m) A[r][lane] = fma(-f, A[c][lane], A[r][lane]);
+                __syncwarp();
             }
-            const double t = b[c];
-            b[c] = b[piv];
-            b[piv] = t;
-        }
-        for (int r = c + 1; r < m; r++) {
-            const double f = A[r * m + c] / A[c * m + c];
-            for (int k = c; k < m; k++) A[r * m + k] -= f * A[c * m + k];
-            b[r] -= f * b[c];
-        }
     }
-    if (ok)
-        for (int c = m - 1; c >= 0; c--) {
-            double sum = b[c];
-            for (int k = c + 1; k < m; k++) sum -= A[c * m + k] * b[k];
-            b[c] = sum / A[c * m + c];
+    if (ok && lane == 0)
+        for (int c = m - 1; c >= 0; --c) {
+            double v = A[c][m];
+            for (int k = c + 1; k < m; ++k) v = fma(-A[c][k], x[k], v);
+            x[c] = v / A[c][c];
         }
-    for (int k = 0; k < nd; k++) cvec[k] = ok ? (k < nhist ? b[k] : 0.0) : (k == head ? 1.0 : 0.0);
+    __syncwarp();
+    if (lane < nd) cvec[lane] = ok ? (lane < nhist ? x[lane] : 0.0) : (lane == head ? 1.0 : 0.0);
+}
+
+// out = sum_k c_k Fh_k over the nhist kept Fock matrices
+__global__ void diis_mix_kernel(int64_t nn, const double* __restrict__ Fh, const double* __restrict__ c, int nhist,
+                                double* __restrict__ out)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nn) return;
+    double s = 0.0;
+    for (int k = 0; k < nhist; ++k) s = fma(__ldg(c + k), Fh[k * nn + i], s);
+    out[i] = s;
 }
 
 constexpr int SP2_MIN = 8;  // smallest basis whose iteration densities come from purification by default
@@ -647,7 +918,13 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     const int64_t nn = (int64_t)n * n;
     HF_CHECK(in.nocc >= 0 && in.nocc <= n, HFGPU_ERR_INVALID, "nocc out of range");
     if (in.begin) in.begin(in.hook_user);
-    DBuf<double> G(nn, st), F(nn, st), Fw(nn, st), Sw(nn, st), Pold(nn, st), scal(4, st);
+    DBuf<double> G(nn, st), F(nn, st), Fw(nn, st), Sw(nn, st), Pold(nn, st), partial(RED_MAX_BLOCKS * RED_MAX, st);
+    DBuf<unsigned> redcount(1, st);
+    redcount.zero();
+    const RedWork red{partial.p, redcount.p};
+    const unsigned rb = red_blocks(nn);
+    DBuf<ScfReport> rep(1, st);
+    ScfReport* h = (ScfReport*)ctx.pinned(Context::PIN_SCF, sizeof(ScfReport));
     DBuf<int> info(1, st);
     info.zero();  // written by dsygvd; the own eigensolver reports errors by exception
     if (in.dP0)
@@ -661,12 +938,11 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
 
     const bool diis = in.accel == HFGPU_SCF_DIIS;
     const int nd = std::max(2, std::min(in.diis_size, 20));
-    DBuf<double> Fh, Eh, Y, bvec, cvec, Bd;
+    DBuf<double> Fh, Eh, Y, cvec, Bd;
     if (diis) {
         Fh.alloc((size_t)nd * nn, st);
         Eh.alloc((size_t)nd * nn, st);
         Y.alloc(nn, st);
-        bvec.alloc(nd, st);
         cvec.alloc(nd, st);
         Bd.alloc((size_t)nd * nd, st);
         Bd.zero();
@@ -678,7 +954,7 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     Purifier pur;
     Eigh eig;
     const bool own_eigh = in.eigensolver == 0 && Eigh::supported(ctx, n);
-    if (in.purify || own_eigh) pur.setup(ctx, n, in.nocc, in.dS);
+    if (in.purify || own_eigh) pur.setup(ctx, n, in.nocc, in.dS, rep.p, h);
     if (own_eigh) eig.setup(ctx, n);
     const double* Xorth = pur.X.p;
     // Densities of the iterations: with the own eigensolver they too come from FP64
@@ -707,12 +983,12 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
 
     std::vector<double> Escf;
     ScfOut out;
-    // incremental Fock builds: Gacc = G(Pacc); each iteration adds G(P - Pacc)
+    // incremental Fock builds: Gacc = G(Pold); each iteration adds G(P - Pold)
     const bool inc = in.direct_jk && in.inc_screen > 0;
-    DBuf<double> Gacc, Pacc;
+    DBuf<double> Gacc, D;
     if (inc) {
         Gacc.alloc(nn, st);
-        Pacc.alloc(nn, st);
+        D.alloc(nn, st);
     }
     // near convergence (dP < 100 tolP) every build is a full one, so the last
     // iterations converge exactly like the full-build SCF
@@ -724,58 +1000,50 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     if (in.end) in.end(in.hook_user);
     for (int it = 1; it <= in.nscf; ++it) {
         const double* Gcur = G.p;
+        double* acc = nullptr;
         if (inc) {
             last_full = it == 1 || endgame || since_full >= in.inc_rebuild;
             if (last_full) {
                 in.direct_jk(ctx, in.direct_ctx, dP, Gacc.p, 0.0);
+                Gcur = Gacc.p;
                 since_full = 0;
             } else {
-                sub_kernel<<<nblk(nn), 256, 0, st>>>(nn, dP, Pacc.p, Pacc.p);  // Pacc <- P - Pacc
-                count_launch();
-                in.direct_jk(ctx, in.direct_ctx, Pacc.p, G.p, in.inc_screen);
-                add_kernel<<<nblk(nn), 256, 0, st>>>(nn, Gacc.p, G.p, Gacc.p);
-                count_launch();
+                in.direct_jk(ctx, in.direct_ctx, D.p, G.p, in.inc_screen);
+                acc = Gacc.p;
                 ++since_full;
             }
-            HF_CUDA(cudaMemcpyAsync(Pacc.p, dP, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
-            Gcur = Gacc.p;
         } else if (in.direct_jk) {
             in.direct_jk(ctx, in.direct_ctx, dP, G.p, 0.0);
         } else {
             jk_from_packed(ctx, n, in.d_int2, dP, G.p);
         }
         ctx.trace_mark("fock");
-        add_kernel<<<nblk(nn), 256, 0, st>>>(nn, in.dH, Gcur, F.p);
-        count_launch();
-        reduce(ctx, 0, nn, dP, in.dH, F.p, scal.p);  // E0
-        const double* Fsolve = F.p;
         // the first iteration of a P = 0 start has a commutator that vanishes
         // trivially: keep it out of the DIIS history
-        if (diis && (it >= 2 || in.dP0)) {
-            const double one = 1.0, zero = 0.0;
+        const bool extrapolate = diis && (it >= 2 || in.dP0);
+        fock_kernel<<<rb, RED_BLOCK, 0, st>>>(nn, in.dH, Gcur, acc, dP, F.p, extrapolate ? Fh.p + head * nn : nullptr,
+                                              Pold.p, red, rep.p);
+        count_launch();
+        HF_CUDA(cudaGetLastError());
+        const double* Fsolve = F.p;
+        if (extrapolate) {
             // error = F P S - S P F = Y - Y^T with Y = F P S
             gemm(ctx, false, false, n, n, n, 1.0, F.p, n, dP, n, 0.0, G.p, n);
             gemm(ctx, false, false, n, n, n, 1.0, G.p, n, in.dS, n, 0.0, Y.p, n);
-            double* ek = Eh.p + (size_t)head * nn;
-            comm_kernel<<<nblk(nn), 256, 0, st>>>(n, Y.p, ek);
-            count_launch();
-            HF_CUDA(cudaMemcpyAsync(Fh.p + (size_t)head * nn, F.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
             nhist = std::min(nhist + 1, nd);
-            // new row of B: <e_k, e_head>; the DIIS system is solved on the device
-            HF_CUBLAS(cublasDgemv(ctx.blas, CUBLAS_OP_T, (int)nn, nd, &one, Eh.p, (int)nn, ek, 1, &zero, bvec.p, 1));
-            diis_solve_kernel<<<1, 32, 0, st>>>(nd, nhist, head, Bd.p, bvec.p, cvec.p);
+            diis_error_kernel<<<rb, RED_BLOCK, 0, st>>>(n, Y.p, Eh.p, nd, nhist, head, Bd.p, cvec.p, red);
             count_launch();
             HF_CUDA(cudaGetLastError());
             ctx.trace_mark("diis error");
             if (nhist >= 2) {
-                HF_CUBLAS(cublasDgemv(ctx.blas, CUBLAS_OP_N, (int)nn, nhist, &one, Fh.p, (int)nn, cvec.p, 1, &zero,
-                                      Y.p, 1));
+                diis_mix_kernel<<<nblk(nn), 256, 0, st>>>(nn, Fh.p, cvec.p, nhist, Y.p);
+                count_launch();
+                HF_CUDA(cudaGetLastError());
                 Fsolve = Y.p;
             }
             head = (head + 1) % nd;
             ctx.trace_mark("diis extrap");
         }
-        HF_CUDA(cudaMemcpyAsync(Pold.p, dP, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
         if (sp2_density) {
             // with the purify option, FP32 steps while the density is still far from converged
             pur.density(ctx, Fsolve, dP, in.purify && it > 1 && !endgame && last_dP > 1e-4);
@@ -786,25 +1054,28 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
         }
         last_F = Fsolve;
         ctx.trace_mark("density");
-        reduce(ctx, 1, nn, dP, Pold.p, nullptr, scal.p + 1);  // dP
-        double h[2];
+        auto report = [&] {  // dP, and everything the host reads of this iteration
+            density_change_kernel<<<rb, RED_BLOCK, 0, st>>>(nn, dP, Pold.p, inc ? D.p : nullptr, red, rep.p);
+            count_launch();
+            HF_CUDA(cudaGetLastError());
+            HF_CUDA(cudaMemcpyAsync(h, rep.p, sizeof(ScfReport), cudaMemcpyDeviceToHost, st));
+        };
+        report();
         int hinfo = 0;
-        scal.download(h, 2);
-        info.download(&hinfo, 1);
+        if (!own_eigh) info.download(&hinfo, 1);  // dsygvd's; the own eigensolver throws
         HF_CUDA(cudaStreamSynchronize(st));
         if (sp2_density && !pur.converged(!in.purify)) {
             HF_CHECK(!in.purify, HFGPU_ERR_LINALG, "density purification did not converge (no gap?)");
             eigh(Fsolve, Fw.p, in.nocc);
             form_density(ctx, n, in.nocc, Fw.p, dP);
-            reduce(ctx, 1, nn, dP, Pold.p, nullptr, scal.p + 1);
-            scal.download(h, 2);
+            report();
             HF_CUDA(cudaStreamSynchronize(st));
         }
         ctx.trace_mark("convergence");
         HF_CHECK(hinfo == 0, HFGPU_ERR_LINALG,
                  "eigh: dsygvd returned info = " + std::to_string(hinfo) +
                      (hinfo > n ? " (S is not positive definite)" : ""));
-        const double E0 = h[0], dPv = h[1];
+        const double E0 = h->E0, dPv = h->dP;
         last_dP = dPv;
         if (dPv < 100 * in.tolP) endgame = true;
         Escf.push_back(E0);
@@ -835,7 +1106,7 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
             }
         }
         if (!diis && in.alpha != 1.0) {
-            mix_kernel<<<nblk(nn), 256, 0, st>>>(nn, in.alpha, Pold.p, dP);
+            mix_kernel<<<nblk(nn), 256, 0, st>>>(nn, in.alpha, Pold.p, dP, inc ? D.p : nullptr);
             count_launch();
         }
     }
@@ -852,8 +1123,12 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
 
 double device_dot(Context& ctx, int64_t nn, const double* A, const double* B)
 {
-    DBuf<double> s(1, ctx.stream);
-    reduce(ctx, 2, nn, A, B, nullptr, s.p);
+    DBuf<double> s(1, ctx.stream), partial(RED_MAX_BLOCKS * RED_MAX, ctx.stream);
+    DBuf<unsigned> count(1, ctx.stream);
+    count.zero();
+    dot_kernel<<<red_blocks(nn), RED_BLOCK, 0, ctx.stream>>>(nn, A, B, RedWork{partial.p, count.p}, s.p);
+    count_launch();
+    HF_CUDA(cudaGetLastError());
     double h = 0;
     s.download(&h, 1);
     HF_CUDA(cudaStreamSynchronize(ctx.stream));
