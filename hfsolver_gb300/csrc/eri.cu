@@ -168,10 +168,10 @@ static float elapsed(cudaEvent_t a, cudaEvent_t b)
     return ms;
 }
 
-// lanes per quartet for kb x kk primitive quartets: enough independent work per
+// lanes per quartet for kprod primitive quartets: enough independent work per
 // lane (between target and 2 target primitive quartets) without idling the rest
 // of the warp
-static int pick_split(int64_t kprod, int target = 16)
+static int pick_split(int64_t kprod, int target)
 {
     int s = 1;
     while (s < 32 && kprod >= 2 * (int64_t)target * s) s <<= 1;
@@ -183,6 +183,61 @@ static int class_G(int tb, int tk)
     int nab = ncart(ptype_la(tb)) * ncart(ptype_lb(tb));
     int ncd = ncart(ptype_la(tk)) * ncart(ptype_lb(tk));
     return ncd / pick_ncd(nab, ncd);
+}
+
+// FP64 instructions of one primitive quartet in one ket chunk's warp: Boys values
+// and R recursion, the chunk's ket sums, their contraction with the bra
+static double chunk_instr(int tb, int tk)
+{
+    const int la = ptype_la(tb), lb = ptype_lb(tb), lc = ptype_la(tk), ld = ptype_lb(tk);
+    const int L = la + lb + lc + ld, ncdt = ncart(lc) * ncart(ld), ncd = pick_ncd(ncart(la) * ncart(lb), ncdt);
+    const double r = (L + 4) * (L + 3) * (L + 2) * (L + 1) / 24.0;  // sum of nherm(l), l <= L
+    return 50 + 1.5 * r + (double)ncd / ncdt * ne_pair(lc, ld) * nherm(la + lb) + ncd * ne_pair(la, lb);
+}
+
+// lanes per quartet of a segment of class (tb, tk): the full-GPU rule's, or more
+// (lanes_in_budget)
+static int split_in_budget(int tb, int tk, int64_t kprod, double budget)
+{
+    const int nab = ncart(ptype_la(tb)) * ncart(ptype_lb(tb));
+    const int sums = nab * pick_ncd(nab, ncart(ptype_la(tk)) * ncart(ptype_lb(tk)));
+    const double instr = chunk_instr(tb, tk);
+    return lanes_in_budget(pick_split(kprod, 16), kprod, budget, [&](int s) {
+        return (double)((kprod + s - 1) / s) * instr + LANE_SUM_INSTR * sums * std::log2((double)s);
+    });
+}
+
+// the budget of a set of classes launched side by side
+static double lane_budget(const Context& ctx, const std::vector<ClassPlan>& classes)
+{
+    double work = 0;
+    for (const ClassPlan& c : classes)
+        for (size_t i = 0; i < c.segs.size(); ++i)
+            work += (double)c.segs[i].nq * c.kprod[i] * class_G(c.tb, c.tk) * chunk_instr(c.tb, c.tk) / 32;
+    return LANE_BUDGET * work / (4.0 * ctx.num_sms);
+}
+
+// lay the warps of a class out, for `target` primitive quartets per lane or by the
+// budget (target 0)
+static void layout_class(Context& ctx, ClassPlan& c, int target, double budget)
+{
+    const int G_ = class_G(c.tb, c.tk);
+    c.nwarps = 0;
+    for (size_t i = 0; i < c.segs.size(); ++i) {
+        Seg& s = c.segs[i];
+        s.split = target > 0 ? pick_split(c.kprod[i], target) : split_in_budget(c.tb, c.tk, c.kprod[i], budget);
+        s.warp0 = c.nwarps;
+        const int64_t qpw = 32 / s.split;
+        c.nwarps += (s.nq + qpw - 1) / qpw * G_;
+    }
+    // the kernels index quartets, warps and prefix sums of a class in 32 bits
+    HF_CHECK(c.nq < (1ll << 31) && c.nwarps < (1ll << 30), HFGPU_ERR_UNSUPPORTED,
+             "quartet class too large for 32-bit indexing");
+    if (c.dsegs.p)
+        c.dsegs.upload(c.segs.data(), c.segs.size());
+    else
+        c.dsegs = to_device(c.segs, ctx.stream);
+    c.lane_target = target;
 }
 
 // McMurchie-Davidson reference flop count of one primitive quartet:
@@ -240,7 +295,7 @@ static std::vector<float> round_up_f32(const std::vector<double>& v)
     return f;
 }
 
-EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
+EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr, bool fixed_lanes)
 {
     cudaStream_t st = ctx.stream;
     auto P = new EriPlan();
@@ -308,34 +363,27 @@ EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
             std::vector<int2> dl;
             std::vector<ClassPlan> dcls;
             for (auto& g : gmap) {
-                int t = g.first.first;
-                ClassPlan c;
-                c.tb = t; c.tk = t;
-                Seg s{};
-                s.warp0 = 0; s.nq = (int64_t)g.second.size(); s.pref0 = (int64_t)dl.size();
-                s.list = 1;
-                s.qoff = 0;
-                s.split = pick_split((int64_t)g.first.second * g.first.second);
-                const int64_t qpw = 32 / s.split;
-                for (int id : g.second) dl.push_back(make_int2(id, id));
-                bool merged = false;
-                for (auto& dc : dcls)
-                    if (dc.tb == t) {
-                        s.warp0 = dc.nwarps;
-                        dc.segs.push_back(s);
-                        dc.nwarps += (s.nq + qpw - 1) / qpw * class_G(t, t);
-                        merged = true;
-                    }
-                if (!merged) {
-                    c.segs.push_back(s);
-                    c.nwarps = (s.nq + qpw - 1) / qpw * class_G(t, t);
+                const int t = g.first.first;
+                if (dcls.empty() || dcls.back().tb != t) {  // gmap: one type after the other
+                    ClassPlan c;
+                    c.tb = c.tk = t;
                     dcls.push_back(std::move(c));
                 }
+                ClassPlan& c = dcls.back();
+                Seg s{};
+                s.nq = (int64_t)g.second.size();
+                s.pref0 = (int64_t)dl.size();
+                s.list = 1;
+                c.segs.push_back(s);
+                c.kprod.push_back((int64_t)g.first.second * g.first.second);
+                c.nq += s.nq;
+                for (int id : g.second) dl.push_back(make_int2(id, id));
             }
+            const double budget = lane_budget(ctx, dcls);
             DBuf<int2> ddl = to_device(dl, st);
             DBuf<double> diag((size_t)P->npair * 36, st);
             diag.zero();
-            for (auto& c : dcls) c.dsegs = to_device(c.segs, st);
+            for (auto& c : dcls) layout_class(ctx, c, 0, budget);
             // one small class per pair type, each latency-bound: side by side
             ctx.fork();
             for (size_t i = 0; i < dcls.size(); ++i)
@@ -384,7 +432,6 @@ EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
             for (int tk = tb; tk < NPTYPE; tk++) {
                 ClassPlan c;
                 c.tb = tb; c.tk = tk;
-                int G_ = class_G(tb, tk);
                 double fl = md_flops(ptype_la(tb), ptype_lb(tb), ptype_la(tk), ptype_lb(tk));
                 for (size_t g1 = 0; g1 < groups.size(); g1++) {
                     if (groups[g1].t != tb) continue;
@@ -423,13 +470,9 @@ EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
                             continue;
                         }
                         s.nq = acc;
-                        s.warp0 = c.nwarps;
                         s.qoff = c.nq;
-                        s.split = pick_split((int64_t)A_.k * B_.k);
                         c.kprod.push_back((int64_t)A_.k * B_.k);
-                        const int64_t qpw = 32 / s.split;
                         c.nq += acc;
-                        c.nwarps += (acc + qpw - 1) / qpw * G_;
                         c.segs.push_back(s);
                         stt.n_quartets += acc;
                         stt.n_bf_quartets += nbf;
@@ -437,14 +480,11 @@ EriPlan* eri_plan_create(Context& ctx, const Basis& b, double thr)
                         stt.flops += (double)acc * A_.k * B_.k * fl;
                     }
                 }
-                if (!c.segs.empty()) {
-                    // the kernels index quartets, warps and prefix sums of a class in 32 bits
-                    HF_CHECK(c.nq < (1ll << 31) && c.nwarps < (1ll << 30), HFGPU_ERR_UNSUPPORTED,
-                             "quartet class too large for 32-bit indexing");
-                    c.dsegs = to_device(c.segs, st);
-                    P->classes.push_back(std::move(c));
-                }
+                if (!c.segs.empty()) P->classes.push_back(std::move(c));
             }
+        P->fixed_lanes = fixed_lanes;
+        P->lane_budget = fixed_lanes ? INFINITY : lane_budget(ctx, P->classes);
+        for (ClassPlan& c : P->classes) layout_class(ctx, c, 0, P->lane_budget);
         P->prefix = to_device(prefix, st);
         P->h_prefix = prefix;
         P->nmol = 1;
@@ -708,45 +748,29 @@ static int block_size(int tb, int tk)
     return ncart(ptype_la(tb)) * ncart(ptype_lb(tb)) * ncart(ptype_la(tk)) * ncart(ptype_lb(tk));
 }
 
-// lay the warps of a class out again for another lanes-per-quartet target
-static void layout_class(Context& ctx, ClassPlan& c, int target)
-{
-    const int G_ = class_G(c.tb, c.tk);
-    c.nwarps = 0;
-    for (size_t i = 0; i < c.segs.size(); ++i) {
-        Seg& s = c.segs[i];
-        s.split = pick_split(c.kprod[i], target);
-        s.warp0 = c.nwarps;
-        const int64_t qpw = 32 / s.split;
-        c.nwarps += (s.nq + qpw - 1) / qpw * G_;
-    }
-    HF_CHECK(c.nwarps < (1ll << 30), HFGPU_ERR_UNSUPPORTED, "quartet class too large for 32-bit indexing");
-    c.dsegs.upload(c.segs.data(), c.segs.size());
-    c.lane_target = target;
-}
-
-// The ERI launch of a class with the tuned lanes-per-quartet target.  On the
-// first molecule of a (class, size bucket) with tuning on, every candidate
-// target is timed on the real launch (the class writes the same values each
-// time) and the fastest is recorded.
-// the class's lanes-per-quartet layout: tuned once per (class, size bucket) by
-// timing the candidates on the main stream, then laid out for the winner
+// The class's lanes-per-quartet layout: by the plan's budget, or with tuning on the
+// fastest target.  On the first molecule of a (class, size bucket) every candidate is
+// timed on the real launch (the class writes the same values each time) and the
+// choice recorded: the built-in layout (0), unless another target gains more than a
+// twentieth (alone on the GPU a class likes more lanes than beside the others: 8
+// waters take 7.8 ms built in, 8.1 with each class's fastest).
 static void eri_class_layout(Context& ctx, EriPlan* P, ClassPlan& c, double* d_out, double* blocks)
 {
-    int target = 16;
-    if (ctx.tune && c.nq > 0) {
+    int target = 0;
+    if (ctx.tune && !P->fixed_lanes && c.nq > 0) {
         const int bucket = tune_bucket(c.nq);
         if (!tune_get(TUNE_ERI, c.tb, c.tk, bucket, &target)) {
             cudaEvent_t a, b;
             HF_CUDA(cudaEventCreate(&a));
             HF_CUDA(cudaEventCreate(&b));
+            launch_class(ctx, P, c, MODE_PACKED, d_out, nullptr, blocks);  // warm
             float best = 1e30f;
-            for (int cand : {4, 8, 16, 32, 64}) {
-                layout_class(ctx, c, cand);
+            for (int cand : {0, 4, 8, 16, 32, 64}) {
+                layout_class(ctx, c, cand, P->lane_budget);
                 HF_CUDA(cudaEventRecord(a, ctx.stream));
                 launch_class(ctx, P, c, MODE_PACKED, d_out, nullptr, blocks);
                 HF_CUDA(cudaEventRecord(b, ctx.stream));
-                const float ms = elapsed(a, b);
+                const float ms = elapsed(a, b) * (cand ? 1.05f : 1.0f);
                 if (ms < best) {
                     best = ms;
                     target = cand;
@@ -757,7 +781,7 @@ static void eri_class_layout(Context& ctx, EriPlan* P, ClassPlan& c, double* d_o
             tune_set(TUNE_ERI, c.tb, c.tk, bucket, target);
         }
     }
-    if (c.lane_target != target) layout_class(ctx, c, target);
+    if (c.lane_target != target) layout_class(ctx, c, target, P->lane_budget);
 }
 
 // The ERI pass in two halves: eri_compute_start tunes and lays out the classes
@@ -934,11 +958,10 @@ EriPlan* eri_plan_merge(Context& ctx, const std::vector<EriPlan*>& plans)
                         }
                     }
                 if (c.segs.empty()) continue;
-                HF_CHECK(c.nq < (1ll << 31), HFGPU_ERR_UNSUPPORTED, "quartet class too large for 32-bit indexing");
-                c.dsegs = to_device(c.segs, st);
-                layout_class(ctx, c, 16);
                 M->classes.push_back(std::move(c));
             }
+        M->lane_budget = lane_budget(ctx, M->classes);
+        for (ClassPlan& c : M->classes) layout_class(ctx, c, 0, M->lane_budget);
         HF_CUDA(cudaStreamSynchronize(st));
         return M;
     } catch (...) {

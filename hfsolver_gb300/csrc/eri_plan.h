@@ -14,13 +14,33 @@ struct ClassPlan {
     int tb, tk;
     std::vector<Seg> segs;
     std::vector<int64_t> kprod;  // primitive quartets per quartet, per segment
-    int lane_target = 16;        // primitive quartets per lane that the splits were laid out for
+    int lane_target = 0;         // primitive quartets per lane that the splits were laid out for (0: by lane_budget)
     int64_t nwarps = 0;
     int64_t nq = 0;     // quartets of the class
     int64_t boff = 0;   // offset of the class's blocks in EriPlan::blocks
     int64_t qbase = 0;  // offset of the class's quartets in EriPlan::qlist
     DBuf<Seg> dsegs;
 };
+
+// Lanes per quartet: from s on, doubled while the quartet's serial chain (chain(s):
+// FP64 instructions in a row with s lanes, sums over the lanes included) is over the
+// budget and gets shorter by it.  The budget is a share of the launches' FP64 work
+// per pipe: an instruction holds a pipe for 64 clocks whatever its lanes do, so a
+// chain that is short against the whole pass costs nothing, and a longer one is the
+// time of the pass.  Every doubling costs sums over lanes and idle lanes, so a pass
+// that fills the GPU keeps s.  Measured (ms, with 16 to 32 primitive quartets a lane
+// at every size, then so): ERI of 1, 2, 3, 4 and 8 waters 0.83, 0.90, 1.11, 1.6, 7.8
+// and 0.21, 0.36, 0.70, 1.36, 7.8; gradient of 1, 2, 3 and 9 waters 2.55, 2.38, 3.59,
+// 52.8 and 0.73, 1.46, 3.27, 52.8.  Shares of 0.06 and 0.5: ERI of 3 waters 0.73 and
+// 0.83, gradient of 2 waters 1.76 and 2.02.
+constexpr double LANE_BUDGET = 0.2;     // share of the pass's work per FP64 pipe
+constexpr double LANE_SUM_INSTR = 1.6;  // a shuffle and add of one value, in FP64 instructions (105 clocks)
+template <class Chain>
+int lanes_in_budget(int s, int64_t nprim, double budget, Chain&& chain)
+{
+    while (s < 32 && s < nprim && chain(s) > budget && chain(2 * s) < chain(s)) s <<= 1;
+    return s;
+}
 
 struct EriPlan {
     Basis basis;
@@ -40,6 +60,8 @@ struct EriPlan {
     DBuf<int> gpairs;
     DBuf<int64_t> prefix;
     std::vector<ClassPlan> classes;
+    double lane_budget = 0;    // of the plan's classes, in FP64 instructions (lanes_in_budget)
+    bool fixed_lanes = false;  // lanes per quartet by primitive counts alone, never tuned
     DBuf<double> blocks;  // class-wise quartet blocks, kept for the SCF's Fock builds
     DBuf<int2> qlist;     // (bra, ket) pair ids of every kept quartet, class by class
     DBuf<int> pair_mol;   // batched plans: the molecule of every pair

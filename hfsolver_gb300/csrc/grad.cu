@@ -407,13 +407,33 @@ static GradKernelFn get_grad_kernel(int tb, int tk, bool withp)
     return table[tb][tk](withp);
 }
 
+// FP64 instructions of the ordered class (tb | tk) in one ket chunk's warp: a
+// primitive quartet's ket sums, and the contraction of one bra primitive pair
+struct GradInstr {
+    double prim, contract;
+    GradInstr(int tb, int tk)
+    {
+        const int la = ptype_la(tb), lb = ptype_lb(tb), lc = ptype_la(tk), ld = ptype_lb(tk);
+        const int L = la + lb + lc + ld + 1, ncdt = ncart(lc) * ncart(ld), ncd = grad_ncd(tb, tk);
+        const double r = (L + 4) * (L + 3) * (L + 2) * (L + 1) / 24.0;  // sum of nherm(l), l <= L
+        prim = 50 + 1.5 * r + (double)ncd / ncdt * ne_pair(lc, ld) * nherm(la + lb + 1);
+        contract = 6.0 * ncd * ne_pair(la, lb);
+    }
+};
+
 // lanes per quartet: enough primitive quartets per lane (16 to 32), so that a
-// quartet with many primitives does not hold its warp long after the others
-static int grad_split(int kb, int kk)
+// quartet with many primitives does not hold its warp long after the others, or more
+// (lanes_in_budget)
+static int grad_split(int kb, int kk, const GradInstr& in, double budget)
 {
     int s = 1;
     while (s < 32 && (int64_t)kb * kk >= 2 * 16 * (int64_t)s) s <<= 1;
-    return s;
+    return lanes_in_budget(s, (int64_t)kb * kk, budget, [&](int s) {
+        const int nkc = s > kb ? (s + kb - 1) / kb : 1;  // slices of the ket primitives (grad_quartet)
+        const int items = (kb * nkc + s - 1) / s;
+        return items * (double)((kk + nkc - 1) / nkc) * in.prim + items * in.contract +
+               6 * LANE_SUM_INSTR * std::log2((double)s);
+    });
 }
 
 // the max dynamic shared memory of the kernels that have been raised so far
@@ -472,6 +492,18 @@ void eri_gradient(Context& ctx, EriPlan* P, const double* dP, double* d_grad, fl
     };
     std::vector<Launch> launches;
     std::vector<Seg> segs;
+    double budget = 0;
+    for (const ClassPlan& c : P->classes)
+        for (int side = 0; side < 2; ++side) {
+            const int tb = side == 0 ? c.tb : c.tk, tk = side == 0 ? c.tk : c.tb;
+            const int G = ncart(ptype_la(tk)) * ncart(ptype_lb(tk)) / grad_ncd(tb, tk);
+            const GradInstr in(tb, tk);
+            for (const Seg& s : c.segs) {
+                const int kbra = P->pK[P->h_gpairs[s.bra0]], kket = P->pK[P->h_gpairs[s.ket0]];
+                budget += (double)s.nq * G * (kbra * kket * in.prim + (side == 0 ? kbra : kket) * in.contract) / 32;
+            }
+        }
+    budget *= LANE_BUDGET / (4.0 * ctx.num_sms);
     for (int i = (int)P->classes.size() - 1; i >= 0; --i) {
         const ClassPlan& c = P->classes[i];
         if (c.nq == 0) continue;
@@ -489,7 +521,8 @@ void eri_gradient(Context& ctx, EriPlan* P, const double* dP, double* d_grad, fl
                 HF_CHECK(s0.list == 0, HFGPU_ERR_UNSUPPORTED, "gradient expects prefix-mode segments");
                 Seg s = s0;
                 const int kbra = P->pK[P->h_gpairs[s0.bra0]], kket = P->pK[P->h_gpairs[s0.ket0]];
-                s.split = side == 0 ? grad_split(kbra, kket) : grad_split(kket, kbra);
+                const GradInstr in(tb, tk);
+                s.split = side == 0 ? grad_split(kbra, kket, in, budget) : grad_split(kket, kbra, in, budget);
                 s.warp0 = l.nwarps;
                 const int64_t qpw = 32 / s.split;
                 l.nwarps += (s.nq + qpw - 1) / qpw * G;

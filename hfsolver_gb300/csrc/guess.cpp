@@ -36,12 +36,14 @@ static std::vector<double> atom_density(Context& ctx, int Z)
     cudaStream_t st = ctx.stream;
     DBuf<double> dS(nn, st), dT(nn, st), dV(nn, st), dH(nn, st);
     const double zero = 0.0;
-    onee_compute(ctx, b, 1, &Z, &zero, &zero, &zero, dS.p, dT.p, dV.p);
+    // fixed orders of summation: which of an open p level's orbitals are filled is up to
+    // rounding, and the guess should not depend on launch shapes
+    onee_compute(ctx, b, 1, &Z, &zero, &zero, &zero, dS.p, dT.p, dV.p, nullptr, true);
     const double one = 1.0;
     HF_CUBLAS(cublasDgeam(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, n, n, &one, dT.p, n, &one, dV.p, n, dH.p, n));
     DBuf<double> dI(packed_size(n), st);
     dI.zero();
-    std::unique_ptr<EriPlan, void (*)(EriPlan*)> plan(eri_plan_create(ctx, b, 0.0), eri_plan_destroy);
+    std::unique_ptr<EriPlan, void (*)(EriPlan*)> plan(eri_plan_create(ctx, b, 0.0, true), eri_plan_destroy);
     eri_compute_packed(ctx, plan.get(), dI.p, nullptr);
     const int nel = (Z % 2 == 0 || Z == 1) ? Z : Z - 1;  // closed shell: the atom, or its cation
     ScfIn in;

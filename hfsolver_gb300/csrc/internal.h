@@ -227,7 +227,8 @@ class EriEngine;  // eri.cu
 
 // Device-side basis + shell pairs + screened quartet segments for one molecule.
 struct EriPlan;
-EriPlan* eri_plan_create(Context& ctx, const Basis& b, double schwarz);
+// fixed_lanes: sums in an order that depends on the basis alone, not on the GPU's size or tuning
+EriPlan* eri_plan_create(Context& ctx, const Basis& b, double schwarz, bool fixed_lanes = false);
 void eri_plan_destroy(EriPlan* p);
 EriStats eri_plan_stats(const EriPlan* p);
 // all unique (ij|kl) into the packed array d_out (device, zeroed by the caller)
@@ -249,7 +250,8 @@ float screen_f32(double s);
 // (on: the stream to run on, ctx.stream if null; the results are ready in stream
 // order there, the host does not wait)
 void onee_compute(Context& ctx, const Basis& b, int natoms, const int* atno, const double* x,
-                  const double* y, const double* z, double* dS, double* dT, double* dV, cudaStream_t on = nullptr);
+                  const double* y, const double* z, double* dS, double* dT, double* dV, cudaStream_t on = nullptr,
+                  bool fixed_lanes = false);
 
 // J/K (jk.cu): G = J - K/2 from packed integrals and density P (device)
 void jk_from_packed(Context& ctx, int n, const double* d_int2, const double* dP, double* dG);

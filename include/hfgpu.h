@@ -301,9 +301,9 @@ int hfgpu_rhf_batch(int nmol, const int *natoms, const int *atno, const double *
 
 /* The autotuner's table as text, one line per tuned (kernel, quartet class,
  * size bucket): "<eri|digest> <bra pair type> <ket pair type> <log2 quartets>
- * <choice>" (choice: primitive quartets per lane for eri, row splits for
- * digest).  Writes at most len bytes including the terminating NUL and returns
- * the length of the whole text. */
+ * <choice>" (choice: primitive quartets per lane for eri, 0 for the built-in
+ * layout; row splits for digest).  Writes at most len bytes including the
+ * terminating NUL and returns the length of the whole text. */
 int64_t hfgpu_autotune_table(char *buf, int64_t len);
 /* forget every tuned shape */
 void hfgpu_autotune_clear(void);
