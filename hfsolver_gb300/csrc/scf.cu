@@ -85,9 +85,18 @@ struct Sp2Sync {
     int err, steps;
     double trace;  // tr X of the result
 };
+// the course of an FP64 purification from F: X_0 = shift I - scale F; dif = ||F - Fprev||_F
+// where there is an Fprev; per step w = tr(X - X^2)
+// and tr X before it, and its stretch alpha (negative: a 2X - X^2 step)
+constexpr int SP2_LOG = 64;
+struct Sp2Log {
+    double scale, shift, dif, alpha[SP2_LOG];
+    long long w[SP2_LOG], tr[SP2_LOG];  // in units of 2^-50
+};
 struct ScfReport {
     double E0, dP;
     Sp2Sync sp2[2];  // density purification: [0] FP32, [1] FP64
+    Sp2Log log;
 };
 
 // F = H + G (with acc: G is added to the running acc first, F = H + acc), F's copy in the
@@ -233,7 +242,7 @@ struct __align__(16) Sp2Slot {
     long long a, c;
 };
 struct __align__(16) Sp2Bounds {
-    double tr, nrm, lo, hi;
+    double tr, nrm, lo, hi, dif, pad;
 };
 // The shares are summed as integers: a warp-wide FP64 add holds its sub-partition's pipe
 // 64 cycles and a shuffle sum of two doubles takes a thousand, a third of a step.  (|X| <= 1
@@ -255,6 +264,17 @@ enum { SP2_FROM_F = 0, SP2_FROM_F32 = 1 };
 // and the number of k-slices ks each output's dot product is split into (their partial
 // sums meet in shared memory) are chosen so that the FP64 work spreads evenly over the SMs
 // and over each SM's four sub-partitions (sp2_shape).
+// Stretched steps: of an earlier F (Fprev) the last occupied energy is known to be at most
+// homo and the first virtual one at least lumo (sp2_gap); F's are within ||F - Fprev||_F
+// of them.  With the virtual states' X in [0, l] and the occupied ones' in [1 - m, 1], the
+// square of a X + (1 - a) I, a = 2 / (2 - l), maps 0 and l to the same (l / (2 - l))^2
+// where X^2 leaves l^2, and keeps the order and [0, 1]; I - (I - a X)^2, a = 2 / (2 - m),
+// does the same for the holes.  The larger of l and m is taken until both are below
+// SP2_STRETCH; the plain recursion ends the work.  l, m and a are one thread's work while
+// the block waits at the barrier.  (Rubensson, J. Chem. Theory Comput. 7, 1233 (2011).)
+// Steps of a density: 28 plain and 19 stretched (1 water, from the eleventh of 48
+// iterations on), 30 and 19 (6 waters), 31 and 18 (16 waters); all FP64 purifications of an
+// SCF of 1, 6, 9 and 16 waters 5.8, 9.9, 20.0 and 23.4 ms plain, 4.9, 8.8, 17.3 and 17.1 so.
 // Once tr(X - X^2) < tol_idem the recursion takes `polish` (0 or 2) more steps, one
 // square and one 2X - X^2: an occupation 1 - d goes to 1 - 2d and 1 - 4d^2 (or 1 - d^2
 // and 1 - 2d^2), one at d to the mirror image, so a sum of 1e-7 left by the test ends
@@ -264,7 +284,8 @@ enum { SP2_FROM_F = 0, SP2_FROM_F32 = 1 };
 // instruction outside the dot products (sums, tests) lengthens it by 64 cycles.  Per
 // purification of 28 steps, with the bounds and X_0 in a chain of small kernels before:
 // 25 functions 0.154 -> 0.11 ms, 50: 0.20 -> 0.14, 150: 0.54 -> 0.38; the 17 densities of
-// an 8-water SCF (8 of them FP32 first) 7.4 -> 5.3 ms, the 18 of 16 waters 31.3 -> 26.7.
+// an 8-water SCF (8 of them FP32 first) 7.4 -> 5.3 ms, the 18 of 16 waters 31.3 -> 26.7 (all
+// steps plain).
 // x^2 in units of 2^-50: the scale goes to x's exponent (|x| < 2^-900 counts as zero)
 __device__ __forceinline__ long long square_fixed(double x)
 {
@@ -273,16 +294,21 @@ __device__ __forceinline__ long long square_fixed(double x)
     return __double2ll_rn(y * y);
 }
 
+constexpr double SP2_STRETCH = 0.02;  // (0.1: a step more at times; below, a is 1.01 and less)
+
 template <typename T, int FROM>
 __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int ks, const void* src, T* X0, T* X1,
                                                    Sp2Slot* slots, int maxs, double tol_idem, double tol_n, int polish,
-                                                   Sp2Sync* sync)
+                                                   Sp2Sync* sync, const double* Fprev, double homo, double lumo,
+                                                   Sp2Log* log)
 {
     extern __shared__ __align__(16) unsigned char sp2_smem[];
     __shared__ long long red[2][32];
-    __shared__ double rb[4][32], tot[2];
-    __shared__ long long s_trace;
+    __shared__ double rb[5][32], tot[4];
+    __shared__ long long s_trace, s_w;
     __shared__ int s_go, s_conv, s_square;
+    __shared__ int s_stretch;      // this step: 0 plain, 1 stretched square, 2 stretched 2X - X^2
+    __shared__ double s_alpha[4];  // its a, and the factors of X^2, X and I
     const int ld = n + 1, nblk = gridDim.x;
     T* Ar = (T*)sp2_smem;    // rows i0 .. i0+tt-1 of X_k, all k
     T* Bc = Ar + tt * ld;    // columns j0 .. j0+tt-1 (rows by symmetry)
@@ -317,6 +343,29 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
         __syncthreads();
         return s_go != 0;
     };
+    // the next step's stretch from l and m, which go on to the step's results (one thread).
+    // a in single precision, l and m for the a taken; non-negative doubles compare as integers
+    double l = 0.0, m = 0.0;
+    auto stretch = [&] {
+        int k = 0;
+        const long long li = __double_as_longlong(l), mi = __double_as_longlong(m);
+        if (max(li, mi) > __double_as_longlong(SP2_STRETCH)) {
+            k = li >= mi ? 1 : 2;
+            const double x = k == 1 ? l : m, y = k == 1 ? m : l;
+            const double a = (double)__fdividef(2.0f, 2.0f - (float)x);
+            const double q = 1.0 - a, p = fma(a, x, q), r = fma(-a, y, 1.0);
+            s_alpha[0] = a;
+            s_alpha[1] = k == 1 ? a * a : -a * a;
+            s_alpha[2] = (k == 1 ? q : 1.0) * (a + a);
+            const double qq = q * q, pp = p * p, small = fma(-r, r, 1.0);
+            s_alpha[3] = k == 1 ? qq : 0.0;
+            const double big = __double_as_longlong(qq) > __double_as_longlong(pp) ? qq : pp;
+            l = k == 1 ? big : small;
+            m = k == 1 ? small : big;
+        }
+        s_stretch = k;
+    };
+    const bool planner = threadIdx.x == blockDim.x - 1;  // (not of warp 0: the block has two at least)
     // the block's share of the traces into its slot of set `set`, then the barrier
     auto share = [&](long long a, long long c, int set, unsigned epoch) {
 #pragma unroll
@@ -336,6 +385,7 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
             }
             slots[set * nblk + blockIdx.x] = Sp2Slot{a, c};
         }
+        if (planner) stretch();
         return barrier(epoch);
     };
     // What step `it` does, from tr X and ||X||^2 in units of 2^-50 (one thread, in integers:
@@ -343,6 +393,7 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
     const long long N = (long long)nocc << 50, tol_i = fixed(tol_idem), tol_t = fixed(tol_n);
     auto decide = [&](long long a, long long c) {
         s_trace = a;
+        s_w = a - c;
         s_conv = llabs(a - c) < tol_i && llabs(a - N) < tol_t;
         s_square = llabs(c - N) <= llabs(2 * a - c - N);
     };
@@ -369,13 +420,17 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
     double scale = 0.0, shift = 0.0;  // X_0 = shift I - scale F
     if (FROM == SP2_FROM_F) {
         const double* F = (const double*)src;
-        double tr = 0, nrm = 0, lo = 1e300, hi = -1e300;
+        double tr = 0, nrm = 0, lo = 1e300, hi = -1e300, dif = 0;
         for (int r = (int)blockIdx.x * nw + warp; r < n; r += nblk * nw) {  // one warp per row (column: F is symmetric)
             double s = 0, q = 0;
             for (int k = lane; k < n; k += 32) {
                 const double f = F[k + (int64_t)r * n];
                 s += fabs(f);
                 q = fma(f, f, q);
+                if (Fprev) {
+                    const double d = f - Fprev[k + (int64_t)r * n];
+                    dif = fma(d, d, dif);
+                }
             }
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) {
@@ -390,7 +445,11 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
                 nrm += q;
             }
         }
+        if (Fprev)
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) dif += __shfl_xor_sync(0xffffffffu, dif, d);
         if (lane == 0) {
+            rb[4][warp] = dif;
             rb[0][warp] = tr;
             rb[1][warp] = nrm;
             rb[2][warp] = lo;
@@ -403,16 +462,18 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
                 nrm += rb[1][w];
                 lo = fmin(lo, rb[2][w]);
                 hi = fmax(hi, rb[3][w]);
+                dif += rb[4][w];
             }
-            bounds[blockIdx.x] = Sp2Bounds{tr, nrm, lo, hi};
+            bounds[blockIdx.x] = Sp2Bounds{tr, nrm, lo, hi, dif, 0.0};
         }
         if (!barrier(++epoch)) return;
         if (warp == 0) {
-            tr = nrm = 0;
+            tr = nrm = dif = 0;
             lo = 1e300, hi = -1e300;
             for (int s = lane; s < nblk; s += 32) {
                 const double2* p = reinterpret_cast<const double2*>(bounds + s);
                 const double2 u = __ldcg(p), v = __ldcg(p + 1);
+                if (Fprev) dif += __ldcg(p + 2).x;
                 tr += u.x;
                 nrm += u.y;
                 lo = fmin(lo, v.x);
@@ -424,17 +485,37 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
                 nrm += __shfl_xor_sync(0xffffffffu, nrm, d);
                 lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, d));
                 hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+                if (Fprev) dif += __shfl_xor_sync(0xffffffffu, dif, d);
             }
             if (lane == 0) {  // X_0 = shift I - scale F, its trace and squared norm
                 const double sc = 1.0 / (hi - lo), sf = hi * sc;
                 decide(fixed(n * sf - sc * tr), fixed(n * sf * sf - 2.0 * sf * sc * tr + sc * sc * nrm));
                 tot[0] = sc;
                 tot[1] = sf;
+                tot[2] = tot[3] = 0.0;
+                if (Fprev) {
+                    const double e = sqrt(dif);
+                    const double l0 = fmax(sf - sc * (lumo - e), 0.0), m0 = fmax(1.0 - sf + sc * (homo + e), 0.0);
+                    if (l0 + m0 < 1.0) {  // (also false for NaN)
+                        tot[2] = l0;
+                        tot[3] = m0;
+                    }
+                }
+                if (log && blockIdx.x == 0) {
+                    log->scale = sc;
+                    log->shift = sf;
+                    log->dif = sqrt(dif);
+                }
             }
         }
         __syncthreads();
         scale = tot[0];
         shift = tot[1];
+        if (planner) {
+            l = tot[2];
+            m = tot[3];
+            stretch();  // (read after the first panels' __syncthreads)
+        }
     } else {
         long long tr = 0, nrm = 0;
         const float* S = (const float*)src;
@@ -508,8 +589,15 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
             }
             return;
         }
+        const int st = left < 0 ? s_stretch : 0;
         // the last of the polishing steps is the opposite of the one before it
-        const bool square = left == 1 ? !last_square : sq;
+        const bool square = st ? st == 1 : left == 1 ? !last_square : sq;
+        if (log && blockIdx.x == 0 && threadIdx.x == 0 && it < SP2_LOG) {
+            const double a = st ? s_alpha[0] : 1.0;
+            log->w[it] = s_w;
+            log->tr[it] = s_trace;
+            log->alpha[it] = square ? a : -a;
+        }
         last_square = square;
         if (left > 0) --left;
         T acc = 0;
@@ -526,7 +614,9 @@ __global__ void __launch_bounds__(1024) sp2_kernel(int n, int nocc, int tt, int 
         }
         long long pt = 0, pn = 0;
         if (own) {
-            const T x = square ? acc : T(2) * Ar[ty * ld + j] - acc;
+            const T y = Ar[ty * ld + j];
+            const T x = st ? (T)fma(s_alpha[1], (double)acc, fma(s_alpha[2], (double)y, i == j ? s_alpha[3] : 0.0))
+                           : square ? acc : T(2) * y - acc;
             Xn[i + (int64_t)j * n] = x;
             if (ti != tj) Xn[j + (int64_t)i * n] = x;
             if (i == j) pt = fixed((double)x);
@@ -683,6 +773,42 @@ static Sp2Shape sp2_shape(Context& ctx, int n)
     return cache[{ctx.device, n}] = best;
 }
 
+// Bounds on the last occupied and the first virtual energy of F from the course of its
+// purification in `steps` steps to a projector of the right trace: before step i every
+// eigenvalue x of X_i has x (1 - x) <= w_i = tr(X_i - X_i^2), so where nocc of them are
+// near 1 the virtual ones are below (1 - sqrt(1 - 4 w_i)) / 2 and the occupied ones as
+// close to 1; the inverse steps take both to X_0 and F.  Late steps have few eigenvalues left in w_i and are the
+// tightest; 1e-5 and up is far above w_i's rounding.  false: none, or no gap left.
+static bool sp2_gap(const Sp2Log& log, int steps, int nocc, double& homo, double& lumo)
+{
+    double l0 = 1.0, h0 = 0.0;
+    if (steps > SP2_LOG) return false;
+    for (int i = 0; i < steps; ++i) {
+        const double w = (double)log.w[i] / SP2_UNIT * (1.0 + 1e-6);
+        if (!(w > 1e-5 && w < 0.2)) continue;
+        // (all but w / 0.72 of the trace is the number of eigenvalues near 1)
+        if (std::fabs((double)log.tr[i] / SP2_UNIT - nocc) > 0.2) continue;
+        double x = 0.5 * (1.0 - std::sqrt(1.0 - 4.0 * w)), y = 1.0 - x;
+        for (int j = i - 1; j >= 0; --j) {
+            const double a = std::fabs(log.alpha[j]);
+            if (log.alpha[j] > 0) {
+                x = (std::sqrt(x) - 1.0 + a) / a;
+                y = (std::sqrt(y) - 1.0 + a) / a;
+            } else {
+                x = (1.0 - std::sqrt(1.0 - x)) / a;
+                y = (1.0 - std::sqrt(1.0 - y)) / a;
+            }
+        }
+        l0 = std::min(l0, x);
+        h0 = std::max(h0, y);
+    }
+    l0 += 1e-8;  // far above the rounding of the steps
+    h0 -= 1e-8;
+    homo = (log.shift - h0) / log.scale;
+    lumo = (log.shift - l0) / log.scale;
+    return l0 < h0;
+}
+
 struct Purifier {
     int n = 0, nocc = 0;
     int tile = 0;  // persistent-kernel tile edge (sp2_shape); -1: per-step fallback
@@ -690,6 +816,10 @@ struct Purifier {
     DBuf<double> X, T1, T2, T3, B, tr;  // orthogonaliser L^-T and work
     DBuf<float> Xf;                     // FP32 iterate of the coarse steps
     DBuf<Sp2Slot> slots;
+    // X^T F X of this density, and of the one whose bounds (sp2_gap) are known
+    DBuf<double> Fx, Fprev;
+    bool gap = false, from_f = false;
+    double homo = 0, lumo = 0;
     ScfReport* rep = nullptr;         // device: barriers and outcome, cleared before each density()
     const ScfReport* hrep = nullptr;  // its host copy, read by converged()
     void setup(Context& ctx, int n_, int nocc_, const double* dS, ScfReport* rep_, const ScfReport* hrep_)
@@ -709,12 +839,14 @@ struct Purifier {
     }
     // One cooperative launch of the whole recursion, barrier state slot `which`.
     template <typename T, int FROM>
-    void run(Context& ctx, const void* src, T* X0, T* X1, double tol_idem, double tol_n, int polish, int which)
+    void run(Context& ctx, const void* src, T* X0, T* X1, double tol_idem, double tol_n, int polish, int which,
+             const double* prev = nullptr, Sp2Log* log = nullptr)
     {
         int n_ = n, nocc_ = nocc, tt_ = tile, ks_ = kslices, maxs = MAXS;
         Sp2Slot* sl = slots.p;
         Sp2Sync* sp = rep->sp2 + which;
-        void* args[] = {&n_, &nocc_, &tt_, &ks_, &src, &X0, &X1, &sl, &maxs, &tol_idem, &tol_n, &polish, &sp};
+        void* args[] = {&n_, &nocc_, &tt_, &ks_, &src, &X0, &X1, &sl, &maxs, &tol_idem, &tol_n, &polish, &sp,
+                        &prev, &homo, &lumo, &log};
         HF_CUDA(cudaLaunchCooperativeKernel((const void*)sp2_kernel<T, FROM>, dim3(sp2_tiles(n, tile)),
                                             dim3(sp2_threads(tile, kslices)), args,
                                             sp2_smem_bytes(n, tile, kslices, sizeof(T)), ctx.stream));
@@ -732,7 +864,18 @@ struct Purifier {
         pending = false;
         HF_CHECK(hrep->sp2[0].err == 0 && hrep->sp2[1].err == 0, HFGPU_ERR_CUDA,
                  "density purification: grid barrier timed out");
-        return fabs(hrep->sp2[1].trace - nocc) < 1e-6 && !(strict && hrep->sp2[1].steps >= MAXS);
+        const bool idem = hrep->sp2[1].steps < MAXS, trace = fabs(hrep->sp2[1].trace - nocc) < 1e-6;
+        if (from_f) {  // the bounds of this F for the next
+            double h = 0, l = 0;
+            const bool found = idem && trace && sp2_gap(hrep->log, hrep->sp2[1].steps, nocc, h, l);
+            // a stretched course reaches back with the bounds it was given at best: the
+            // last ones moved by the change of F are tighter once that is small
+            homo = gap && found ? std::min(h, homo + hrep->log.dif) : h;
+            lumo = gap && found ? std::max(l, lumo - hrep->log.dif) : l;
+            gap = found;
+            std::swap(Fx, Fprev);
+        }
+        return trace && !(strict && !idem);
     }
     // is the whole recursion one cooperative launch at this size?
     bool one_launch(Context& ctx)
@@ -755,21 +898,26 @@ struct Purifier {
         cudaStream_t st = ctx.stream;
         // X is upper triangular: X^T F sums k <= i, (X^T F) X k <= j and is symmetric
         gemm(ctx, true, false, n, n, n, 1.0, X.p, n, dF, n, 0.0, T1.p, n, GEMM_K_LE_I);
-        gemm(ctx, false, false, n, n, n, 1.0, T1.p, n, X.p, n, 0.0, T2.p, n, GEMM_K_LE_J | GEMM_SYMMETRIC);
+        const bool one = one_launch(ctx);
+        if (one && !slots.p) {
+            slots.alloc(5 * (size_t)sp2_tiles(n, tile), st);  // two sets, and the bounds
+            T3.alloc(nn, st);
+            Fx.alloc(nn, st);
+            Fprev.alloc(nn, st);
+        }
+        double* f = one ? Fx.p : T2.p;
+        gemm(ctx, false, false, n, n, n, 1.0, T1.p, n, X.p, n, 0.0, f, n, GEMM_K_LE_J | GEMM_SYMMETRIC);
         ctx.trace_mark("sp2 X^T F X");
-        if (one_launch(ctx)) {
-            if (!slots.p) {
-                slots.alloc(4 * (size_t)sp2_tiles(n, tile), st);  // two sets, and the bounds
-                T3.alloc(nn, st);
-            }
+        if (one) {
             if (coarse) {
                 if (Xf.n < (size_t)(2 * nn)) Xf.alloc(2 * nn, st);
-                run<float, SP2_FROM_F>(ctx, T2.p, Xf.p, Xf.p + nn, 1e-3, 1e-3, 0, 0);
+                run<float, SP2_FROM_F>(ctx, f, Xf.p, Xf.p + nn, 1e-3, 1e-3, 0, 0);
                 ctx.trace_mark("sp2 fp32");
                 run<double, SP2_FROM_F32>(ctx, Xf.p, T1.p, T3.p, 1e-7, 1e-6, 2, 1);
             } else {
-                run<double, SP2_FROM_F>(ctx, T2.p, T1.p, T3.p, 1e-7, 1e-6, 2, 1);
+                run<double, SP2_FROM_F>(ctx, f, T1.p, T3.p, 1e-7, 1e-6, 2, 1, gap ? Fprev.p : nullptr, &rep->log);
             }
+            from_f = !coarse;
             ctx.trace_mark("sp2 fp64");
             pending = true;
         } else {
