@@ -23,27 +23,39 @@ namespace hfgpu {
 
 static const int64_t BLOCK_ROWS = 1 << 20;  // GEMM rows of a block
 
-// out[c][r] = in[r][c] for a rows x cols row-major matrix (32 x 32 tiles through
-// shared memory, both sides coalesced)
-__global__ void transpose_kernel(const double* __restrict__ in, int64_t rows, int64_t cols, double* __restrict__ out)
+// out[c][r] = in[r][c] for a rows x cols row-major matrix: 32 x 32 tiles through shared
+// memory, both sides coalesced, a thread's loads in flight together.  Bound: DRAM (16
+// waters, 80200 x 25600, 32.8 GB both ways: 5.2 -> 4.9 ms of 4.8 at copy speed; tiles
+// of 64 6.4).
+constexpr int TP_T = 32;
+__global__ void __launch_bounds__(256) transpose_kernel(const double* __restrict__ in, int64_t rows, int64_t cols,
+                                                        double* __restrict__ out)
 {
-    __shared__ double t[32][33];
-    const int64_t c0 = (int64_t)blockIdx.x * 32, r0 = (int64_t)blockIdx.y * 32;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int64_t r = r0 + y, c = c0 + threadIdx.x;
-        if (r < rows && c < cols) t[y][threadIdx.x] = in[r * cols + c];
+    __shared__ double t[TP_T][TP_T + 1];
+    const int64_t c0 = (int64_t)blockIdx.x * TP_T, r0 = (int64_t)blockIdx.y * TP_T;
+    const int x = threadIdx.x % TP_T, y0 = threadIdx.x / TP_T;
+    constexpr int DY = 256 / TP_T;
+    double v[TP_T / DY];
+#pragma unroll
+    for (int k = 0; k < TP_T / DY; ++k) {
+        const int64_t r = r0 + y0 + k * DY, c = c0 + x;
+        v[k] = r < rows && c < cols ? __ldcs(in + r * cols + c) : 0.0;
     }
+#pragma unroll
+    for (int k = 0; k < TP_T / DY; ++k) t[y0 + k * DY][x] = v[k];
     __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int64_t c = c0 + y, r = r0 + threadIdx.x;
-        if (r < rows && c < cols) out[c * rows + r] = t[threadIdx.x][y];
+#pragma unroll
+    for (int k = 0; k < TP_T / DY; ++k) {
+        const int y = y0 + k * DY;
+        const int64_t c = c0 + y, r = r0 + x;
+        if (r < rows && c < cols) out[c * rows + r] = t[x][y];
     }
 }
 
 void transpose_device(Context& ctx, const double* in, int64_t rows, int64_t cols, double* out)
 {
-    const dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
-    transpose_kernel<<<grid, dim3(32, 8), 0, ctx.stream>>>(in, rows, cols, out);
+    const dim3 grid((unsigned)((cols + TP_T - 1) / TP_T), (unsigned)((rows + TP_T - 1) / TP_T));
+    transpose_kernel<<<grid, 256, 0, ctx.stream>>>(in, rows, cols, out);
     count_launch();
     HF_CUDA(cudaGetLastError());
 }
@@ -98,14 +110,18 @@ void ao2mo_sliced(Context& ctx, int n, const double* d_int2, const double* C1, i
 }
 
 // one block per pair i >= j: sum_ab (ia|jb) [2 (ia|jb) - (ib|ja)] / (e_i + e_j - e_a - e_b)
-// from T[j][b][i][a] (relative error of each term ~1e-14 from the refined reciprocal).  For fixed (i, j) the v x v block X[b][a] = (ia|jb) has rows
-// of consecutive a; (ib|ja) = X[a][b] is its transpose.  32 x 32 tiles of X and of
-// the mirrored tile are staged in shared memory with coalesced row reads, so T is
-// read with unit stride instead of one scattered element per (ib|ja).
+// from T[j][b][i][a] (relative error of each term ~1e-14 from the refined reciprocal).
+// For fixed (i, j) the v x v block X[b][a] = (ia|jb) has rows of consecutive a, and
+// (ib|ja) = X[a][b] is its transpose: 32 x 32 tiles of X and of the mirrored tile are
+// staged in shared memory with coalesced row reads.  (a, b) and (b, a) have one
+// denominator, so tiles below the diagonal stand for both:
+//   x (2x - y) + y (2y - x) = 2 ((x - y)^2 + x y).
+// Bound: the FP64 pipe (9 instructions per two terms; 10 per term with each (a, b) on
+// its own): 8 and 16 waters 0.52 and 6.5 -> 0.33 and 3.4 ms.
 __global__ void __launch_bounds__(256) mp2_pair_energy_kernel(int o, int v, const double* __restrict__ T,
                                                              const double* __restrict__ eps, double* partial)
 {
-    __shared__ double A[32][33], B[32][33];
+    __shared__ double A[32][33], B[32][33], eb[32];
     // block p = the pair i >= j (p = i (i + 1) / 2 + j): the (j, i) block holds the
     // same terms with a and b exchanged ((jb|ia) = (ia|jb)), so it counts twice
     const int p = blockIdx.x;
@@ -113,35 +129,49 @@ __global__ void __launch_bounds__(256) mp2_pair_energy_kernel(int o, int v, cons
     while (i * (i + 1) / 2 > p) --i;
     while ((i + 1) * (i + 2) / 2 <= p) ++i;
     const int j = p - i * (i + 1) / 2;
-    (void)o;
     const double eij = eps[i] + eps[j];
     const int64_t rs = (int64_t)o * v;  // stride between consecutive b (rows of X)
     const double* X = T + ((int64_t)j * v * o + i) * v;  // X[b][a] = X[b * rs + a]
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-    double s = 0.0;
+    double s_diag = 0.0, s_off = 0.0;
     for (int b0 = 0; b0 < v; b0 += 32)
-        for (int a0 = 0; a0 < v; a0 += 32) {
-            for (int r = ty; r < 32; r += 8) {
-                const int b = b0 + r, a = a0 + tx;
-                A[r][tx] = (b < v && a < v) ? X[b * rs + a] : 0.0;    // X[b0 + r][a0 + tx]
-                const int bb = a0 + r, aa = b0 + tx;
-                B[r][tx] = (bb < v && aa < v) ? X[bb * rs + aa] : 0.0;  // X[a0 + r][b0 + tx]
+        for (int a0 = 0; a0 <= b0; a0 += 32) {
+            const bool off = a0 != b0;
+            double va[4], vb[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = ty + 8 * k, b = b0 + r, a = a0 + tx, bb = a0 + r, aa = b0 + tx;
+                va[k] = (b < v && a < v) ? X[b * rs + a] : 0.0;            // X[b0 + r][a0 + tx]
+                vb[k] = off && bb < v && aa < v ? X[bb * rs + aa] : va[k];  // X[a0 + r][b0 + tx]
             }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                A[ty + 8 * k][tx] = va[k];
+                B[ty + 8 * k][tx] = vb[k];
+            }
+            if (ty == 0) eb[tx] = b0 + tx < v ? eps[o + b0 + tx] : 0.0;
+            const double da = a0 + tx < v ? eij - eps[o + a0 + tx] : 0.0;
             __syncthreads();
-            for (int r = ty; r < 32; r += 8) {
-                const int b = b0 + r, a = a0 + tx;
-                if (b < v && a < v) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = ty + 8 * k;
+                if (b0 + r < v && a0 + tx < v) {
                     const double x = A[r][tx], y = B[tx][r];  // (ia|jb), (ib|ja)
-                    const double d = eij - eps[o + a] - eps[o + b];
+                    const double d = da - eb[r];
                     // 1/d: FP32 reciprocal (24 bits) and one Newton step in FP64
                     // (~48 bits), instead of an FP64 division on the narrow FP64 pipe
                     const double r0 = (double)__frcp_rn((float)d);
                     const double rd = r0 * fma(-d, r0, 2.0);
-                    s = fma(x * (2 * x - y), rd, s);
+                    const double u = x - y;
+                    if (off)
+                        s_off = fma(fma(u, u, x * y), rd, s_off);
+                    else
+                        s_diag = fma(x * (x + u), rd, s_diag);
                 }
             }
             __syncthreads();
         }
+    const double s = fma(2.0, s_off, s_diag);
     __shared__ double sh[256];
     sh[threadIdx.x] = s;
     __syncthreads();

@@ -708,8 +708,9 @@ void sliced_gemm_settle(Context& ctx)
 // this GPU's narrow FP64 pipe).
 // Folding a stored row (elements kl = (la, si), la >= si, kl < len) onto basis
 // indices: a warp takes one run kl = tri(la) .. tri(la) + la (consecutive si,
-// coalesced loads); each element counts for si (shared-memory atomicMax,
-// distinct per lane) and, as the run's maximum, for la.
+// coalesced loads); the run's maximum counts for la, and a
+// lane keeps those of its own si = lane + 32 j over all runs of its warp in registers
+// (a shared-memory atomicMax per element otherwise).
 __device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
 // the same straight from memory: the upper 32-bit word of the element, loaded as an integer
 __device__ __forceinline__ unsigned abs_hi_at(const double* p)
@@ -727,8 +728,10 @@ __device__ __forceinline__ unsigned warp_max_u32(unsigned v)
 // one CTA per stored row a: PACKED rows are the lower triangle of the packed
 // integrals (row a = M[a][0 .. a], at a (a + 1) / 2); otherwise rows of length
 // len_full at src + a * ld.  out[a * n + idx] = folded maximum.
-template <bool PACKED>
-__global__ void row_max_tri_kernel(const double* __restrict__ src, int64_t ld, int len_full, int n, unsigned* out)
+// NJ: runs of up to 32 NJ elements.
+template <bool PACKED, int NJ>
+__global__ void __launch_bounds__(256) row_max_tri_kernel(const double* __restrict__ src, int64_t ld, int len_full,
+                                                          int n, unsigned* out)
 {
     extern __shared__ unsigned smax32[];
     const int a = blockIdx.x;
@@ -737,29 +740,64 @@ __global__ void row_max_tri_kernel(const double* __restrict__ src, int64_t ld, i
     for (int i = threadIdx.x; i < n; i += blockDim.x) smax32[i] = 0u;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    constexpr int NG = NJ < 4 ? NJ : 4;  // loads of a run in flight
+    unsigned own[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) own[j] = 0u;
     for (int la = warp; la < n; la += nw) {
         const int t0 = la * (la + 1) / 2;
         if (t0 >= len) break;  // later runs start further out
         const int smx = min(len - 1 - t0, la);
         unsigned m = 0u;
-        for (int si = lane; si <= smx; si += 32) {
-            const unsigned v = abs_hi_at(row + t0 + si);
-            atomicMax(&smax32[si], v);
-            m = max(m, v);
-        }
-        m = warp_max_u32(m);
+#pragma unroll
+        for (int j0 = 0; j0 < NJ; j0 += NG)
+            if (32 * j0 <= smx) {
+                unsigned v[NG];
+#pragma unroll
+                for (int j = 0; j < NG; ++j) {
+                    const int si = lane + 32 * (j0 + j);
+                    v[j] = si <= smx ? abs_hi_at(row + t0 + si) : 0u;
+                }
+#pragma unroll
+                for (int j = 0; j < NG; ++j) {
+                    own[j0 + j] = max(own[j0 + j], v[j]);
+                    m = max(m, v[j]);
+                }
+            }
+        m = __reduce_max_sync(0xffffffffu, m);
         if (lane == 0) atomicMax(&smax32[la], m);
     }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+        if (lane + 32 * j < n) atomicMax(&smax32[lane + 32 * j], own[j]);
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) out[(int64_t)a * n + i] = smax32[i];
 }
 
+template <bool PACKED>
+static void row_max_tri(Context& ctx, const double* src, int64_t ld, int len_full, int n, int64_t rows, unsigned* out)
+{
+    HF_CHECK(n <= 512, HFGPU_ERR_UNSUPPORTED, "row maxima: basis too large");
+    auto kernel = n <= 64    ? row_max_tri_kernel<PACKED, 2>
+                  : n <= 128 ? row_max_tri_kernel<PACKED, 4>
+                  : n <= 256 ? row_max_tri_kernel<PACKED, 8>
+                  : n <= 384 ? row_max_tri_kernel<PACKED, 12>
+                             : row_max_tri_kernel<PACKED, 16>;
+    kernel<<<(unsigned)rows, 256, n * sizeof(unsigned), ctx.stream>>>(src, ld, len_full, n, out);
+    count_launch();
+    HF_CUDA(cudaGetLastError());
+}
+
 // the column part of the packed rows: M[a][b] = M[b][a] for b > a lives in
 // stored row b.  A CTA takes 32 consecutive a (one per lane, so a warp's loads of
-// row b are one 256-byte segment); its warps stride over b.  Each element counts
-// for both indices of pair b, in shared memory laid out [idx][lane] (padded);
-// the block's maxima are merged into out by atomicMax.
-__global__ void row_max_cols_kernel(const double* __restrict__ ints, int npair, int n, unsigned* out)
+// row b are one 256-byte segment); a warp takes pairs b = (la, si) of COLS_LA
+// consecutive la and COLS_SI consecutive si: their la maxima stay in registers and
+// the si ones are merged before they go to shared memory, laid out [idx][lane]
+// (padded), so an element costs 1 / COLS_LA of an atomicMax there instead of two.
+// The block's maxima are merged into out by atomicMax.
+constexpr int COLS_LA = 4, COLS_SI = 64, COLS_THREADS = 256, COLS_SPLIT = 4;
+__global__ void __launch_bounds__(COLS_THREADS) row_max_cols_kernel(const double* __restrict__ ints, int npair, int n,
+                                                            unsigned* out)
 {
     extern __shared__ unsigned smax32[];  // n x 33
     const int a0 = blockIdx.x * 32;
@@ -767,29 +805,41 @@ __global__ void row_max_cols_kernel(const double* __restrict__ ints, int npair, 
     for (int i = threadIdx.x; i < n * 33; i += blockDim.x) smax32[i] = 0u;
     __syncthreads();
     const int a = a0 + lane;
-    // the warp's stored rows b = b0, b0 + nw, ...: the pair (la, si) of b and the
-    // row's offset b (b + 1) / 2 are carried along by additions (64-bit multiplies
-    // and divisions are slow on this GPU)
-    int b = a0 + 1 + warp;
-    int la = (int)((sqrtf(8.0f * (float)b + 1.0f) - 1.0f) * 0.5f);
-    while (la * (la + 1) / 2 > b) --la;
-    while ((la + 1) * (la + 2) / 2 <= b) ++la;
-    int si = b - la * (la + 1) / 2;
-    const double* rowb = ints + (((int64_t)b * (b + 1)) >> 1);
-    for (; b < npair; ) {
-        if (a < b) {
-            const unsigned v = abs_hi_at(rowb + a);
-            atomicMax(&smax32[la * 33 + lane], v);
-            atomicMax(&smax32[si * 33 + lane], v);
+    int first = (int)((sqrtf(8.0f * (float)a0 + 1.0f) - 1.0f) * 0.5f);  // the la of pair a0
+    while (first * (first + 1) / 2 > a0) --first;
+    while ((first + 1) * (first + 2) / 2 <= a0) ++first;
+    const int nseg = (n + COLS_SI - 1) / COLS_SI, g0 = first / COLS_LA, ng = (n + COLS_LA - 1) / COLS_LA;
+    for (int t = blockIdx.y * nw + warp; t < (ng - g0) * nseg; t += nw * gridDim.y) {
+        const int la0 = (ng - 1 - t / nseg) * COLS_LA, s0 = t % nseg * COLS_SI;  // the longest runs first
+        const int s1 = min(s0 + COLS_SI, min(la0 + COLS_LA, n));
+        unsigned m[COLS_LA];
+        int b[COLS_LA];
+        const double* p[COLS_LA];  // element (b, a): advances by b + 1 with b
+#pragma unroll
+        for (int u = 0; u < COLS_LA; ++u) {
+            m[u] = 0u;
+            b[u] = (la0 + u) * (la0 + u + 1) / 2 + s0;
+            p[u] = ints + (((int64_t)b[u] * (b[u] + 1)) >> 1) + a;
         }
-        // advance by nw: row offset (b + 1) + (b + 2) + ... + (b + nw)
-        rowb += (int64_t)nw * b + (nw * (nw + 1)) / 2;
-        b += nw;
-        si += nw;
-        while (si > la) {  // la grows by one for every la + 1 pairs
-            si -= la + 1;
-            ++la;
+#pragma unroll 2
+        for (int s = s0; s < s1; ++s) {
+            unsigned v[COLS_LA];
+#pragma unroll
+            for (int u = 0; u < COLS_LA; ++u) {
+                v[u] = (la0 + u < n && s <= la0 + u && b[u] > a) ? abs_hi_at(p[u]) : 0u;
+                p[u] += ++b[u];
+            }
+            unsigned x = 0u;
+#pragma unroll
+            for (int u = 0; u < COLS_LA; ++u) {
+                m[u] = max(m[u], v[u]);
+                x = max(x, v[u]);
+            }
+            atomicMax(&smax32[s * 33 + lane], x);
         }
+#pragma unroll
+        for (int u = 0; u < COLS_LA; ++u)
+            if (la0 + u < n) atomicMax(&smax32[(la0 + u) * 33 + lane], m[u]);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n * 32; i += blockDim.x) {
@@ -802,16 +852,18 @@ __global__ void row_max_cols_kernel(const double* __restrict__ ints, int npair, 
 void packed_row_max(Context& ctx, const double* ints, int n, unsigned* out)
 {
     const int npair = n * (n + 1) / 2;
-    row_max_tri_kernel<true><<<(unsigned)npair, 256, n * sizeof(unsigned), ctx.stream>>>(ints, 0, 0, n, out);
-    count_launch();
-    HF_CUDA(cudaGetLastError());
+    row_max_tri<true>(ctx, ints, 0, 0, n, npair, out);
     const size_t smem = (size_t)n * 33 * sizeof(unsigned);
     static std::once_flag once;
     std::call_once(once, [] {
         cudaFuncSetAttribute(row_max_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     });
     HF_CHECK(smem <= 200 * 1024, HFGPU_ERR_UNSUPPORTED, "row maxima: basis too large");
-    row_max_cols_kernel<<<(unsigned)((npair + 31) / 32), 1024, smem, ctx.stream>>>(ints, npair, n, out);
+    // the first pairs have a whole triangle of rows: COLS_SPLIT CTAs share each 32 of them.
+    // Both passes of 16 waters read 51 GB, 7.6 ms at copy speed: 11.7 -> 10.1 ms (8 waters
+    // 0.83 -> 0.74); one CTA of 1024 threads per 32 pairs 11.7, 1.13
+    const dim3 grid((unsigned)((npair + 31) / 32), COLS_SPLIT);
+    row_max_cols_kernel<<<grid, COLS_THREADS, smem, ctx.stream>>>(ints, npair, n, out);
     count_launch();
     HF_CUDA(cudaGetLastError());
 }
@@ -819,9 +871,7 @@ void packed_row_max(Context& ctx, const double* ints, int n, unsigned* out)
 void sympair_row_max(Context& ctx, const double* Zt, int64_t ldz, int64_t nq, int n, unsigned* out)
 {
     const int npair = n * (n + 1) / 2;
-    row_max_tri_kernel<false><<<(unsigned)nq, 256, n * sizeof(unsigned), ctx.stream>>>(Zt, ldz, npair, n, out);
-    count_launch();
-    HF_CUDA(cudaGetLastError());
+    row_max_tri<false>(ctx, Zt, ldz, npair, n, nq, out);
 }
 
 // one warp per row: the upper word of max |x| over the row's K elements
