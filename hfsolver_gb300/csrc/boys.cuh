@@ -4,13 +4,20 @@
 // the GPU way, from the mathematics:
 //   * 0 <= T < BOYS_TMAX: Taylor expansion about the nearest grid point
 //     T_k = k h (h = 1/16, |d| <= 1/32), using dF_m/dT = -F_{m+1}:
-//         F_M(T) = sum_{j<8} F_{M+j}(T_k) (-d)^j / j!,
-//     e^{-T} = e^{-T_k} sum_{j<8} (-d)^j / j!, then the downward recursion
+//         F_M(T) = sum_{j<8} F_{M+j}(T_k) (-d)^j / j!
+//     with the coefficients of each M in a table of its own (one run of memory per
+//     T_k, nothing left to scale), e^{-T} = e^{-T_k} sum_{j<8} (-d)^j / j!, then the
+//     downward recursion
 //     F_m = (2T F_{m+1} + e^{-T}) / (2m+1)  (Shavitt's eq. 24).  Truncation
 //     error <= (1/32)^8/8! ~ 2e-17 relative.
 //   * T >= BOYS_TMAX: F_0 = sqrt(pi/T)/2 (erf(sqrt T) = 1 to < 1e-22) and the
 //     upward recursion F_{m+1} = ((2m+1) F_m - e^{-T}) / (2T); here e^{-T}
 //     contributes < 1e-11 relative, so an FP32 exponential is exact enough.
+// The light quartet classes spend most of their FP64 instructions here (34 of the 45 of
+// a primitive (ss|ss)): with the d^j / j! formed first and F's columns shared by all M
+// the sums took 29 and the grid index 5, so 14 and 4.  ERI of 8 and 16 waters 7.8 and
+// 41.2 -> 6.8 and 36.2 ms, two-electron gradient of 9 waters 52.9 -> 49.3 ms (with the
+// shorter rsqrt_nr).
 // The grid values F_m(T_k) are made on the host in extended precision
 // (boys_table.cpp) from the convergent series
 //     F_m(T) = e^{-T} sum_i (2T)^i / ((2m+1)(2m+3)...(2m+2i+1)).
@@ -23,11 +30,11 @@ namespace hfgpu {
 
 constexpr int BOYS_MMAX = 12;                    // largest m a kernel may ask for
 constexpr int BOYS_NTAYLOR = 8;                  // Taylor terms
-constexpr int BOYS_NCOL = BOYS_MMAX + BOYS_NTAYLOR;  // F_0 .. F_{MMAX+7}
-constexpr int BOYS_STRIDE = BOYS_NCOL + 1;       // + e^{-T_k}
+constexpr int BOYS_STRIDE = BOYS_NTAYLOR + 2;    // F_{M+j}(T_k) / j!, e^{-T_k}, unused: 16-byte loads
 constexpr double BOYS_H = 1.0 / 16.0;
 constexpr double BOYS_TMAX = 50.0;
 constexpr int BOYS_NROW = 801;                   // T_k = k/16, k = 0..800
+constexpr int BOYS_SIZE = (BOYS_MMAX + 1) * BOYS_NROW * BOYS_STRIDE;  // [M][k][]
 
 #ifdef __CUDACC__
 // F[0..M] = pref * F_m(T) * s^m  (s = -2 alpha for the Hermite R integrals)
@@ -36,21 +43,31 @@ __device__ __forceinline__ void boys_scaled(double T, double pref, double s, con
                                             double (&F)[M + 1])
 {
     static_assert(M <= BOYS_MMAX, "Boys order beyond table");
-    if (T < BOYS_TMAX) {
-        int k = __double2int_rn(T * 16.0);
-        double d = (double)k * BOYS_H - T;  // -(T - T_k)
-        const double* row = tab + k * BOYS_STRIDE;
-        double w[BOYS_NTAYLOR];
-        w[0] = 1.0;
+    // T >= 0: its upper word orders like it, and the grid index comes out of the low word
+    // of 16 T + 1.5 2^52 (compares and conversions would run on the FP64 pipe)
+    static_assert(BOYS_TMAX == 50.0, "upper word of 50.0");
+    if (__double2hiint(T) < 0x40490000) {
+        constexpr double MAGIC = 6755399441055744.0;
+        const double t = fma(T, 1.0 / BOYS_H, MAGIC);
+        const int k = __double2loint(t);
+        const double d = fma(t - MAGIC, BOYS_H, -T);  // -(T - T_k)
+        const double2* row = reinterpret_cast<const double2*>(tab + (M * BOYS_NROW + k) * BOYS_STRIDE);
+        double c[BOYS_NTAYLOR + 2];
 #pragma unroll
-        for (int j = 1; j < BOYS_NTAYLOR; ++j) w[j] = w[j - 1] * d * (1.0 / j);
-        double fm = 0.0, ex = 0.0;
-#pragma unroll
-        for (int j = BOYS_NTAYLOR - 1; j >= 0; --j) {
-            fm = fma(__ldg(row + M + j), w[j], fm);
-            ex += w[j];
+        for (int j = 0; j < BOYS_NTAYLOR + (M > 0 ? 2 : 0); j += 2) {
+            const double2 v = __ldg(row + j / 2);
+            c[j] = v.x;
+            c[j + 1] = v.y;
         }
-        double e = ex * __ldg(row + BOYS_NCOL);
+        constexpr double INV[BOYS_NTAYLOR] = {1.0,       1.0,         1.0 / 2.0,   1.0 / 6.0,
+                                              1.0 / 24.0, 1.0 / 120.0, 1.0 / 720.0, 1.0 / 5040.0};  // 1 / j!
+        double fm = c[BOYS_NTAYLOR - 1], ex = INV[BOYS_NTAYLOR - 1];
+#pragma unroll
+        for (int j = BOYS_NTAYLOR - 2; j >= 0; --j) {
+            fm = fma(d, fm, c[j]);
+            ex = fma(d, ex, INV[j]);
+        }
+        const double e = M > 0 ? ex * c[BOYS_NTAYLOR] : 0.0;
         F[M] = fm;
 #pragma unroll
         for (int m = M - 1; m >= 0; --m) F[m] = fma(2.0 * T, F[m + 1], e) * (1.0 / (2 * m + 1));
@@ -78,7 +95,7 @@ __device__ __forceinline__ void boys_scaled(double T, double pref, double s, con
 
 #endif
 
-// Host: build the table (BOYS_NROW x BOYS_STRIDE doubles).
+// Host: build the table (BOYS_SIZE doubles).
 void boys_make_table(double* tab);
 
 }  // namespace hfgpu

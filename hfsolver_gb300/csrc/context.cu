@@ -101,7 +101,7 @@ static Context* make_context(int dev)
         HF_CUDA(cudaEventCreateWithFlags(&c->join_ev[i], cudaEventDisableTiming));
     }
     HF_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
-    std::vector<double> tab((size_t)BOYS_NROW * BOYS_STRIDE);
+    std::vector<double> tab((size_t)BOYS_SIZE);
     boys_make_table(tab.data());
     HF_CUDA(cudaMalloc((void**)&c->boys, tab.size() * sizeof(double)));
     HF_CUDA(cudaMemcpy(c->boys, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));

@@ -129,43 +129,6 @@ __global__ void grad_pair_kernel(const int* __restrict__ sL, const int* __restri
     }
 }
 
-__device__ static void boys_rt(int M, double T, double pref, double s, const double* __restrict__ tab, double* F)
-{
-    if (T < BOYS_TMAX) {
-        const int k = __double2int_rn(T * 16.0);
-        const double d = (double)k * BOYS_H - T;
-        const double* row = tab + k * BOYS_STRIDE;
-        double w[BOYS_NTAYLOR];
-        w[0] = 1.0;
-#pragma unroll
-        for (int j = 1; j < BOYS_NTAYLOR; ++j) w[j] = w[j - 1] * d * (1.0 / j);
-        double fm = 0.0, ex = 0.0;
-#pragma unroll
-        for (int j = BOYS_NTAYLOR - 1; j >= 0; --j) {
-            fm = fma(__ldg(row + M + j), w[j], fm);
-            ex += w[j];
-        }
-        const double e = ex * __ldg(row + BOYS_NCOL);
-        F[M] = fm;
-        for (int m = M - 1; m >= 0; --m) F[m] = fma(2.0 * T, F[m + 1], e) / (double)(2 * m + 1);
-    } else {
-        const double r = rsqrt_nr(T);
-        const double e = (T < 103.0) ? (double)expf(-(float)T) : 0.0;
-        const double inv2t = 0.5 * r * r;
-        double f = 0.88622692545275801364 * r;
-        F[0] = f;
-        for (int m = 0; m < M; ++m) {
-            f = fma((double)(2 * m + 1), f, -e) * inv2t;
-            F[m + 1] = f;
-        }
-    }
-    double sc = pref;
-    for (int m = 0; m <= M; ++m) {
-        F[m] *= sc;
-        sc *= s;
-    }
-}
-
 // ------------------------------------------------------------- two-electron part
 // (the class kernels: grad_kernel.cuh and gen/grad_class_*.cu)
 

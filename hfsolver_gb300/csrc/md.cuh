@@ -88,15 +88,13 @@ constexpr int NPTYPE = 6;
 
 // ------------------------------------------------------------- FP64 helpers
 #ifdef __CUDACC__
-// 1/sqrt(s) for s > 0 in FP64: an FP32 seed refined by two Newton steps
-// y <- y (3 - s y^2) / 2, each doubling the number of correct bits.
+// 1/sqrt(s) for s > 0 in FP64: an FP32 seed y refined once, with e = 1 - s y^2 of about
+// 2^-22, by the first terms of (1 - e)^{-1/2} = 1 + e/2 + 3 e^2/8 + O(e^3)
 __device__ __forceinline__ double rsqrt_nr(double s)
 {
-    double y = (double)rsqrtf((float)s);
-    double h = 0.5 * s;
-    y = y * fma(-h * y, y, 1.5);
-    y = y * fma(-h * y, y, 1.5);
-    return y;
+    const double y = (double)rsqrtf((float)s);
+    const double e = fma(-(s * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // R_tuv(p, PC) for t+u+v <= L (Helgaker et al. eqs. 9.9.18-9.9.20), compile-time L
