@@ -67,10 +67,17 @@ using KernelFn = void (*)(EriArgs);
 constexpr int ERI_BLOCK = 128;
 constexpr double TWO_PI_2_5 = 34.986836655249725;  // 2 pi^{5/2}
 
+// Ket component pairs per chunk.  Every chunk forms the Boys values and R_tuv of its
+// primitive quartets again (155 FP64 instructions of (pp|pp) beside 70 per ket pair),
+// and accumulators in registers cost no time: dependent FMAs of one warp keep an FP64
+// pipe busy.  So as many as the registers hold: 54 doubles, and for a pp bra, whose R
+// and Hermite sums are small, all 81 of (pp|pp).  ERI of 1, 3, 8 and 16 waters with at
+// most 36: 0.19, 0.61, 6.8 and 36.2 ms, so 0.22, 0.53, 5.8 and 31.3 (81 for every class:
+// 0.32, 0.55, 5.7 and longer Schwarz bounds).
 __host__ __device__ constexpr int pick_ncd(int nab, int ncd)
 {
     for (int n = ncd; n >= 1; --n)
-        if (ncd % n == 0 && nab * n <= 36) return n;
+        if (ncd % n == 0 && nab * n <= (nab == 9 ? 81 : 54)) return n;
     return 1;
 }
 

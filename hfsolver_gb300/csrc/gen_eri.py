@@ -79,7 +79,7 @@ def ne_pair(la, lb):
 
 def pick_ncd(nab, ncd):
     for n in range(ncd, 0, -1):
-        if ncd % n == 0 and nab * n <= 36:
+        if ncd % n == 0 and nab * n <= (81 if nab == 9 else 54):
             return n
     return 1
 

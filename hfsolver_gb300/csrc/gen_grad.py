@@ -35,7 +35,7 @@ sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 from gen_eri import PTYPES, box, cart, eoff, gen_R, herm_list, hidx, ncart, nherm  # noqa: E402
 
 GR_HDR = 20   # alpha, beta, p, Px, Py, Pz, K_ab, unused, c_a K_ab (6), c_b (6)
-XCAP = 48     # accumulators X per thread: ket component pairs per chunk x bra Hermite indices
+XCAP = 60     # accumulators X per thread: ket component pairs per chunk x bra Hermite indices
 
 
 def grad_ncd(tb, tk):

@@ -29,7 +29,13 @@
 namespace hfgpu {
 
 constexpr int GR_HDR = 20;  // alpha, beta, p, Px, Py, Pz, K_ab, unused, c_a K_ab (6), c_b (6)
-constexpr int GRAD_XCAP = 48;
+// accumulators X per thread: ket component pairs per chunk times bra Hermite indices.
+// Every chunk forms the Boys values and R_tuv again (240 FP64 instructions of (pp|pp)
+// beside 73 per ket pair): 60 holds three ket pairs of a pp or ds bra, six of a ps one.
+// Two-electron gradient of 1, 3 and 9 waters: 0.70, 2.99 and 49.3 ms with 48; 0.78, 2.74 and
+// 44.8 with 60; 0.97, 2.57 and 42.8 with 90; 1.19, 2.58 and 41.4 with 105 (the long
+// straight-line bodies of few chunks run once a warp in a small molecule).
+constexpr int GRAD_XCAP = 60;
 constexpr int GRAD_BLK = 128;
 
 HD constexpr int grad_table(int la, int lb) { return (la + 1) * (lb + 1) * (la + lb + 2); }
