@@ -201,9 +201,9 @@ def run_reference(args):
 # kernel for one molecule, from the ncu capture summarised under profiles/
 # (keyed by roofline entry and basis size).
 KERNEL_TRAFFIC = {
-    ("step1", 200): {"bytes_per_molecule": 4.3775e9, "bytes_per_launch": 1.0944e9,
+    ("step1", 200): {"bytes_per_molecule": 4.3840e9, "bytes_per_launch": 1.0960e9,
                      "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4 step-1 launches of one "
-                               "8-water molecule (profiles/gather_gemm_traffic_water8.md)"},
+                               "8-water molecule (profiles/kernels_water8.md)"},
 }
 
 def measured_peaks():
@@ -296,7 +296,7 @@ def run_gpu(args):
         "eri": {"kernel": "eri_class_kernel (21 classes, one ERI pass)", "bound": "fp64",
                 "achieved": r["eri_flops"] / (eri_ms * 1e-3) / 1e12, "peak": peak.value, "unit": "TFLOP/s",
                 "peak_source": "measured on this GPU by hfgpu_probe_fp64_tflops", "ms": eri_ms},
-        "fock": {"kernel": "digest_kernel / digest_wide_kernel (21 classes, + symmetrize), one full Fock build",
+        "fock": {"kernel": "digest_kernel (21 classes in three launches, + symmetrize), one full Fock build",
                  "bound": "fp64", "achieved": 12.0 * elems / (full_ms * 1e-3) / 1e12, "peak": peak.value,
                  "unit": "TFLOP/s", "peak_source": "measured on this GPU by hfgpu_probe_fp64_tflops", "ms": fock_ms,
                  "ms_per_full_build": full_ms, "full_builds": nfull, "builds": r["niter"],
@@ -319,7 +319,7 @@ def run_gpu(args):
     if s1_ms > 0:
         nl = avg("n_tc_step1")
         executed1 = 2.0 * 21 * (n * (n + 1) / 2 * n) * o * n
-        roof["step1"] = {"kernel": "sliced_gemm_gather_kernel<PackedRowsBlocked> (AO->MO step 1: packed ERIs "
+        roof["step1"] = {"kernel": "gather_gemm_kernel<PackedRowsBlocked> (AO->MO step 1: packed ERIs "
                                    "gathered and sliced inside a tcgen05 GEMM)",
                          "bound": "tensor", "achieved": 3.0 * dense_q[0] / (s1_ms * 1e-3) / 1e12,
                          "peak": bf16_peak, "unit": "TFLOP/s", "peak_source": peak_src, "ms": s1_ms,

@@ -260,7 +260,7 @@ class RHFOptions:
     schwarz: float = 0.0
     mp2: str = "fp64"          # "none" | "fp64" | "split_bf16"
     mp2_nocc: int = 0          # <= 0: sum(Z)/2
-    purify: bool = False       # SP2 density purification instead of an eigensolve per iteration
+    purify: bool = False       # FP32 purification steps while far from convergence; needs a gap
     batch_streams: int = 0     # rhf_batch: molecules per wave (<= 0: 32), or in flight at once with batch_fused=False (<= 0: 8)
     batch_fused: bool = True   # rhf_batch: waves sharing one ERI and one Fock-build launch per quartet class
     incremental: bool = False  # Fock builds from screened density differences

@@ -190,15 +190,16 @@ int hfgpu_find_pole_diag(int n, const double *moint2, const double *lam, int noc
 /* FP64-accurate C = A B on the tcgen05 tensor cores (the kernel behind the
  * mixed-precision transform): A row-major M x K, Bt = B^T row-major N x K
  * (B column-major), C row-major M x N; 1 <= K <= 512.  Rows of A and columns
- * of B are split exactly into six 7-bit bf16 digits with a power-of-two scale;
+ * of B are rounded to six balanced 7-bit bf16 digits with a power-of-two scale;
  * the result agrees with an FP64 GEMM to about 2^-42 K max|A_r.| max|B_.c|. */
 int hfgpu_dgemm_sliced(int64_t M, int N, int K, const double *A, const double *Bt, double *C);
 
 /* MBPT2 energy from the packed AO integrals and the orbitals: the
  * transform_int2 + mbpt2 sequence of the reference's tests
  * (src/mbpt.f90:11-79, :154-159) without the packed MO array; only (ia|jb) is
- * formed.  precision: HFGPU_MP2_FP64 (cuBLAS DGEMM) or HFGPU_MP2_SPLIT_BF16
- * (tensor cores, exact 7-bit bf16 slicing). */
+ * formed.  Both precisions run on the tensor cores by exact 7-bit bf16 slicing:
+ * HFGPU_MP2_FP64 with nine digits per factor, 2^-62 of a row's scale (above 455
+ * functions on FP64 GEMMs), HFGPU_MP2_SPLIT_BF16 with six, 2^-42. */
 int hfgpu_mp2_energy(int n, const double *int2, const double *C, const double *lam, int nocc,
                      int precision, double *E2);
 
@@ -217,8 +218,10 @@ typedef struct {
     double schwarz;      /* quartet cut on sqrt((ab|ab)(cd|cd)); 0 = none (reference) */
     int mp2;             /* HFGPU_MP2_* */
     int mp2_nocc;        /* occupied orbitals passed to MBPT2; <= 0: sum(Z)/2 */
-    int purify;          /* 1: density by SP2 purification (GEMMs only) in each iteration and one
-                            final dsygvd for the orbitals; 0: dsygvd every iteration (reference) */
+    int purify;          /* 1: density by SP2 purification in each iteration, with FP32 steps while
+                            far from convergence and an error without a gap; 0: the occupied
+                            eigenvectors' density to rounding (FP64 purification where it
+                            converges, else an eigensolve).  One eigensolve at the end */
     int batch_streams;   /* hfgpu_rhf_batch: molecules in flight at once, each on its own
                             streams; <= 0: 8 */
     int incremental;     /* 1: Fock builds from density differences, each quartet's bounded
