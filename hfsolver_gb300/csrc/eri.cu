@@ -753,7 +753,7 @@ static int block_size(int tb, int tk)
 // timed on the real launch (the class writes the same values each time) and the
 // choice recorded: the built-in layout (0), unless another target gains more than a
 // twentieth (alone on the GPU a class likes more lanes than beside the others: 8
-// waters take 7.8 ms built in, 8.1 with each class's fastest).
+// waters took 7.8 ms built in, 8.1 with each class's fastest, when that was measured).
 static void eri_class_layout(Context& ctx, EriPlan* P, ClassPlan& c, double* d_out, double* blocks)
 {
     int target = 0;
