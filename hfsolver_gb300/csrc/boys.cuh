@@ -43,10 +43,12 @@ __device__ __forceinline__ void boys_scaled(double T, double pref, double s, con
                                             double (&F)[M + 1])
 {
     static_assert(M <= BOYS_MMAX, "Boys order beyond table");
-    // T >= 0: its upper word orders like it, and the grid index comes out of the low word
-    // of 16 T + 1.5 2^52 (compares and conversions would run on the FP64 pipe)
+    // the upper word of T >= 0 orders like T, and the grid index comes out of the low word
+    // of 16 T + 1.5 2^52 (compares and conversions would run on the FP64 pipe); -0 is in
+    // the table, a NaN or a negative T is not
     static_assert(BOYS_TMAX == 50.0, "upper word of 50.0");
-    if (__double2hiint(T) < 0x40490000) {
+    const unsigned hi = (unsigned)__double2hiint(T);
+    if (hi < 0x40490000u || hi == 0x80000000u) {
         constexpr double MAGIC = 6755399441055744.0;
         const double t = fma(T, 1.0 / BOYS_H, MAGIC);
         const int k = __double2loint(t);
