@@ -266,7 +266,7 @@ __device__ __forceinline__ void cut8(const double (&x)[8], unsigned amax_hi, uin
 // to be cut: 16 waters, step 1 70 ms; see the kernel.)
 template <int NSL>
 __global__ void slice_kernel(const double* __restrict__ A, int64_t ld, int64_t rows, int K, int T, int ksteps,
-                             uint16_t* planes, int* rexp)
+                             uint16_t* planes, int* rexp, unsigned* rmax)
 {
     const int lane = threadIdx.x & 31;
     const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -277,7 +277,10 @@ __global__ void slice_kernel(const double* __restrict__ A, int64_t ld, int64_t r
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
         const int e = row_exponent(m);
-        if (lane == 0) rexp[r] = e;
+        if (lane == 0) {
+            rexp[r] = e;
+            rmax[r] = m;
+        }
         const int nt = (int)(r / T), c = (int)(r - (int64_t)nt * T);
         for (int k = lane; k < K; k += 32) {
             const uint64_t U = biased_digits<NSL>((uint64_t)__double_as_longlong(row[k]), e);
@@ -560,6 +563,100 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
+// ------------------------------------------------------------------ nine digits: entries in FP64
+// Digits stand for finite numbers only: where a row of A or a column of B holds an Inf or
+// a NaN the fixed-point sums mean nothing.  With nine digits, which stand in for plain
+// FP64, such entries are formed again as FP64 sums in the order of k, as the FP64 GEMM
+// (dgemm_rows.cu) forms them.  A block walks 128-row tiles of the output, lists the
+// entries to redo and does them 256 at a time, one per thread, so that its warps are full
+// however the entries lie.
+struct Fp64Args {
+    const double* b;  // rows of B^T, stride ldb
+    int64_t ldb;
+    const unsigned* bmax;
+    int K, N, M;
+    double* out;
+    OutMap om;
+};
+
+constexpr int FP64_THREADS = 256, FP64_CHUNK = 4 * FP64_THREADS;
+constexpr unsigned ROW_DEAD = 0xFFFFFFFFu, HI_INF = 0x7FF00000u;
+
+// must the entry of a row and a column whose largest |x| have these upper words be
+// formed in FP64?
+__device__ __forceinline__ bool needs_fp64(unsigned am, unsigned bm)
+{
+    return am >= HI_INF || bm >= HI_INF;
+}
+
+template <class Src>
+__global__ void __launch_bounds__(FP64_THREADS) fp64_entries_kernel(const Src src, const Fp64Args g)
+{
+    __shared__ int2 list[FP64_THREADS + FP64_CHUNK];
+    __shared__ int count;
+    __shared__ unsigned amax[BM];
+    const int t = threadIdx.x, R = (int)g.om.R;
+    auto redo = [&](int2 e) {
+        typename Src::Row w{};
+        unsigned m;
+        src.open(e.x, g.M, w, m);
+        const double* b = g.b + e.y * g.ldb;
+        double s = 0.0;
+        int k = 0;
+        for (; k + 8 <= g.K; k += 8) {
+            double x[8];
+            src.load8(w, k, x);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s = fma(x[j], __ldg(b + k + j), s);
+        }
+        for (; k < g.K; ++k) s = fma(src.at(w, k), __ldg(b + k), s);
+        int64_t off;
+        src.place(e.x, g.M, R, g.om.ld, off, m);
+        g.out[off + (int64_t)e.y * (R > 0 ? R : 1)] = s;
+    };
+    if (t == 0) count = 0;
+    const int ntm = (g.M + BM - 1) / BM;
+    for (int tile = blockIdx.x; tile < ntm; tile += gridDim.x) {
+        __syncthreads();  // the last tile's amax
+        if (t < BM) {
+            int64_t off;
+            unsigned m;
+            amax[t] = src.place(tile * BM + t, g.M, R, g.om.ld, off, m) ? m : ROW_DEAD;
+        }
+        __syncthreads();
+        for (int e0 = 0; e0 < BM * g.N; e0 += FP64_CHUNK) {
+            for (int e = e0 + t; e < min(e0 + FP64_CHUNK, BM * g.N); e += FP64_THREADS) {
+                // the outputs' order: rows fastest in blocks of R rows, else columns
+                const int r = R > 0 ? e & (BM - 1) : e / g.N, c = R > 0 ? e / BM : e - r * g.N;
+                const unsigned am = amax[r];
+                if (am != ROW_DEAD && needs_fp64(am, __ldg(g.bmax + c)))
+                    list[atomicAdd(&count, 1)] = make_int2(tile * BM + r, c);
+            }
+            __syncthreads();
+            int have = count;
+            __syncthreads();
+            if (have >= FP64_THREADS) {
+                for (; have >= FP64_THREADS; have -= FP64_THREADS) redo(list[have - FP64_THREADS + t]);
+                if (t == 0) count = have;
+                __syncthreads();
+            }
+        }
+    }
+    __syncthreads();
+    if (t < count) redo(list[t]);
+}
+
+template <class Src>
+static void fp64_entries(Context& ctx, const Src& src, int M, int K, const Sliced& B, double* out, OutMap om)
+{
+    HF_CHECK(B.rows < (1 << 20), HFGPU_ERR_UNSUPPORTED, "sliced GEMM: column count");
+    const Fp64Args g{B.src, B.ld, B.rmax.p, K, (int)B.rows, M, out, om};
+    const unsigned grid = (unsigned)std::min((M + BM - 1) / BM, ctx.num_sms * 8);
+    fp64_entries_kernel<Src><<<grid, FP64_THREADS, 0, ctx.stream>>>(src, g);
+    count_launch();
+    HF_CUDA(cudaGetLastError());
+}
+
 // ------------------------------------------------------------------ host side
 int slice_kmax(int digits) { return digits == SLICE_MIXED ? SliceFmt<6>::KMAX : SliceFmt<9>::KMAX; }
 
@@ -589,14 +686,17 @@ void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld,
     const size_t need = (size_t)digits * s.rows_pad * s.ksteps * BK;
     s.planes.alloc(need, ctx.stream);
     s.rexp.alloc(s.rows_pad, ctx.stream);
+    s.rmax.alloc(s.rows_pad, ctx.stream);
+    s.src = A;
+    s.ld = ld;
     HF_CUDA(cudaMemsetAsync(s.planes.p, 0, need * sizeof(__nv_bfloat16), ctx.stream));
     const int64_t warps = std::min<int64_t>(rows, (int64_t)ctx.num_sms * 64);
     const unsigned blocks = (unsigned)std::max<int64_t>(1, (warps * 32 + 255) / 256);
     uint16_t* pl = reinterpret_cast<uint16_t*>(s.planes.p);
     if (digits == SLICE_MIXED)
-        slice_kernel<6><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p);
+        slice_kernel<6><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p, s.rmax.p);
     else
-        slice_kernel<9><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p);
+        slice_kernel<9><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p, s.rmax.p);
     count_launch();
     HF_CUDA(cudaGetLastError());
 }
@@ -662,6 +762,7 @@ static void gather_gemm_n(Context& ctx, const Src& src, int64_t M, int64_t M_row
     HF_CUDA(cudaGetLastError());
     HF_CUDA(cudaEventRecord(t.b, ctx.stream));
     ctx.tc_events.push_back(t);
+    if constexpr (NSL == SLICE_FP64) fp64_entries(ctx, src, g.M, K, B, out, om);
 }
 
 template <class Src>

@@ -1,0 +1,80 @@
+"""Entries of the plain FP64 transform that digits cannot hold: what the four contractions
+of transform_int2 give in FP64, entry by entry."""
+import numpy as np
+import pytest
+
+import hfsolver_gb300 as hf
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(n, int2):
+    m = n * (n + 1) // 2
+    M = np.zeros((m, m), dtype=int2.dtype)
+    k, l = np.tril_indices(m)
+    M[k, l] = int2
+    M[l, k] = int2
+    return M
+
+
+def _transform(n, int2, C):
+    """Packed MO integrals by the four contractions one after the other, plain sums in the
+    operands' type."""
+    i = np.arange(n)
+    hi, lo = np.maximum(i[:, None], i[None, :]), np.minimum(i[:, None], i[None, :])
+    pair = hi * (hi + 1) // 2 + lo
+    with np.errstate(all="ignore"):
+        X = _pairs(n, int2)[:, pair]  # [p][la][si]
+        Y = (X[:, :, :, None] * C[None, None, :, :]).sum(2)  # [p][la][j]
+        Z = (Y[:, :, :, None] * C[None, :, None, :]).sum(1)  # [p][j][b]
+        W = (Z[pair][:, :, :, :, None] * C[None, :, None, None, :]).sum(1)  # [mu][j][b][i]
+        T = (W[:, :, :, :, None] * C[:, None, None, None, :]).sum(0)  # [j][b][i][a]
+    a, b = np.tril_indices(n)
+    k, l = np.tril_indices(len(a))
+    # the packed element (ij|kl), ij >= kl, is taken from T[i][j][k][l]
+    return T[a[k], b[k], a[l], b[l]]
+
+
+@pytest.mark.parametrize("n", [3, 18, 21])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("where", ["int2", "C", "both"])
+def test_nan_and_inf_go_through(n, bad, where):
+    """An Inf or a NaN reaches the same outputs with the same values as in FP64 sums, zeros
+    of C included (0 Inf is a NaN); an entry without one is left as it is."""
+    rng = np.random.default_rng(n)
+    m = n * (n + 1) // 2
+    int2 = rng.standard_normal(m * (m + 1) // 2)
+    C = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    C[0, n // 2] = 0.0
+    if where != "C":
+        int2[int2.size // 3] = bad
+    if where != "int2":
+        C[n - 1, n - 2] = bad
+    want, got = _transform(n, int2, C), hf.transform_int2(int2, C)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(np.isinf(got), np.isinf(want))
+    inf = np.isinf(want)
+    assert np.array_equal(got[inf], want[inf])
+    ok = np.isfinite(want)
+    # n 2^-52 of the largest integral times sums of n entries of C in each of four steps
+    assert np.all(np.abs(got[ok] - want[ok]) <= 4 * n * 2.0 ** -52 * 8 * n * n)
+
+
+def test_nan_reaches_the_fp64_energy():
+    n = 24
+    m = n * (n + 1) // 2
+    rng = np.random.default_rng(5)
+    int2 = rng.standard_normal(m * (m + 1) // 2)
+    int2[100] = np.nan
+    C = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    lam = np.sort(rng.standard_normal(n))
+    assert np.isnan(hf.mp2_energy(int2, C, lam, 5))
+
+
+def test_a_step_that_overflows_stays_infinite():
+    """Integrals of 1e300 and C of 1e10: every sum beyond the largest double is Inf from
+    the first step on, as in FP64, not turned back into numbers by the next."""
+    n = 19
+    m = n * (n + 1) // 2
+    out = hf.transform_int2(np.full(m * (m + 1) // 2, 1e300), np.full((n, n), 1e10))
+    assert np.all(np.isposinf(out))
