@@ -1,10 +1,12 @@
 // Plain FP64 AO -> MO transform: the drop-in beside the mixed-precision path.
 //
 // Up to slice_kmax(9) = 455 functions every contraction is the sliced tensor-core GEMM
-// with nine digits per factor (tcgemm.cu), which keeps 2^-62 of a row's scale and sums
-// exactly: at 20 to 48 functions the transformed integrals are within 1e-16 (2-norm) of
-// 113-bit arithmetic, where FP64 GEMMs left 3e-16, and GB300's FP64 pipe (2 FMAs per
-// clock per SM) no longer bounds it: 6 waters' MBPT2 34 -> 6 ms, 8 waters' 137 -> 19 ms.
+// with nine digits per factor (tcgemm.cu): exact sums of elements kept to 2^-62 of their
+// row's scale, and entries too small against the scales for that formed in FP64, so that
+// each is as good as an FP64 sum.  GB300's FP64 pipe (2 FMAs per clock per SM) is left with
+// the latter: none to speak of for dense factors (transform_int2 of 100 random orbitals
+// 72 -> 16 ms), about 57% of steps 1 and 3 and 18% of steps 2 and 4 for 6 waters, whose
+// orbitals and integrals are local (MBPT2 34 -> 18 ms; 8 waters 137 -> 74).
 //
 // Beyond that the same half transform over mu >= nu pairs runs on FP64 GEMMs whose A
 // rows are gathered straight from where the transform keeps them (gather_rows.cuh): the

@@ -9,7 +9,8 @@
 // weight and are accumulated together in group t (t < NSL); every group's FP32 sum
 // is exact; the epilogue recombines the groups in int64 and applies the row and
 // column scales.  Six digits (21 products) keep each entry to 2^-42 of its row's or
-// column's scale; nine digits (45 products) keep 2^-62, more than an FP64 entry has.
+// column's scale; nine digits (45 products) keep 2^-62, and entries that are small against
+// those scales are formed again in FP64 (fp64_entries_kernel).
 //
 // Kernel: persistent CTAs, one per SM, walk the 128 x T output tiles; a K step of 32
 // is one pipeline stage.
@@ -18,7 +19,7 @@
 //     the 64-byte-swizzled K-major layout the MMA reads (16-byte chunk c of row r at
 //     c ^ ((r >> 1) & 3)).  Thread t: row t % 128, K quarter t / 128 (8 elements, one
 //     chunk per plane); the elements of the next two steps are in flight.
-//   * B: its digit planes are stacked as NSL T rows of one K-major tile (one bulk copy
+//   * B: its planes are stacked as PLANES T rows of one K-major tile (one bulk copy
 //     a stage, laid out by slice_kernel), so that digit plane i of A multiplies
 //     consecutive planes of B in one product: column block j lands on group i + j by
 //     starting at TMEM column (i + j) T.  The groups are taken in slots of three, so
@@ -29,7 +30,7 @@
 //   * The 17th warp issues the B loads (ahead, into every free stage) and the products.
 //   * Producers read the accumulators of a finished tile back (tcgen05.ld) after they
 //     have filled the first stage of the next one, so that the products have a stage to
-//     go on with; with NSL T <= 256 columns two sets of accumulators fit TMEM and the
+//     go on with; with PLANES T <= 256 columns two sets of accumulators fit TMEM and the
 //     products go on meanwhile too.
 // Bound: the producers' instructions (gather, cut, read back), then shared-memory
 // bandwidth (a 32 k step of 80 columns reads 180 KB for its products beside the 78 KB
@@ -58,7 +59,11 @@ constexpr uint32_t TMEM_COLS = 512;
 constexpr int WAIT_SPINS = 1 << 20;  // of up to 2 us each
 constexpr int GATHER_PRODUCERS = 512, PRODUCER_WARPS = GATHER_PRODUCERS / 32;
 constexpr int GATHER_THREADS = GATHER_PRODUCERS + 32;
-constexpr int MAX_STAGES = 4, MAX_OPS = 18;
+constexpr int MAX_STAGES = 4, MAX_OPS = 19;
+// planes of a stage: the digits, and with nine the magnitudes (scaled_abs) whose product
+// tells which entries the digits are good enough for
+template <int NSL>
+constexpr int PLANES = NSL + (NSL == SLICE_FP64 ? 1 : 0);
 
 // ------------------------------------------------------------------ PTX helpers
 __device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -240,6 +245,9 @@ __device__ __forceinline__ void digit_words(uint64_t Ua, uint64_t Ub, uint32_t (
     }
 }
 
+constexpr unsigned HI_INF = 0x7FF00000u, HI_NORMAL = 1u << 20;  // upper words
+constexpr int FAR_EXPONENT = 1 << 20;
+
 // row exponent from the upper word of the largest |x| of the row: |x| < 2^e for every
 // x in the row (0 for a row without normal numbers, whose digits are all zero)
 __device__ __forceinline__ int row_exponent(unsigned amax_hi)
@@ -247,27 +255,45 @@ __device__ __forceinline__ int row_exponent(unsigned amax_hi)
     return amax_hi < (1u << 20) ? 0 : (int)(amax_hi >> 20) - 1022;
 }
 
+// |x| 2^-e < 1 as bf16, rounded down (0 below 2^-126)
+__device__ __forceinline__ uint32_t scaled_abs(double x, int e)
+{
+    const int u = ((__double2hiint(x) & 0x7FFFFFFF) >> 13) - ((896 + e) << 7);
+    return u < 128 ? 0u : (uint32_t)u;
+}
+
+// the digits (and magnitudes) of two elements as packed bf16
+template <int NSL>
+__device__ __forceinline__ void cut2(double x0, double x1, int e, uint32_t (&w)[PLANES<NSL>])
+{
+    uint32_t d[NSL];
+    digit_words<NSL>(biased_digits<NSL>((uint64_t)__double_as_longlong(x0), e),
+                     biased_digits<NSL>((uint64_t)__double_as_longlong(x1), e), d);
+#pragma unroll
+    for (int t = 0; t < NSL; ++t) w[t] = d[t];
+    if constexpr (NSL == SLICE_FP64) w[NSL] = scaled_abs(x0, e) | scaled_abs(x1, e) << 16;
+}
+
 // the digits of 8 consecutive elements of a row whose largest |x| has upper word amax_hi
 template <int NSL>
-__device__ __forceinline__ void cut8(const double (&x)[8], unsigned amax_hi, uint32_t (&w)[4][NSL])
+__device__ __forceinline__ void cut8(const double (&x)[8], unsigned amax_hi, uint32_t (&w)[4][PLANES<NSL>])
 {
     const int e = row_exponent(amax_hi);
 #pragma unroll
-    for (int j = 0; j < 8; j += 2)
-        digit_words<NSL>(biased_digits<NSL>((uint64_t)__double_as_longlong(x[j]), e),
-                         biased_digits<NSL>((uint64_t)__double_as_longlong(x[j + 1]), e), w[j / 2]);
+    for (int j = 0; j < 8; j += 2) cut2<NSL>(x[j], x[j + 1], e, w[j / 2]);
 }
 
 // ------------------------------------------------------------------ slicing of B
 // One warp per row (a column of B): its exponent, then every element's digits, laid out
-// as the GEMM's stages take them: per column tile and K step, NSL T rows (plane major)
+// as the GEMM's stages take them: per column tile and K step, PLANES T rows (plane major)
 // of 32 bf16, already swizzled, so that a stage's B is one contiguous bulk copy.  (As
 // NSL tensor-map tiles of T 64-byte rows a step's B took longer to arrive than its A
 // to be cut: 16 waters, step 1 70 ms; see the kernel.)
 template <int NSL>
 __global__ void slice_kernel(const double* __restrict__ A, int64_t ld, int64_t rows, int K, int T, int ksteps,
-                             uint16_t* planes, int* rexp, unsigned* rmax)
+                             uint16_t* planes, int* rexp, double* b)
 {
+    constexpr int NP = PLANES<NSL>;
     const int lane = threadIdx.x & 31;
     const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nwarp) {
@@ -277,26 +303,37 @@ __global__ void slice_kernel(const double* __restrict__ A, int64_t ld, int64_t r
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
         const int e = row_exponent(m);
-        if (lane == 0) {
-            rexp[r] = e;
-            rmax[r] = m;
-        }
+        // with nine digits, columns that digits cannot hold are told apart by their exponent
+        if (lane == 0) rexp[r] = NSL == SLICE_FP64 && (m >= HI_INF || m < HI_NORMAL) ? FAR_EXPONENT : e;
         const int nt = (int)(r / T), c = (int)(r - (int64_t)nt * T);
         for (int k = lane; k < K; k += 32) {
-            const uint64_t U = biased_digits<NSL>((uint64_t)__double_as_longlong(row[k]), e);
-            uint32_t w[NSL];
-            digit_words<NSL>(U, U, w);
+            if (NSL == SLICE_FP64) b[k * rows + r] = row[k];
+            uint32_t w[NP];
+            cut2<NSL>(row[k], row[k], e, w);
 #pragma unroll
-            for (int t = 0; t < NSL; ++t) {
+            for (int t = 0; t < NP; ++t) {
                 const int row = t * T + c;
                 const int chunk = ((k & 31) >> 3) ^ ((row >> 1) & 3);  // 64-byte swizzle
-                planes[(((int64_t)nt * ksteps + (k >> 5)) * (NSL * T) + row) * BK + chunk * 8 + (k & 7)] = (uint16_t)w[t];
+                planes[(((int64_t)nt * ksteps + (k >> 5)) * (NP * T) + row) * BK + chunk * 8 + (k & 7)] = (uint16_t)w[t];
             }
         }
     }
 }
 
 // ------------------------------------------------------------------ GEMM kernel
+// Nine digits stand in for plain FP64, so every entry has to be as good as an FP64 sum,
+// which is within K 2^-53 S of it, S = sum_k |A_rk B_kc|.  Digits keep an element to 2^-63
+// of its row's 2^e and leave out the products i + j >= 9, less than 1.01 2^-60 of 2^(ea + eb)
+// each k: 1.26 K 2^(ea + eb - 60) in all, a third of K 2^-53 S where S = 2^(ea + eb - 5).  (On
+// the average, sqrt(K) 2^(ea + eb - 63), the two meet there: rounding leaves about
+// 2^-54.5 S in an FP64 sum of terms of random sign.)  Entries with a smaller S, their row
+// and column large in different places as with orbitals on distant molecules, are left
+// to fp64_entries_kernel: the magnitudes' product is S to 2 parts in 2^7, from below.  So
+// are those whose scales leave FP64's range, and every entry of a row or column with
+// an Inf or a NaN, which digits cannot hold, or with subnormals alone.
+constexpr float FP64_S = 1.0f / 32;
+constexpr long long TO_REDO = 0x7FF8DEADBEEF5EEDll;
+
 struct GatherArgs {
     const unsigned char* b;  // B's stages (slice_kernel)
     int K, ksteps;
@@ -321,6 +358,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
     __shared__ uint4 ops[MAX_OPS];
     __shared__ uint32_t tslot;
     __shared__ int s_ok;
+    constexpr int NP = PLANES<NSL>;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int T = g.T, nst = g.nst, nbuf = g.nbuf, ksteps = g.ksteps;
     if (tid == 0) {
@@ -344,8 +382,11 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
                                       (uint32_t)((first - i) * T * (BK * 2) >> 4), idesc(((g1 - first) * T + 15) & ~15));
             }
         }
+        if (NP > NSL)  // magnitudes: a group of their own
+            ops[k] = make_uint4((uint32_t)(NSL * T) | 0x80000000u, (uint32_t)(NSL * (A_TILE >> 4)),
+                                (uint32_t)(NSL * T * (BK * 2) >> 4), idesc(T));
     }
-    const int nops = g.slot == NSL ? NSL : NSL == 6 ? 9 : 18;
+    const int nops = (g.slot == NSL ? NSL : NSL == 6 ? 9 : 18) + NP - NSL;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&tslot)),
                      "r"(TMEM_COLS));
@@ -356,7 +397,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
     fence_after();
     const uint32_t tmem = tslot;
     auto stage_a = [&](int s) { return smem + s * g.stage; };
-    auto stage_b = [&](int s) { return smem + s * g.stage + NSL * A_TILE; };
+    auto stage_b = [&](int s) { return smem + s * g.stage + NP * A_TILE; };
 
     bool ok = true;
     if (warp == PRODUCER_WARPS) {
@@ -369,7 +410,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
             int ahead = 0;                 // loads issued beyond the step being multiplied
             int last_load = -1, last_load_use = 0, last_commit = -1, last_commit_use = 0;
             int s = 0, use = 0, lt = 0;
-            const int b_bytes = NSL * T * BK * 2;
+            const int b_bytes = NP * T * BK * 2;
             for (int tile = blockIdx.x; tile < g.ntiles && ok; tile += gridDim.x, ++lt) {
                 const int buf = nbuf == 2 ? lt & 1 : 0;
                 const uint32_t acc = tmem + (uint32_t)(buf * 256);
@@ -479,15 +520,15 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
             int64_t off = 0;
             unsigned amax = 0;
             const bool lv = src.place(mt * BM + (warp & 3) * 32 + lane, g.M, (int)g.om.R, g.om.ld, off, amax);
-            const int er = row_exponent(amax) - SliceFmt<NSL>::SHIFT;
+            const int er = NSL == SLICE_FP64 && amax >= HI_INF ? FAR_EXPONENT : row_exponent(amax);
             double* orow = g.out + off;
             if (!mbar_wait(&acc_full[buf], (uint32_t)(nbuf == 2 ? lt >> 1 : lt) & 1u)) return false;
             fence_after();
             const uint32_t ta = tmem + (uint32_t)(buf * 256) + ((uint32_t)((warp & 3) * 32) << 16);
             for (int c0 = (warp >> 2) * 4; c0 < T && n0 + c0 < g.N; c0 += PRODUCER_WARPS) {
-                uint32_t f[NSL][4];
+                uint32_t f[NP][4];
 #pragma unroll
-                for (int t = 0; t < NSL; ++t) tmem_ld4(ta + (uint32_t)(t * T + c0), f[t]);
+                for (int t = 0; t < NP; ++t) tmem_ld4(ta + (uint32_t)(t * T + c0), f[t]);
                 tmem_wait_ld(f);
                 const int c = n0 + c0;
 #pragma unroll
@@ -495,8 +536,14 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
                     uint32_t a[NSL];
 #pragma unroll
                     for (int t = 0; t < NSL; ++t) a[t] = f[t][i];
-                    if (lv && c + i < g.N)
-                        orow[(int64_t)(c + i) * cstep] = recombine<NSL>(a, er + __ldg(g.eb + c + i));
+                    if (lv && c + i < g.N) {
+                        const int E = er + __ldg(g.eb + c + i);
+                        double v = recombine<NSL>(a, E - SliceFmt<NSL>::SHIFT);
+                        if constexpr (NSL == SLICE_FP64)
+                            if ((unsigned)(E + 800) > 1600u || (amax != 0u && __uint_as_float(f[NSL][i]) < FP64_S))
+                                v = __longlong_as_double(TO_REDO);
+                        orow[(int64_t)(c + i) * cstep] = v;
+                    }
                 }
             }
             fence_before();
@@ -515,14 +562,14 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
         // this code, with the two buffers swapped after it: two copies, or a second way to
         // cut digits on the FP32 pipe, ran slower from instruction fetches.)
         auto step = [&](double(&x)[8], unsigned& amax) {
-            uint32_t w[4][NSL];
+            uint32_t w[4][NP];
             const bool has = ks * BK + part * 8 < g.K;
             if (has) cut8<NSL>(x, amax, w);
             fetch(x, amax);  // in flight while this step is stored and the next one is cut
             if (use > 0 && !mbar_wait(&empty[s], (uint32_t)(use - 1) & 1u)) return ok = false;
             unsigned char* dst = stage_a(s) + prow * 64 + chunk * 16;
 #pragma unroll
-            for (int t = 0; t < NSL; ++t)
+            for (int t = 0; t < NP; ++t)
                 *reinterpret_cast<uint4*>(dst + t * A_TILE) =
                     has ? make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]) : make_uint4(0u, 0u, 0u, 0u);
             // the tensor core reads shared memory through the async proxy
@@ -564,72 +611,72 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
 }
 
 // ------------------------------------------------------------------ nine digits: entries in FP64
-// Digits stand for finite numbers only: where a row of A or a column of B holds an Inf or
-// a NaN the fixed-point sums mean nothing.  With nine digits, which stand in for plain
-// FP64, such entries are formed again as FP64 sums in the order of k, as the FP64 GEMM
-// (dgemm_rows.cu) forms them.  A block walks 128-row tiles of the output, lists the
-// entries to redo and does them 256 at a time, one per thread, so that its warps are full
-// however the entries lie.
+// Forms the entries that the GEMM left as TO_REDO as FP64 sums in the order of k, as the
+// FP64 GEMM (dgemm_rows.cu) forms them.  A block walks 128-row tiles of the output, lists
+// them and does them 256 at a time, one per thread, so that its warps are full however the
+// entries lie.
 struct Fp64Args {
-    const double* b;  // rows of B^T, stride ldb
-    int64_t ldb;
-    const unsigned* bmax;
+    const double* b;  // K x N: the lanes of a warp mostly have one row and different columns, or the reverse
     int K, N, M;
     double* out;
     OutMap om;
 };
 
 constexpr int FP64_THREADS = 256, FP64_CHUNK = 4 * FP64_THREADS;
-constexpr unsigned ROW_DEAD = 0xFFFFFFFFu, HI_INF = 0x7FF00000u;
-
-// must the entry of a row and a column whose largest |x| have these upper words be
-// formed in FP64?
-__device__ __forceinline__ bool needs_fp64(unsigned am, unsigned bm)
-{
-    return am >= HI_INF || bm >= HI_INF;
-}
 
 template <class Src>
 __global__ void __launch_bounds__(FP64_THREADS) fp64_entries_kernel(const Src src, const Fp64Args g)
 {
     __shared__ int2 list[FP64_THREADS + FP64_CHUNK];
-    __shared__ int count;
-    __shared__ unsigned amax[BM];
+    __shared__ int count, tiny[BM];
+    __shared__ int64_t off[BM];
     const int t = threadIdx.x, R = (int)g.om.R;
+    const int64_t cstep = R > 0 ? R : 1;
     auto redo = [&](int2 e) {
         typename Src::Row w{};
         unsigned m;
         src.open(e.x, g.M, w, m);
-        const double* b = g.b + e.y * g.ldb;
+        const double* b = g.b + e.y;
         double s = 0.0;
         int k = 0;
         for (; k + 8 <= g.K; k += 8) {
             double x[8];
             src.load8(w, k, x);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s = fma(x[j], __ldg(b + k + j), s);
+            for (int j = 0; j < 8; ++j) s = fma(x[j], __ldg(b + (k + j) * g.N), s);
         }
-        for (; k < g.K; ++k) s = fma(src.at(w, k), __ldg(b + k), s);
-        int64_t off;
-        src.place(e.x, g.M, R, g.om.ld, off, m);
-        g.out[off + (int64_t)e.y * (R > 0 ? R : 1)] = s;
+        for (; k < g.K; ++k) s = fma(src.at(w, k), __ldg(b + k * g.N), s);
+        int64_t o;
+        src.place(e.x, g.M, R, g.om.ld, o, m);
+        g.out[o + e.y * cstep] = s;
     };
     if (t == 0) count = 0;
     const int ntm = (g.M + BM - 1) / BM;
     for (int tile = blockIdx.x; tile < ntm; tile += gridDim.x) {
-        __syncthreads();  // the last tile's amax
+        __syncthreads();  // the last tile's off and tiny
         if (t < BM) {
-            int64_t off;
-            unsigned m;
-            amax[t] = src.place(tile * BM + t, g.M, R, g.om.ld, off, m) ? m : ROW_DEAD;
+            unsigned m = 0u;
+            const bool live = src.place(tile * BM + t, g.M, R, g.om.ld, off[t], m);
+            if (!live) off[t] = -1;
+            tiny[t] = live && m == 0u ? -1 : 0;
+        }
+        __syncthreads();
+        // the maxima are upper words: of a row with 0 there, is anything left below?
+        if (tiny[t % BM]) {
+            typename Src::Row w{};
+            unsigned m, any = 0u;
+            src.open(tile * BM + t % BM, g.M, w, m);
+#pragma unroll 8
+            for (int k = t / BM; k < g.K; k += FP64_THREADS / BM) any |= (unsigned)__double2loint(src.at(w, k));
+            if (any) tiny[t % BM] = 1;
         }
         __syncthreads();
         for (int e0 = 0; e0 < BM * g.N; e0 += FP64_CHUNK) {
             for (int e = e0 + t; e < min(e0 + FP64_CHUNK, BM * g.N); e += FP64_THREADS) {
                 // the outputs' order: rows fastest in blocks of R rows, else columns
                 const int r = R > 0 ? e & (BM - 1) : e / g.N, c = R > 0 ? e / BM : e - r * g.N;
-                const unsigned am = amax[r];
-                if (am != ROW_DEAD && needs_fp64(am, __ldg(g.bmax + c)))
+                if (off[r] < 0) continue;
+                if (tiny[r] > 0 || __double_as_longlong(g.out[off[r] + c * cstep]) == TO_REDO)
                     list[atomicAdd(&count, 1)] = make_int2(tile * BM + r, c);
             }
             __syncthreads();
@@ -650,7 +697,7 @@ template <class Src>
 static void fp64_entries(Context& ctx, const Src& src, int M, int K, const Sliced& B, double* out, OutMap om)
 {
     HF_CHECK(B.rows < (1 << 20), HFGPU_ERR_UNSUPPORTED, "sliced GEMM: column count");
-    const Fp64Args g{B.src, B.ld, B.rmax.p, K, (int)B.rows, M, out, om};
+    const Fp64Args g{B.b.p, K, (int)B.rows, M, out, om};
     const unsigned grid = (unsigned)std::min((M + BM - 1) / BM, ctx.num_sms * 8);
     fp64_entries_kernel<Src><<<grid, FP64_THREADS, 0, ctx.stream>>>(src, g);
     count_launch();
@@ -660,6 +707,8 @@ static void fp64_entries(Context& ctx, const Src& src, int M, int K, const Slice
 // ------------------------------------------------------------------ host side
 int slice_kmax(int digits) { return digits == SLICE_MIXED ? SliceFmt<6>::KMAX : SliceFmt<9>::KMAX; }
 
+static int slice_planes(int digits) { return digits == SLICE_MIXED ? PLANES<SLICE_MIXED> : PLANES<SLICE_FP64>; }
+
 // Columns of a tile for N columns of B: the fewest tiles (every tile gathers and cuts
 // the A rows again) that fit the TMEM columns, evenly filled, a multiple of 16 (the
 // granularity of a product's columns); or 40, for 33 to 40 columns of six digits: 240
@@ -668,7 +717,7 @@ int slice_kmax(int digits) { return digits == SLICE_MIXED ? SliceFmt<6>::KMAX : 
 static int tile_columns(int64_t N, int digits)
 {
     if (digits == SLICE_MIXED && N > 32 && N <= 40) return 40;
-    const int most = (int)TMEM_COLS / digits / 16 * 16;  // 80 with six digits, 48 with nine
+    const int most = (int)TMEM_COLS / slice_planes(digits) / 16 * 16;  // 80 with six digits, 48 with nine
     const int64_t ntn = (N + most - 1) / most;
     return (int)(((N + ntn - 1) / ntn + 15) / 16 * 16);
 }
@@ -683,20 +732,18 @@ void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld,
     s.tile = tile_columns(rows, digits);
     s.rows_pad = (rows + s.tile - 1) / s.tile * s.tile;
     s.ksteps = (K + BK - 1) / BK;
-    const size_t need = (size_t)digits * s.rows_pad * s.ksteps * BK;
+    const size_t need = (size_t)slice_planes(digits) * s.rows_pad * s.ksteps * BK;
     s.planes.alloc(need, ctx.stream);
     s.rexp.alloc(s.rows_pad, ctx.stream);
-    s.rmax.alloc(s.rows_pad, ctx.stream);
-    s.src = A;
-    s.ld = ld;
+    if (digits == SLICE_FP64) s.b.alloc((size_t)rows * K, ctx.stream);
     HF_CUDA(cudaMemsetAsync(s.planes.p, 0, need * sizeof(__nv_bfloat16), ctx.stream));
     const int64_t warps = std::min<int64_t>(rows, (int64_t)ctx.num_sms * 64);
     const unsigned blocks = (unsigned)std::max<int64_t>(1, (warps * 32 + 255) / 256);
     uint16_t* pl = reinterpret_cast<uint16_t*>(s.planes.p);
     if (digits == SLICE_MIXED)
-        slice_kernel<6><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p, s.rmax.p);
+        slice_kernel<6><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p, s.b.p);
     else
-        slice_kernel<9><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p, s.rmax.p);
+        slice_kernel<9><<<blocks, 256, 0, ctx.stream>>>(A, ld, rows, K, s.tile, s.ksteps, pl, s.rexp.p, s.b.p);
     count_launch();
     HF_CUDA(cudaGetLastError());
 }
@@ -719,13 +766,13 @@ static void gather_gemm_n(Context& ctx, const Src& src, int64_t M, int64_t M_row
     HF_CHECK((std::is_same_v<Src, DenseRowsG> || om.R == K), HFGPU_ERR_INVALID, "gather GEMM: output placement");
     g.M = (int)M;
     g.ntiles = (int)ntiles;
-    g.nbuf = NSL * g.T <= 256 ? 2 : 1;
+    g.nbuf = PLANES<NSL> * g.T <= 256 ? 2 : 1;
     // slots of three groups where every product's columns are a multiple of 16; else all
     // groups in one: a padded product then writes only past the last group, into the 8
     // spare columns of a set (and reads B rows of the next plane)
     g.slot = g.T % 16 == 0 ? 3 : NSL;
     HF_CHECK(g.slot == 3 || NSL * g.T + 8 <= 256, HFGPU_ERR_INVALID, "gather GEMM: tile columns");
-    g.stage = (NSL * A_TILE + NSL * g.T * BK * 2 + 1023) / 1024 * 1024;  // the digit planes of A and of B
+    g.stage = (PLANES<NSL> * (A_TILE + g.T * BK * 2) + 1023) / 1024 * 1024;  // the planes of A and of B
     g.eb = B.rexp.p;
     g.out = out;
     g.om = om;

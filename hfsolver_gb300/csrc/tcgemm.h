@@ -20,15 +20,12 @@ int slice_kmax(int digits);
 
 // The B operand of a sliced GEMM: the rows of B^T cut into bf16 digit planes, laid out
 // as the GEMM's pipeline stages (whole tiles of `tile` columns, K steps of 32), plus
-// one power-of-two exponent per row and the upper word of the row's largest |x|.  With
-// nine digits the GEMM also reads the rows themselves (src, stride ld), which have to
-// outlive it.
+// one power-of-two exponent per row; with nine digits also a plane of magnitudes, and B
+// itself in FP64.
 struct Sliced {
     DBuf<__nv_bfloat16> planes;
     DBuf<int> rexp;
-    DBuf<unsigned> rmax;
-    const double* src = nullptr;
-    int64_t ld = 0;
+    DBuf<double> b;  // [k][row]
     int64_t rows = 0, rows_pad = 0;
     int K = 0, ksteps = 0, digits = 0, tile = 0;
 };

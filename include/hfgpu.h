@@ -197,9 +197,11 @@ int hfgpu_dgemm_sliced(int64_t M, int N, int K, const double *A, const double *B
 /* MBPT2 energy from the packed AO integrals and the orbitals: the
  * transform_int2 + mbpt2 sequence of the reference's tests
  * (src/mbpt.f90:11-79, :154-159) without the packed MO array; only (ia|jb) is
- * formed.  Both precisions run on the tensor cores by exact 7-bit bf16 slicing:
- * HFGPU_MP2_FP64 with nine digits per factor, 2^-62 of a row's scale (above 455
- * functions on FP64 GEMMs), HFGPU_MP2_SPLIT_BF16 with six, 2^-42. */
+ * formed.  HFGPU_MP2_FP64: every product entry as good as an FP64 sum of its
+ * terms (on the tensor cores by exact 7-bit bf16 slicing with nine digits per
+ * factor where that keeps it, 2^-62 of a row's scale, else in FP64; above 455
+ * functions FP64 GEMMs); HFGPU_MP2_SPLIT_BF16: six digits, 2^-42 of a row's
+ * scale. */
 int hfgpu_mp2_energy(int n, const double *int2, const double *C, const double *lam, int nocc,
                      int precision, double *E2);
 

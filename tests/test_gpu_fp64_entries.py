@@ -78,3 +78,47 @@ def test_a_step_that_overflows_stays_infinite():
     m = n * (n + 1) // 2
     out = hf.transform_int2(np.full(m * (m + 1) // 2, 1e300), np.full((n, n), 1e10))
     assert np.all(np.isposinf(out))
+
+
+def _fragments(rng, n):
+    """Two halves 1e-7 of each other in every index and C without a block between them."""
+    i, j = np.tril_indices(n)
+    h = n // 2
+    s = np.where(i < h, 1.0, 1e-7) * np.where(j < h, 1.0, 1e-7)
+    k, l = np.tril_indices(len(i))
+    C = np.zeros((n, n))
+    C[:h, :h] = np.linalg.qr(rng.standard_normal((h, h)))[0]
+    C[h:, h:] = np.linalg.qr(rng.standard_normal((n - h, n - h)))[0]
+    return rng.uniform(0.5, 1.0, len(k)) * s[k] * s[l], C
+
+
+def _graded(rng, n):
+    """Integrals of sixteen decades and coefficients of twelve, without an order."""
+    m = n * (n + 1) // 2
+    k = m * (m + 1) // 2
+    return rng.standard_normal(k) * 10.0 ** (-16.0 * rng.random(k)), rng.standard_normal((n, n)) * 10.0 ** (-12.0 * rng.random((n, n)))
+
+
+def _scaled(a, c):
+    def make(rng, n):
+        m = n * (n + 1) // 2
+        return a * rng.standard_normal(m * (m + 1) // 2), c * rng.standard_normal((n, n))
+    return make
+
+
+@pytest.mark.parametrize("make", [_fragments, _graded, _scaled(1e-290, 1.0), _scaled(1e-150, 1e-35), _scaled(3e-320, 1e5),
+                                  _scaled(1e280, 1e2), _scaled(1.0, 1.0)],
+                         ids=["fragments", "graded", "tiny", "small", "subnormal", "huge", "plain"])
+@pytest.mark.parametrize("n", [6, 18, 25])
+def test_every_entry_is_as_good_as_an_fp64_sum(n, make):
+    """Against extended precision, entry by entry: four sums of n terms, each within n 2^-53
+    of the sum of the terms' magnitudes (twice that covers products of the four factors),
+    and half the smallest subnormal for each product that underflows, through the steps
+    that follow it."""
+    int2, C = make(np.random.default_rng(n), n)
+    got = hf.transform_int2(int2, C).astype(np.longdouble)
+    X, D = int2.astype(np.longdouble), C.astype(np.longdouble)
+    want, scale = _transform(n, X, D), _transform(n, np.abs(X), np.abs(D))
+    q = n * np.longdouble(np.max(np.abs(C)))
+    under = n * np.longdouble(2.0 ** -1074) * (1 + q + q * q + q * q * q)
+    assert np.all(np.abs(got - want) <= 8 * n * np.longdouble(2.0 ** -53) * scale + under)
