@@ -201,6 +201,20 @@ def boys(maxm, T):
     return F
 
 
+def half_transform(int2, C, nocc, path):
+    """(ia|jb) as T[j][b][i][a] by FP64 GEMMs (path 0) or sliced GEMMs with path = 6 or 9
+    digits (diagnostic, see hfgpu_half_transform)."""
+    int2 = _f64(int2)
+    C = np.asfortranarray(C, dtype=np.float64)
+    n = C.shape[0]
+    if int2.size != packed_size(n):
+        raise ValueError("int2 has the wrong length")
+    v = n - nocc if nocc < n else n
+    T = np.zeros((nocc, v, nocc, v))
+    _check(_lib.lib().hfgpu_half_transform(n, _d(int2), C.ctypes.data_as(_dp), int(nocc), int(path), _d(T)))
+    return T
+
+
 def formG(P, int2):
     """G = J - K/2 from the packed integrals (scf.f90:26-58)."""
     P = np.asfortranarray(P, dtype=np.float64)

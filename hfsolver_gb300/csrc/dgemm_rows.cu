@@ -174,13 +174,9 @@ void dgemm_rowmajor(Context& ctx, int64_t m, int n, int k, double alpha, const d
 // rows per operand block (Y and W), as in the mixed transform
 static const int64_t FP64_BLOCK_ROWS = 1 << 20;
 
-void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,
+void ao2mo_rows(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,
                 double* T)
 {
-    if (n <= slice_kmax(SLICE_FP64)) {
-        ao2mo_sliced(ctx, n, d_int2, C1, n1, C2, n2, SLICE_FP64, T);
-        return;
-    }
     cudaStream_t st = ctx.stream;
     HF_CHECK(n <= 4096, HFGPU_ERR_UNSUPPORTED, "FP64 transform supports up to 4096 functions");
     const int64_t npair = (int64_t)n * (n + 1) / 2;
@@ -214,6 +210,15 @@ void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int
         dgemm_rows(ctx, rows4, nqb * n1, n, C2, 1, n, n2, T + q0 * n1 * n2, OutMap{0, n2});
         ctx.trace_mark("fp64 step 4");
     }
+}
+
+void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,
+                double* T)
+{
+    if (n <= slice_kmax(SLICE_FP64))
+        ao2mo_sliced(ctx, n, d_int2, C1, n1, C2, n2, SLICE_FP64, T);
+    else
+        ao2mo_rows(ctx, n, d_int2, C1, n1, C2, n2, T);
 }
 
 }  // namespace hfgpu

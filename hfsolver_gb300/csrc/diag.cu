@@ -7,6 +7,8 @@
 //    limit.  Launching fewer blocks than the barrier expects makes its wait run
 //    out: every block then returns with the error flag set, and the host
 //    reports HFGPU_ERR_CUDA with the context still usable.
+//  * hfgpu_half_transform: (ia|jb) by a chosen one of the three transforms, so that
+//    they can be compared with each other at any size.
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -15,6 +17,8 @@
 #include "boys.cuh"
 #include "gridsync.cuh"
 #include "internal.h"
+#include "scf.h"
+#include "tcgemm.h"
 
 namespace hfgpu {
 
@@ -130,5 +134,29 @@ extern "C" int hfgpu_grid_barrier_check(int launched_blocks, int expected_blocks
         HF_CHECK(herr == 0, HFGPU_ERR_CUDA,
                  "grid barrier timed out after " + std::to_string(limit_ms) + " ms (" +
                      std::to_string(launched_blocks) + " of " + std::to_string(expected_blocks) + " blocks arrived)");
+    });
+}
+
+extern "C" int hfgpu_half_transform(int n, const double* int2, const double* C, int nocc, int path, double* T)
+{
+    return guarded([&] {
+        HF_CHECK(n >= 1 && nocc >= 1 && nocc <= n, HFGPU_ERR_INVALID, "hfgpu_half_transform: invalid sizes");
+        HF_CHECK(path == 0 || ((path == SLICE_MIXED || path == SLICE_FP64) && n <= slice_kmax(path)), HFGPU_ERR_INVALID,
+                 "hfgpu_half_transform: path is 0, 6 (n <= 512) or 9 (n <= 455)");
+        HF_CHECK(int2 && C && T, HFGPU_ERR_INVALID, "hfgpu_half_transform: NULL array");
+        Context& ctx = context();
+        std::lock_guard<std::recursive_mutex> lk(ctx.call_mutex);
+        const int64_t np = packed_size(n);
+        const int n1 = nocc, n2 = nocc < n ? n - nocc : n;
+        DBuf<double> dI(np, ctx.stream), dC((size_t)n * n, ctx.stream), dT((size_t)n1 * n2 * n1 * n2, ctx.stream);
+        dI.upload(int2, np);
+        dC.upload(C, (size_t)n * n);
+        const double* C2 = nocc < n ? dC.p + (size_t)n * nocc : dC.p;
+        if (path == 0)
+            ao2mo_rows(ctx, n, dI.p, dC.p, n1, C2, n2, dT.p);
+        else
+            ao2mo_sliced(ctx, n, dI.p, dC.p, n1, C2, n2, path, dT.p);
+        dT.download(T, dT.n);
+        HF_CUDA(cudaStreamSynchronize(ctx.stream));
     });
 }

@@ -52,6 +52,9 @@ double device_dot(Context& ctx, int64_t nn, const double* A, const double* B);
 // packed AO integrals.  Output layout [i][a][j][b].
 void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* dC1, int n1, const double* dC2, int n2,
                 double* d_out);
+// the same by FP64 GEMMs whatever the size (dgemm_rows.cu)
+void ao2mo_rows(Context& ctx, int n, const double* d_int2, const double* dC1, int n1, const double* dC2, int n2,
+                double* d_out);
 // C[m][n] = alpha A[m][k] B[k][n] + beta C, row-major FP64 with leading
 // dimensions lda, ldb, ldc: the row-gathered FP64 GEMM of dgemm_rows.cu
 void dgemm_rowmajor(Context& ctx, int64_t m, int n, int k, double alpha, const double* A, int64_t lda,

@@ -337,6 +337,13 @@ int hfgpu_boys(int maxm, int64_t nt, const double *T, double *F);
  * code; it tests the failure path that replaces a hang. */
 int hfgpu_grid_barrier_check(int launched_blocks, int expected_blocks, double limit_ms, double *elapsed_ms);
 
+/* (ia|jb) from the packed AO integrals by one of the transforms behind
+ * hfgpu_mp2_energy and hfgpu_transform_int2 (src/mbpt.f90:11-79), whatever the
+ * size would choose: i, j over the first nocc columns of C, a, b over the others (all
+ * columns for nocc = n), T[j][b][i][a] (C order).  path: 0 FP64 GEMMs, 9 or 6 the
+ * tensor cores with that many digits (n <= 455 and 512). */
+int hfgpu_half_transform(int n, const double *int2, const double *C, int nocc, int path, double *T);
+
 #ifdef __cplusplus
 }
 #endif
