@@ -1,6 +1,6 @@
 // Plain FP64 AO -> MO transform: the drop-in beside the mixed-precision path.
 //
-// Up to slice_kmax(9) = 455 functions every contraction is the sliced tensor-core GEMM
+// From 28 up to slice_kmax(9) = 455 functions every contraction is the sliced tensor-core GEMM
 // with nine digits per factor (tcgemm.cu): exact sums of elements kept to 2^-62 of their
 // row's scale, and entries too small against the scales for that formed in FP64, so that
 // each is as good as an FP64 sum.  GB300's FP64 pipe (2 FMAs per clock per SM) is left with
@@ -8,7 +8,7 @@
 // 72 -> 16 ms), about 57% of steps 1 and 3 and 18% of steps 2 and 4 for 6 waters, whose
 // orbitals and integrals are local (MBPT2 34 -> 18 ms; 8 waters 137 -> 74).
 //
-// Beyond that the same half transform over mu >= nu pairs runs on FP64 GEMMs whose A
+// Below and beyond the same half transform over mu >= nu pairs runs on FP64 GEMMs whose A
 // rows are gathered straight from where the transform keeps them (gather_rows.cuh): the
 // packed AO integrals, Z transposed, or dense rows.
 //   1. Y[p][j][la] = sum_si (mu nu|la si) C1[si, j]        p = pair(mu >= nu)
@@ -215,7 +215,11 @@ void ao2mo_rows(Context& ctx, int n, const double* d_int2, const double* C1, int
 void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,
                 double* T)
 {
-    if (n <= slice_kmax(SLICE_FP64))
+    // Below 28 functions the FP64 GEMMs are a single wave of blocks and the sliced ones' cutting,
+    // row maxima and second pass 0.06 ms of launches: transform_int2 of 10, 24 and 28
+    // functions 0.12, 0.26, 0.39 ms with FP64 GEMMs, 0.18, 0.28, 0.36 with digits.
+    constexpr int DIGITS_MIN = 28;
+    if (n >= DIGITS_MIN && n <= slice_kmax(SLICE_FP64))
         ao2mo_sliced(ctx, n, d_int2, C1, n1, C2, n2, SLICE_FP64, T);
     else
         ao2mo_rows(ctx, n, d_int2, C1, n1, C2, n2, T);

@@ -35,10 +35,20 @@ def _transform(n, int2, C):
     return T[a[k], b[k], a[l], b[l]]
 
 
-@pytest.mark.parametrize("n", [3, 18, 21])
+def _got(route, n, int2, C):
+    """The packed MO integrals by transform_int2, or from the transform with nine digits."""
+    if route == "call":
+        return hf.transform_int2(int2, C)
+    T = hf.half_transform(int2, C, n, 9)
+    a, b = np.tril_indices(n)
+    k, l = np.tril_indices(len(a))
+    return T[a[k], b[k], a[l], b[l]]
+
+
+@pytest.mark.parametrize("n,route", [(3, "call"), (3, "digits"), (18, "digits"), (21, "digits"), (30, "call")])
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
 @pytest.mark.parametrize("where", ["int2", "C", "both"])
-def test_nan_and_inf_go_through(n, bad, where):
+def test_nan_and_inf_go_through(n, route, bad, where):
     """An Inf or a NaN reaches the same outputs with the same values as in FP64 sums, zeros
     of C included (0 Inf is a NaN); an entry without one is left as it is."""
     rng = np.random.default_rng(n)
@@ -50,7 +60,7 @@ def test_nan_and_inf_go_through(n, bad, where):
         int2[int2.size // 3] = bad
     if where != "int2":
         C[n - 1, n - 2] = bad
-    want, got = _transform(n, int2, C), hf.transform_int2(int2, C)
+    want, got = _transform(n, int2, C), _got(route, n, int2, C)
     assert np.array_equal(np.isnan(got), np.isnan(want))
     assert np.array_equal(np.isinf(got), np.isinf(want))
     inf = np.isinf(want)
@@ -61,7 +71,7 @@ def test_nan_and_inf_go_through(n, bad, where):
 
 
 def test_nan_reaches_the_fp64_energy():
-    n = 24
+    n = 29
     m = n * (n + 1) // 2
     rng = np.random.default_rng(5)
     int2 = rng.standard_normal(m * (m + 1) // 2)
@@ -74,7 +84,7 @@ def test_nan_reaches_the_fp64_energy():
 def test_a_step_that_overflows_stays_infinite():
     """Integrals of 1e300 and C of 1e10: every sum beyond the largest double is Inf from
     the first step on, as in FP64, not turned back into numbers by the next."""
-    n = 19
+    n = 29
     m = n * (n + 1) // 2
     out = hf.transform_int2(np.full(m * (m + 1) // 2, 1e300), np.full((n, n), 1e10))
     assert np.all(np.isposinf(out))
@@ -109,16 +119,32 @@ def _scaled(a, c):
 @pytest.mark.parametrize("make", [_fragments, _graded, _scaled(1e-290, 1.0), _scaled(1e-150, 1e-35), _scaled(3e-320, 1e5),
                                   _scaled(1e280, 1e2), _scaled(1.0, 1.0)],
                          ids=["fragments", "graded", "tiny", "small", "subnormal", "huge", "plain"])
-@pytest.mark.parametrize("n", [6, 18, 25])
-def test_every_entry_is_as_good_as_an_fp64_sum(n, make):
+@pytest.mark.parametrize("n,route", [(6, "call"), (6, "digits"), (18, "digits"), (25, "digits"), (29, "call")])
+def test_every_entry_is_as_good_as_an_fp64_sum(n, route, make):
     """Against extended precision, entry by entry: four sums of n terms, each within n 2^-53
     of the sum of the terms' magnitudes (twice that covers products of the four factors),
     and half the smallest subnormal for each product that underflows, through the steps
     that follow it."""
     int2, C = make(np.random.default_rng(n), n)
-    got = hf.transform_int2(int2, C).astype(np.longdouble)
+    got = _got(route, n, int2, C).astype(np.longdouble)
     X, D = int2.astype(np.longdouble), C.astype(np.longdouble)
     want, scale = _transform(n, X, D), _transform(n, np.abs(X), np.abs(D))
     q = n * np.longdouble(np.max(np.abs(C)))
     under = n * np.longdouble(2.0 ** -1074) * (1 + q + q * q + q * q * q)
     assert np.all(np.abs(got - want) <= 8 * n * np.longdouble(2.0 ** -53) * scale + under)
+
+
+@pytest.mark.parametrize("n", [4, 15, 24])
+def test_small_transforms_launch_no_cutting_kernels(n):
+    """A small basis takes the kernels of the FP64 GEMM transform alone."""
+    from hfsolver_gb300 import _lib
+
+    L = _lib.lib()
+    m = n * (n + 1) // 2
+    int2, C = np.ones(m * (m + 1) // 2), np.eye(n)
+    k = [L.hfgpu_kernel_launches()]
+    hf.half_transform(int2, C, n, 0)
+    k.append(L.hfgpu_kernel_launches())
+    hf.transform_int2(int2, C)
+    k.append(L.hfgpu_kernel_launches())
+    assert k[2] - k[1] == k[1] - k[0] + 1  # and the packing
