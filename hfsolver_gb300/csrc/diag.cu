@@ -7,6 +7,8 @@
 //    limit.  Launching fewer blocks than the barrier expects makes its wait run
 //    out: every block then returns with the error flag set, and the host
 //    reports HFGPU_ERR_CUDA with the context still usable.
+//  * hfgpu_dgemm_digits: the sliced GEMM with six or nine digits, and with a limit on
+//    its waits that can be set so low that they run out.
 //  * hfgpu_half_transform: (ia|jb) by a chosen one of the three transforms, so that
 //    they can be compared with each other at any size.
 #include <algorithm>
@@ -157,6 +159,31 @@ extern "C" int hfgpu_half_transform(int n, const double* int2, const double* C, 
         else
             ao2mo_sliced(ctx, n, dI.p, dC.p, n1, C2, n2, path, dT.p);
         dT.download(T, dT.n);
+        HF_CUDA(cudaStreamSynchronize(ctx.stream));
+    });
+}
+
+extern "C" int hfgpu_dgemm_digits(int64_t M, int N, int K, const double* A, const double* Bt, double* C, int digits,
+                                  int spins)
+{
+    return guarded([&] {
+        HF_CHECK(M >= 1 && N >= 1 && (digits == SLICE_MIXED || digits == SLICE_FP64) && K >= 1 && K <= slice_kmax(digits),
+                 HFGPU_ERR_INVALID, "hfgpu_dgemm_digits: need M, N >= 1 and 1 <= K <= 512 (6 digits) or 455 (9 digits)");
+        HF_CHECK(A && Bt && C, HFGPU_ERR_INVALID, "hfgpu_dgemm_digits: NULL array");
+        Context& ctx = context();
+        std::lock_guard<std::recursive_mutex> lk(ctx.call_mutex);
+        DBuf<double> dA((size_t)M * K, ctx.stream), dB((size_t)N * K, ctx.stream), dC((size_t)M * N, ctx.stream);
+        dA.upload(A, dA.n);
+        dB.upload(Bt, dB.n);
+        dC.zero();
+        Sliced sb;
+        slice_dense(ctx, dB.p, N, K, K, digits, sb);
+        if (spins >= 0) sb.spins = spins;
+        DBuf<unsigned> rmax((size_t)M, ctx.stream);
+        dense_row_max(ctx, dA.p, M, K, K, rmax.p);
+        sliced_gemm_dense(ctx, dA.p, M, K, K, rmax.p, sb, dC.p, OutMap{0, N});
+        sliced_gemm_settle(ctx);
+        dC.download(C, dC.n);
         HF_CUDA(cudaStreamSynchronize(ctx.stream));
     });
 }

@@ -57,6 +57,7 @@ constexpr int BM = 128, BK = 32;
 constexpr int A_TILE = BM * BK * 2;  // 8 KiB: one digit plane of a stage
 constexpr uint32_t TMEM_COLS = 512;
 constexpr int WAIT_SPINS = 1 << 20;  // of up to 2 us each
+constexpr int COPY_SPINS = 1 << 10;  // for a copy in flight, which needs microseconds
 constexpr int GATHER_PRODUCERS = 512, PRODUCER_WARPS = GATHER_PRODUCERS / 32;
 constexpr int GATHER_THREADS = GATHER_PRODUCERS + 32;
 constexpr int MAX_STAGES = 4, MAX_OPS = 19;
@@ -102,10 +103,10 @@ __device__ __forceinline__ bool mbar_try_wait_ns(uint64_t* bar, uint32_t phase, 
     return ok != 0;
 }
 
-// bounded wait on an mbarrier phase; false after WAIT_SPINS polls
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase)
+// bounded wait on an mbarrier phase; false after `spins` polls
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, int spins = WAIT_SPINS)
 {
-    for (int i = 0; i < WAIT_SPINS; ++i)
+    for (int i = 0; i < spins; ++i)
         if (mbar_try_wait_ns(bar, phase, 2000)) return true;
     return false;
 }
@@ -343,6 +344,7 @@ struct GatherArgs {
     double* out;
     OutMap om;
     int* err;
+    int spins;  // of a wait (WAIT_SPINS; fewer to test what follows when one runs out)
 };
 
 template <class Src, int NSL>
@@ -408,7 +410,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
             int ks_l = 0;                  // its K step
             int tile_l = blockIdx.x;       // its tile
             int ahead = 0;                 // loads issued beyond the step being multiplied
-            int last_load = -1, last_load_use = 0, last_commit = -1, last_commit_use = 0;
+            int last_commit = -1, last_commit_use = 0;
             int s = 0, use = 0, lt = 0;
             const int b_bytes = NP * T * BK * 2;
             for (int tile = blockIdx.x; tile < g.ntiles && ok; tile += gridDim.x, ++lt) {
@@ -419,7 +421,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
                         if (sl_use > 0) {
                             const uint32_t ph = (uint32_t)(sl_use - 1) & 1u;
                             if (ahead == 0) {
-                                if (!mbar_wait(&empty[sl], ph)) {
+                                if (!mbar_wait(&empty[sl], ph, g.spins)) {
                                     ok = false;
                                     break;
                                 }
@@ -430,8 +432,6 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
                         mbar_expect_tx(&full[sl], b_bytes);
                         bulk_load(stage_b(sl), g.b + (int64_t)((tile_l % g.ntn) * ksteps + ks_l) * b_bytes, b_bytes,
                                   &full[sl]);
-                        last_load = sl;
-                        last_load_use = sl_use;
                         ++ahead;
                         if (++sl == nst) {
                             sl = 0;
@@ -444,12 +444,12 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
                     }
                     if (!ok) break;
                     if (ks == 0 && lt >= nbuf) {  // the tile that used these accumulators has been read back
-                        if (!mbar_wait(&acc_empty[buf], (uint32_t)(lt / nbuf - 1) & 1u)) {
+                        if (!mbar_wait(&acc_empty[buf], (uint32_t)(lt / nbuf - 1) & 1u, g.spins)) {
                             ok = false;
                             break;
                         }
                     }
-                    if (!mbar_wait(&full[s], (uint32_t)use & 1u)) {
+                    if (!mbar_wait(&full[s], (uint32_t)use & 1u, g.spins)) {
                         ok = false;
                         break;
                     }
@@ -474,14 +474,19 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
                     }
                 }
             }
+            // every B copy and all products in flight land before shared memory and TMEM go
+            // (a stage whose producers gave up never fills: its copy is waited out)
             if (!ok) {
                 atomicExch(&s_ok, 0);
-                // B copies and products still in flight land before shared memory and TMEM go
-                // (bounded; a stage whose producers gave up never fills: its copy is waited
-                // out by the spin limit)
-                if (last_load >= 0) mbar_wait(&full[last_load], (uint32_t)last_load_use & 1u);
-                if (last_commit >= 0) mbar_wait(&empty[last_commit], (uint32_t)last_commit_use & 1u);
+                for (; ahead > 0; --ahead) {
+                    mbar_wait(&full[s], (uint32_t)use & 1u, COPY_SPINS);
+                    if (++s == nst) {
+                        s = 0;
+                        ++use;
+                    }
+                }
             }
+            if (last_commit >= 0) mbar_wait(&empty[last_commit], (uint32_t)last_commit_use & 1u);
         }
     } else {
         const int prow = tid & (BM - 1), part = tid / BM;  // row of the tile, K quarter of a stage
@@ -522,7 +527,9 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
             const bool lv = src.place(mt * BM + (warp & 3) * 32 + lane, g.M, (int)g.om.R, g.om.ld, off, amax);
             const int er = NSL == SLICE_FP64 && amax >= HI_INF ? FAR_EXPONENT : row_exponent(amax);
             double* orow = g.out + off;
-            if (!mbar_wait(&acc_full[buf], (uint32_t)(nbuf == 2 ? lt >> 1 : lt) & 1u)) return false;
+            // (lanes that disagreed on a wait would part before the warp's next barrier)
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[buf], (uint32_t)(nbuf == 2 ? lt >> 1 : lt) & 1u, g.spins)))
+                return false;
             fence_after();
             const uint32_t ta = tmem + (uint32_t)(buf * 256) + ((uint32_t)((warp & 3) * 32) << 16);
             for (int c0 = (warp >> 2) * 4; c0 < T && n0 + c0 < g.N; c0 += PRODUCER_WARPS) {
@@ -566,7 +573,8 @@ __global__ void __launch_bounds__(GATHER_THREADS, 1)
             const bool has = ks * BK + part * 8 < g.K;
             if (has) cut8<NSL>(x, amax, w);
             fetch(x, amax);  // in flight while this step is stored and the next one is cut
-            if (use > 0 && !mbar_wait(&empty[s], (uint32_t)(use - 1) & 1u)) return ok = false;
+            if (use > 0 && !__all_sync(0xFFFFFFFFu, mbar_wait(&empty[s], (uint32_t)(use - 1) & 1u, g.spins)))
+                return ok = false;
             unsigned char* dst = stage_a(s) + prow * 64 + chunk * 16;
 #pragma unroll
             for (int t = 0; t < NP; ++t)
@@ -729,6 +737,7 @@ void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld,
     s.rows = rows;
     s.K = K;
     s.digits = digits;
+    s.spins = WAIT_SPINS;
     s.tile = tile_columns(rows, digits);
     s.rows_pad = (rows + s.tile - 1) / s.tile * s.tile;
     s.ksteps = (K + BK - 1) / BK;
@@ -797,6 +806,7 @@ static void gather_gemm_n(Context& ctx, const Src& src, int64_t M, int64_t M_row
         HF_CUDA(cudaMemsetAsync(ctx.tc_err, 0, sizeof(int), ctx.stream));
     }
     g.err = ctx.tc_err;
+    g.spins = B.spins;
     Context::TcTimer t;
     HF_CUDA(cudaEventCreate(&t.a));
     HF_CUDA(cudaEventCreate(&t.b));

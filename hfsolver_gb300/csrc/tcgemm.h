@@ -28,6 +28,7 @@ struct Sliced {
     DBuf<double> b;  // [k][row]
     int64_t rows = 0, rows_pad = 0;
     int K = 0, ksteps = 0, digits = 0, tile = 0;
+    int spins = 0;  // polls of the GEMM's waits before it gives up
 };
 // rows of a row-major FP64 matrix (stride ld)
 void slice_dense(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, int digits, Sliced& s);

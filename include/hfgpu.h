@@ -337,6 +337,13 @@ int hfgpu_boys(int maxm, int64_t nt, const double *T, double *F);
  * code; it tests the failure path that replaces a hang. */
 int hfgpu_grid_barrier_check(int launched_blocks, int expected_blocks, double limit_ms, double *elapsed_ms);
 
+/* hfgpu_dgemm_sliced with digits = 6 or 9 (K <= 512 and 455).  spins >= 0: polls of
+ * each of the kernel's waits before it gives up; with 0 they all run out, the kernel
+ * leaves with its copies landed and the call returns HFGPU_ERR_CUDA, the device staying
+ * usable.  spins < 0: the limit every other call has. */
+int hfgpu_dgemm_digits(int64_t M, int N, int K, const double *A, const double *Bt, double *C, int digits,
+                       int spins);
+
 /* (ia|jb) from the packed AO integrals by one of the transforms behind
  * hfgpu_mp2_energy and hfgpu_transform_int2 (src/mbpt.f90:11-79), whatever the
  * size would choose: i, j over the first nocc columns of C, a, b over the others (all
