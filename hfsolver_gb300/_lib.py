@@ -83,6 +83,7 @@ SIGNATURES = {
     "hfgpu_autotune_clear": (None, []),
     "hfgpu_boys": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, _dp, _dp]),
     "hfgpu_grid_barrier_check": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_double, _dp]),
+    "hfgpu_fail_allocation": (None, [ctypes.c_int]),
     "hfgpu_dgemm_digits": (ctypes.c_int, [ctypes.c_int64, ctypes.c_int, ctypes.c_int, _dp, _dp, _dp, ctypes.c_int,
                                           ctypes.c_int]),
     "hfgpu_half_transform": (ctypes.c_int, [ctypes.c_int, _dp, _dp, ctypes.c_int, ctypes.c_int, _dp]),

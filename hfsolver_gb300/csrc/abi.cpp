@@ -586,12 +586,13 @@ int hfgpu_dgemm_sliced(int64_t M, int N, int K, const double* A, const double* B
         DBuf<double> dA((size_t)M * K, ctx.stream), dB((size_t)N * K, ctx.stream), dC((size_t)M * N, ctx.stream);
         dA.upload(A, (size_t)M * K);
         dB.upload(Bt, (size_t)N * K);
+        SlicedRun run(ctx);
         Sliced sb;
         slice_dense(ctx, dB.p, N, K, K, SLICE_MIXED, sb);
         DBuf<unsigned> rmax((size_t)M, ctx.stream);
         dense_row_max(ctx, dA.p, M, K, K, rmax.p);
         sliced_gemm_dense(ctx, dA.p, M, K, K, rmax.p, sb, dC.p, OutMap{0, N});
-        sliced_gemm_settle(ctx);
+        run.settle();
         dC.download(C, (size_t)M * N);
         HF_CUDA(cudaStreamSynchronize(ctx.stream));
     });

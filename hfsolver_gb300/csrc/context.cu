@@ -20,6 +20,13 @@ static std::atomic<int64_t> g_launches{0};
 void count_launch(int n) { g_launches += n; }
 int64_t launches_counted() { return g_launches.load(); }
 
+static thread_local int g_fail_allocation = 0;  // allocations of this thread until one fails
+void allocation_check()
+{
+    if (g_fail_allocation > 0 && --g_fail_allocation == 0)
+        throw Error(HFGPU_ERR_NOMEM, "device allocation failed (hfgpu_fail_allocation)");
+}
+
 static std::mutex g_ctx_mutex;
 static std::vector<Context*> g_ctx;
 
@@ -207,4 +214,5 @@ void Context::join()
 
 extern "C" const char* hfgpu_last_error(void) { return hfgpu::g_last_error.c_str(); }
 extern "C" int hfgpu_version(void) { return 1; }
+extern "C" void hfgpu_fail_allocation(int k) { hfgpu::g_fail_allocation = k > 0 ? k : 0; }
 extern "C" int64_t hfgpu_kernel_launches(void) { return hfgpu::g_launches.load(); }

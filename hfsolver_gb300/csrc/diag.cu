@@ -176,13 +176,14 @@ extern "C" int hfgpu_dgemm_digits(int64_t M, int N, int K, const double* A, cons
         dA.upload(A, dA.n);
         dB.upload(Bt, dB.n);
         dC.zero();
+        SlicedRun run(ctx);
         Sliced sb;
         slice_dense(ctx, dB.p, N, K, K, digits, sb);
         if (spins >= 0) sb.spins = spins;
         DBuf<unsigned> rmax((size_t)M, ctx.stream);
         dense_row_max(ctx, dA.p, M, K, K, rmax.p);
         sliced_gemm_dense(ctx, dA.p, M, K, K, rmax.p, sb, dC.p, OutMap{0, N});
-        sliced_gemm_settle(ctx);
+        run.settle();
         dC.download(C, dC.n);
         HF_CUDA(cudaStreamSynchronize(ctx.stream));
     });

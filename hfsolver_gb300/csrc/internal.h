@@ -50,6 +50,9 @@ void set_last_error(const std::string& m);
     } while (0)
 
 // ---------------------------------------------------------------- device buffers
+// throws where hfgpu_fail_allocation asked for it (context.cu)
+void allocation_check();
+
 template <class T>
 struct DBuf {
     T* p = nullptr;
@@ -71,8 +74,10 @@ struct DBuf {
     {
         release();
         st = s;
+        if (!count) return;
+        allocation_check();
+        HF_CUDA(cudaMallocAsync((void**)&p, count * sizeof(T), s));
         n = count;
-        if (count) HF_CUDA(cudaMallocAsync((void**)&p, count * sizeof(T), s));
     }
     void zero() { if (n) HF_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), st)); }
     void upload(const T* h, size_t count)
@@ -136,8 +141,8 @@ struct Context {
     double stat_fock_ms = 0, stat_tc_ms = 0, stat_tc_flops = 0;
     // the gather-fed GEMM over the packed integrals (transform step 1) alone
     double stat_tc_step1_ms = 0, stat_tc_step1_n = 0;
-    // event pairs around sliced GEMMs and their error flag (device), read by
-    // sliced_gemm_settle() at the end of a transform instead of after each GEMM
+    // event pairs around the sliced GEMMs of the call in progress and their error flag
+    // (device), read at its end instead of after each GEMM (SlicedRun)
     struct TcTimer {
         cudaEvent_t a, b;
         double flops;

@@ -64,6 +64,7 @@ void ao2mo_sliced(Context& ctx, int n, const double* d_int2, const double* C1, i
                   int digits, double* T)
 {
     cudaStream_t st = ctx.stream;
+    SlicedRun run(ctx);
     const int64_t npair = (int64_t)n * (n + 1) / 2, nq = (int64_t)n1 * n2;
     Sliced B1, B2;
     slice_dense(ctx, C1, n1, n, n, digits, B1);  // rows of B^T = columns of C1
@@ -106,7 +107,7 @@ void ao2mo_sliced(Context& ctx, int n, const double* d_int2, const double* C1, i
         sliced_gemm_dense(ctx, W.p, nqb * n1, n, n, dmax.p, B2, T + q0 * n1 * n2, OutMap{0, n2});
         ctx.trace_mark("mp2 step 4");
     }
-    sliced_gemm_settle(ctx);
+    run.settle();
 }
 
 // one block per pair i >= j: sum_ab (ia|jb) [2 (ia|jb) - (ib|ja)] / (e_i + e_j - e_a - e_b)

@@ -832,7 +832,18 @@ static void gather_gemm(Context& ctx, const Src& src, int64_t M, int64_t M_rows,
         gather_gemm_n<Src, 9>(ctx, src, M, M_rows, K, B, out, om);
 }
 
-void sliced_gemm_settle(Context& ctx)
+SlicedRun::~SlicedRun()
+{
+    if (ctx.tc_events.empty()) return;  // settled
+    for (auto& t : ctx.tc_events) {
+        cudaEventDestroy(t.a);
+        cudaEventDestroy(t.b);
+    }
+    ctx.tc_events.clear();
+    if (ctx.tc_err) cudaMemsetAsync(ctx.tc_err, 0, sizeof(int), ctx.stream);  // after the GEMMs
+}
+
+void SlicedRun::settle()
 {
     int h = 0;
     if (ctx.tc_err) {

@@ -52,9 +52,18 @@ void sliced_gemm_dense(Context& ctx, const double* A, int64_t rows, int K, int64
 void packed_row_max(Context& ctx, const double* ints, int n, unsigned* out);
 void dense_row_max(Context& ctx, const double* A, int64_t rows, int K, int64_t ld, unsigned* out);
 void sympair_row_max(Context& ctx, const double* Zt, int64_t ldz, int64_t nq, int n, unsigned* out);
-// wait for the sliced GEMMs queued so far: adds their times to the context's
-// counters and throws if one of them timed out
-void sliced_gemm_settle(Context& ctx);
+// Held around the sliced GEMMs of a call.  settle() waits for them, adds their times to
+// the context's counters and throws if one of them timed out; where an exception ends
+// the call between two of them, what they left in the context goes with this object.
+class SlicedRun {
+    Context& ctx;
+
+public:
+    explicit SlicedRun(Context& c) : ctx(c) {}
+    SlicedRun(const SlicedRun&) = delete;
+    ~SlicedRun();
+    void settle();
+};
 // (ia|jb) by the half transform on sliced GEMMs of `digits` digits, T[j][b][i][a]
 // (mp2_mixed.cu); n <= slice_kmax(digits)
 void ao2mo_sliced(Context& ctx, int n, const double* d_int2, const double* C1, int n1, const double* C2, int n2,

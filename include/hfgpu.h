@@ -337,6 +337,10 @@ int hfgpu_boys(int maxm, int64_t nt, const double *T, double *F);
  * code; it tests the failure path that replaces a hang. */
 int hfgpu_grid_barrier_check(int launched_blocks, int expected_blocks, double limit_ms, double *elapsed_ms);
 
+/* The k-th device allocation that the calling thread makes from now on fails once with
+ * HFGPU_ERR_NOMEM, on the host; k <= 0: none does. */
+void hfgpu_fail_allocation(int k);
+
 /* hfgpu_dgemm_sliced with digits = 6 or 9 (K <= 512 and 455).  spins >= 0: polls of
  * each of the kernel's waits before it gives up; with 0 they all run out, the kernel
  * leaves with its copies landed and the call returns HFGPU_ERR_CUDA, the device staying
