@@ -1258,11 +1258,8 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
             count_launch();
         }
     }
-    // orbitals of the last Fock matrix
-    if ((sp2_density || own_eigh) && last_F) {
-        eigh(last_F, Fw.p, 0);
-        if (sp2_density && !in.purify) form_density(ctx, n, in.nocc, Fw.p, dP);
-    }
+    // not converged: orbitals of the last Fock matrix, and P as the last iteration left it (mixed)
+    if ((sp2_density || own_eigh) && last_F) eigh(last_F, Fw.p, 0);
     HF_CUDA(cudaMemcpyAsync(dC, Fw.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
     HF_CUDA(cudaStreamSynchronize(st));
     out.converged = false;
