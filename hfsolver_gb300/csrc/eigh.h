@@ -32,6 +32,7 @@ struct Eigh {
     void setup(Context& ctx, int n_);
     // ncol: eigenvectors formed (the lowest ncol; all eigenvalues always); <= 0: all
     void solve(Context& ctx, const double* X, const double* F, double* C, double* lam, int ncol = 0);
+    const double* energies() const { return hbuf + 2 * n; }  // of the last solve (host)
     ~Eigh();
 };
 

@@ -842,7 +842,7 @@ struct Purifier {
     void run(Context& ctx, const void* src, T* X0, T* X1, double tol_idem, double tol_n, int polish, int which,
              const double* prev = nullptr, Sp2Log* log = nullptr)
     {
-        int n_ = n, nocc_ = nocc, tt_ = tile, ks_ = kslices, maxs = MAXS;
+        int n_ = n, nocc_ = nocc, tt_ = tile, ks_ = kslices, maxs = limit;
         Sp2Slot* sl = slots.p;
         Sp2Sync* sp = rep->sp2 + which;
         void* args[] = {&n_, &nocc_, &tt_, &ks_, &src, &X0, &X1, &sl, &maxs, &tol_idem, &tol_n, &polish, &sp,
@@ -856,6 +856,13 @@ struct Purifier {
     // travels to the host with the iteration's report.
     bool pending = false;
     static constexpr int MAXS = 160;
+    // Steps that the recursion may take (even), and its estimate for a spectrum of this
+    // width and gap: each step shrinks their ratio 1.24 times.  Where an eigensolve can take
+    // over, more than eigensolve_limit() steps are slower than it: 4 us a step at 25 functions,
+    // 6 us at 75 and 13 us at 150 against 0.2, 0.7 and 2 ms.
+    int limit = MAXS;
+    int eigensolve_limit() const { return std::min(MAXS, std::max(40, 20 + 5 * n / 4) & ~1); }
+    static double steps_for(double width, double gap) { return gap > 0 ? 9.0 + 10.9 * std::log10(1.5 * width / gap) : 1e9; }
     // Did the last density() end with tr X = nocc?  strict: and by the idempotency
     // test, not at the step limit.  (True when nothing is pending.)
     bool converged(bool strict)
@@ -864,7 +871,7 @@ struct Purifier {
         pending = false;
         HF_CHECK(hrep->sp2[0].err == 0 && hrep->sp2[1].err == 0, HFGPU_ERR_CUDA,
                  "density purification: grid barrier timed out");
-        const bool idem = hrep->sp2[1].steps < MAXS, trace = fabs(hrep->sp2[1].trace - nocc) < 1e-6;
+        const bool idem = hrep->sp2[1].steps < limit, trace = fabs(hrep->sp2[1].trace - nocc) < 1e-6;
         if (from_f) {  // the bounds of this F for the next
             double h = 0, l = 0;
             const bool found = idem && trace && sp2_gap(hrep->log, hrep->sp2[1].steps, nocc, h, l);
@@ -1116,6 +1123,12 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     // stays.
     const bool sp2_density = in.purify || (own_eigh && in.nocc > 0 && in.nocc < n && n >= SP2_MIN &&
                                            in.tolP >= 1e-11 && pur.one_launch(ctx));
+    // A purification that found no gap is not tried again until the energies of the
+    // eigensolves after it show one (and after the third such not at all): 20 iterations of
+    // 25 functions without a gap, or with one of 1e-6, took 19 and 10 ms, 6.3 with eigensolves alone.
+    bool rest = false;
+    int misses = 0;
+    if (sp2_density && !in.purify) pur.limit = pur.eigensolve_limit();
     // orbitals C (may alias F) and energies of F C = S C diag(lam); with the own
     // eigensolver only the lowest ncol orbitals are formed (ncol <= 0: all)
     auto eigh = [&](const double* Fm, double* Cm, int ncol) {
@@ -1192,7 +1205,8 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
             head = (head + 1) % nd;
             ctx.trace_mark("diis extrap");
         }
-        if (sp2_density) {
+        const bool sp2_now = sp2_density && !rest;
+        if (sp2_now) {
             // with the purify option, FP32 steps while the density is still far from converged
             pur.density(ctx, Fsolve, dP, in.purify && it > 1 && !endgame && last_dP > 1e-4);
         } else {
@@ -1212,8 +1226,14 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
         int hinfo = 0;
         if (!own_eigh) info.download(&hinfo, 1);  // dsygvd's; the own eigensolver throws
         HF_CUDA(cudaStreamSynchronize(st));
-        if (sp2_density && !pur.converged(!in.purify)) {
+        if (rest) {
+            const double* w = eig.energies();
+            rest = misses >= 3 || Purifier::steps_for(w[n - 1] - w[0], w[in.nocc] - w[in.nocc - 1]) > pur.limit - 6;
+        }
+        if (sp2_now && !pur.converged(!in.purify)) {
             HF_CHECK(!in.purify, HFGPU_ERR_LINALG, "density purification did not converge (no gap?)");
+            rest = true;
+            ++misses;
             eigh(Fsolve, Fw.p, in.nocc);
             form_density(ctx, n, in.nocc, Fw.p, dP);
             report();
