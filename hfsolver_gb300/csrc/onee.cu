@@ -85,7 +85,8 @@ __device__ __forceinline__ void lane_sums(double (&acc)[N], int split)
 
 // One group of split lanes per shell pair (A, B) of one pair type (l_A >= l_B) and
 // blockIdx.y: 0 forms S and T, y > 0 adds the attraction of nuclei
-// [(y - 1) atoms, y atoms) to V (zeroed by the caller) atomically.  The 1-D tables
+// [(y - 1) atoms, y atoms) to V (zeroed by the caller) atomically, or with vrow > 0 writes
+// it to a matrix of its own at V + (y - 1) vrow.  The 1-D tables
 // of a primitive pair serve every component pair, and the Boys values and R_tuv of
 // a nucleus serve every component pair as well.  A == B: only component pairs with
 // a >= b are formed (both triangle entries are written from them).
@@ -100,7 +101,7 @@ template <int LA, int LB>
 __global__ void __launch_bounds__(64) onee_shell_kernel(ShellOne sh, const int2* __restrict__ pairs, OneeSegs segs,
                                                         int n, int nat, int atoms, const int* __restrict__ Z,
                                                         const double* __restrict__ C, const double* __restrict__ boys,
-                                                        double* S, double* T, double* V)
+                                                        double* S, double* T, double* V, int64_t vrow)
 {
     constexpr double PI = 3.14159265358979323846;
     constexpr int NA = ncart(LA), NB = ncart(LB), L = LA + LB;
@@ -233,9 +234,24 @@ __global__ void __launch_bounds__(64) onee_shell_kernel(ShellOne sh, const int2*
             const int x = fa[i], y = fb[j];
             if (x < 0 || y < 0 || (A == B && i < j)) continue;
             const int64_t o1 = x + (int64_t)y * n, o2 = y + (int64_t)x * n;
+            if (vrow > 0) {
+                double* Vr = V + (blockIdx.y - 1) * vrow;
+                Vr[o1] = Vr[o2] = vacc[i * NB + j];
+                continue;
+            }
             atomicAdd(V + o1, vacc[i * NB + j]);
             if (o2 != o1) atomicAdd(V + o2, vacc[i * NB + j]);
         }
+}
+
+// V = the sum of the block rows' matrices, in their order
+__global__ void onee_sum_kernel(int64_t nn, int rows, const double* __restrict__ part, double* __restrict__ V)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nn) return;
+    double s = 0.0;
+    for (int r = 0; r < rows; ++r) s += part[r * nn + i];
+    V[i] = s;
 }
 
 // nuclei per block row: ONEE_ATOMS share a primitive pair's 1-D tables, unless that
@@ -317,7 +333,17 @@ void onee_compute(Context& ctx, const Basis& b, int nat, const int* atno, const 
     auto dZ = to_device(Z, st);
     auto dC = to_device(C, st);
     ShellOne sh{dL.p, dn.p, dp0.p, dc0.p, df0.p, dxyz.p, dal.p, dco.p, dcf.p};
-    if (dV) HF_CUDA(cudaMemsetAsync(dV, 0, sizeof(double) * n * n, st));
+    // a nucleus per block row: the rows' matrices are summed in order, so that V does not
+    // change from call to call (as one block row's does not; with more nuclei a row, 9
+    // waters and up, the rows meet in atomics)
+    const int64_t nn = (int64_t)n * n;
+    DBuf<double> parts;
+    if (dV && wide && nat > 0)
+        parts.alloc((size_t)(nn * nat), st);
+    else if (dV)
+        HF_CUDA(cudaMemsetAsync(dV, 0, sizeof(double) * nn, st));
+    double* v = parts.p ? parts.p : dV;
+    const int64_t vrow = parts.p ? nn : 0;
     // one small launch per pair type: side by side, the longest first
     const unsigned rows = 1 + (dV ? (unsigned)((nat + atoms - 1) / atoms) : 0u);
     static_assert(NPTYPE <= Context::NAUX, "one side stream per pair type");
@@ -329,7 +355,7 @@ void onee_compute(Context& ctx, const Basis& b, int nat, const int* atno, const 
         cudaStream_t on_t = ctx.aux[t];
         if (on_t != st) HF_CUDA(cudaStreamWaitEvent(on_t, ctx.fork_ev, 0));
         auto launch = [&](auto kernel) {
-            kernel<<<grid, 64, 0, on_t>>>(sh, pp, segs[t], n, nat, atoms, dZ.p, dC.p, ctx.boys, dS, dT, dV);
+            kernel<<<grid, 64, 0, on_t>>>(sh, pp, segs[t], n, nat, atoms, dZ.p, dC.p, ctx.boys, dS, dT, v, vrow);
         };
         switch (t) {
             case 0: launch(onee_shell_kernel<0, 0>); break;
@@ -346,6 +372,11 @@ void onee_compute(Context& ctx, const Basis& b, int nat, const int* atno, const 
     // st frees the tables: after every launch
     for (int t = 0; t < NPTYPE; ++t)
         if (segs[t].nwarps && ctx.aux[t] != st) HF_CUDA(cudaStreamWaitEvent(st, ctx.join_ev[t], 0));
+    if (parts.p) {
+        onee_sum_kernel<<<(unsigned)((nn + 127) / 128), 128, 0, st>>>(nn, nat, parts.p, dV);
+        count_launch();
+        HF_CUDA(cudaGetLastError());
+    }
 }
 
 }  // namespace hfgpu
