@@ -285,7 +285,8 @@ void onee_compute(Context& ctx, const Basis& b, int nat, const int* atno, const 
     // shell pairs by pair type, the larger angular momentum first, most primitives first
     const bool wide = !fixed_lanes &&
                       (int64_t)ns * (ns + 1) / 2 * ((nat + ONEE_ATOMS - 1) / ONEE_ATOMS) / 32 < (int64_t)ctx.num_sms * 4;
-    const int atoms = wide ? 1 : ONEE_ATOMS;
+    // (block rows past 65535 are not launchable: point charges by the ten thousand share them)
+    const int atoms = std::max(wide ? 1 : ONEE_ATOMS, (nat + 65533) / 65534);
     std::vector<int2> pairs;
     int off[NPTYPE] = {};
     OneeSegs segs[NPTYPE] = {};
@@ -338,14 +339,15 @@ void onee_compute(Context& ctx, const Basis& b, int nat, const int* atno, const 
     // waters and up, the rows meet in atomics)
     const int64_t nn = (int64_t)n * n;
     DBuf<double> parts;
+    const int vrows = (nat + atoms - 1) / atoms;
     if (dV && wide && nat > 0)
-        parts.alloc((size_t)(nn * nat), st);
+        parts.alloc((size_t)(nn * vrows), st);
     else if (dV)
         HF_CUDA(cudaMemsetAsync(dV, 0, sizeof(double) * nn, st));
     double* v = parts.p ? parts.p : dV;
     const int64_t vrow = parts.p ? nn : 0;
     // one small launch per pair type: side by side, the longest first
-    const unsigned rows = 1 + (dV ? (unsigned)((nat + atoms - 1) / atoms) : 0u);
+    const unsigned rows = 1 + (dV ? (unsigned)vrows : 0u);
     static_assert(NPTYPE <= Context::NAUX, "one side stream per pair type");
     HF_CUDA(cudaEventRecord(ctx.fork_ev, st));
     for (int t = NPTYPE - 1; t >= 0; --t) {
@@ -373,7 +375,7 @@ void onee_compute(Context& ctx, const Basis& b, int nat, const int* atno, const 
     for (int t = 0; t < NPTYPE; ++t)
         if (segs[t].nwarps && ctx.aux[t] != st) HF_CUDA(cudaStreamWaitEvent(st, ctx.join_ev[t], 0));
     if (parts.p) {
-        onee_sum_kernel<<<(unsigned)((nn + 127) / 128), 128, 0, st>>>(nn, nat, parts.p, dV);
+        onee_sum_kernel<<<(unsigned)((nn + 127) / 128), 128, 0, st>>>(nn, vrows, parts.p, dV);
         count_launch();
         HF_CUDA(cudaGetLastError());
     }
