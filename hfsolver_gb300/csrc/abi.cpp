@@ -155,6 +155,7 @@ static void rhf_impl(int natoms, const int* atno, const double* xyz, const hfgpu
         // the one-electron integrals run on a side stream, under the ERI plan's
         // host work (pair lists, quartet classes); joined before H is formed
         ctx.fork();
+        SideStreams onee(&ctx);
         onee_compute(ctx, b, natoms, atno, x.data(), y.data(), z.data(), dS.p, dT.p, dV.p, ctx.aux[0]);
         // integrals, resident in HBM for the whole SCF (in a wave: the wave's arrays)
         DBuf<double> dI;
@@ -166,6 +167,7 @@ static void rhf_impl(int natoms, const int* atno, const double* xyz, const hfgpu
         EriStats es;
         std::unique_ptr<EriPlan, void (*)(EriPlan*)> plan(eri_plan_create(ctx, b, opt.schwarz), eri_plan_destroy);
         ctx.join();
+        onee.joined();
         {
             const double one = 1.0;
             HF_CUBLAS(cublasDgeam(ctx.blas, CUBLAS_OP_N, CUBLAS_OP_N, n, n, &one, dT.p, n, &one, dV.p, n, dH.p, n));

@@ -174,6 +174,21 @@ struct Context {
     // threads on one context run one after another (handles and stream are shared)
     std::recursive_mutex call_mutex;
 };
+// Work queued on a context's side streams, over buffers that outlive this object: where
+// an exception comes before joined(), it is waited for, so that they are not freed under it.
+class SideStreams {
+    Context* ctx;
+
+public:
+    explicit SideStreams(Context* c) : ctx(c) {}
+    SideStreams(const SideStreams&) = delete;
+    void joined() { ctx = nullptr; }
+    ~SideStreams()
+    {
+        for (int i = 0; ctx && i < Context::NAUX; ++i) cudaStreamSynchronize(ctx->aux[i]);
+    }
+};
+
 // C = alpha op(A) op(B) + beta C in FP64, column-major: the own small-matrix
 // kernel for m, n, k <= 512 (gemm_small.cu), cuBLAS beyond
 // flags: what the caller knows of the operands.  GEMM_K_LE_I: op(A)(i, k) = 0 for k > i;

@@ -1072,6 +1072,7 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     const int n = in.n;
     const int64_t nn = (int64_t)n * n;
     HF_CHECK(in.nocc >= 0 && in.nocc <= n, HFGPU_ERR_INVALID, "nocc out of range");
+    SideStreams beside(in.begin ? &ctx : nullptr);  // until `end`
     if (in.begin) in.begin(in.hook_user);
     DBuf<double> G(nn, st), F(nn, st), Fw(nn, st), Sw(nn, st), Pold(nn, st), partial(RED_MAX_BLOCKS * RED_MAX, st);
     DBuf<unsigned> redcount(1, st);
@@ -1159,6 +1160,7 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     const double* last_F = nullptr;  // the Fock matrix of the last eigensolve
     ctx.trace_mark("scf setup");
     if (in.end) in.end(in.hook_user);
+    beside.joined();
     for (int it = 1; it <= in.nscf; ++it) {
         const double* Gcur = G.p;
         double* acc = nullptr;
