@@ -580,10 +580,8 @@ static DigestClass digest_class(const EriPlan* P, const ClassPlan& c, int split,
     d.nq = (int)c.nq;
     d.split = split;
     d.rounds = rounds;
-    d.nseg = (int)c.segs.size();
-    d.segs = c.dsegs.p;
     d.blocks = P->blocks.p + c.boff;
-    d.qlist = P->qlist.p ? P->qlist.p + c.qbase : nullptr;
+    d.qlist = P->qlist.p + c.qbase;
     return d;
 }
 
@@ -719,8 +717,6 @@ void eri_digest(Context& ctx, EriPlan* P, const double* dP, double* dG, double s
     DigestArgs a{};
     a.sh = P->shdev();
     a.pr = P->prdev();
-    a.gpairs = P->gpairs.p;
-    a.prefix = P->prefix.p;
     a.P = dP;
     a.n = n;
     a.Gh = Gh.p;
@@ -1089,8 +1085,6 @@ static void batch_digest_launches(Context& ctx, EriPlan* P, BatchDigest& t, cuda
     DigestArgs a{};
     a.sh = P->shdev();
     a.pr = P->prdev();
-    a.gpairs = P->gpairs.p;
-    a.prefix = P->prefix.p;
     a.Q = P->dQf.p;
     a.mol_n = t.mol_n.p;
     a.mol_P = t.mol_P.p;

@@ -37,19 +37,13 @@ struct DigestClass {
     int nq;       // quartets (below 2^31, checked when the plan is made)
     int split;    // warps that share the bra component rows of the same 32 x rounds quartets
     int rounds;   // a warp screens rounds x 32 quartets and digests the survivors (1 to 8)
-    int nseg;
-    const Seg* segs;
     const double* blocks;
-    // the (bra, ket) pair ids of every quartet, written by the ERI pass (null: found
-    // by searching the segments)
-    const int2* qlist;
+    const int2* qlist;  // the (bra, ket) pair ids of every quartet, written by the ERI pass
 };
 
 struct DigestArgs {
     ShellDev sh;
     PairDev pr;
-    const int* gpairs;
-    const int64_t* prefix;
     const double* P;
     int n;
     double* Gh;  // Jh (n x n), then Kh
@@ -111,33 +105,13 @@ __device__ __forceinline__ bool digest_mol(const DigestArgs& a, int mol, DigestM
     return true;
 }
 
-// quartet qg of the class: its bra and ket pair ids and its molecule, from the
-// list the ERI pass wrote, else by searching the segments and prefix sums
+// quartet qg of the class: its bra and ket pair ids and its molecule
 __device__ __forceinline__ void digest_quartet(const DigestArgs& a, const DigestClass& c, int qg, int& bra, int& ket, int& mol)
 {
-    if (c.qlist) {
-        const int2 e = __ldg(c.qlist + qg);
-        bra = e.x;
-        ket = e.y;
-        mol = a.pair_mol ? __ldg(a.pair_mol + bra) : 0;
-        return;
-    }
-    int lo = 0, hi = c.nseg - 1;  // last segment with qoff <= qg
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if ((int)(c.segs[mid].qoff) <= qg) lo = mid; else hi = mid - 1;
-    }
-    const Seg sg = c.segs[lo];
-    const int q = qg - (int)sg.qoff;
-    mol = sg.mol;
-    const int64_t* pf = a.prefix + sg.pref0;
-    int l2 = 0, h2 = sg.nbra - 1;
-    while (l2 < h2) {
-        const int mid = (l2 + h2 + 1) >> 1;
-        if ((int)pf[mid] <= q) l2 = mid; else h2 = mid - 1;
-    }
-    bra = a.gpairs[sg.bra0 + l2];
-    ket = a.gpairs[sg.ket0 + (q - (int)pf[l2])];
+    const int2 e = __ldg(c.qlist + qg);
+    bra = e.x;
+    ket = e.y;
+    mol = a.pair_mol ? __ldg(a.pair_mol + bra) : 0;
 }
 
 // true if the quartet's whole contribution is below the screening threshold:
