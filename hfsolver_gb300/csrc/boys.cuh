@@ -15,9 +15,8 @@
 //     contributes < 1e-11 relative, so an FP32 exponential is exact enough.
 // The light quartet classes spend most of their FP64 instructions here (34 of the 45 of
 // a primitive (ss|ss)): with the d^j / j! formed first and F's columns shared by all M
-// the sums took 29 and the grid index 5, so 14 and 4.  ERI of 8 and 16 waters 7.8 and
-// 41.2 -> 6.8 and 36.2 ms, two-electron gradient of 9 waters 52.9 -> 49.3 ms (with the
-// shorter rsqrt_nr).
+// the sums took 29 and the grid index 5, so 14 and 4 (ERI of 8 waters 13% faster, with
+// the shorter rsqrt_nr).
 // The grid values F_m(T_k) are made on the host in extended precision
 // (boys_table.cpp) from the convergent series
 //     F_m(T) = e^{-T} sum_i (2T)^i / ((2m+1)(2m+3)...(2m+2i+1)).

@@ -29,10 +29,10 @@ struct ClassPlan {
 // chain that is short against the whole pass costs nothing, and a longer one is the
 // time of the pass.  Every doubling costs sums over lanes and idle lanes, so a pass
 // that fills the GPU keeps s.  Measured (ms, with 16 to 32 primitive quartets a lane
-// at every size, then so; the Boys tables and chunks of that time, 8 waters are 5.8 now): ERI of 1, 2, 3, 4 and 8 waters 0.83, 0.90, 1.11, 1.6, 7.8
-// and 0.21, 0.36, 0.70, 1.36, 7.8; gradient of 1, 2, 3 and 9 waters 2.55, 2.38, 3.59,
-// 52.8 and 0.73, 1.46, 3.27, 52.8.  Shares of 0.06 and 0.5: ERI of 3 waters 0.73 and
-// 0.83, gradient of 2 waters 1.76 and 2.02.
+// at every size, and so): ERI of 1, 2, 3, 4 and 8 waters 1.32, 1.38, 1.43, 1.65, 5.84
+// and 0.22, 0.31, 0.52, 1.10, 5.84; two-electron gradient of 1, 2, 3 and 9 waters 3.23, 2.70,
+// 3.48, 44.7 and 0.80, 1.40, 2.81, 44.9.  Shares of 0.06 and 0.5: ERI of 3 waters 0.58 and
+// 0.65, gradient of 2 waters 1.71 and 1.91.
 constexpr double LANE_BUDGET = 0.2;     // share of the pass's work per FP64 pipe
 constexpr double LANE_SUM_INSTR = 1.6;  // a shuffle and add of one value, in FP64 instructions (105 clocks)
 template <class Chain>

@@ -95,8 +95,8 @@ __device__ __forceinline__ void lane_sums(double (&acc)[N], int split)
 // whatever its lanes do, and a thread that walks a pair's 36 primitive pairs over
 // four nuclei runs ~4000 of them in a row.  With one thread per pair and the types one
 // after the other the six launches took 1.24 ms for 2 waters (and held up the Schwarz
-// bounds on their stream); so, the whole set-up of 1, 2, 3 and 8 waters went from 1.20,
-// 1.52, 1.6 and 2.6 ms to 0.43, 0.50, 0.60 and 1.85.
+// bounds on their stream); so, the whole set-up of 1, 2, 3 and 8 waters is 0.46, 0.52,
+// 0.62 and 1.8 ms (1.20, 1.52, 1.6 and 2.6 with those launches).
 template <int LA, int LB>
 __global__ void __launch_bounds__(64) onee_shell_kernel(ShellOne sh, const int2* __restrict__ pairs, OneeSegs segs,
                                                         int n, int nat, int atoms, const int* __restrict__ Z,

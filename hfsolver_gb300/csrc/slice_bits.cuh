@@ -4,7 +4,7 @@
 // Y = round(x 2^(F - e)), |Y| <= 2^F, and cut into N balanced digits of radix 128,
 // Y = sum_t d_t 2^(7 (N - 1 - t)), every digit an integer that bf16 holds exactly:
 //   N = 6, F = 42: |d_0| <= 128, -64 <= d_t <= 63 below it (the mixed-precision path)
-//   N = 9, F = 62: |d_0| <= 64, the same below (FP64 accuracy: 2^-62 of the row's scale)
+//   N = 9, F = 62: |d_0| <= 64, the same below (the plain FP64 path; 2^-62 of the row's scale)
 // Digits are balanced rather than sign and magnitude for two reasons.  The sum over
 // K of all digit products of one group i + j = t stays below 2^24, so FP32
 // accumulation is exact for every input: N = 6: (2 128 64 + 4 64 64) K <= 2^24 for

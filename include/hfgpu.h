@@ -162,7 +162,8 @@ int hfgpu_formG(int n, const double *P, const double *int2, double *G);
 int hfgpu_formG_device_noalloc(int n, const double *d_int2, const double *d_P, double *d_G, void *cuda_stream);
 
 /* replaces transform_int2, src/mbpt.f90:11-79: (mu nu|la si) -> (ij|kl) over
- * all orbitals, both arrays packed.  FP64. */
+ * all orbitals, both arrays packed.  FP64: in each of the four contractions an
+ * entry is within n 2^-53 of its terms' magnitudes, and Inf and NaN go through. */
 int hfgpu_transform_int2(int n, const double *int2, const double *C, double *moint2);
 
 /* replaces mbpt2, src/mbpt.f90:154-159 (term1, src/mbpt2.f90:8-31):
