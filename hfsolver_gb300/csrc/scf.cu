@@ -858,10 +858,13 @@ struct Purifier {
     static constexpr int MAXS = 160;
     // Steps that the recursion may take (even), and its estimate for a spectrum of this
     // width and gap: each step shrinks their ratio 1.24 times.  Where an eigensolve can take
-    // over, more than eigensolve_limit() steps are slower than it: 4 us a step at 25 functions,
-    // 6 us at 75 and 13 us at 150 against 0.2, 0.7 and 2 ms.
+    // over, more than slow() steps are slower than it: 4 us a step at 25 functions, 6 us at
+    // 75 and 13 us at 150 against 0.2, 0.7 and 2 ms.  One such density costs little (of one
+    // water's Fock matrices after the core Hamiltonian the first has a gap of 0.0045 and takes 52
+    // steps, the others 24 to 38), so it is given up at twice as many.
     int limit = MAXS;
-    int eigensolve_limit() const { return std::min(MAXS, std::max(40, 20 + 5 * n / 4) & ~1); }
+    int slow() const { return std::min(MAXS, std::max(40, 20 + 5 * n / 4)); }
+    int steps() const { return hrep->sp2[1].steps; }
     static double steps_for(double width, double gap) { return gap > 0 ? 9.0 + 10.9 * std::log10(1.5 * width / gap) : 1e9; }
     // Did the last density() end with tr X = nocc?  strict: and by the idempotency
     // test, not at the step limit.  (True when nothing is pending.)
@@ -1124,12 +1127,13 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
     // stays.
     const bool sp2_density = in.purify || (own_eigh && in.nocc > 0 && in.nocc < n && n >= SP2_MIN &&
                                            in.tolP >= 1e-11 && pur.one_launch(ctx));
-    // A purification that found no gap is not tried again until the energies of the
-    // eigensolves after it show one (and after the third such not at all): 20 iterations of
-    // 25 functions without a gap, or with one of 1e-6, took 19 and 10 ms, 6.3 with eigensolves alone.
+    // After a purification that found no gap, or two slow ones in a row, none is tried until
+    // the energies of the eigensolves instead of it show a gap for a fast one (and after the
+    // third such not at all): 20 iterations of 25 functions without a gap, or with one of 1e-6,
+    // took 19 and 10 ms, 6.3 with eigensolves alone.
     bool rest = false;
-    int misses = 0;
-    if (sp2_density && !in.purify) pur.limit = pur.eigensolve_limit();
+    int misses = 0, slow = 0;
+    if (sp2_density && !in.purify) pur.limit = std::min(Purifier::MAXS, 2 * pur.slow());
     // orbitals C (may alias F) and energies of F C = S C diag(lam); with the own
     // eigensolver only the lowest ncol orbitals are formed (ncol <= 0: all)
     auto eigh = [&](const double* Fm, double* Cm, int ncol) {
@@ -1230,12 +1234,16 @@ ScfOut run_scf(Context& ctx, const ScfIn& in, double* dC, double* dP, double* dL
         HF_CUDA(cudaStreamSynchronize(st));
         if (rest) {
             const double* w = eig.energies();
-            rest = misses >= 3 || Purifier::steps_for(w[n - 1] - w[0], w[in.nocc] - w[in.nocc - 1]) > pur.limit - 6;
+            rest = misses >= 3 || Purifier::steps_for(w[n - 1] - w[0], w[in.nocc] - w[in.nocc - 1]) > pur.slow() - 6;
         }
-        if (sp2_now && !pur.converged(!in.purify)) {
-            HF_CHECK(!in.purify, HFGPU_ERR_LINALG, "density purification did not converge (no gap?)");
+        const bool fell_back = sp2_now && !pur.converged(!in.purify);
+        slow = sp2_now && !in.purify && pur.steps() > pur.slow() ? slow + 1 : 0;
+        if (fell_back || slow >= 2) {
             rest = true;
             ++misses;
+        }
+        if (fell_back) {
+            HF_CHECK(!in.purify, HFGPU_ERR_LINALG, "density purification did not converge (no gap?)");
             eigh(Fsolve, Fw.p, in.nocc);
             form_density(ctx, n, in.nocc, Fw.p, dP);
             report();

@@ -48,3 +48,11 @@ def test_purification_returns_with_the_gap():
     eig, sp2 = _launches(n, nocc, H, int2, 20, 1e-12), _launches(n, nocc, H, int2, 20, 1e-9)
     alone = _launches(n, nocc, *_system(n, nocc, 0.0, 0.0), 20, 1e-9)
     assert sp2 <= eig - 3 * 16 and alone > eig - 3
+
+
+def test_one_narrow_gap_costs_no_eigensolve():
+    """A first Fock matrix with a gap of 1e-4 (70 steps) and wide ones after it take the same
+    kernels as wide ones throughout."""
+    n, nocc = 24, 8
+    k = [_launches(n, nocc, *_system(n, nocc, gap, 0.02), 12, 1e-9) for gap in (1e-4, 0.5)]
+    assert k[0] == k[1]
