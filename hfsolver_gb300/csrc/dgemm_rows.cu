@@ -1,6 +1,6 @@
 // Plain FP64 AO -> MO transform: the drop-in beside the mixed-precision path.
 //
-// From 28 up to slice_kmax(9) = 455 functions every contraction is the sliced tensor-core GEMM
+// From 28 (36) up to slice_kmax(9) = 455 functions every contraction is the sliced tensor-core GEMM
 // with nine digits per factor (tcgemm.cu): exact sums of elements kept to 2^-62 of their
 // row's scale, and entries too small against the scales for that formed in FP64, so that
 // each is as good as an FP64 sum.  GB300's FP64 pipe (2 FMAs per clock per SM) is left with
@@ -216,10 +216,12 @@ void ao2mo_fp64(Context& ctx, int n, const double* d_int2, const double* C1, int
                 double* T)
 {
     // Below 28 functions the FP64 GEMMs are a single wave of blocks and the sliced ones' cutting,
-    // row maxima and second pass 0.06 ms of launches: transform_int2 of 10, 24 and 28
-    // functions 0.12, 0.26, 0.39 ms with FP64 GEMMs, 0.18, 0.28, 0.36 with digits.
-    constexpr int DIGITS_MIN = 28;
-    if (n >= DIGITS_MIN && n <= slice_kmax(SLICE_FP64))
+    // row maxima and second pass 0.06 ms of launches: all (ij|kl) of 10, 24 and 28 functions 0.12,
+    // 0.26, 0.39 ms with FP64 GEMMs, 0.18, 0.28, 0.36 with digits.  With a part of the orbitals
+    // on each side the line is later: a fifth occupied, 28, 32 and 40 functions 0.20, 0.21,
+    // 0.40 and 0.22, 0.23, 0.28.
+    const int digits_min = n1 == n ? 28 : 36;
+    if (n >= digits_min && n <= slice_kmax(SLICE_FP64))
         ao2mo_sliced(ctx, n, d_int2, C1, n1, C2, n2, SLICE_FP64, T);
     else
         ao2mo_rows(ctx, n, d_int2, C1, n1, C2, n2, T);

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 def test_gemm_counters_after_a_failed_transform(precision):
     """Each device allocation of an MBPT2 energy fails in turn, some of them between two sliced
     GEMMs: the next call counts its own GEMMs only."""
-    n, o = 30, 6
+    n, o = 40, 6
     m = n * (n + 1) // 2
     rng = np.random.default_rng(2)
     int2 = rng.standard_normal(m * (m + 1) // 2)

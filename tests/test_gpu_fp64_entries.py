@@ -71,7 +71,7 @@ def test_nan_and_inf_go_through(n, route, bad, where):
 
 
 def test_nan_reaches_the_fp64_energy():
-    n = 29
+    n = 37
     m = n * (n + 1) // 2
     rng = np.random.default_rng(5)
     int2 = rng.standard_normal(m * (m + 1) // 2)
@@ -148,3 +148,18 @@ def test_small_transforms_launch_no_cutting_kernels(n):
     hf.transform_int2(int2, C)
     k.append(L.hfgpu_kernel_launches())
     assert k[2] - k[1] == k[1] - k[0] + 1  # and the packing
+
+
+@pytest.mark.parametrize("n,o", [(25, 5), (30, 6), (35, 17)])
+def test_small_half_transforms_launch_no_cutting_kernels(n, o):
+    from hfsolver_gb300 import _lib
+
+    L = _lib.lib()
+    m = n * (n + 1) // 2
+    int2, C = np.ones(m * (m + 1) // 2), np.eye(n)
+    k = [L.hfgpu_kernel_launches()]
+    hf.half_transform(int2, C, o, 0)
+    k.append(L.hfgpu_kernel_launches())
+    hf.mp2_energy(int2, C, np.arange(n) - o + 0.5, o)
+    k.append(L.hfgpu_kernel_launches())
+    assert k[2] - k[1] == k[1] - k[0] + 1  # and the energy
