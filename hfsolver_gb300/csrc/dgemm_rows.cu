@@ -5,8 +5,8 @@
 // row's scale, and entries too small against the scales for that formed in FP64, so that
 // each is as good as an FP64 sum.  GB300's FP64 pipe (2 FMAs per clock per SM) is left with
 // the latter: none to speak of for dense factors (transform_int2 of 100 random orbitals
-// 72 -> 16 ms), about 57% of steps 1 and 3 and 18% of steps 2 and 4 for 6 waters, whose
-// orbitals and integrals are local (MBPT2 34 -> 18 ms; 8 waters 137 -> 74).
+// 72 -> 16 ms), 37, 11, 56 and 16% of the four steps for 6 waters, whose orbitals and
+// integrals are local (MBPT2 34 -> 18 ms; 8 waters 137 -> 74).
 //
 // Below and beyond the same half transform over mu >= nu pairs runs on FP64 GEMMs whose A
 // rows are gathered straight from where the transform keeps them (gather_rows.cuh): the
