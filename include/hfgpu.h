@@ -202,7 +202,7 @@ int hfgpu_dgemm_sliced(int64_t M, int N, int K, const double *A, const double *B
  * terms (on the tensor cores by exact 7-bit bf16 slicing with nine digits per
  * factor where that keeps it, 2^-62 of a row's scale, else in FP64; above 455
  * functions FP64 GEMMs); HFGPU_MP2_SPLIT_BF16: six digits, 2^-42 of a row's
- * scale. */
+ * scale, for finite input (digits do not carry Inf and NaN). */
 int hfgpu_mp2_energy(int n, const double *int2, const double *C, const double *lam, int nocc,
                      int precision, double *E2);
 
